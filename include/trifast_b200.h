@@ -265,6 +265,14 @@ int trifast_check_device_status(void* stream);
  * exception without a synchronisation per call.  (No reference counterpart.) */
 int trifast_snapshot_device_status(uint32_t* host_word, void* stream);
 
+/* The same without anything enqueued per call: *host_word becomes the address of a pinned
+ * word (owned by the library, one per device, zero at first) that the kernels themselves
+ * write when a wait gives up (and the next call's first kernel again while the status is set).  A binding
+ * looks at it at the start of each call; when it is non-zero it calls
+ * trifast_check_device_status() and then sets the word to zero.  The first call on a device
+ * allocates the word: make it outside stream capture.  (No reference counterpart.) */
+int trifast_host_status_word(uint32_t** host_word);
+
 /* Test support for that path: launches one warp that waits, with the same bounded
  * wait the kernels use, on a barrier nobody arrives on; after limit_us
  * microseconds (1 .. 100000) the wait gives up, the kernel sets the status word

@@ -13,6 +13,7 @@ import torch
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_HERE, "libtrifast_b200.so")
+OPS_PATH = os.path.join(_HERE, "libtrifast_b200_torch.so")   # the PyTorch operators (csrc/torch_ops.cpp)
 
 DTYPE_CODE = {torch.float32: 0, torch.bfloat16: 1, torch.float16: 2}
 KERNEL_AUTO, KERNEL_SIMT, KERNEL_TCGEN05 = 0, 1, 2
@@ -82,6 +83,7 @@ SIGNATURES = {
     "trifast_db_finalize": (C.c_int, [_P(Shape), C.c_void_p, _P(T4), C.c_void_p]),
     "trifast_check_device_status": (C.c_int, [C.c_void_p]),
     "trifast_snapshot_device_status": (C.c_int, [C.c_void_p, C.c_void_p]),
+    "trifast_host_status_word": (C.c_int, [_P(_P(C.c_uint32))]),
     "trifast_db_push_reduce": (C.c_int, [_P(PushReduce), C.c_void_p]),
     "trifast_db_push_reduce_staging_floats": (C.c_size_t, [C.c_int64, C.c_int32]),
     "trifast_debug_wait_probe": (C.c_int, [C.c_uint32, C.c_void_p]),
@@ -119,9 +121,8 @@ def check(rc: int, what: str) -> None:
         raise RuntimeError(f"{what}: {status_str(rc)} (status {rc}{detail})")
 
 
-# Per-device pinned host word that mirrors the device status word (see
-# trifast_snapshot_device_status in the header): the library copies the status
-# into it after every operator call, and the next call looks at it first.
+# Per-device pinned host word that the kernels write when a bounded wait gives up (see
+# trifast_host_status_word in the header): every operator call looks at it first.
 _status_words: dict = {}
 
 
@@ -131,33 +132,30 @@ def _status_word(device) -> torch.Tensor:
         idx = torch.cuda.current_device()
     w = _status_words.get(idx)
     if w is None:
-        w = torch.zeros(1, dtype=torch.int32).pin_memory()
+        p = _P(C.c_uint32)()
+        with torch.cuda.device(idx):
+            check(load().trifast_host_status_word(C.byref(p)), "trifast_host_status_word")
+        word = C.cast(p, _P(C.c_int32 * 1)).contents       # owned by the library
+        w = torch.frombuffer(word, dtype=torch.int32)
         _status_words[idx] = w
     return w
 
 
 def raise_if_device_gave_up(device) -> None:
-    """First thing in every operator call.  If an earlier kernel on this device gave
-    up on one of its bounded waits, its outputs (and those of every launch since) were
-    never written: read and clear the status and raise, instead of returning
-    uninitialised memory.  Costs one host-memory read when nothing is wrong."""
+    """First thing in every call of this package (the operators do the same natively).  If an
+    earlier kernel on this device gave up on one of its bounded waits, its outputs (and those
+    of every launch since) were never written: read and clear the status and raise, instead
+    of returning uninitialised memory.  Costs one host-memory read when nothing is wrong."""
     w = _status_word(device)
     if int(w[0]) == 0:
         return
-    w.zero_()
     with torch.cuda.device(device):
         load().trifast_check_device_status(
             C.c_void_p(torch.cuda.current_stream(device).cuda_stream))
+    w.zero_()
     raise RuntimeError(
         "trifast_b200: " + status_str(-11) + " in an earlier call on this device; the results "
         "of that call and of the calls after it are invalid (status cleared, retry is possible)")
-
-
-def snapshot_status(device, stream: C.c_void_p) -> None:
-    """Last thing in every operator call: enqueue the copy of the status word."""
-    with torch.cuda.device(device):
-        check(load().trifast_snapshot_device_status(C.c_void_p(_status_word(device).data_ptr()),
-                                                    stream), "trifast_snapshot_device_status")
 
 
 def kernel_choice() -> int:

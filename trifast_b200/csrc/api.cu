@@ -4,6 +4,7 @@
 
 #include <float.h>
 #include <math.h>
+#include <stddef.h>
 
 #include <mutex>
 
@@ -12,7 +13,7 @@
 namespace trifast {
 namespace {
 
-__device__ unsigned int g_device_status;  // OR of DeviceStatusBits
+__device__ DeviceStatus g_device_status;  // bits: OR of DeviceStatusBits
 
 constexpr int kMaxDevices = 64;
 // SMs the persistent dq / dk / dv kernels leave free under TRIFAST_FLAG_SHARE_GPU: their
@@ -21,7 +22,11 @@ constexpr int kMaxDevices = 64;
 constexpr int kSharedGpuSms = 8;
 unsigned int* g_status_ptr[kMaxDevices];
 int g_arch_major[kMaxDevices];
+int g_sm_count[kMaxDevices];
 std::once_flag g_once[kMaxDevices];
+unsigned int* g_host_word[kMaxDevices];   // pinned mirrors of the status words (DeviceStatus::host)
+cudaError_t g_host_word_error[kMaxDevices];
+std::once_flag g_host_word_once[kMaxDevices];
 
 // Per-device set-up, once: address of the status word and the compute capability.
 int device_setup(int* dev_out, unsigned int** status) {
@@ -33,6 +38,7 @@ int device_setup(int* dev_out, unsigned int** status) {
     int major = 0;
     cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
     g_arch_major[dev] = major;
+    cudaDeviceGetAttribute(&g_sm_count[dev], cudaDevAttrMultiProcessorCount, dev);
   });
   if (!g_status_ptr[dev]) return TRIFAST_ERR_LAUNCH;
   if (g_arch_major[dev] != 10) return TRIFAST_ERR_ARCH;
@@ -319,6 +325,13 @@ int cuda_rc(cudaError_t e) {
 }
 
 }  // namespace
+
+int sm_count() {
+  int dev;
+  unsigned int* status;
+  return device_setup(&dev, &status) == TRIFAST_OK && g_sm_count[dev] > 0 ? g_sm_count[dev] : 148;
+}
+
 }  // namespace trifast
 
 using namespace trifast;
@@ -561,6 +574,30 @@ int trifast_snapshot_device_status(uint32_t* host_word, void* stream) {
   if (rc) return rc;
   return cuda_rc(cudaMemcpyAsync(host_word, status, sizeof(uint32_t), cudaMemcpyDeviceToHost,
                                  (cudaStream_t)stream));
+}
+
+int trifast_host_status_word(uint32_t** host_word) {
+  if (!host_word) return TRIFAST_ERR_NULL;
+  int dev;
+  unsigned int* status;
+  int rc = device_setup(&dev, &status);
+  if (rc) return rc;
+  std::call_once(g_host_word_once[dev], [dev, status] {
+    void* p = nullptr;
+    cudaError_t e = cudaHostAlloc(&p, sizeof(uint32_t), cudaHostAllocPortable | cudaHostAllocMapped);
+    if (e == cudaSuccess) {
+      *(volatile uint32_t*)p = 0;
+      void* d = nullptr;   // the address kernels write to (the same one under unified addressing)
+      e = cudaHostGetDevicePointer(&d, p, 0);
+      if (e == cudaSuccess)
+        e = cudaMemcpy((char*)status + offsetof(DeviceStatus, host), &d, sizeof(d), cudaMemcpyHostToDevice);
+    }
+    g_host_word[dev] = e == cudaSuccess ? (unsigned int*)p : nullptr;
+    g_host_word_error[dev] = e;
+  });
+  if (!g_host_word[dev]) return cuda_rc(g_host_word_error[dev]);
+  *host_word = g_host_word[dev];
+  return TRIFAST_OK;
 }
 
 int trifast_debug_wait_probe(uint32_t limit_us, void* stream) {

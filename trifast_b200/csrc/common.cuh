@@ -6,6 +6,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "../../include/trifast_b200.h"
 
 namespace trifast {
@@ -64,7 +66,15 @@ template <> __device__ __forceinline__ __half from_f32<__half>(float x) {
 }
 
 // Kernels whose bounded waits give up OR a non-zero code into a device status
-// word (they never trap); its address is handed to them as a kernel argument.
+// word (they never trap); its address is handed to them as a kernel argument.  Next to the
+// word lies the address of a pinned host word, or null: whoever sets the status also writes
+// it there (and the prepare kernels repeat it while it stays set), so that a binding learns
+// of the time-out from host memory, without a copy enqueued behind each call.
+struct DeviceStatus {
+  unsigned int bits;
+  unsigned int unused;
+  unsigned int* host;
+};
 enum DeviceStatusBits : unsigned int {
   kStatusTimeoutFwd = 1u,
   kStatusTimeoutBwdDb = 2u,
@@ -74,5 +84,43 @@ enum DeviceStatusBits : unsigned int {
   kStatusTimeoutProbe = 32u,
   kStatusTimeoutPushReduce = 64u,
 };
+
+// (out of line, so that the cold path leaves the code of the kernels' loops alone)
+static __device__ __noinline__ void mirror_status(unsigned int* status, unsigned int bits) {
+  unsigned int* host = reinterpret_cast<DeviceStatus*>(status)->host;
+  if (host) {
+    *reinterpret_cast<volatile unsigned int*>(host) = bits;
+    __threadfence_system();
+  }
+}
+// For the prepare kernels, which run first in a call.
+__device__ __forceinline__ void repeat_status(unsigned int* status) {
+  const unsigned int bits = *reinterpret_cast<volatile unsigned int*>(status);
+  if (bits != 0u) mirror_status(status, bits);
+}
+__device__ __forceinline__ void set_status(unsigned int* status, unsigned int bits) {
+  mirror_status(status, atomicOr(status, bits) | bits);
+}
+
+// SMs of the current device.
+int sm_count();
+
+// Opts a kernel in to `bytes` of dynamic shared memory: one runtime call per kernel, device
+// and growth of the size, not one per launch.
+template <auto Kernel>
+cudaError_t opt_in_smem(int bytes) {
+  static std::atomic<int> have[64];
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+  if (have[dev].load(std::memory_order_acquire) >= bytes) return cudaSuccess;
+  e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e != cudaSuccess) return e;
+  int seen = have[dev].load(std::memory_order_relaxed);
+  while (seen < bytes && !have[dev].compare_exchange_weak(seen, bytes, std::memory_order_release)) {
+  }
+  return cudaSuccess;
+}
 
 }  // namespace trifast

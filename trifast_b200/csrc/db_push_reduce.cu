@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(1024) db_push_reduce_kernel(PushReduceParams p
   }
   announce(p, p.counters + 0, 0);
   if (!await(p, 0, &gave_up)) {
-    if (threadIdx.x == 0) atomicOr(status, (unsigned int)kStatusTimeoutPushReduce);
+    if (threadIdx.x == 0) set_status(status, kStatusTimeoutPushReduce);
     return;
   }
 
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(1024) db_push_reduce_kernel(PushReduceParams p
   }
   announce(p, p.counters + 1, kMaxWorld);
   if (!await(p, kMaxWorld, &gave_up)) {
-    if (threadIdx.x == 0) atomicOr(status, (unsigned int)kStatusTimeoutPushReduce);
+    if (threadIdx.x == 0) set_status(status, kStatusTimeoutPushReduce);
   }
 }
 

@@ -82,8 +82,9 @@ __device__ __forceinline__ void axpy_smem(float a, const float* sm, float* reg) 
 // ---------------------------------------------------------------------------
 __global__ void rowfull_kernel(MaskView mask, int n, int n_rows, uint8_t* rowfull,
                                uint32_t* maskbits, uint32_t* maskbits_lin, int mask_words,
-                               uint32_t* rowrange) {
+                               uint32_t* rowrange, unsigned int* status) {
   const int bi = blockIdx.x;
+  if (bi == 0 && threadIdx.x == 0) repeat_status(status);
   const int b = bi / n_rows, i = bi % n_rows;
   const uint8_t* row = mask.p + b * mask.sb + (int64_t)i * mask.si;
   __shared__ int first_open, last_open;
@@ -845,7 +846,7 @@ cudaError_t simt_forward(const FwdArgs& a, cudaStream_t s) {
 cudaError_t bwd_prepare(const BwdArgs& a, cudaStream_t s) {
   const Dims& dm = a.dm;
   rowfull_kernel<<<dm.batch * dm.n_rows, 128, 0, s>>>(a.mask, dm.n, dm.n_rows, a.rowfull, a.maskbits,
-                                                      a.maskbits_lin, a.mask_words, a.rowrange);
+                                                      a.maskbits_lin, a.mask_words, a.rowrange, a.status);
   if (a.bias_t) {
     dim3 grid((dm.n + 63) / 64, (dm.n + 63) / 64, dm.batch * dm.heads);
     bias_transpose_kernel<<<grid, 256, 0, s>>>(a.bias, (uint16_t*)a.bias_t, dm.heads, dm.n,
@@ -871,7 +872,7 @@ cudaError_t fwd_prepare(const FwdArgs& a, cudaStream_t s) {
   // the live key-tile range of every row always; the packed masks, row flags and the padded
   // bias copy only where the workspace holds them (n % 8 != 0)
   rowfull_kernel<<<dm.batch * dm.n_rows, 128, 0, s>>>(a.mask, dm.n, dm.n_rows, a.rowfull, a.maskbits,
-                                                      nullptr, a.mask_words, a.rowrange);
+                                                      nullptr, a.mask_words, a.rowrange, a.status);
   if (a.bias_pad) {
     dim3 grid(1, dm.n, dm.batch * dm.heads);
     bias_pad_kernel<<<grid, 256, 0, s>>>(a.bias, (uint16_t*)a.bias_pad, dm.heads, dm.n, dm.n_pad);

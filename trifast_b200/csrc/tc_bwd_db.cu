@@ -361,7 +361,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
     const long long t0 = clock64();
     while (clock64() - t0 < 4000000LL) {
     }
-    if (tid == 0) atomicOr(status, (unsigned int)kStatusTimeoutBwdDb);
+    if (tid == 0) set_status(status, kStatusTimeoutBwdDb);
     __syncthreads();
   }
   if (warp == kMmaWarp) {
@@ -398,8 +398,8 @@ cudaError_t launch_db(const BwdArgs& a, cudaStream_t stream) {
       return cudaErrorInvalidValue;
   }
   const int smem = Cfg::smem_bytes();
-  auto kern = tc_db_kernel<T, D, NS>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  constexpr auto kern = tc_db_kernel<T, D, NS>;
+  cudaError_t e = opt_in_smem<kern>(smem);
   if (e != cudaSuccess) return e;
   const int t = (dm.n + 127) / 128;
   const int total = t * t * a.splits * dm.batch * dm.heads;

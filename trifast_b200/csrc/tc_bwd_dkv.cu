@@ -448,7 +448,7 @@ tc_dkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
     const long long t0 = clock64();
     while (clock64() - t0 < 4000000LL) {
     }
-    if (tid == 0) atomicOr(status, (unsigned int)kStatusTimeoutBwdDkv);
+    if (tid == 0) set_status(status, kStatusTimeoutBwdDkv);
     __syncthreads();
   }
   if (warp == 4 * R + 1) {
@@ -495,17 +495,14 @@ cudaError_t launch_dkv(const BwdArgs& a, cudaStream_t stream) {
       return cudaErrorInvalidValue;
   }
   const int smem = Cfg::smem_bytes();
-  auto kern = tc_dkv_kernel<T, D, R, NS>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  constexpr auto kern = tc_dkv_kernel<T, D, R, NS>;
+  cudaError_t e = opt_in_smem<kern>(smem);
   if (e != cudaSuccess) return e;
   ItemGrid items;
   items.nkt = (dm.n + kBKeys - 1) / kBKeys;
   items.nrp = (dm.n_rows + R - 1) / R;
   items.total = items.nkt * items.nrp * dm.batch * dm.heads;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (sms <= 0) sms = 148;
+  int sms = sm_count();
   sms = sms - a.reserve_sms > 0 ? sms - a.reserve_sms : 1;
   const int grid = items.total < sms ? items.total : sms;
   kern<<<grid, Cfg::kThreads, smem, stream>>>(mk, mv, mq, mdo, mbt, mlse, mdelta, a.dk, a.dv,

@@ -445,20 +445,13 @@ tc_dq_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
     const long long t0 = clock64();
     while (clock64() - t0 < 4000000LL) {
     }
-    if (tid == 0) atomicOr(status, (unsigned int)kStatusTimeoutBwdDq);
+    if (tid == 0) set_status(status, kStatusTimeoutBwdDq);
     __syncthreads();
   }
   if (warp == 4 * R + 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
-}
-
-int sm_count_dq() {
-  int dev = 0, c = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
-  return c > 0 ? c : 148;
 }
 
 template <typename T, int D, int NS>
@@ -493,14 +486,14 @@ cudaError_t launch_dq(const BwdArgs& a, cudaStream_t stream) {
       return cudaErrorInvalidValue;
   }
   const int smem = Cfg::smem_bytes(dm.n);
-  auto kern = tc_dq_kernel<T, D, NS>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  constexpr auto kern = tc_dq_kernel<T, D, NS>;
+  cudaError_t e = opt_in_smem<kern>(smem);
   if (e != cudaSuccess) return e;
   ItemGrid items;
   items.njt = (dm.n + kBJ - 1) / kBJ;
   items.nrp = (dm.n_rows + 1) / 2;
   items.total = items.njt * items.nrp * dm.batch * dm.heads;
-  const int sms = sm_count_dq() - a.reserve_sms > 0 ? sm_count_dq() - a.reserve_sms : 1;
+  const int sms = sm_count() - a.reserve_sms > 0 ? sm_count() - a.reserve_sms : 1;
   const int grid = items.total < sms ? items.total : sms;
   kern<<<grid, Cfg::kThreads, smem, stream>>>(mq, mdo, mk, mv, mbias, a.dq, a.lse, a.delta,
                                               a.rowfull, a.maskbits, a.mask_words, dm, items, a.status);

@@ -659,7 +659,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
     const long long t0 = clock64();
     while (clock64() - t0 < 4000000LL) {
     }
-    if (tid == 0) atomicOr(status, (unsigned int)kStatusTimeoutBwdFused);
+    if (tid == 0) set_status(status, kStatusTimeoutBwdFused);
     __syncthreads();
   }
   if (warp == 9) {
@@ -707,8 +707,8 @@ cudaError_t launch_fused(const BwdArgs& a, cudaStream_t stream) {
       return cudaErrorInvalidValue;
   }
   const int smem = Cfg::smem_bytes();
-  auto kern = tc_dqkv_kernel<T, D, NS, SB>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  constexpr auto kern = tc_dqkv_kernel<T, D, NS, SB>;
+  cudaError_t e = opt_in_smem<kern>(smem);
   if (e != cudaSuccess) return e;
   FusedGrid grid;
   grid.total = dm.batch * dm.heads * dm.n_rows;
@@ -718,10 +718,7 @@ cudaError_t launch_fused(const BwdArgs& a, cudaStream_t stream) {
   grid.jsc = 2 * Cfg::kMaxJTiles;
   grid.nch = (grid.njt + Cfg::kMaxJTiles - 1) / Cfg::kMaxJTiles;
   if (grid.nch > 1 && !a.kv_scratch) return cudaErrorInvalidValue;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (sms <= 0) sms = 148;
+  int sms = sm_count();
   if (sms > kFusedMaxCtas) sms = kFusedMaxCtas;  // the dK / dV scratch is sized for this many CTAs
   int ctas = grid.total < sms ? grid.total : sms;
   if (a.reserve_sms > 0) {

@@ -591,26 +591,13 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     const long long t0 = clock64();
     while (clock64() - t0 < 4000000LL) {
     }
-    if (tid == 0) atomicOr(status, (unsigned int)kStatusTimeoutFwd);
+    if (tid == 0) set_status(status, kStatusTimeoutFwd);
     __syncthreads();
   }
   if (warp == 4 * R + 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
-}
-
-int sm_count() {
-  static int count[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return 148;
-  if (count[dev] == 0) {
-    int c = 0;
-    cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev);
-    count[dev] = c > 0 ? c : 148;
-  }
-  return count[dev];
 }
 
 template <typename T, int D, int R, int NS>
@@ -643,8 +630,10 @@ cudaError_t launch(const FwdArgs& a, cudaStream_t stream) {
   }
   const int smem = Cfg::smem_bytes(dm.n);
   const bool two = Cfg::mask_bufs(dm.n) == 2;
-  auto kern = two ? tc_fwd_kernel<T, D, R, NS, 2> : tc_fwd_kernel<T, D, R, NS, 1>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  constexpr auto kern2 = tc_fwd_kernel<T, D, R, NS, 2>;
+  constexpr auto kern1 = tc_fwd_kernel<T, D, R, NS, 1>;
+  const auto kern = two ? kern2 : kern1;
+  cudaError_t e = two ? opt_in_smem<kern2>(smem) : opt_in_smem<kern1>(smem);
   if (e != cudaSuccess) return e;
   ItemGrid items;
   items.njt = (dm.n + kBJ - 1) / kBJ;

@@ -461,7 +461,7 @@ tc_fwd_d128_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
     const long long t0 = clock64();
     while (clock64() - t0 < 4000000LL) {
     }
-    if (tid == 0) atomicOr(status, (unsigned int)kStatusTimeoutFwd);
+    if (tid == 0) set_status(status, kStatusTimeoutFwd);
     __syncthreads();
   }
   if (warp == 9) {
@@ -496,17 +496,14 @@ cudaError_t launch128(const FwdArgs& a, cudaStream_t stream) {
                              a.bias_pad ? st_pad : st_user, box4, CU_TENSOR_MAP_SWIZZLE_128B))
       return cudaErrorInvalidValue;
   }
-  auto kern = tc_fwd_d128_kernel<T>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  constexpr auto kern = tc_fwd_d128_kernel<T>;
+  cudaError_t e = opt_in_smem<kern>(kSmemBytes);
   if (e != cudaSuccess) return e;
   Grid128 items;
   items.njt = (dm.n + 127) / 128;
   items.njp = (items.njt + 1) / 2;
   items.total = items.njp * dm.n_rows * dm.batch * dm.heads;
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (sms <= 0) sms = 148;
+  const int sms = sm_count();
   const int grid = items.total < sms ? items.total : sms;
   kern<<<grid, 384, kSmemBytes, stream>>>(mq, mk, mv, mbias, a.o, a.lse, a.rowfull, a.maskbits,
                                           a.mask_words, a.rowrange, dm, items, a.status);

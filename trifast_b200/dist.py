@@ -86,7 +86,6 @@ class CudaKernels:
                 C.byref(_lib.t5(dv)), C.c_void_p(ws.data_ptr()), C.c_size_t(ws.numel()),
                 _stream(q))
         _lib.check(rc, "trifast_backward_dqkv")
-        _lib.snapshot_status(q.device, _stream(q))
         return dq, dk, dv
 
     def db_finalize(self, db_f32, dtype):

@@ -257,7 +257,6 @@ class HostPipeline:
         cur.wait_stream(self.s_out)
         cur.wait_stream(self.s_run)
         cur.wait_stream(self.s_in)
-        L.snapshot_status(self.device, C.c_void_p(cur.cuda_stream))
         self.kernel_launches = launches
         return out
 

@@ -4,14 +4,16 @@ Mirrors the reference's ``src/trifast/torch.py``: a forward op returning
 ``(o, lse)`` (``_triangle_attention``, :17-65), a backward op returning
 ``(dq, dk, dv, db, dmask)`` (``triangle_attention_bwd``, :68-182), autograd glue
 (:185-217) and the public ``triangle_attention`` (:220-228).  The ops live in the
-``trifast_b200`` namespace so the reference can be imported beside them.  All
-compute happens in the CUDA library behind the C ABI (``_lib.py``); this module
-only checks arguments, allocates outputs and passes pointers and strides.
+``trifast_b200`` namespace so the reference can be imported beside them.  They are native
+(``csrc/torch_ops.cpp``): argument checks, allocation and autograd run without
+Python, and all compute happens in the CUDA library behind the C ABI.  The checks
+below serve the layers that call the C ABI from Python (``dist.py``).
 """
 
 from __future__ import annotations
 
 import ctypes as C
+import os
 
 import torch
 
@@ -98,92 +100,40 @@ def _stream(t):
     return C.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
 
 
-@torch.library.custom_op("trifast_b200::triangle_attention", mutates_args=(), device_types="cuda")
-def _triangle_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b: torch.Tensor,
-                        mask: torch.Tensor) -> tuple[torch.Tensor, torch.Tensor]:
-    bs, h, n_rows, n, d = _check_inputs(q, k, v, b, mask)
-    lib = _lib.load()
-    _lib.raise_if_device_gave_up(q.device)
-    q, k, v, b = _prep5(q), _prep5(k), _prep5(v), _prep4(b)
-    m8 = _prep_mask(mask)
-    o = torch.empty((bs, h, n_rows, n, d), dtype=q.dtype, device=q.device)
-    lse = torch.empty((bs, h, n_rows, n), dtype=torch.float32, device=q.device)
-    shp = _lib.make_shape(bs, h, n, n_rows, d, q.dtype)
-    ws_bytes = lib.trifast_forward_workspace_bytes(C.byref(shp))   # 0 on the CUDA-core plan
-    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device) if ws_bytes else None
-    with torch.cuda.device(q.device):
-        rc = lib.trifast_forward(C.byref(shp), C.byref(_lib.t5(q)), C.byref(_lib.t5(k)),
-                                 C.byref(_lib.t5(v)), C.byref(_lib.t4(b)),
-                                 C.byref(_lib.mask_view(m8)), C.byref(_lib.t5(o)),
-                                 C.c_void_p(lse.data_ptr()),
-                                 C.c_void_p(ws.data_ptr() if ws is not None else None),
-                                 C.c_size_t(ws_bytes), _stream(q))
-    _lib.check(rc, "trifast_forward")
-    _lib.snapshot_status(q.device, _stream(q))
-    return o, lse
+def _load_ops():
+    """The operators (csrc/torch_ops.cpp: schema, CUDA implementations, autograd) and their fake
+    kernels.  Without the built library every call raises with build instructions."""
+    if not os.path.exists(_lib.OPS_PATH):
+        def missing(*_args):
+            raise RuntimeError(
+                f"{_lib.OPS_PATH} not found: build it with `python -m trifast_b200.build` "
+                "(needs nvcc; there is no fallback path)")
+        return missing, missing
+    torch.ops.load_library(_lib.OPS_PATH)
+
+    @torch.library.register_fake("trifast_b200::triangle_attention")
+    def _(q, k, v, b, mask):
+        bs, h, n_rows, n, d = q.shape
+        return (q.new_empty((bs, h, n_rows, n, d)),
+                q.new_empty((bs, h, n_rows, n), dtype=torch.float32))
+
+    def grads(q, k, v, b):
+        return tuple(torch.empty_like(t, memory_format=torch.contiguous_format) for t in (q, k, v, b))
+
+    @torch.library.register_fake("trifast_b200::triangle_attention_grads")
+    def _(do, q, k, v, b, o, l, mask):
+        return grads(q, k, v, b)
+
+    @torch.library.register_fake("trifast_b200::triangle_attention_backward")
+    def _(do, q, k, v, b, o, l, mask):
+        return grads(q, k, v, b) + (torch.empty_like(mask, memory_format=torch.contiguous_format),)
+
+    ops = torch.ops.trifast_b200
+    return ops.triangle_attention.default, ops.triangle_attention_backward.default
 
 
-@_triangle_attention.register_fake
-def _(q, k, v, b, mask):
-    bs, h, n_rows, n, d = q.shape
-    return (q.new_empty((bs, h, n_rows, n, d)),
-            q.new_empty((bs, h, n_rows, n), dtype=torch.float32))
-
-
-@torch.library.custom_op("trifast_b200::triangle_attention_backward", mutates_args=(),
-                         device_types="cuda")
-def triangle_attention_bwd(do: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
-                           b: torch.Tensor, o: torch.Tensor, l: torch.Tensor, mask: torch.Tensor
-                           ) -> tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor,
-                                      torch.Tensor]:
-    bs, h, n_rows, n, d = _check_inputs(q, k, v, b, mask)
-    _check_saved(do, q, o, l)
-    lib = _lib.load()
-    _lib.raise_if_device_gave_up(q.device)
-    do, q, k, v, o, b = _prep5(do), _prep5(q), _prep5(k), _prep5(v), _prep5(o), _prep4(b)
-    m8 = _prep_mask(mask)
-    l = l.contiguous()
-    dq, dk, dv = (torch.empty((bs, h, n_rows, n, d), dtype=q.dtype, device=q.device)
-                  for _ in range(3))
-    db = torch.empty((bs, h, n, n), dtype=q.dtype, device=q.device)
-    dmask = torch.zeros_like(mask)   # mask has no gradient; the reference returns zeros too
-    shp = _lib.make_shape(bs, h, n, n_rows, d, q.dtype)
-    ws_bytes = lib.trifast_backward_workspace_bytes(C.byref(shp))
-    ws = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-    with torch.cuda.device(q.device):
-        rc = lib.trifast_backward(
-            C.byref(shp), C.byref(_lib.t5(do)), C.byref(_lib.t5(q)), C.byref(_lib.t5(k)),
-            C.byref(_lib.t5(v)), C.byref(_lib.t4(b)), C.byref(_lib.mask_view(m8)),
-            C.byref(_lib.t5(o)), C.c_void_p(l.data_ptr()), C.byref(_lib.t5(dq)),
-            C.byref(_lib.t5(dk)), C.byref(_lib.t5(dv)), C.byref(_lib.t4(db)),
-            C.c_void_p(ws.data_ptr()), C.c_size_t(ws_bytes), _stream(q))
-    _lib.check(rc, "trifast_backward")
-    _lib.snapshot_status(q.device, _stream(q))
-    return dq, dk, dv, db, dmask
-
-
-@triangle_attention_bwd.register_fake
-def _(do, q, k, v, b, o, l, mask):
-    return (torch.empty_like(q, memory_format=torch.contiguous_format),
-            torch.empty_like(k, memory_format=torch.contiguous_format),
-            torch.empty_like(v, memory_format=torch.contiguous_format),
-            torch.empty_like(b, memory_format=torch.contiguous_format),
-            torch.empty_like(mask, memory_format=torch.contiguous_format))
-
-
-def _setup_context(ctx, inputs, output):
-    q, k, v, b, mask = inputs
-    o, l = output
-    ctx.save_for_backward(q, k, v, b, mask, o, l)
-
-
-def _backward(ctx, do, _dlse):
-    q, k, v, b, mask, o, l = ctx.saved_tensors
-    dq, dk, dv, db, _ = triangle_attention_bwd(do, q, k, v, b, o, l, mask)
-    return dq, dk, dv, db, None
-
-
-_triangle_attention.register_autograd(_backward, setup_context=_setup_context)
+# (q, k, v, bias, mask) -> (o, lse), and (do, q, k, v, bias, o, lse, mask) -> (dq, dk, dv, db, dmask)
+_triangle_attention, triangle_attention_bwd = _load_ops()
 
 
 def triangle_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, b: torch.Tensor,
