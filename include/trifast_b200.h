@@ -120,8 +120,10 @@ typedef struct trifast_plan {
   int32_t db_row_splits; /* row groups whose db partials are summed in fixed order */
   int32_t bwd_fused;     /* 1: dq, dk, dv come from one kernel (one exponential per score) */
   int32_t bwd_chunks;    /* query chunks a row is walked in by that kernel (1: dQ of a row fits TMEM) */
-  int32_t fwd_kernel;    /* trifast_kernel of the forward: differs from `kernel` for head dim 128,
-                            whose forward has tensor-core tiles and whose backward has not */
+  int32_t fwd_kernel;    /* trifast_kernel of the forward: differs from `kernel` for head dim 128.
+                            There `kernel` names the plan that sizes the backward's workspace; with
+                            TRIFAST_KERNEL_AUTO, 16-bit inputs and n >= 64 its tensor-core kernels
+                            run inside that workspace */
 } trifast_plan;
 
 /* Library version as major*10000 + minor*100 + patch. */

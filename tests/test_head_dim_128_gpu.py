@@ -130,3 +130,49 @@ def test_tensor_core_family_cannot_be_forced_onto_the_backward():
     plan = _lib.Plan()
     assert _lib.load().trifast_pick_plan(C.byref(shp), C.byref(plan)) == 0
     assert plan.fwd_kernel == _lib.KERNEL_TCGEN05 and plan.kernel == _lib.KERNEL_SIMT
+
+
+BWD_SHAPES = [  # (n, h, rows, dtype, mask)
+    (64, 1, None, torch.bfloat16, "none"),         # the smallest: half a resident tile, one step
+    (96, 2, None, torch.float16, "random"),        # second step half empty
+    (128, 1, 9, torch.bfloat16, "padding"),        # fewer rows than two splits of db
+    (193, 2, None, torch.bfloat16, "random"),      # ragged: padded bias copy, a one-column step
+    (328, 1, None, torch.float16, "padding"),      # dropped key tiles: zero-filled dk, dv
+    (640, 2, 24, torch.bfloat16, "ranges"),        # live ranges differ row by row
+    (1000, 1, 40, torch.bfloat16, "random"),       # 64 tiles: row splits in clusters, items > CTAs
+]
+
+
+@pytest.mark.parametrize("n,h,rows,dtype,mask", BWD_SHAPES)
+def test_backward_on_tensor_cores(n, h, rows, dtype, mask):
+    """Against the fp64 oracle and the CUDA-core kernels; exact zeros at dropped keys; bitwise
+    the same twice (db is summed over row splits in a fixed order)."""
+    from tests.helpers import abi_backward
+    rows = rows or n
+    q, k, v, b, m = _inputs(n, h, rows, dtype, mask, seed=n)
+    do = torch.randn(q.shape, generator=torch.Generator().manual_seed(2)).to(dtype)
+    dev = [t.to(DEV) for t in (q, k, v, b, m)]
+    o = torch.empty_like(dev[0])
+    lse = torch.empty(q.shape[:4], dtype=torch.float32, device=DEV)
+    abi_forward(*dev, o, lse)
+
+    def grads(kernel=None):
+        out = [torch.full_like(dev[0], float("nan")) for _ in range(3)] + [torch.full_like(dev[3], float("nan"))]
+        abi_backward(do.to(DEV), *dev, o, lse, *out, kernel=kernel)
+        torch.cuda.synchronize()
+        return [t.float().cpu() for t in out]
+
+    got, again, simt = grads(), grads(), grads(_lib.KERNEL_SIMT)
+    f = [t.float() for t in (q, k, v, b)]
+    _, _, ref = orc.forward_backward_chunked(f[0], f[1], f[2], f[3], m, do=do.float(), rows_per_chunk=8,
+                                             acc_dtype=torch.float64)
+    qq, kk, vv, bb = (t.detach().clone().requires_grad_(True) for t in (q, k, v, b))
+    orc.attention_reference_port(qq, kk, vv, bb, m).backward(do)
+    pt = [t.grad.float() for t in (qq, kk, vv, bb)]
+    for nm, x, y, z, r_, p in zip(("dq", "dk", "dv", "db"), got, again, simt, ref, pt):
+        assert torch.isfinite(x).all(), nm
+        assert torch.equal(x, y), nm
+        assert_within_pt_error(x, p, r_, DTYPE_EPS[dtype], f"d=128 n={n} {nm}")
+        assert max_abs(x, z) <= 3 * (max_abs(z, r_) + DTYPE_EPS[dtype]), f"d=128 n={n} {nm} vs CUDA cores"
+    sel = (m & ~m.all(dim=-1)[..., None])[:, None, :, :, None].expand_as(got[1])
+    assert not sel.any() or float(got[1][sel].abs().max()) == float(got[2][sel].abs().max()) == 0.0

@@ -161,6 +161,15 @@ FwdWorkspace carve_fwd(const trifast_shape* s, const trifast_plan& plan) {
   return w;
 }
 
+// Head dim 128: the backward's tensor-core kernels work inside the workspace of the CUDA-core
+// plan (row splits of db are summed in a cluster and the bias needs no transposed copy), plus
+// the padded bias copy for ragged n.  plan.kernel stays CUDA cores: they take what these
+// kernels do not (n below a quarter tile, bias rows TMA cannot address).
+bool wants_bwd_d128(const trifast_shape* s) {
+  return s->dtype != TRIFAST_F32 && s->d == 128 && s->n >= kMinTensorCoreN &&
+         s->kernel == TRIFAST_KERNEL_AUTO;
+}
+
 Workspace carve(const trifast_shape* s, const trifast_plan& plan) {
   Workspace w;
   const size_t n_pad = (size_t)(s->n + 7) / 8 * 8;  // row pitch of the vectors and bias copies
@@ -187,7 +196,7 @@ Workspace carve(const trifast_shape* s, const trifast_plan& plan) {
   w.bias_t_off = off;
   if (w.has_bias_t) off = align_up(off + bias_copy, 256);
   // bias copy with a 16-byte row pitch, when the bias rows themselves are not
-  w.has_bias_pad = w.has_bias_t && s->n % 8 != 0;
+  w.has_bias_pad = (w.has_bias_t || wants_bwd_d128(s)) && s->n % 8 != 0;
   w.bias_pad_off = off;
   if (w.has_bias_pad) off = align_up(off + bias_copy, 256);
   w.partial_off = off;
@@ -211,8 +220,9 @@ int pick_plan(const trifast_shape* s, trifast_plan* p) {
   // d = 16 tiles.
   const bool tc_ok = half && (s->d == 16 || s->d == 32 || s->d == 64) && s->n >= kMinTensorCoreN &&
                      !(s->d == 16 && (s->flags & TRIFAST_FLAG_SPLIT_BWD));
-  // Head dim 128 has tensor-core tiles in the forward only: its backward stays on the CUDA
-  // cores (`kernel`), and asking for the tensor-core family fails in the backward entry points.
+  // Head dim 128: `kernel` names the family whose workspace the backward is given, CUDA cores
+  // (see wants_bwd_d128), and asking for the tensor-core family fails in the backward entry
+  // points.
   const bool tc_fwd_only = half && s->d == 128 && s->n >= kMinTensorCoreN;
   int kernel = s->kernel;
   if (kernel == TRIFAST_KERNEL_AUTO) kernel = tc_ok ? TRIFAST_KERNEL_TCGEN05 : TRIFAST_KERNEL_SIMT;
@@ -452,6 +462,11 @@ int trifast_backward_db(const trifast_shape* shape, const trifast_t5* d_o, const
   a.db_f32 = db_f32;
   cudaStream_t s = (cudaStream_t)stream;
   if ((rc = cuda_rc(bwd_prepare(a, s)))) return rc;
+  if (wants_bwd_d128(shape) && tc_bwd_d128_supported(a)) {
+    const int64_t t = (shape->n + 127) / 128;
+    a.splits = tc_db_cluster_splits(t * t * shape->heads * shape->batch, shape->n_rows, sm_count());
+    return cuda_rc(tc_bwd_db(a, s));
+  }
   bool tc = c.plan.kernel == TRIFAST_KERNEL_TCGEN05;
   if (tc && !tc_backward_supported(a)) {
     if (shape->kernel == TRIFAST_KERNEL_TCGEN05) return TRIFAST_ERR_KERNEL_CHOICE;
@@ -479,6 +494,10 @@ int trifast_backward_dqkv(const trifast_shape* shape, const trifast_t5* d_o, con
   a.dk = make_view(dk);
   a.dv = make_view(dv);
   cudaStream_t s = (cudaStream_t)stream;
+  if (wants_bwd_d128(shape) && tc_bwd_d128_supported(a)) {
+    if ((rc = cuda_rc(tc_bwd_d128_dq(a, s)))) return rc;
+    return cuda_rc(tc_bwd_d128_dkv(a, s));
+  }
   bool tc = c.plan.kernel == TRIFAST_KERNEL_TCGEN05;
   if (tc && !tc_backward_supported(a)) {
     if (shape->kernel == TRIFAST_KERNEL_TCGEN05) return TRIFAST_ERR_KERNEL_CHOICE;

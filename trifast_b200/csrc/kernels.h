@@ -70,6 +70,11 @@ bool tc_backward_supported(const BwdArgs& a);
 cudaError_t tc_bwd_dq(const BwdArgs& a, cudaStream_t s);
 cudaError_t tc_bwd_dkv(const BwdArgs& a, cudaStream_t s);
 cudaError_t tc_bwd_db(const BwdArgs& a, cudaStream_t s);
+int tc_db_cluster_splits(int64_t tiles, int n_rows, int sms);   // d = 128: row splits summed in a cluster
+// head dim 128 (its db: tc_bwd_db)
+bool tc_bwd_d128_supported(const BwdArgs& a);
+cudaError_t tc_bwd_d128_dq(const BwdArgs& a, cudaStream_t s);
+cudaError_t tc_bwd_d128_dkv(const BwdArgs& a, cudaStream_t s);
 // dq, dk and dv in one pass over the scores
 bool tc_bwd_fused_supported(const BwdArgs& a);
 int tc_bwd_fused_chunks(int n, int d);             // query chunks per row (1: dQ of a row fits TMEM)

@@ -38,20 +38,45 @@ constexpr int kRegsLaunch = 96, kRegsIssue = 32, kRegsMath = 112;
 static_assert(512 * kRegsMath + 128 * kRegsIssue <= 640 * kRegsLaunch, "setmaxnreg pool");
 constexpr int kTmaWarp = 16, kMmaWarp = 17;
 
+// D = 128: a row of a tile is two 128-byte swizzle spans, and a stage holds one 64-element half
+// of the four tiles (KS = 2 stages per pair row, accumulated by the MMAs).
 template <int D, int NS>
 struct DbCfg {
-  static constexpr int kRowBytes = D * 2;
+  static constexpr int KS = D > 64 ? 2 : 1;
+  static constexpr int DS = D / KS;                       // head-dim elements per stage
+  static constexpr int kRowBytes = DS * 2;
   static constexpr int kTileBytes = 128 * kRowBytes;
   static constexpr int kVecBytes = 128 * 4;
   static constexpr int kStageBytes = 4 * kTileBytes + 2 * kVecBytes;   // multiple of 1024
   static constexpr int kThreads = 640;
-  static constexpr uint64_t kSwz = RowSwizzle<D>::kDesc;
+  static constexpr uint64_t kSwz = RowSwizzle<DS>::kDesc;
   static constexpr int kSbo = 8 * kRowBytes;
   static constexpr int kLiveBytes = 8192;   // one bit per row of the split (n_rows <= 65535)
   static int smem_bytes() { return 1024 + 1024 + NS * kStageBytes + kLiveBytes; }
+  // Row splits summed inside a cluster: every CTA leaves its 128 x 128 partial in its own
+  // shared memory (over the stages; rows padded by 4 floats against bank conflicts).
+  static constexpr int kPartPitch = 132;
+  static_assert(128 * kPartPitch * 4 <= NS * kStageBytes, "cluster partial");
 };
 
-template <typename T, int D, int NS>
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster4(uint32_t local_addr, uint32_t cta) {
+  uint32_t addr;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(local_addr), "r"(cta));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+
+// kCluster: the CTAs of a cluster are the row splits of one tile; their partials are summed in
+// split order through distributed shared memory and `out` gets the sum, so that neither
+// partials in global memory nor a reduce kernel are needed.
+template <typename T, int D, int NS, bool kCluster>
 __global__ void __launch_bounds__(640, 1)
 tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
              const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
@@ -83,7 +108,9 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
   auto nlse_off = [&](int s) -> uint32_t { return stage_off(s) + 4 * Cfg::kTileBytes; };
   auto delta_off = [&](int s) -> uint32_t { return nlse_off(s) + Cfg::kVecBytes; };
 
-  if (*reinterpret_cast<volatile unsigned int*>(status) != 0u) return;
+  // (a cluster's CTAs must all reach its barriers: they skip the rows instead)
+  if (!kCluster && *reinterpret_cast<volatile unsigned int*>(status) != 0u) return;
+  volatile int* skip = reinterpret_cast<volatile int*>(gbase + 264);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tiles_k = (n + 127) / 128;
@@ -95,13 +122,14 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
   };
   // item order: tile fastest, then split, then (b, h): the CTAs running together work
   // on the same rows of the same (b, h), so the Q/dO/K/V row tiles are shared in L2
+  // (split fastest with clusters, whose CTAs are consecutive)
   auto decode = [&](int w) {
     Item im;
-    const int tile = w % tiles;
+    const int tile = kCluster ? (w / splits) % tiles : w % tiles;
     const int rest = w / tiles;
     im.jt = tile / tiles_k;
     im.kt = tile % tiles_k;
-    im.split = rest % splits;
+    im.split = kCluster ? w % splits : rest % splits;
     im.bh = rest / splits;
     im.b = im.bh / dm.heads;
     im.h = im.bh % dm.heads;
@@ -120,6 +148,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
       mbar_init(bar(S_FREE + u), 16);
     }
     *abort_flag = 0;
+    if (kCluster) *skip = *reinterpret_cast<volatile unsigned int*>(status) != 0u;
     mbar_fence_init();
   }
   if (warp == kMmaWarp) {
@@ -157,6 +186,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  const bool skipped = kCluster && *skip != 0;
 
   if (warp >= kTmaWarp) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
@@ -165,24 +195,25 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
       if (lane == 0) {
         const Item im = decode(blockIdx.x);
         int g = 0;
-        bool stop = false;
+        bool stop = skipped;
         for (int r0 = 0; r0 < im.nrows && !stop; r0 += 32) {
-        for (uint32_t bits = live[r0 >> 5]; bits != 0u; bits &= bits - 1u) {
-          {
+        for (uint32_t bits = live[r0 >> 5]; bits != 0u && !stop; bits &= bits - 1u) {
+          for (int c = 0; c < Cfg::KS; ++c) {
             const int s = g % NS, i = im.i_begin + r0 + __ffs(bits) - 1;
             if (g >= NS && !mbar_wait(bar(EMPTY + s), ((g / NS) - 1) & 1, abort_flag)) {
               stop = true;
               break;
             }
+            const int c0 = c * Cfg::DS;
             mbar_arrive_expect_tx(bar(FULL + s), Cfg::kStageBytes);
-            tma_load_5d(q_tile(s), &map_q, bar(FULL + s), 0, im.jt * 128, i, im.h, im.b);
-            tma_load_5d(do_tile(s), &map_do, bar(FULL + s), 0, im.jt * 128, i, im.h, im.b);
-            tma_load_5d(k_tile(s), &map_k, bar(FULL + s), 0, im.kt * 128, i, im.h, im.b);
-            tma_load_5d(v_tile(s), &map_v, bar(FULL + s), 0, im.kt * 128, i, im.h, im.b);
+            tma_load_5d(q_tile(s), &map_q, bar(FULL + s), c0, im.jt * 128, i, im.h, im.b);
+            tma_load_5d(do_tile(s), &map_do, bar(FULL + s), c0, im.jt * 128, i, im.h, im.b);
+            tma_load_5d(k_tile(s), &map_k, bar(FULL + s), c0, im.kt * 128, i, im.h, im.b);
+            tma_load_5d(v_tile(s), &map_v, bar(FULL + s), c0, im.kt * 128, i, im.h, im.b);
             tma_load_4d(base + nlse_off(s), &map_nlse, bar(FULL + s), im.jt * 128, i, im.h, im.b);
             tma_load_4d(base + delta_off(s), &map_delta, bar(FULL + s), im.jt * 128, i, im.h, im.b);
+            ++g;
           }
-          ++g;
         }
         }
       }
@@ -191,31 +222,35 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
       if (lane == 0) {
         constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
         constexpr uint32_t idesc = make_idesc(128, 128, kBf16, false, false);
-        bool ok = true;
+        bool ok = !skipped;
         {
           const int nrows = decode(blockIdx.x).nrows;
           int g = 0;
           for (int r0 = 0; r0 < nrows && ok; r0 += 32) {
           for (uint32_t bits = live[r0 >> 5]; bits != 0u && ok; bits &= bits - 1u) {
-            const int s = g % NS, u = g & 1;
-            ok = mbar_wait(bar(FULL + s), (g / NS) & 1, abort_flag);
-            if (ok && g >= 2) ok = mbar_wait(bar(S_FREE + u), ((g >> 1) - 1) & 1, abort_flag);
+            const int u = g & 1;
+            if (g >= 2) ok = mbar_wait(bar(S_FREE + u), ((g >> 1) - 1) & 1, abort_flag);
+            for (int c = 0; c < Cfg::KS && ok; ++c) {
+              const int sg = g * Cfg::KS + c, s = sg % NS;
+              ok = mbar_wait(bar(FULL + s), (sg / NS) & 1, abort_flag);
+              if (!ok) break;
+              tc_fence_after();
+#pragma unroll
+              for (int kk = 0; kk < Cfg::DS / 16; ++kk) {
+                const uint64_t aq = make_smem_desc(q_tile(s) + kk * 32, 16, Cfg::kSbo, Cfg::kSwz);
+                const uint64_t bk = make_smem_desc(k_tile(s) + kk * 32, 16, Cfg::kSbo, Cfg::kSwz);
+                umma_ss(tmem_base + u * 256, aq, bk, idesc, c > 0 || kk > 0);
+              }
+#pragma unroll
+              for (int kk = 0; kk < Cfg::DS / 16; ++kk) {
+                const uint64_t ag = make_smem_desc(do_tile(s) + kk * 32, 16, Cfg::kSbo, Cfg::kSwz);
+                const uint64_t bv = make_smem_desc(v_tile(s) + kk * 32, 16, Cfg::kSbo, Cfg::kSwz);
+                umma_ss(tmem_base + u * 256 + 128, ag, bv, idesc, c > 0 || kk > 0);
+              }
+              if (c == Cfg::KS - 1) umma_commit(bar(S_FULL + u));
+              umma_commit(bar(EMPTY + s));
+            }
             if (!ok) break;
-            tc_fence_after();
-#pragma unroll
-            for (int kk = 0; kk < D / 16; ++kk) {
-              const uint64_t aq = make_smem_desc(q_tile(s) + kk * 32, 16, Cfg::kSbo, Cfg::kSwz);
-              const uint64_t bk = make_smem_desc(k_tile(s) + kk * 32, 16, Cfg::kSbo, Cfg::kSwz);
-              umma_ss(tmem_base + u * 256, aq, bk, idesc, kk > 0);
-            }
-#pragma unroll
-            for (int kk = 0; kk < D / 16; ++kk) {
-              const uint64_t ag = make_smem_desc(do_tile(s) + kk * 32, 16, Cfg::kSbo, Cfg::kSwz);
-              const uint64_t bv = make_smem_desc(v_tile(s) + kk * 32, 16, Cfg::kSbo, Cfg::kSwz);
-              umma_ss(tmem_base + u * 256 + 128, ag, bv, idesc, kk > 0);
-            }
-            umma_commit(bar(S_FULL + u));
-            umma_commit(bar(EMPTY + s));
             ++g;
           }
           }
@@ -230,7 +265,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
     const float c1 = dm.scale * kLog2e;
     const float uniform = 1.f / (float)n;
 
-    bool ok = true;
+    bool ok = !skipped;
     {
       const Item im = decode(blockIdx.x);
       const int b = im.b, h = im.h, kt = im.kt;
@@ -273,13 +308,22 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
       int g = 0;
       for (int r0 = 0; r0 < im.nrows && ok; r0 += 32) {
       for (uint32_t bits = live[r0 >> 5]; bits != 0u; bits &= bits - 1u) {
-        const int s = g % NS, u = g & 1, i = im.i_begin + r0 + __ffs(bits) - 1;
+        // (with KS stages per row the vectors are read from the last one; the earlier ones are
+        // released as they come, untouched)
+        const int sg = g * Cfg::KS + Cfg::KS - 1;
+        const int s = sg % NS, u = g & 1, i = im.i_begin + r0 + __ffs(bits) - 1;
         // per-row inputs that do not come through shared memory (consumed after the
         // barrier waits below, which hide their latency)
         const uint32_t mw =
             __ldg(maskbits + ((int64_t)b * dm.n_rows + i) * mask_words + kt * 4 + quarter);
         const bool row_full = rowfull[b * dm.n_rows + i] != 0;
-        ok = __all_sync(0xffffffffu, mbar_wait(bar(FULL + s), (g / NS) & 1, abort_flag));
+        if (Cfg::KS > 1) {
+          const int s0 = (sg - 1) % NS;
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(FULL + s0), ((sg - 1) / NS) & 1, abort_flag));
+          if (!ok) break;
+          if (lane == 0) mbar_arrive(bar(EMPTY + s0));
+        }
+        ok = __all_sync(0xffffffffu, mbar_wait(bar(FULL + s), (sg / NS) & 1, abort_flag));
         if (!ok) break;
         const float nl = reinterpret_cast<const float*>(gbase + nlse_off(s))[row];
         const float dl = reinterpret_cast<const float*>(gbase + delta_off(s))[row];
@@ -340,7 +384,16 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
         ++g;
       }
       }
-      if (ok && n_store > 0) {
+      if (kCluster) {
+        // the last row's S_FULL has completed every load and MMA that used the stages, for all
+        // warps alike once the cluster barrier below is passed; here a named barrier of the
+        // elementwise warps orders their last reads of the vectors before the partials
+        asm volatile("bar.sync 1, 512;" ::: "memory");
+        float* part = reinterpret_cast<float*>(gbase + tiles_off) + row * Cfg::kPartPitch + quarter * 32;
+#pragma unroll
+        for (int c = 0; c < 32; c += 4)
+          *reinterpret_cast<float4*>(part + c) = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
+      } else if (ok && n_store > 0) {
         if (n_store == 32 && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
 #pragma unroll
           for (int c = 0; c < 32; c += 4)
@@ -352,6 +405,40 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
         }
       }
     }
+  }
+
+  if (kCluster) {
+    // each CTA sums its share of the tile's rows over the cluster, in split order; the second
+    // barrier keeps a CTA's shared memory alive until its readers are done
+    __syncwarp();
+    cluster_sync();
+    const Item im = decode(blockIdx.x);
+    const int share = 128 / splits, r0 = im.split * share;
+    if (!skipped && *abort_flag == 0) {
+      for (int idx = tid; idx < share * 32; idx += Cfg::kThreads) {
+        const int r = r0 + (idx >> 5), c = (idx & 31) * 4;
+        const uint32_t at = base + tiles_off + (r * Cfg::kPartPitch + c) * 4;
+        float4 sum = ld_cluster4(at, 0);
+        for (int k = 1; k < splits; ++k) {
+          const float4 v = ld_cluster4(at, k);
+          sum.x += v.x;
+          sum.y += v.y;
+          sum.z += v.z;
+          sum.w += v.w;
+        }
+        const int j = im.jt * 128 + r, key = im.kt * 128 + c;
+        if (j < n && key < n) {
+          float* dst = out + ((int64_t)im.bh * n + j) * n + key;
+          if (key + 4 <= n && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+            *reinterpret_cast<float4*>(dst) = sum;
+          } else {
+            const float e[4] = {sum.x, sum.y, sum.z, sum.w};
+            for (int k = 0; k < 4 && key + k < n; ++k) dst[k] = e[k];
+          }
+        }
+      }
+    }
+    cluster_sync();
   }
 
   // ---------------------------------------------------------------- teardown
@@ -370,7 +457,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
   }
 }
 
-template <typename T, int D, int NS>
+template <typename T, int D, int NS, bool kCluster = false>
 cudaError_t launch_db(const BwdArgs& a, cudaStream_t stream) {
   using Cfg = DbCfg<D, NS>;
   const Dims& dm = a.dm;
@@ -379,8 +466,8 @@ cudaError_t launch_db(const BwdArgs& a, cudaStream_t stream) {
   CUtensorMap mq, mdo, mk, mv, mnl, mdl;
   const uint64_t dims5[5] = {(uint64_t)D, (uint64_t)dm.n, (uint64_t)dm.n_rows, (uint64_t)dm.heads,
                              (uint64_t)dm.batch};
-  const uint32_t box[5] = {(uint32_t)D, 128, 1, 1, 1};
-  const CUtensorMapSwizzle swz = (CUtensorMapSwizzle)RowSwizzle<D>::kTma;
+  const uint32_t box[5] = {(uint32_t)Cfg::DS, 128, 1, 1, 1};
+  const CUtensorMapSwizzle swz = (CUtensorMapSwizzle)RowSwizzle<Cfg::DS>::kTma;
   auto map5 = [&](CUtensorMap* m, const View5& v) {
     const uint64_t st[4] = {(uint64_t)v.sj * eb, (uint64_t)v.si * eb, (uint64_t)v.sh * eb,
                             (uint64_t)v.sb * eb};
@@ -398,19 +485,35 @@ cudaError_t launch_db(const BwdArgs& a, cudaStream_t stream) {
       return cudaErrorInvalidValue;
   }
   const int smem = Cfg::smem_bytes();
-  constexpr auto kern = tc_db_kernel<T, D, NS>;
+  constexpr auto kern = tc_db_kernel<T, D, NS, kCluster>;
   cudaError_t e = opt_in_smem<kern>(smem);
   if (e != cudaSuccess) return e;
   const int t = (dm.n + 127) / 128;
   const int total = t * t * a.splits * dm.batch * dm.heads;
   const int grid = total;  // one item per CTA
-  float* out = a.splits > 1 ? a.db_partials : a.db_f32;
+  float* out = a.splits > 1 && !kCluster ? a.db_partials : a.db_f32;
   View4 bias = a.bias;
   if (a.bias_pad) {  // the copy with a 16-byte row pitch: its rows can be read 16 bytes at a time
     bias.p = (char*)a.bias_pad;
     bias.sj = dm.n_pad;
     bias.sh = (int64_t)dm.n * dm.n_pad;
     bias.sb = bias.sh * dm.heads;
+  }
+  if (kCluster) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = a.splits;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(Cfg::kThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, mq, mdo, mk, mv, mnl, mdl, bias, (const uint8_t*)a.rowfull,
+                              (const uint32_t*)a.maskbits_lin, a.mask_words, (const uint32_t*)a.rowrange,
+                              out, a.splits, dm, a.status);
   }
   kern<<<grid, Cfg::kThreads, smem, stream>>>(mq, mdo, mk, mv, mnl, mdl, bias, a.rowfull,
                                               a.maskbits_lin, a.mask_words, a.rowrange, out, a.splits,
@@ -420,9 +523,27 @@ cudaError_t launch_db(const BwdArgs& a, cudaStream_t stream) {
 
 }  // namespace
 
+// Row splits of a tile when a cluster sums them (a power of two up to 8, the portable cluster
+// size): the count whose rounds of CTAs over the SMs, each lasting a split's rows and about
+// six rows' time of prologue and exchange, end first.
+int tc_db_cluster_splits(int64_t tiles, int n_rows, int sms) {
+  int best = 1;
+  int64_t best_cost = INT64_MAX;
+  for (int s = 1; s <= 8 && n_rows / s >= 8; s *= 2) {
+    const int64_t cost = ((tiles * s + sms - 1) / sms) * ((n_rows + s - 1) / s + 6);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = s;
+    }
+  }
+  return best;
+}
+
 cudaError_t tc_bwd_db(const BwdArgs& a, cudaStream_t s) {
   const bool bf16 = a.dtype == TRIFAST_BF16;
   if (!a.neg_lse2 || !a.maskbits_lin) return cudaErrorInvalidValue;
+  if (a.dm.d == 128)
+    return bf16 ? launch_db<__nv_bfloat16, 128, 3, true>(a, s) : launch_db<__half, 128, 3, true>(a, s);
   if (a.dm.d == 16)
     return bf16 ? launch_db<__nv_bfloat16, 16, 4>(a, s) : launch_db<__half, 16, 4>(a, s);
   if (a.dm.d == 32)
