@@ -407,3 +407,25 @@ def test_step_can_be_captured_in_a_cuda_graph(n, d, dtype):
     for name, x, y in zip(NAMES, replayed, eager):
         assert torch.isfinite(x.float()).all(), name
         assert torch.equal(x, y), f"{name}: graph replay differs from the eager step"
+
+
+@pytest.mark.parametrize("n,d,dtype", [
+    (3, 32, torch.float32), (32, 32, torch.float32), (33, 32, torch.float32),     # either side of the small tiles
+    (64, 16, torch.float32), (65, 64, torch.float32), (97, 128, torch.float32),   # one streamed tile, a remainder
+    (130, 32, torch.float32), (63, 32, torch.bfloat16), (31, 64, torch.float16),  # rows 4 bytes off; 16-bit inputs
+])
+def test_cuda_core_kernels_at_their_tile_edges(n, d, dtype):
+    torch.manual_seed(n + d)
+    h = 2
+    q, k, v = (torch.randn(1, h, n, n, d).to(dtype) for _ in range(3))
+    b = torch.randn(1, h, n, n).to(dtype)
+    m = torch.rand(1, n, n) < 0.3
+    m[0, n // 2] = True                                   # a fully masked row
+    do = torch.randn(1, h, n, n, d).to(dtype)
+    dev = [t.to(DEV).requires_grad_(True) for t in (q, k, v, b)]
+    o = triangle_attention(*dev, m.to(DEV))
+    got = (o,) + torch.autograd.grad(o, dev, do.to(DEV))
+    got = tuple(t.detach().float().cpu() for t in got)
+    ref_o, _ = orc.forward(q, k, v, b, m, torch.float64)
+    ref = (ref_o,) + orc.backward(do, q, k, v, b, m, torch.float64)
+    check(dtype, got, ref, None if dtype == torch.float32 else run_pt(q, k, v, b, m, do), f"edge n={n} d={d}")

@@ -237,21 +237,27 @@ int pick_plan(const trifast_shape* s, trifast_plan* p) {
     p->stages = (s->d <= 32) ? 3 : 2;
   } else {
     p->block_j = 64;
-    p->block_k = (s->d <= 32) ? 32 : 16;
+    p->block_k = (s->d <= 32) ? 64 : 32;
     p->rows_per_cta = 1;
     p->stages = 1;
   }
-  // db: CTAs = tiles * splits.  Split the local rows until the grid covers the
-  // 148 SMs twice (CUDA-core kernel, 32 x 32 tiles, several CTAs per SM) or four
-  // times (tensor-core kernel, 128 x 128 tiles, one CTA per SM), but never below
-  // 8 rows per split and at most 16 splits.
+  // db: CTAs = tiles * splits.  Tensor-core kernel (128 x 128 tiles, one CTA per SM): split the
+  // local rows until the grid covers the 148 SMs four times, but never below 8 rows per split
+  // and at most 16 splits.  CUDA-core kernel (64 x 64 tiles, 32 x 32 for n <= 32, two CTAs per
+  // SM): until 256 CTAs, down to 2 rows per split (a row is a whole product there, and small
+  // problems have few), while the partials stay below 5 MiB (beyond that their traffic shows,
+  // and the largest problem that fits a fixed workspace would shrink).
   const bool tc_db = kernel == TRIFAST_KERNEL_TCGEN05;
-  const int tile = tc_db ? 128 : 32;
-  const int64_t want = tc_db ? 592 : 296;
+  const int tile = tc_db ? 128 : s->n <= 32 ? 32 : 64;
+  const int64_t want = tc_db ? 592 : 256;
+  const int min_rows = tc_db ? 8 : 2;
   const int64_t t = (s->n + tile - 1) / tile;
-  const int64_t tiles = t * t * s->batch * s->heads;
+  const int64_t bh = (int64_t)s->batch * s->heads, tiles = t * t * bh;
+  const int64_t db_bytes = bh * s->n * s->n * (int64_t)sizeof(float);
   int splits = 1;
-  while (splits < 16 && tiles * splits < want && s->n_rows / (splits * 2) >= 8) splits *= 2;
+  while (splits < 16 && tiles * splits < want && s->n_rows / (splits * 2) >= min_rows &&
+         (tc_db || db_bytes * splits * 2 <= (5 << 20)))
+    splits *= 2;
   p->db_row_splits = splits;
   // dq, dk, dv from one kernel on the tensor-core path; a row whose dQ (D fp32 columns
   // per 128 queries) does not fit in TMEM beside the other accumulators (192 + 2 D

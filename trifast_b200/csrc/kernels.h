@@ -50,7 +50,7 @@ struct BwdArgs {
   unsigned int* status;
 };
 
-// CUDA-core kernels (simt_kernels.cu): any dtype, any n, d in {16, 32, 64, 128}.
+// CUDA-core kernels (simt_attention.cu) and the kernels around both families (support_kernels.cu): any dtype, any n, d in {16, 32, 64, 128}.
 cudaError_t simt_forward(const FwdArgs& a, cudaStream_t s);
 cudaError_t bwd_prepare(const BwdArgs& a, cudaStream_t s);   // delta, row flags, masks, bias copies
 cudaError_t fwd_prepare(const FwdArgs& a, cudaStream_t s);   // row flags, masks, padded bias
