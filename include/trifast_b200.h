@@ -74,7 +74,13 @@ typedef enum trifast_flags {
   /* Not a debug switch: set by row-sharded callers.  trifast_backward_dqkv then leaves 8 SMs
    * free, so that the all-reduce of db launched beside it (another stream) finds room to run
    * at once instead of after it.  (No reference counterpart: the reference is single-GPU.) */
-  TRIFAST_FLAG_SHARE_GPU = 2
+  TRIFAST_FLAG_SHARE_GPU = 2,
+  /* The bias and mask arguments of the forward and backward calls point to the longer
+   * descriptors trifast_t4_strided and trifast_mask_strided: any non-negative strides, the
+   * innermost dimension's included (a projection's (b, n, n, h) output seen as (b, h, n, n), a
+   * transposed pair map).  The workspaces then hold packed copies where the kernels need them;
+   * the size functions look at this flag. */
+  TRIFAST_FLAG_STRIDED = 8
 } trifast_flags;
 /* With TRIFAST_FLAG_SHARE_GPU, bits 8-15 of `flags` hold the number of SMs to leave free
  * (0 = 8): as many as the collective beside the kernel has CTAs that must run at once. */
@@ -109,6 +115,17 @@ typedef struct trifast_mask {
   const uint8_t* data;
   int64_t stride[2];
 } trifast_mask;
+
+/* The same with a stride for k as well: what a trifast_t4* bias and a trifast_mask* point to
+ * under TRIFAST_FLAG_STRIDED. */
+typedef struct trifast_t4_strided {
+  void* data;
+  int64_t stride[4];
+} trifast_t4_strided;
+typedef struct trifast_mask_strided {
+  const uint8_t* data;
+  int64_t stride[3];
+} trifast_mask_strided;
 
 /* Tile plan chosen by the heuristic (host only; no device needed). */
 typedef struct trifast_plan {

@@ -429,3 +429,24 @@ def test_cuda_core_kernels_at_their_tile_edges(n, d, dtype):
     ref_o, _ = orc.forward(q, k, v, b, m, torch.float64)
     ref = (ref_o,) + orc.backward(do, q, k, v, b, m, torch.float64)
     check(dtype, got, ref, None if dtype == torch.float32 else run_pt(q, k, v, b, m, do), f"edge n={n} d={d}")
+
+
+@pytest.mark.parametrize("n,d,dtype", [(48, 32, torch.float32), (40, 32, torch.bfloat16), (64, 32, torch.bfloat16),
+                                       (131, 16, torch.float16), (136, 64, torch.bfloat16), (200, 128, torch.bfloat16)])
+def test_strided_bias_and_mask_equal_dense_copies(n, d, dtype):
+    """A permuted, a misaligned and an expanded bias with a transposed mask: packed by the
+    prepare kernels, bit for bit the results of dense copies."""
+    torch.manual_seed(n)
+    h = 3
+    q, k, v, do = (torch.randn(1, h, n, n, d, device=DEV).to(dtype) for _ in range(4))
+    m = (torch.rand(1, n, n, device=DEV) < 0.3).transpose(1, 2)
+    wide = torch.randn(1, h, n, n + 3, device=DEV).to(dtype)
+    for b in (torch.randn(1, n, n, h, device=DEV).to(dtype).permute(0, 3, 1, 2), wide[..., 1:n + 1],
+              torch.randn(1, 1, n, n, device=DEV).to(dtype).transpose(2, 3).expand(1, h, n, n)):
+        res = []
+        for bias, mask in ((b, m), (b.contiguous(), m.contiguous())):
+            leaves = [t.detach().requires_grad_(True) for t in (q, k, v, bias)]
+            o = triangle_attention(*leaves, mask)
+            res.append((o.detach(),) + torch.autograd.grad(o, leaves, do))
+        for nm, x, y in zip(NAMES, *res):
+            assert torch.equal(x, y), nm

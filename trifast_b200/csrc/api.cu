@@ -66,7 +66,8 @@ int check_shape(const trifast_shape* s) {
   if (s->dtype < TRIFAST_F32 || s->dtype > TRIFAST_F16) return TRIFAST_ERR_DTYPE;
   if (s->kernel < TRIFAST_KERNEL_AUTO || s->kernel > TRIFAST_KERNEL_TCGEN05)
     return TRIFAST_ERR_KERNEL_CHOICE;
-  if (s->flags & ~(TRIFAST_FLAG_SPLIT_BWD | TRIFAST_FLAG_SHARE_GPU | 0xff00)) return TRIFAST_ERR_KERNEL_CHOICE;
+  if (s->flags & ~(TRIFAST_FLAG_SPLIT_BWD | TRIFAST_FLAG_SHARE_GPU | TRIFAST_FLAG_STRIDED | 0xff00))
+    return TRIFAST_ERR_KERNEL_CHOICE;
   if ((s->flags & 0xff00) && !(s->flags & TRIFAST_FLAG_SHARE_GPU)) return TRIFAST_ERR_KERNEL_CHOICE;
   return TRIFAST_OK;
 }
@@ -101,8 +102,24 @@ int check_t4(const trifast_t4* t, const trifast_shape* s) {
   return TRIFAST_OK;
 }
 
+bool strided(const trifast_shape* s) { return (s->flags & TRIFAST_FLAG_STRIDED) != 0; }
+
+int check_bias(const trifast_t4* t, const trifast_shape* s) {
+  if (!strided(s)) return check_t4(t, s);
+  if (!t || !t->data) return TRIFAST_ERR_NULL;
+  if (((uintptr_t)t->data) & (elem_bytes(s->dtype) - 1)) return TRIFAST_ERR_ALIGN;
+  for (int a = 0; a < 4; ++a)
+    if (reinterpret_cast<const trifast_t4_strided*>(t)->stride[a] < 0) return TRIFAST_ERR_STRIDE;
+  return TRIFAST_OK;
+}
+
 int check_mask(const trifast_mask* m, const trifast_shape* s) {
   if (!m || !m->data) return TRIFAST_ERR_NULL;
+  if (strided(s)) {
+    for (int a = 0; a < 3; ++a)
+      if (reinterpret_cast<const trifast_mask_strided*>(m)->stride[a] < 0) return TRIFAST_ERR_STRIDE;
+    return TRIFAST_OK;
+  }
   if (m->stride[0] < 0 || m->stride[1] < s->n) return TRIFAST_ERR_STRIDE;
   return TRIFAST_OK;
 }
@@ -147,7 +164,7 @@ FwdWorkspace carve_fwd(const trifast_shape* s, const trifast_plan& plan) {
   w.rowrange_off = off;
   off = (off + (size_t)s->batch * s->n_rows * sizeof(uint32_t) + 255) / 256 * 256;
   w.total = off;
-  w.bias_pad = s->n % 8 != 0;
+  w.bias_pad = s->n % 8 != 0 || strided(s);
   w.masks = w.bias_pad || s->d == 128;   // the head-dim-128 forward always reads prepared masks
   if (!w.masks) return w;
   const size_t n_pad = (size_t)(s->n + 7) / 8 * 8;
@@ -196,7 +213,7 @@ Workspace carve(const trifast_shape* s, const trifast_plan& plan) {
   w.bias_t_off = off;
   if (w.has_bias_t) off = align_up(off + bias_copy, 256);
   // bias copy with a 16-byte row pitch, when the bias rows themselves are not
-  w.has_bias_pad = (w.has_bias_t || wants_bwd_d128(s)) && s->n % 8 != 0;
+  w.has_bias_pad = (w.has_bias_t || wants_bwd_d128(s)) && (s->n % 8 != 0 || strided(s));
   w.bias_pad_off = off;
   if (w.has_bias_pad) off = align_up(off + bias_copy, 256);
   w.partial_off = off;
@@ -289,7 +306,7 @@ int fill_bwd(const trifast_shape* shape, const Common& c, const trifast_t5* d_o,
              const float* lse, void* workspace, size_t workspace_bytes, BwdArgs* a) {
   int rc;
   if ((rc = check_t5(d_o, shape)) || (rc = check_t5(q, shape)) || (rc = check_t5(k, shape)) ||
-      (rc = check_t5(v, shape)) || (rc = check_t4(bias, shape)) || (rc = check_mask(mask, shape)))
+      (rc = check_t5(v, shape)) || (rc = check_bias(bias, shape)) || (rc = check_mask(mask, shape)))
     return rc;
   if (o && (rc = check_t5(o, shape))) return rc;
   if (!lse) return TRIFAST_ERR_NULL;
@@ -305,8 +322,8 @@ int fill_bwd(const trifast_shape* shape, const Common& c, const trifast_t5* d_o,
   a->k = make_view(k);
   a->v = make_view(v);
   if (o) a->o = make_view(o);
-  a->bias = make_view(bias);
-  a->mask = make_view(mask);
+  a->bias = bias_view(bias, shape->flags);
+  a->mask = mask_view(mask, shape->flags);
   a->lse = lse;
   char* base = (char*)workspace;
   a->delta = (float*)(base + w.delta_off);
@@ -338,6 +355,45 @@ int cuda_rc(cudaError_t e) {
   if (e == cudaSuccess) return TRIFAST_OK;
   g_last_cuda_error = e;
   return TRIFAST_ERR_LAUNCH;
+}
+
+// The kernels a backward runs on.
+enum BwdKernels { kBwdSimt, kBwdFused, kBwdSplit, kBwdD128 };
+
+int pick_bwd(const trifast_shape* shape, const Common& c, BwdArgs* a, BwdKernels* kern) {
+  if (wants_bwd_d128(shape) && tc_bwd_d128_supported(*a)) {
+    const int64_t t = (shape->n + 127) / 128;
+    a->splits = tc_db_cluster_splits(t * t * shape->heads * shape->batch, shape->n_rows, sm_count());
+    *kern = kBwdD128;
+    return TRIFAST_OK;
+  }
+  *kern = kBwdSimt;
+  if (c.plan.kernel != TRIFAST_KERNEL_TCGEN05) return TRIFAST_OK;
+  if (!tc_backward_supported(*a))
+    return shape->kernel == TRIFAST_KERNEL_TCGEN05 ? TRIFAST_ERR_KERNEL_CHOICE : TRIFAST_OK;
+  *kern = c.plan.bwd_fused && tc_bwd_fused_supported(*a) ? kBwdFused : kBwdSplit;
+  return TRIFAST_OK;
+}
+
+// db into a.db_f32, or its row-split partials into a.db_partials
+int run_db(const BwdArgs& a, BwdKernels kern, cudaStream_t s) {
+  return cuda_rc(kern == kBwdSimt ? simt_bwd_db(a, s) : tc_bwd_db(a, s));
+}
+
+int run_dqkv(const BwdArgs& a, BwdKernels kern, cudaStream_t s) {
+  int rc;
+  switch (kern) {
+    case kBwdFused: return cuda_rc(tc_bwd_dqkv_fused(a, s));
+    case kBwdD128:
+      if ((rc = cuda_rc(tc_bwd_d128_dq(a, s)))) return rc;
+      return cuda_rc(tc_bwd_d128_dkv(a, s));
+    case kBwdSplit:
+      if ((rc = cuda_rc(tc_bwd_dq(a, s)))) return rc;
+      return cuda_rc(tc_bwd_dkv(a, s));
+    default:
+      if ((rc = cuda_rc(simt_bwd_dq(a, s)))) return rc;
+      return cuda_rc(simt_bwd_dkv(a, s));
+  }
 }
 
 }  // namespace
@@ -411,7 +467,7 @@ int trifast_forward(const trifast_shape* shape, const trifast_t5* q, const trifa
   int rc = check_shape(shape);
   if (rc) return rc;
   if ((rc = check_t5(q, shape)) || (rc = check_t5(k, shape)) || (rc = check_t5(v, shape)) ||
-      (rc = check_t5(o, shape)) || (rc = check_t4(bias, shape)) || (rc = check_mask(mask, shape)))
+      (rc = check_t5(o, shape)) || (rc = check_bias(bias, shape)) || (rc = check_mask(mask, shape)))
     return rc;
   if (!lse) return TRIFAST_ERR_NULL;
   Common c;
@@ -424,8 +480,8 @@ int trifast_forward(const trifast_shape* shape, const trifast_t5* q, const trifa
   a.k = make_view(k);
   a.v = make_view(v);
   a.o = make_view(o);
-  a.bias = make_view(bias);
-  a.mask = make_view(mask);
+  a.bias = bias_view(bias, shape->flags);
+  a.mask = mask_view(mask, shape->flags);
   a.lse = lse;
   a.dm = c.dm;
   a.dtype = shape->dtype;
@@ -448,7 +504,11 @@ int trifast_forward(const trifast_shape* shape, const trifast_t5* q, const trifa
       if (shape->kernel == TRIFAST_KERNEL_TCGEN05) return TRIFAST_ERR_KERNEL_CHOICE;
       return cuda_rc(simt_forward(a, s));
     }
-    if (w.total && (rc = cuda_rc(fwd_prepare(a, s)))) return rc;
+    // up to 128 keys are one tile, which every row walks: nothing to prepare but copies
+    if (shape->n <= 128 && !w.masks)
+      a.rowrange = nullptr;
+    else if ((rc = cuda_rc(fwd_prepare(a, s))))
+      return rc;
     return cuda_rc(d128 ? tc_forward_d128(a, s) : tc_forward(a, c.plan, s));
   }
   return cuda_rc(simt_forward(a, s));
@@ -467,19 +527,11 @@ int trifast_backward_db(const trifast_shape* shape, const trifast_t5* d_o, const
     return rc;
   a.db_f32 = db_f32;
   cudaStream_t s = (cudaStream_t)stream;
-  if ((rc = cuda_rc(bwd_prepare(a, s)))) return rc;
-  if (wants_bwd_d128(shape) && tc_bwd_d128_supported(a)) {
-    const int64_t t = (shape->n + 127) / 128;
-    a.splits = tc_db_cluster_splits(t * t * shape->heads * shape->batch, shape->n_rows, sm_count());
-    return cuda_rc(tc_bwd_db(a, s));
-  }
-  bool tc = c.plan.kernel == TRIFAST_KERNEL_TCGEN05;
-  if (tc && !tc_backward_supported(a)) {
-    if (shape->kernel == TRIFAST_KERNEL_TCGEN05) return TRIFAST_ERR_KERNEL_CHOICE;
-    tc = false;
-  }
-  if ((rc = cuda_rc(tc ? tc_bwd_db(a, s) : simt_bwd_db(a, s)))) return rc;
-  return cuda_rc(db_reduce_splits(a, s));
+  BwdKernels kern;
+  if ((rc = pick_bwd(shape, c, &a, &kern)) || (rc = cuda_rc(bwd_prepare(a, s))) ||
+      (rc = run_db(a, kern, s)))
+    return rc;
+  return kern == kBwdD128 ? TRIFAST_OK : cuda_rc(db_reduce_splits(a, s));
 }
 
 int trifast_backward_dqkv(const trifast_shape* shape, const trifast_t5* d_o, const trifast_t5* q,
@@ -499,19 +551,9 @@ int trifast_backward_dqkv(const trifast_shape* shape, const trifast_t5* d_o, con
   a.dq = make_view(dq);
   a.dk = make_view(dk);
   a.dv = make_view(dv);
-  cudaStream_t s = (cudaStream_t)stream;
-  if (wants_bwd_d128(shape) && tc_bwd_d128_supported(a)) {
-    if ((rc = cuda_rc(tc_bwd_d128_dq(a, s)))) return rc;
-    return cuda_rc(tc_bwd_d128_dkv(a, s));
-  }
-  bool tc = c.plan.kernel == TRIFAST_KERNEL_TCGEN05;
-  if (tc && !tc_backward_supported(a)) {
-    if (shape->kernel == TRIFAST_KERNEL_TCGEN05) return TRIFAST_ERR_KERNEL_CHOICE;
-    tc = false;
-  }
-  if (tc && c.plan.bwd_fused && tc_bwd_fused_supported(a)) return cuda_rc(tc_bwd_dqkv_fused(a, s));
-  if ((rc = cuda_rc(tc ? tc_bwd_dq(a, s) : simt_bwd_dq(a, s)))) return rc;
-  return cuda_rc(tc ? tc_bwd_dkv(a, s) : simt_bwd_dkv(a, s));
+  BwdKernels kern;
+  if ((rc = pick_bwd(shape, c, &a, &kern))) return rc;
+  return run_dqkv(a, kern, (cudaStream_t)stream);
 }
 
 int trifast_db_finalize(const trifast_shape* shape, const float* db_f32, const trifast_t4* db,
@@ -520,7 +562,7 @@ int trifast_db_finalize(const trifast_shape* shape, const float* db_f32, const t
   if (rc) return rc;
   if (!db_f32) return TRIFAST_ERR_NULL;
   if ((rc = check_t4(db, shape))) return rc;
-  return cuda_rc(db_cast(db_f32, make_view(db), shape->dtype, shape->batch, shape->heads,
+  return cuda_rc(db_cast(db_f32, 1, make_view(db), shape->dtype, shape->batch, shape->heads,
                          shape->n, (cudaStream_t)stream));
 }
 
@@ -537,18 +579,23 @@ int trifast_backward(const trifast_shape* shape, const trifast_t5* d_o, const tr
   if ((rc = check_t5(dq, shape)) || (rc = check_t5(dk, shape)) || (rc = check_t5(dv, shape)) ||
       (rc = check_t4(db, shape)))
     return rc;
-  trifast_plan plan;
-  if ((rc = pick_plan(shape, &plan))) return rc;
-  const Workspace w = carve(shape, plan);
-  if (!workspace || workspace_bytes < w.total) return TRIFAST_ERR_WORKSPACE;
-  float* db_f32 = (float*)((char*)workspace + w.db_off);
-  if ((rc = trifast_backward_db(shape, d_o, q, k, v, bias, mask, o, lse, db_f32, workspace,
-                                workspace_bytes, stream)))
+  Common c;
+  if ((rc = common_setup(shape, &c))) return rc;
+  if (!o) return TRIFAST_ERR_NULL;
+  BwdArgs a;
+  if ((rc = fill_bwd(shape, c, d_o, q, k, v, bias, mask, o, lse, workspace, workspace_bytes, &a)))
     return rc;
-  if ((rc = trifast_backward_dqkv(shape, d_o, q, k, v, bias, mask, lse, dq, dk, dv, workspace,
-                                  workspace_bytes, stream)))
+  a.dq = make_view(dq);
+  a.dk = make_view(dk);
+  a.dv = make_view(dv);
+  cudaStream_t s = (cudaStream_t)stream;
+  BwdKernels kern;
+  if ((rc = pick_bwd(shape, c, &a, &kern)) || (rc = cuda_rc(bwd_prepare(a, s))) ||
+      (rc = run_db(a, kern, s)) || (rc = run_dqkv(a, kern, s)))
     return rc;
-  return trifast_db_finalize(shape, db_f32, db, stream);
+  const bool partials = a.splits > 1 && kern != kBwdD128;
+  return cuda_rc(db_cast(partials ? a.db_partials : a.db_f32, partials ? a.splits : 1, make_view(db),
+                         shape->dtype, shape->batch, shape->heads, shape->n, s));
 }
 
 int trifast_check_device_status(void* stream) {

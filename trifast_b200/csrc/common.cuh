@@ -21,15 +21,16 @@ struct View5 {
   char* p;
   int64_t sb, sh, si, sj;
 };
-// (b, h, j, k) view with element strides; k contiguous.
+// (b, h, j, k) view with element strides; sk is 1 except for a caller's bias under
+// TRIFAST_FLAG_STRIDED.
 struct View4 {
   char* p;
-  int64_t sb, sh, sj;
+  int64_t sb, sh, sj, sk;
 };
-// (b, i, k) byte mask.
+// (b, i, k) byte mask; sk as above.
 struct MaskView {
   const uint8_t* p;
-  int64_t sb, si;
+  int64_t sb, si, sk;
 };
 
 struct Dims {
@@ -43,10 +44,23 @@ inline View5 make_view(const trifast_t5* t) {
   return View5{(char*)t->data, t->stride[0], t->stride[1], t->stride[2], t->stride[3]};
 }
 inline View4 make_view(const trifast_t4* t) {
-  return View4{(char*)t->data, t->stride[0], t->stride[1], t->stride[2]};
+  return View4{(char*)t->data, t->stride[0], t->stride[1], t->stride[2], 1};
 }
 inline MaskView make_view(const trifast_mask* t) {
-  return MaskView{t->data, t->stride[0], t->stride[1]};
+  return MaskView{t->data, t->stride[0], t->stride[1], 1};
+}
+
+// The bias and mask of a call: with TRIFAST_FLAG_STRIDED the descriptors are the longer
+// structs, whose innermost dimension has a stride of its own.
+inline View4 bias_view(const trifast_t4* t, int flags) {
+  View4 v = make_view(t);
+  if (flags & TRIFAST_FLAG_STRIDED) v.sk = reinterpret_cast<const trifast_t4_strided*>(t)->stride[3];
+  return v;
+}
+inline MaskView mask_view(const trifast_mask* t, int flags) {
+  MaskView v = make_view(t);
+  if (flags & TRIFAST_FLAG_STRIDED) v.sk = reinterpret_cast<const trifast_mask_strided*>(t)->stride[2];
+  return v;
 }
 
 template <typename T> __device__ __forceinline__ float to_f32(T x);

@@ -58,7 +58,8 @@ cudaError_t simt_bwd_db(const BwdArgs& a, cudaStream_t s);
 cudaError_t simt_bwd_dq(const BwdArgs& a, cudaStream_t s);
 cudaError_t simt_bwd_dkv(const BwdArgs& a, cudaStream_t s);
 cudaError_t db_reduce_splits(const BwdArgs& a, cudaStream_t s);
-cudaError_t db_cast(const float* db_f32, View4 db, int dtype, int batch, int heads, int n,
+// db in its own type: the sum of `splits` partials in order (1: db_f32 itself)
+cudaError_t db_cast(const float* partials, int splits, View4 db, int dtype, int batch, int heads, int n,
                     cudaStream_t s);
 
 // tcgen05 kernels (tc_*.cu): bf16 / fp16.

@@ -110,11 +110,11 @@ __device__ __forceinline__ void stage_rows(float* dst, const T* src, int64_t str
   }
 }
 
-// ROWS x COLS values of a matrix with contiguous columns (a bias tile), zeros outside
-// valid_r x valid_c.  `wide`: the matrix allows 16-byte accesses.
+// ROWS x COLS values of a matrix (a bias tile), zeros outside valid_r x valid_c.  `wide`: its
+// columns are contiguous and its rows allow 16-byte accesses.
 template <typename T, int P, int ROWS, int COLS, int NT>
-__device__ __forceinline__ void stage_matrix(float* dst, const T* src, int64_t stride, int valid_r,
-                                             int valid_c, bool wide) {
+__device__ __forceinline__ void stage_matrix(float* dst, const T* src, int64_t stride, int64_t stride_c,
+                                             int valid_r, int valid_c, bool wide) {
   if constexpr (std::is_same<T, float>::value) {
     if (wide) {
 #pragma unroll 1
@@ -131,9 +131,9 @@ __device__ __forceinline__ void stage_matrix(float* dst, const T* src, int64_t s
     const int r = idx / COLS, c = idx % COLS;
     const bool ok = r < valid_r && c < valid_c;
     if constexpr (std::is_same<T, float>::value)
-      cp_async<4>(smem_addr(dst + r * P + c), src + (ok ? r * stride + c : 0), ok);
+      cp_async<4>(smem_addr(dst + r * P + c), src + (ok ? r * stride + c * stride_c : 0), ok);
     else
-      dst[r * P + c] = ok ? to_f32<T>(src[r * stride + c]) : 0.f;
+      dst[r * P + c] = ok ? to_f32<T>(src[r * stride + c * stride_c]) : 0.f;
   }
 }
 
@@ -254,7 +254,7 @@ __device__ __forceinline__ const T* bias_ptr(const View4& t, int b, int h, int j
 }
 template <typename T>
 __device__ __forceinline__ bool wide_bias(const View4& t, int n) {
-  return std::is_same<T, float>::value && n % 4 == 0 && t.sj % 4 == 0 && t.sh % 4 == 0 && t.sb % 4 == 0 &&
+  return std::is_same<T, float>::value && t.sk == 1 && n % 4 == 0 && t.sj % 4 == 0 && t.sh % 4 == 0 && t.sb % 4 == 0 &&
          (reinterpret_cast<uintptr_t>(t.p) & 15) == 0;
 }
 
@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(kThreads) simt_fwd_kernel(View5 q, View5 k, Vi
   const Place<D, R> at;
   const uint8_t* mrow = mask.p + b * mask.sb + (int64_t)i * mask.si;
   int open = 0;
-  for (int c = threadIdx.x; c < n; c += kThreads) open |= mrow[c] == 0;
+  for (int c = threadIdx.x; c < n; c += kThreads) open |= mrow[c * mask.sk] == 0;
   const bool row_full = !__syncthreads_or(open);
   const bool wide = wide_bias<T>(bias, n);
 
@@ -331,11 +331,11 @@ __global__ void __launch_bounds__(kThreads) simt_fwd_kernel(View5 q, View5 k, Vi
     float* d = buf(u);
     stage_rows<T, D, F::P, F::TS, kThreads>(d, row_ptr<const T>(k, b, h, i, k0), k.sj, valid);
     stage_rows<T, D, F::P, F::TS, kThreads>(d + S::kStr, row_ptr<const T>(v, b, h, i, k0), v.sj, valid);
-    stage_matrix<T, S::kBiasP, F::BR, F::TS, kThreads>(d + 2 * S::kStr, bias_ptr<T>(bias, b, h, j0) + k0,
-                                                       bias.sj, n - j0, valid, wide);
+    stage_matrix<T, S::kBiasP, F::BR, F::TS, kThreads>(d + 2 * S::kStr, bias_ptr<T>(bias, b, h, j0) + k0 * bias.sk,
+                                                       bias.sj, bias.sk, n - j0, valid, wide);
     if (threadIdx.x < F::TS) {
       const int c = threadIdx.x;
-      d[2 * S::kStr + S::kBias + c] = (c < valid && (row_full || mrow[k0 + c] == 0)) ? 1.f : 0.f;
+      d[2 * S::kStr + S::kBias + c] = (c < valid && (row_full || mrow[(k0 + c) * mask.sk] == 0)) ? 1.f : 0.f;
     }
   };
   auto work = [&](int, int u) {
@@ -457,11 +457,11 @@ __global__ void __launch_bounds__(kThreads) simt_bwd_kernel(View5 a1, View5 a2, 
     stage_rows<T, D, F::P, F::TS, kThreads>(d, row_ptr<const T>(b1, b, h, i, s0), b1.sj, valid);
     stage_rows<T, D, F::P, F::TS, kThreads>(d + S::kStr, row_ptr<const T>(b2, b, h, i, s0), b2.sj, valid);
     if constexpr (kKv)
-      stage_matrix<T, S::kBiasP, F::TS, F::BR, kThreads>(d + 2 * S::kStr, bias_ptr<T>(bias, b, h, s0) + r0,
-                                                         bias.sj, valid, n - r0, wide);
+      stage_matrix<T, S::kBiasP, F::TS, F::BR, kThreads>(d + 2 * S::kStr, bias_ptr<T>(bias, b, h, s0) + r0 * bias.sk,
+                                                         bias.sj, bias.sk, valid, n - r0, wide);
     else
-      stage_matrix<T, S::kBiasP, F::BR, F::TS, kThreads>(d + 2 * S::kStr, bias_ptr<T>(bias, b, h, r0) + s0,
-                                                         bias.sj, n - r0, valid, wide);
+      stage_matrix<T, S::kBiasP, F::BR, F::TS, kThreads>(d + 2 * S::kStr, bias_ptr<T>(bias, b, h, r0) + s0 * bias.sk,
+                                                         bias.sj, bias.sk, n - r0, valid, wide);
     if (kKv && threadIdx.x < F::TS) {
       const int c = threadIdx.x, cc = min(s0 + c, n - 1);
       d[2 * S::kStr + S::kBias + c] = lse_row[cc];
@@ -543,7 +543,7 @@ __global__ void __launch_bounds__(TILE / EA * (TILE / EC), 2) simt_db_kernel(Vie
 #pragma unroll
     for (int c = 0; c < EC; ++c) {
       const int j = j0 + y + S::TY * a, key = k0 + x + S::TX * c;
-      bv[a][c] = (j < n && key < n) ? to_f32<T>(bias_ptr<T>(bias, b, h, j)[key]) : 0.f;
+      bv[a][c] = (j < n && key < n) ? to_f32<T>(bias_ptr<T>(bias, b, h, j)[key * bias.sk]) : 0.f;
       acc[a][c] = 0.f;
     }
   auto buf = [&](int u) { return sm + u * S::kBuf; };

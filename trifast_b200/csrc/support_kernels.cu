@@ -1,5 +1,10 @@
-// Small kernels around the attention kernels of both families: row flags and packed key
-// masks, delta, bias copies, the sum of db's row splits and its cast.
+// Small kernels around the attention kernels of both families: one prepare kernel per call
+// (row flags, packed key masks, live key-tile ranges, bias copies, delta) and the sum of db's
+// row splits with its cast.
+//
+// On small problems every launch counts (about 3 us of host time and 2 us of device time each):
+// the parts of the prepare step are independent of one another, so they are block ranges of
+// one launch, and the sum over row splits writes the gradient in its own type.
 
 #include <math.h>
 
@@ -10,32 +15,31 @@
 namespace trifast {
 namespace {
 
-constexpr float kMinusInf = -INFINITY;
-constexpr float kMaxInit = -1e30f;  // finite start of the running max: exp(-inf - m) stays 0, never NaN
+constexpr int kPrepThreads = 256;
+constexpr float kLog2e = 1.4426950408889634f;
 
-template <typename T>
-__device__ __forceinline__ const T* row5(const View5& t, int b, int h, int i, int j) {
-  return (const T*)t.p + b * t.sb + h * t.sh + (int64_t)i * t.si + (int64_t)j * t.sj;
-}
-template <typename T>
-__device__ __forceinline__ T* row5w(const View5& t, int b, int h, int i, int j) {
-  return (T*)t.p + b * t.sb + h * t.sh + (int64_t)i * t.si + (int64_t)j * t.sj;
-}
-template <typename T>
-__device__ __forceinline__ const T* row4(const View4& t, int b, int h, int j) {
-  return (const T*)t.p + b * t.sb + h * t.sh + (int64_t)j * t.sj;
-}
+struct Prep {
+  MaskView mask;
+  View4 bias;
+  uint8_t* rowfull;
+  uint32_t *maskbits, *maskbits_lin, *rowrange;
+  int mask_words;
+  uint16_t *bias_t, *bias_pad;
+  Dims dm;
+  unsigned int* status;
+  // block ranges, in this order: one row of the mask each; 64 x 64 bias tiles; the rest delta
+  int mask_blocks, bias_tiles, bias_blocks;
+};
 
 // ---------------------------------------------------------------------------
-// rowfull[b, i] = 1 when every key of pair row i is masked.
+// One pair row of the mask: rowfull = 1 when every key is masked, the packed key masks, the
+// range of 128-key tiles that hold an open key.
 // ---------------------------------------------------------------------------
-__global__ void rowfull_kernel(MaskView mask, int n, int n_rows, uint8_t* rowfull,
-                               uint32_t* maskbits, uint32_t* maskbits_lin, int mask_words,
-                               uint32_t* rowrange, unsigned int* status) {
-  const int bi = blockIdx.x;
-  if (bi == 0 && threadIdx.x == 0) repeat_status(status);
+__device__ void prepare_mask_row(const Prep& a, int bi) {
+  const int n = a.dm.n, n_rows = a.dm.n_rows;
   const int b = bi / n_rows, i = bi % n_rows;
-  const uint8_t* row = mask.p + b * mask.sb + (int64_t)i * mask.si;
+  const uint8_t* row = a.mask.p + b * a.mask.sb + (int64_t)i * a.mask.si;
+  const int64_t sk = a.mask.sk;
   __shared__ int first_open, last_open;
   if (threadIdx.x == 0) {
     first_open = n;
@@ -43,8 +47,8 @@ __global__ void rowfull_kernel(MaskView mask, int n, int n_rows, uint8_t* rowful
   }
   __syncthreads();
   int lo = n, hi = -1;
-  for (int k = threadIdx.x; k < n; k += blockDim.x) {
-    if (row[k] == 0) {
+  for (int k = threadIdx.x; k < n; k += kPrepThreads) {
+    if (row[k * sk] == 0) {
       lo = min(lo, k);
       hi = max(hi, k);
     }
@@ -56,291 +60,313 @@ __global__ void rowfull_kernel(MaskView mask, int n, int n_rows, uint8_t* rowful
   __syncthreads();
   const int open = last_open >= 0;
   if (threadIdx.x == 0) {
-    if (rowfull) rowfull[bi] = open ? 0 : 1;
+    if (a.rowfull) a.rowfull[bi] = open ? 0 : 1;
     // 128-key tiles [first, last + 1) that hold an open key: the tensor-core kernels walk
     // only those.  A fully masked row weighs all n keys: every tile.
-    if (rowrange) {
+    if (a.rowrange) {
       const uint32_t t0 = open ? (uint32_t)(first_open >> 7) : 0u;
       const uint32_t t1 = open ? (uint32_t)(last_open >> 7) + 1u : (uint32_t)((n + 127) >> 7);
-      rowrange[bi] = t0 | (t1 << 16);
+      a.rowrange[bi] = t0 | (t1 << 16);
     }
   }
-  if (!maskbits) return;
+  if (!a.maskbits) return;
   // Packed key mask (bit set = key dropped or beyond n).  A fully masked row keeps
   // all n keys with uniform weight, so only the keys beyond n stay set.  Layout per
   // 128-key chunk c: word c*4 + jb holds, at bit l, key c*128 + 4*l + jb (the order
   // in which a warp reading four mask bytes per lane produces the words).
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int c = warp; c < mask_words / 4; c += blockDim.x >> 5) {
-#pragma unroll
-    for (int jb = 0; jb < 4; ++jb) {
-      const int k = c * 128 + 4 * lane + jb;
-      const int dropped = (k < n) ? (open ? (row[k] != 0) : 0) : 1;
-      const unsigned bits = __ballot_sync(0xffffffffu, dropped);
-      if (lane == 0) maskbits[(int64_t)bi * mask_words + c * 4 + jb] = bits;
-    }
+  for (int w = warp; w < a.mask_words; w += kPrepThreads / 32) {
+    const int k = (w >> 2) * 128 + 4 * lane + (w & 3);
+    const int dropped = (k < n) ? (open ? (row[k * sk] != 0) : 0) : 1;
+    const unsigned bits = __ballot_sync(0xffffffffu, dropped);
+    if (lane == 0) a.maskbits[(int64_t)bi * a.mask_words + w] = bits;
   }
   // The same bits in key order (word w, bit l: key 32 * w + l), when asked for.
-  if (maskbits_lin) {
-    for (int w = warp; w < mask_words; w += blockDim.x >> 5) {
+  if (a.maskbits_lin) {
+    for (int w = warp; w < a.mask_words; w += kPrepThreads / 32) {
       const int k = w * 32 + lane;
-      const int dropped = (k < n) ? (open ? (row[k] != 0) : 0) : 1;
+      const int dropped = (k < n) ? (open ? (row[k * sk] != 0) : 0) : 1;
       const unsigned bits = __ballot_sync(0xffffffffu, dropped);
-      if (lane == 0) maskbits_lin[(int64_t)bi * mask_words + w] = bits;
+      if (lane == 0) a.maskbits_lin[(int64_t)bi * a.mask_words + w] = bits;
     }
   }
 }
 
-// bias_pad[b, h, j, 0..n_pad) = bias[b, h, j, 0..n) (pad = 0): a copy whose row pitch
-// is a multiple of 16 bytes, as TMA needs, for n % 8 != 0.
-__global__ void bias_pad_kernel(View4 bias, uint16_t* out, int heads, int n, int n_pad) {
-  const int bh = blockIdx.z, b = bh / heads, h = bh % heads;
-  const int j = blockIdx.y;
-  const uint16_t* src = (const uint16_t*)bias.p + b * bias.sb + h * bias.sh + (int64_t)j * bias.sj;
-  uint16_t* dst = out + ((int64_t)bh * n + j) * n_pad;
-  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < n_pad; k += gridDim.x * blockDim.x)
-    dst[k] = (k < n) ? src[k] : (uint16_t)0;
-}
-
 // ---------------------------------------------------------------------------
-// delta[b, h, i, j] = sum_d o * dO   (fp32; never rounded to the input dtype)
+// 64 x 64 tile of the bias (2-byte elements) into the copies asked for, both with row pitch
+// n_pad (a multiple of 16 bytes, as TMA needs): bias_t[b, h, k, j] with keys on the rows, and
+// bias_pad[b, h, j, k] where the bias itself cannot be described to TMA.  Elements of the pad
+// columns are zero in bias_pad.
 // ---------------------------------------------------------------------------
-template <typename T, int D>
-__global__ void delta_kernel(View5 o, View5 d_o, const float* lse, float* delta, float* neg_lse2,
-                             Dims dm) {
-  // A group of G threads owns one (b, h, i, j) row of D elements, 16 bytes per thread
-  // and step, so that a warp reads whole 128-byte lines of o and dO.
-  constexpr int kVec = 16 / sizeof(T);   // elements per 16-byte load
-  constexpr int G = (D / kVec) < 4 ? (D / kVec) : 4;
-  constexpr int kSteps = D / (kVec * G);
-  const int64_t total = (int64_t)dm.batch * dm.heads * dm.n_rows * dm.n;
-  const int64_t gid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t idx = gid / G;
-  const int part = (int)(gid % G);
-  const bool valid = idx < total;
-  float acc = 0.f;
-  if (valid) {
-    const int j = idx % dm.n;
-    int64_t r = idx / dm.n;
-    const int i = r % dm.n_rows;
-    r /= dm.n_rows;
-    const int h = r % dm.heads, b = r / dm.heads;
-    const T* po = row5<T>(o, b, h, i, j);
-    const T* pd = row5<T>(d_o, b, h, i, j);
-#pragma unroll
-    for (int st = 0; st < kSteps; ++st) {
-      const int off = (st * G + part) * kVec;
-      const uint4 uo = *reinterpret_cast<const uint4*>(po + off);
-      const uint4 ud = *reinterpret_cast<const uint4*>(pd + off);
-      const T* eo = reinterpret_cast<const T*>(&uo);
-      const T* ed = reinterpret_cast<const T*>(&ud);
-#pragma unroll
-      for (int c = 0; c < kVec; ++c) acc = fmaf(to_f32<T>(eo[c]), to_f32<T>(ed[c]), acc);
-    }
-  }
-#pragma unroll
-  for (int m = G / 2; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-  if (valid && part == 0) {
-    const int64_t out = (idx / dm.n) * dm.n_pad + idx % dm.n;  // row pitch n_pad
-    delta[out] = acc;
-    neg_lse2[out] = -lse[idx] * 1.4426950408889634f;
-  }
-}
-
-// bias_t[b, h, k, j] = bias[b, h, j, k] (row pitch n_pad) for 2-byte elements (the dk/dv kernel reads
-// the bias with keys on the rows).  64 x 64 tiles; 4-byte accesses on both sides when the rows allow it.
-__global__ void __launch_bounds__(256)
-bias_transpose_kernel(View4 bias, uint16_t* out, int heads, int n, int n_pad) {
+__device__ void prepare_bias_tile(const Prep& a, int w) {
   __shared__ uint16_t tile[64][66];
-  const int bh = blockIdx.z, b = bh / heads, h = bh % heads;
+  const int n = a.dm.n, n_pad = a.dm.n_pad;
+  const int k0 = w % a.bias_tiles * 64, j0 = w / a.bias_tiles % a.bias_tiles * 64;
+  const int bh = w / (a.bias_tiles * a.bias_tiles), b = bh / a.dm.heads, h = bh % a.dm.heads;
+  const View4& bias = a.bias;
   const uint16_t* src = (const uint16_t*)bias.p + b * bias.sb + h * bias.sh;
-  uint16_t* dst = out + (int64_t)bh * n * n_pad;
-  const int j0 = blockIdx.y * 64, k0 = blockIdx.x * 64;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
-  const bool pairs_in = (bias.sj % 2 == 0) && (bias.sh % 2 == 0) && (bias.sb % 2 == 0) &&
+  const bool pairs_in = bias.sk == 1 && (bias.sj % 2 == 0) && (bias.sh % 2 == 0) && (bias.sb % 2 == 0) &&
                         ((reinterpret_cast<uintptr_t>(bias.p) & 3) == 0);
-  for (int r = ty; r < 64; r += 8) {
-    const int j = j0 + r, k = k0 + 2 * tx;
+#pragma unroll
+  for (int it = 0; it < 8; ++it) {
+    const int r = ty + 8 * it, j = j0 + r, k = k0 + 2 * tx;
+    uint16_t e0 = 0, e1 = 0;
     if (j < n) {
+      const uint16_t* p = src + (int64_t)j * bias.sj + (int64_t)k * bias.sk;
       if (pairs_in && k + 1 < n) {
-        const uint32_t u = *reinterpret_cast<const uint32_t*>(src + (int64_t)j * bias.sj + k);
-        tile[r][2 * tx] = (uint16_t)(u & 0xffffu);
-        tile[r][2 * tx + 1] = (uint16_t)(u >> 16);
+        const uint32_t u = *reinterpret_cast<const uint32_t*>(p);
+        e0 = (uint16_t)(u & 0xffffu);
+        e1 = (uint16_t)(u >> 16);
       } else {
-        if (k < n) tile[r][2 * tx] = src[(int64_t)j * bias.sj + k];
-        if (k + 1 < n) tile[r][2 * tx + 1] = src[(int64_t)j * bias.sj + k + 1];
+        if (k < n) e0 = p[0];
+        if (k + 1 < n) e1 = p[bias.sk];
       }
     }
+    if (a.bias_pad && j < n && k < n_pad)   // n_pad is even: a pair never straddles it
+      *reinterpret_cast<uint32_t*>(a.bias_pad + ((int64_t)bh * n + j) * n_pad + k) =
+          (uint32_t)e0 | ((uint32_t)e1 << 16);
+    tile[r][2 * tx] = e0;
+    tile[r][2 * tx + 1] = e1;
   }
+  if (!a.bias_t) return;
   __syncthreads();
-  for (int r = ty; r < 64; r += 8) {  // output row k0 + r holds queries j0 .. j0 + 63
-    const int k = k0 + r, j = j0 + 2 * tx;
-    if (k < n) {
-      if (j + 1 < n) {  // n_pad is even and dst 4-byte aligned: a pair never straddles
-        const uint32_t u = (uint32_t)tile[2 * tx][r] | ((uint32_t)tile[2 * tx + 1][r] << 16);
-        *reinterpret_cast<uint32_t*>(dst + (int64_t)k * n_pad + j) = u;
-      } else if (j < n) {
-        dst[(int64_t)k * n_pad + j] = tile[2 * tx][r];
-      }
+  uint16_t* dst = a.bias_t + (int64_t)bh * n * n_pad;
+#pragma unroll
+  for (int it = 0; it < 8; ++it) {  // output row k0 + r holds queries j0 .. j0 + 63
+    const int r = ty + 8 * it, k = k0 + r, j = j0 + 2 * tx;
+    if (k < n && j < n_pad) {
+      const uint32_t u = (uint32_t)tile[2 * tx][r] | ((uint32_t)tile[2 * tx + 1][r] << 16);
+      *reinterpret_cast<uint32_t*>(dst + (int64_t)k * n_pad + j) = u;
     }
   }
 }
 
-// Sum the row-split partials in split order (fixed order => deterministic).
-__global__ void db_reduce_kernel(const float* partials, float* out, int splits, int64_t count) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= count) return;
-  float acc = partials[idx];
-  for (int s = 1; s < splits; ++s) acc += partials[(int64_t)s * count + idx];
-  out[idx] = acc;
+// ---------------------------------------------------------------------------
+// delta[b, h, i, j] = sum_d o * dO (fp32; never rounded to the input dtype) and
+// neg_lse2 = -lse * log2(e), row pitch n_pad.
+// ---------------------------------------------------------------------------
+// A group of G threads owns a (b, h, i, j) row of D elements, 16 bytes per thread and step, so
+// that a warp reads whole 128-byte lines of o and dO; U rows per thread keep several loads in
+// flight (one row at a time read 3.5 TB/s of the 6.5 a copy reaches).
+template <typename T, int D> struct DeltaCfg {
+  static constexpr int kVec = 16 / sizeof(T);   // elements per 16-byte load
+  static constexpr int G = (D / kVec) < 4 ? (D / kVec) : 4;
+  static constexpr int kSteps = D / (kVec * G);
+  static constexpr int U = kSteps == 1 ? 4 : kSteps == 2 ? 2 : 1;
+  static constexpr int kRows = kPrepThreads / G * U;   // rows of a block
+};
+
+// (volatile: the loads of a thread go out together, in this order)
+__device__ __forceinline__ uint4 load_once(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
 }
 
-// four elements per thread (count % 4 == 0)
-__global__ void db_reduce4_kernel(const float4* partials, float4* out, int splits, int64_t count4) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= count4) return;
-  float4 acc = __ldg(partials + idx);
-  for (int s = 1; s < splits; ++s) {  // fixed split order: deterministic
-    const float4 v = __ldg(partials + (int64_t)s * count4 + idx);
-    acc.x += v.x;
-    acc.y += v.y;
-    acc.z += v.z;
-    acc.w += v.w;
+template <typename T, int D>
+__device__ void prepare_delta(const View5& o, const View5& d_o, const float* lse, float* delta,
+                              float* neg_lse2, const Dims& dm, unsigned block) {
+  using C = DeltaCfg<T, D>;
+  const unsigned n = dm.n, n_rows = dm.n_rows, heads = dm.heads;
+  const unsigned total = (unsigned)dm.batch * heads * n_rows * n;   // < 2^31: 16 bytes each fit memory
+  const int part = threadIdx.x % C::G;
+  uint4 uo[C::U][C::kSteps], ud[C::U][C::kSteps];
+  unsigned idx[C::U], row[C::U];
+#pragma unroll
+  for (int u = 0; u < C::U; ++u) {
+    idx[u] = block * C::kRows + u * (kPrepThreads / C::G) + threadIdx.x / C::G;
+    const unsigned at = min(idx[u], total - 1);
+    row[u] = at / n;
+    const unsigned j = at - row[u] * n, i = row[u] % n_rows, bh = row[u] / n_rows;
+    const unsigned h = bh % heads, b = bh / heads;
+    const T* po = (const T*)o.p + b * o.sb + h * o.sh + (int64_t)i * o.si + (int64_t)j * o.sj;
+    const T* pd = (const T*)d_o.p + b * d_o.sb + h * d_o.sh + (int64_t)i * d_o.si + (int64_t)j * d_o.sj;
+#pragma unroll
+    for (int st = 0; st < C::kSteps; ++st) {
+      const int off = (st * C::G + part) * C::kVec;
+      uo[u][st] = load_once(po + off);
+      ud[u][st] = load_once(pd + off);
+    }
   }
-  out[idx] = acc;
+#pragma unroll
+  for (int u = 0; u < C::U; ++u) {
+    float acc = 0.f;
+#pragma unroll
+    for (int st = 0; st < C::kSteps; ++st) {
+      const T* eo = reinterpret_cast<const T*>(&uo[u][st]);
+      const T* ed = reinterpret_cast<const T*>(&ud[u][st]);
+#pragma unroll
+      for (int c = 0; c < C::kVec; ++c) acc = fmaf(to_f32<T>(eo[c]), to_f32<T>(ed[c]), acc);
+    }
+#pragma unroll
+    for (int m = C::G / 2; m > 0; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+    if (idx[u] < total && part == 0) {
+      const int64_t out = (int64_t)row[u] * dm.n_pad + (idx[u] - row[u] * n);
+      delta[out] = acc;
+      neg_lse2[out] = -lse[idx[u]] * kLog2e;
+    }
+  }
 }
 
-// four keys of one row per thread (n % 4 == 0, destination rows 8-byte aligned; T is 16 bits)
-template <typename T>
-__global__ void db_cast4_kernel(const float4* src, View4 db, int heads, int n, int64_t count4) {
+__global__ void __launch_bounds__(kPrepThreads) fwd_prepare_kernel(Prep a) {
+  int w = blockIdx.x;
+  if (w == 0 && threadIdx.x == 0) repeat_status(a.status);
+  if (w < a.mask_blocks) return prepare_mask_row(a, w);
+  prepare_bias_tile(a, w - a.mask_blocks);
+}
+
+template <typename T, int D>
+__global__ void __launch_bounds__(kPrepThreads) bwd_prepare_kernel(Prep a, View5 o, View5 d_o, const float* lse,
+                                                                   float* delta, float* neg_lse2) {
+  int w = blockIdx.x;
+  if (w == 0 && threadIdx.x == 0) repeat_status(a.status);
+  if (w < a.mask_blocks) return prepare_mask_row(a, w);
+  w -= a.mask_blocks;
+  if (w < a.bias_blocks) return prepare_bias_tile(a, w);
+  prepare_delta<T, D>(o, d_o, lse, delta, neg_lse2, a.dm, w - a.bias_blocks);
+}
+
+// ---------------------------------------------------------------------------
+// db: the row-split partials summed in split order (fixed order => deterministic), written as
+// fp32 or in the gradient's type.  kWide: four keys of one row per thread (n % 4 == 0, rows
+// aligned to four elements).
+// ---------------------------------------------------------------------------
+template <typename T, bool kWide>
+__global__ void db_finish_kernel(const float* partials, int splits, View4 db, int heads, int n, int64_t count) {
+  constexpr int V = kWide ? 4 : 1;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= count4) return;
-  const int n4 = n >> 2;
-  const int key = (int)(idx % n4) * 4;
-  int64_t r = idx / n4;
+  if (idx * V >= count) return;
+  float acc[V];
+  for (int s = 0; s < splits; ++s) {
+    if constexpr (kWide) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(partials + s * count) + idx);
+      const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int c = 0; c < V; ++c) acc[c] = s ? acc[c] + e[c] : e[c];
+    } else {
+      const float e = __ldg(partials + s * count + idx);
+      acc[0] = s ? acc[0] + e : e;
+    }
+  }
+  const int per_row = n / V, key = (int)(idx % per_row) * V;
+  int64_t r = idx / per_row;
   const int j = (int)(r % n);
   r /= n;
   const int h = (int)(r % heads), b = (int)(r / heads);
-  const float4 v = __ldg(src + idx);
   T* dst = (T*)db.p + b * db.sb + h * db.sh + (int64_t)j * db.sj + key;
-  const T o4[4] = {from_f32<T>(v.x), from_f32<T>(v.y), from_f32<T>(v.z), from_f32<T>(v.w)};
-  *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(o4);
+  if constexpr (!kWide) {
+    dst[0] = from_f32<T>(acc[0]);
+  } else if constexpr (sizeof(T) == 4) {
+    *reinterpret_cast<float4*>(dst) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  } else {
+    const T o4[4] = {from_f32<T>(acc[0]), from_f32<T>(acc[1]), from_f32<T>(acc[2]), from_f32<T>(acc[3])};
+    *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(o4);
+  }
 }
 
 template <typename T>
-__global__ void db_cast_kernel(const float* src, View4 db, int heads, int n, int64_t count) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= count) return;
-  const int key = idx % n;
-  int64_t r = idx / n;
-  const int j = r % n;
-  r /= n;
-  const int h = r % heads, b = r / heads;
-  T* dst = (T*)db.p + b * db.sb + h * db.sh + (int64_t)j * db.sj;
-  dst[key] = from_f32<T>(src[idx]);
+cudaError_t launch_finish(const float* partials, int splits, View4 db, int batch, int heads, int n, cudaStream_t s) {
+  const int64_t count = (int64_t)batch * heads * n * n;
+  const int64_t row_bytes = 4 * sizeof(T);
+  const bool wide = n % 4 == 0 && db.sj % 4 == 0 && db.sh % 4 == 0 && db.sb % 4 == 0 &&
+                    reinterpret_cast<uintptr_t>(db.p) % row_bytes == 0 &&
+                    (reinterpret_cast<uintptr_t>(partials) & 15) == 0;
+  const int64_t threads = wide ? count / 4 : count;
+  const unsigned blocks = (unsigned)((threads + 255) / 256);
+  if (wide)
+    db_finish_kernel<T, true><<<blocks, 256, 0, s>>>(partials, splits, db, heads, n, count);
+  else
+    db_finish_kernel<T, false><<<blocks, 256, 0, s>>>(partials, splits, db, heads, n, count);
+  return cudaGetLastError();
 }
 
-// ---------------------------------------------------------------------------
-// dispatch on (dtype, d)
-// ---------------------------------------------------------------------------
+Prep make_prep(const MaskView& mask, const View4& bias, const Dims& dm) {
+  Prep p{};
+  p.mask = mask;
+  p.bias = bias;
+  p.dm = dm;
+  p.mask_blocks = dm.batch * dm.n_rows;
+  p.bias_tiles = (dm.n + 63) / 64;
+  return p;
+}
+
 template <typename F>
 cudaError_t dispatch(int dtype, int d, F&& f) {
-#define TRIFAST_D_CASES(T)                                 \
-  switch (d) {                                             \
-    case 16: f((T*)nullptr, std::integral_constant<int, 16>{}); break;   \
-    case 32: f((T*)nullptr, std::integral_constant<int, 32>{}); break;   \
-    case 64: f((T*)nullptr, std::integral_constant<int, 64>{}); break;   \
-    case 128: f((T*)nullptr, std::integral_constant<int, 128>{}); break; \
-    default: return cudaErrorInvalidValue;                 \
-  }
+  auto on_d = [&](auto* tp) -> cudaError_t {
+    switch (d) {
+      case 16: f(tp, std::integral_constant<int, 16>{}); break;
+      case 32: f(tp, std::integral_constant<int, 32>{}); break;
+      case 64: f(tp, std::integral_constant<int, 64>{}); break;
+      case 128: f(tp, std::integral_constant<int, 128>{}); break;
+      default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+  };
   switch (dtype) {
-    case TRIFAST_F32: TRIFAST_D_CASES(float) break;
-    case TRIFAST_BF16: TRIFAST_D_CASES(__nv_bfloat16) break;
-    case TRIFAST_F16: TRIFAST_D_CASES(__half) break;
+    case TRIFAST_F32: return on_d((float*)nullptr);
+    case TRIFAST_BF16: return on_d((__nv_bfloat16*)nullptr);
+    case TRIFAST_F16: return on_d((__half*)nullptr);
     default: return cudaErrorInvalidValue;
   }
-#undef TRIFAST_D_CASES
-  return cudaGetLastError();
 }
 
 }  // namespace
 
 cudaError_t bwd_prepare(const BwdArgs& a, cudaStream_t s) {
   const Dims& dm = a.dm;
-  rowfull_kernel<<<dm.batch * dm.n_rows, 128, 0, s>>>(a.mask, dm.n, dm.n_rows, a.rowfull, a.maskbits,
-                                                      a.maskbits_lin, a.mask_words, a.rowrange, a.status);
-  if (a.bias_t) {
-    dim3 grid((dm.n + 63) / 64, (dm.n + 63) / 64, dm.batch * dm.heads);
-    bias_transpose_kernel<<<grid, 256, 0, s>>>(a.bias, (uint16_t*)a.bias_t, dm.heads, dm.n,
-                                                       dm.n_pad);
-  }
-  if (a.bias_pad) {
-    dim3 grid(1, dm.n, dm.batch * dm.heads);
-    bias_pad_kernel<<<grid, 256, 0, s>>>(a.bias, (uint16_t*)a.bias_pad, dm.heads, dm.n, dm.n_pad);
-  }
+  Prep p = make_prep(a.mask, a.bias, dm);
+  p.rowfull = a.rowfull;
+  p.maskbits = a.maskbits;
+  p.maskbits_lin = a.maskbits_lin;
+  p.mask_words = a.mask_words;
+  p.rowrange = a.rowrange;
+  p.bias_t = (uint16_t*)a.bias_t;
+  p.bias_pad = (uint16_t*)a.bias_pad;
+  p.status = a.status;
+  p.bias_blocks = a.bias_t || a.bias_pad ? p.bias_tiles * p.bias_tiles * dm.batch * dm.heads : 0;
   return dispatch(a.dtype, dm.d, [&](auto* tp, auto dc) {
     using T = std::remove_pointer_t<decltype(tp)>;
     constexpr int D = decltype(dc)::value;
-    constexpr int kVec = 16 / sizeof(T);
-    constexpr int G = (D / kVec) < 4 ? (D / kVec) : 4;
-    const int64_t threads = (int64_t)dm.batch * dm.heads * dm.n_rows * dm.n * G;
-    delta_kernel<T, D><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>(a.o, a.d_o, a.lse, a.delta,
-                                                                       a.neg_lse2, dm);
+    constexpr int kRows = DeltaCfg<T, D>::kRows;
+    const int64_t rows = (int64_t)dm.batch * dm.heads * dm.n_rows * dm.n;
+    const unsigned blocks = (unsigned)(p.mask_blocks + p.bias_blocks + (rows + kRows - 1) / kRows);
+    bwd_prepare_kernel<T, D><<<blocks, kPrepThreads, 0, s>>>(p, a.o, a.d_o, a.lse, a.delta, a.neg_lse2);
   });
 }
 
 cudaError_t fwd_prepare(const FwdArgs& a, cudaStream_t s) {
-  const Dims& dm = a.dm;
   // the live key-tile range of every row always; the packed masks, row flags and the padded
-  // bias copy only where the workspace holds them (n % 8 != 0)
-  rowfull_kernel<<<dm.batch * dm.n_rows, 128, 0, s>>>(a.mask, dm.n, dm.n_rows, a.rowfull, a.maskbits,
-                                                      nullptr, a.mask_words, a.rowrange, a.status);
-  if (a.bias_pad) {
-    dim3 grid(1, dm.n, dm.batch * dm.heads);
-    bias_pad_kernel<<<grid, 256, 0, s>>>(a.bias, (uint16_t*)a.bias_pad, dm.heads, dm.n, dm.n_pad);
-  }
+  // bias copy only where the workspace holds them
+  Prep p = make_prep(a.mask, a.bias, a.dm);
+  p.rowfull = a.rowfull;
+  p.maskbits = a.maskbits;
+  p.mask_words = a.mask_words;
+  p.rowrange = a.rowrange;
+  p.bias_pad = (uint16_t*)a.bias_pad;
+  p.status = a.status;
+  p.bias_blocks = a.bias_pad ? p.bias_tiles * p.bias_tiles * a.dm.batch * a.dm.heads : 0;
+  fwd_prepare_kernel<<<p.mask_blocks + p.bias_blocks, kPrepThreads, 0, s>>>(p);
   return cudaGetLastError();
 }
 
 cudaError_t db_reduce_splits(const BwdArgs& a, cudaStream_t s) {
   if (a.splits <= 1) return cudaSuccess;
-  const int64_t count = (int64_t)a.dm.batch * a.dm.heads * a.dm.n * a.dm.n;
-  if (count % 4 == 0) {  // the partials and db_f32 sit on 256-byte boundaries of the workspace
-    const int64_t c4 = count / 4;
-    db_reduce4_kernel<<<(unsigned)((c4 + 255) / 256), 256, 0, s>>>(
-        reinterpret_cast<const float4*>(a.db_partials), reinterpret_cast<float4*>(a.db_f32), a.splits,
-        c4);
-    return cudaGetLastError();
-  }
-  db_reduce_kernel<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(a.db_partials, a.db_f32,
-                                                                 a.splits, count);
-  return cudaGetLastError();
+  const int64_t n = a.dm.n;
+  const View4 out{(char*)a.db_f32, n * n * a.dm.heads, n * n, n, 1};
+  return launch_finish<float>(a.db_partials, a.splits, out, a.dm.batch, a.dm.heads, a.dm.n, s);
 }
 
-cudaError_t db_cast(const float* db_f32, View4 db, int dtype, int batch, int heads, int n,
+cudaError_t db_cast(const float* partials, int splits, View4 db, int dtype, int batch, int heads, int n,
                     cudaStream_t s) {
-  const int64_t count = (int64_t)batch * heads * n * n;
-  const bool wide = dtype != TRIFAST_F32 && n % 4 == 0 && db.sj % 4 == 0 && db.sh % 4 == 0 &&
-                    db.sb % 4 == 0 && (reinterpret_cast<uintptr_t>(db.p) & 7) == 0 &&
-                    (reinterpret_cast<uintptr_t>(db_f32) & 15) == 0;
-  if (wide) {
-    const int64_t c4 = count / 4;
-    const unsigned blocks4 = (unsigned)((c4 + 255) / 256);
-    const float4* src = reinterpret_cast<const float4*>(db_f32);
-    if (dtype == TRIFAST_BF16)
-      db_cast4_kernel<__nv_bfloat16><<<blocks4, 256, 0, s>>>(src, db, heads, n, c4);
-    else
-      db_cast4_kernel<__half><<<blocks4, 256, 0, s>>>(src, db, heads, n, c4);
-    return cudaGetLastError();
-  }
-  const unsigned blocks = (unsigned)((count + 255) / 256);
   switch (dtype) {
-    case TRIFAST_F32: db_cast_kernel<float><<<blocks, 256, 0, s>>>(db_f32, db, heads, n, count); break;
-    case TRIFAST_BF16: db_cast_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>(db_f32, db, heads, n, count); break;
-    case TRIFAST_F16: db_cast_kernel<__half><<<blocks, 256, 0, s>>>(db_f32, db, heads, n, count); break;
+    case TRIFAST_F32: return launch_finish<float>(partials, splits, db, batch, heads, n, s);
+    case TRIFAST_BF16: return launch_finish<__nv_bfloat16>(partials, splits, db, batch, heads, n, s);
+    case TRIFAST_F16: return launch_finish<__half>(partials, splits, db, batch, heads, n, s);
     default: return cudaErrorInvalidValue;
   }
-  return cudaGetLastError();
 }
 
 }  // namespace trifast

@@ -498,6 +498,7 @@ cudaError_t launch_db(const BwdArgs& a, cudaStream_t stream) {
     bias.sj = dm.n_pad;
     bias.sh = (int64_t)dm.n * dm.n_pad;
     bias.sb = bias.sh * dm.heads;
+    bias.sk = 1;
   }
   if (kCluster) {
     cudaLaunchConfig_t cfg = {};

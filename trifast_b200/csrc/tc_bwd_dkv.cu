@@ -289,7 +289,7 @@ tc_dkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__
         const int key = min(im.kt * kBKeys + t, n - 1);
         KeyState ks;
         ks.row_full = rowfull[im.b * dm.n_rows + i];
-        ks.masked = mask.p[im.b * mask.sb + (int64_t)i * mask.si + key];
+        ks.masked = mask.p[im.b * mask.sb + (int64_t)i * mask.si + key * mask.sk];
         return ks;
       };
       KeyState next_state{0u, 0u};

@@ -178,7 +178,10 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 
   // A wait that gave up in an earlier CTA or launch leaves the status word set:
   // stop doing work until the host has read and cleared it.
-  if (*reinterpret_cast<volatile unsigned int*>(status) != 0u) return;
+  if (*reinterpret_cast<volatile unsigned int*>(status) != 0u) {
+    if (threadIdx.x == 0) repeat_status(status);   // (no prepare kernel runs before small problems)
+    return;
+  }
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 

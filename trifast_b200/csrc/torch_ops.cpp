@@ -95,28 +95,36 @@ Tensor prep5(const Tensor& t) {
   return ok ? t : dense(t);
 }
 
-Tensor prep4(const Tensor& t) {
-  bool ok = t.stride(3) == 1 && t.stride(2) >= t.size(3);
-  for (int a = 0; a < 3 && ok; ++a) ok = t.stride(a) >= 0;
-  return ok ? t : dense(t);
-}
-
-Tensor prep_mask(const Tensor& m) {
-  return m.stride(2) == 1 && m.stride(1) >= m.size(2) ? m : dense(m);
+// Whether the kernels can take the bias and the mask as they lie: innermost stride 1, and, for
+// the 16-bit kernels where no copies are prepared anyway (n a multiple of 8), rows that TMA and
+// 4-byte reads can address.  Anything else (a projection's permuted output, a transposed map,
+// an expanded view) goes in with TRIFAST_FLAG_STRIDED, and the call's prepare kernel makes the
+// copies it needs: no separate copies here.
+bool as_they_lie(const Tensor& b, const Tensor& m, int64_t n) {
+  if (b.stride(3) != 1 || b.stride(2) < n || m.stride(2) != 1 || m.stride(1) < n) return false;
+  if (b.scalar_type() == at::kFloat || n % 8 != 0) return true;
+  bool ok = reinterpret_cast<uintptr_t>(b.const_data_ptr()) % 16 == 0 &&
+            reinterpret_cast<uintptr_t>(m.const_data_ptr()) % 4 == 0;
+  for (int a = 0; a < 3 && ok; ++a) ok = b.stride(a) % 8 == 0 || b.size(a) == 1;
+  for (int a = 0; a < 2 && ok; ++a) ok = m.stride(a) % 4 == 0 || m.size(a) == 1;
+  return ok;
 }
 
 trifast_t5 view5(const Tensor& t) {
   return {const_cast<void*>(t.const_data_ptr()), {t.stride(0), t.stride(1), t.stride(2), t.stride(3)}};
 }
-trifast_t4 view4(const Tensor& t) {
-  return {const_cast<void*>(t.const_data_ptr()), {t.stride(0), t.stride(1), t.stride(2)}};
+trifast_t4_strided view4(const Tensor& t) {
+  return {const_cast<void*>(t.const_data_ptr()), {t.stride(0), t.stride(1), t.stride(2), t.stride(3)}};
 }
-trifast_mask view_mask(const Tensor& m) {
-  return {static_cast<const uint8_t*>(m.const_data_ptr()), {m.stride(0), m.stride(1)}};
+trifast_mask_strided view_mask(const Tensor& m) {
+  return {static_cast<const uint8_t*>(m.const_data_ptr()), {m.stride(0), m.stride(1), m.stride(2)}};
 }
+// (the longer descriptors start with the shorter ones)
+const trifast_t4* ptr(const trifast_t4_strided& v) { return reinterpret_cast<const trifast_t4*>(&v); }
+const trifast_mask* ptr(const trifast_mask_strided& v) { return reinterpret_cast<const trifast_mask*>(&v); }
 
 // Debug overrides of the tile heuristic, read per call like the rest of the binding does.
-trifast_shape make_shape(const Problem& p, at::ScalarType dt) {
+trifast_shape make_shape(const Problem& p, const Tensor& b, const Tensor& mask) {
   int32_t kernel = TRIFAST_KERNEL_AUTO;
   if (const char* e = std::getenv("TRIFAST_B200_KERNEL"); e && *e) {
     if (!strcasecmp(e, "simt"))
@@ -127,9 +135,10 @@ trifast_shape make_shape(const Problem& p, at::ScalarType dt) {
       TORCH_CHECK_VALUE(!strcasecmp(e, "auto"), "TRIFAST_B200_KERNEL=", e);
   }
   const char* f = std::getenv("TRIFAST_B200_FLAGS");
-  const int32_t flags = f && *f ? (int32_t)std::strtol(f, nullptr, 0) : 0;
+  int32_t flags = f && *f ? (int32_t)std::strtol(f, nullptr, 0) : 0;
+  if (!as_they_lie(b, mask, p.n)) flags |= TRIFAST_FLAG_STRIDED;
   return {(int32_t)p.batch, (int32_t)p.heads, (int32_t)p.n, (int32_t)p.rows, (int32_t)p.d,
-          dtype_code(dt), kernel, flags};
+          dtype_code(b.scalar_type()), kernel, flags};
 }
 
 void check_rc(int rc, const char* what) {
@@ -162,22 +171,22 @@ void raise_if_device_gave_up(c10::DeviceIndex dev, cudaStream_t stream) {
 
 // ------------------------------------------------------------------ CUDA implementations
 std::tuple<Tensor, Tensor> forward_cuda(const Tensor& q_, const Tensor& k_, const Tensor& v_,
-                                        const Tensor& b_, const Tensor& mask_) {
-  const Problem p = check_inputs(q_, k_, v_, b_, mask_);
-  const trifast_shape shp = make_shape(p, q_.scalar_type());
+                                        const Tensor& b, const Tensor& mask) {
+  const Problem p = check_inputs(q_, k_, v_, b, mask);
+  const trifast_shape shp = make_shape(p, b, mask);
   const c10::cuda::CUDAGuard guard(q_.device());
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
   raise_if_device_gave_up(q_.device().index(), stream);
-  const Tensor q = prep5(q_), k = prep5(k_), v = prep5(v_), b = prep4(b_), mask = prep_mask(mask_);
+  const Tensor q = prep5(q_), k = prep5(k_), v = prep5(v_);
   Tensor o = at::empty({p.batch, p.heads, p.rows, p.n, p.d}, q.options());
   Tensor lse = at::empty({p.batch, p.heads, p.rows, p.n}, q.options().dtype(at::kFloat));
   const size_t ws_bytes = trifast_forward_workspace_bytes(&shp);  // 0 on the CUDA-core plan
   Tensor ws;
   if (ws_bytes) ws = at::empty({(int64_t)ws_bytes}, q.options().dtype(at::kByte));
   const trifast_t5 tq = view5(q), tk = view5(k), tv = view5(v), to = view5(o);
-  const trifast_t4 tb = view4(b);
-  const trifast_mask tm = view_mask(mask);
-  check_rc(trifast_forward(&shp, &tq, &tk, &tv, &tb, &tm, &to, lse.mutable_data_ptr<float>(),
+  const trifast_t4_strided tb = view4(b);
+  const trifast_mask_strided tm = view_mask(mask);
+  check_rc(trifast_forward(&shp, &tq, &tk, &tv, ptr(tb), ptr(tm), &to, lse.mutable_data_ptr<float>(),
                            ws_bytes ? ws.mutable_data_ptr() : nullptr, ws_bytes, stream),
            "trifast_forward");
   return {o, lse};
@@ -185,9 +194,9 @@ std::tuple<Tensor, Tensor> forward_cuda(const Tensor& q_, const Tensor& k_, cons
 
 std::tuple<Tensor, Tensor, Tensor, Tensor> grads_cuda(const Tensor& do_, const Tensor& q_,
                                                       const Tensor& k_, const Tensor& v_,
-                                                      const Tensor& b_, const Tensor& o_,
-                                                      const Tensor& lse_, const Tensor& mask_) {
-  const Problem p = check_inputs(q_, k_, v_, b_, mask_);
+                                                      const Tensor& b, const Tensor& o_,
+                                                      const Tensor& lse_, const Tensor& mask) {
+  const Problem p = check_inputs(q_, k_, v_, b, mask);
   const auto like_q = [&](const char* name, const Tensor& t) {
     TORCH_CHECK_VALUE(t.sizes() == q_.sizes() && t.scalar_type() == q_.scalar_type(), name,
                       " must be ", q_.sizes(), " ", q_.scalar_type(), "; got ", t.sizes(), " ",
@@ -203,12 +212,12 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> grads_cuda(const Tensor& do_, const T
                     lse_.scalar_type(), " ", lse_.sizes());
   TORCH_CHECK_VALUE(lse_.device() == q_.device(), "lse is on ", lse_.device(), " but q is on ",
                     q_.device());
-  const trifast_shape shp = make_shape(p, q_.scalar_type());
+  const trifast_shape shp = make_shape(p, b, mask);
   const c10::cuda::CUDAGuard guard(q_.device());
   const cudaStream_t stream = at::cuda::getCurrentCUDAStream();
   raise_if_device_gave_up(q_.device().index(), stream);
   const Tensor d_o = prep5(do_), q = prep5(q_), k = prep5(k_), v = prep5(v_), o = prep5(o_),
-               b = prep4(b_), mask = prep_mask(mask_), lse = lse_.contiguous();
+               lse = lse_.contiguous();
   const at::IntArrayRef s5 = q_.sizes();
   Tensor dq = at::empty(s5, q.options()), dk = at::empty(s5, q.options()),
          dv = at::empty(s5, q.options());
@@ -217,10 +226,10 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> grads_cuda(const Tensor& do_, const T
   Tensor ws = at::empty({(int64_t)ws_bytes}, q.options().dtype(at::kByte));
   const trifast_t5 tdo = view5(d_o), tq = view5(q), tk = view5(k), tv = view5(v), to = view5(o),
                    tdq = view5(dq), tdk = view5(dk), tdv = view5(dv);
-  const trifast_t4 tb = view4(b), tdb = view4(db);
-  const trifast_mask tm = view_mask(mask);
-  check_rc(trifast_backward(&shp, &tdo, &tq, &tk, &tv, &tb, &tm, &to, lse.const_data_ptr<float>(),
-                            &tdq, &tdk, &tdv, &tdb, ws.mutable_data_ptr(), ws_bytes, stream),
+  const trifast_t4_strided tb = view4(b), tdb = view4(db);
+  const trifast_mask_strided tm = view_mask(mask);
+  check_rc(trifast_backward(&shp, &tdo, &tq, &tk, &tv, ptr(tb), ptr(tm), &to,
+                            lse.const_data_ptr<float>(), &tdq, &tdk, &tdv, ptr(tdb), ws.mutable_data_ptr(), ws_bytes, stream),
            "trifast_backward");
   return {dq, dk, dv, db};
 }
