@@ -260,7 +260,8 @@ int pick_plan(const trifast_shape* s, trifast_plan* p) {
   }
   // db: CTAs = tiles * splits.  Tensor-core kernel (128 x 128 tiles, one CTA per SM): split the
   // local rows until the grid covers the 148 SMs four times, but never below 8 rows per split
-  // and at most 16 splits.  CUDA-core kernel (64 x 64 tiles, 32 x 32 for n <= 32, two CTAs per
+  // and at most 16 splits (the workspace's share of partials: the backward takes as many as
+  // end first, tc_db_splits).  CUDA-core kernel (64 x 64 tiles, 32 x 32 for n <= 32, two CTAs per
   // SM): until 256 CTAs, down to 2 rows per split (a row is a whole product there, and small
   // problems have few), while the partials stay below 5 MiB (beyond that their traffic shows,
   // and the largest problem that fits a fixed workspace would shrink).
@@ -361,17 +362,21 @@ int cuda_rc(cudaError_t e) {
 enum BwdKernels { kBwdSimt, kBwdFused, kBwdSplit, kBwdD128 };
 
 int pick_bwd(const trifast_shape* shape, const Common& c, BwdArgs* a, BwdKernels* kern) {
-  if (wants_bwd_d128(shape) && tc_bwd_d128_supported(*a)) {
-    const int64_t t = (shape->n + 127) / 128;
-    a->splits = tc_db_cluster_splits(t * t * shape->heads * shape->batch, shape->n_rows, sm_count());
-    *kern = kBwdD128;
-    return TRIFAST_OK;
-  }
   *kern = kBwdSimt;
-  if (c.plan.kernel != TRIFAST_KERNEL_TCGEN05) return TRIFAST_OK;
-  if (!tc_backward_supported(*a))
-    return shape->kernel == TRIFAST_KERNEL_TCGEN05 ? TRIFAST_ERR_KERNEL_CHOICE : TRIFAST_OK;
-  *kern = c.plan.bwd_fused && tc_bwd_fused_supported(*a) ? kBwdFused : kBwdSplit;
+  if (wants_bwd_d128(shape)) {
+    if (!tc_bwd_d128_supported(*a)) return TRIFAST_OK;
+    *kern = kBwdD128;
+  } else {
+    if (c.plan.kernel != TRIFAST_KERNEL_TCGEN05) return TRIFAST_OK;
+    if (!tc_backward_supported(*a))
+      return shape->kernel == TRIFAST_KERNEL_TCGEN05 ? TRIFAST_ERR_KERNEL_CHOICE : TRIFAST_OK;
+    *kern = c.plan.bwd_fused && tc_bwd_fused_supported(*a) ? kBwdFused : kBwdSplit;
+  }
+  const int64_t t = (shape->n + 127) / 128, bh = (int64_t)shape->heads * shape->batch;
+  if (*kern == kBwdD128)   // (summed inside a cluster, without partials)
+    a->splits = tc_db_cluster_splits(t * t * bh, shape->n_rows, sm_count());
+  else                     // (the workspace holds the plan's number of partials)
+    a->splits = tc_db_splits(t * t * bh, shape->n_rows, sm_count(), bh * shape->n * shape->n * 4, c.plan.db_row_splits);
   return TRIFAST_OK;
 }
 

@@ -71,6 +71,7 @@ bool tc_backward_supported(const BwdArgs& a);
 cudaError_t tc_bwd_dq(const BwdArgs& a, cudaStream_t s);
 cudaError_t tc_bwd_dkv(const BwdArgs& a, cudaStream_t s);
 cudaError_t tc_bwd_db(const BwdArgs& a, cudaStream_t s);
+int tc_db_splits(int64_t tiles, int n_rows, int sms, int64_t partial_bytes, int most);
 int tc_db_cluster_splits(int64_t tiles, int n_rows, int sms);   // d = 128: row splits summed in a cluster
 // head dim 128 (its db: tc_bwd_db)
 bool tc_bwd_d128_supported(const BwdArgs& a);

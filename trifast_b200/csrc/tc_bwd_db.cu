@@ -559,16 +559,33 @@ int tc_db_cluster_splits(int64_t tiles, int n_rows, int sms) {
   return best;
 }
 
+// Row splits of a tile whose partials go through global memory (d <= 64), up to `most`: the same
+// estimate with the 9 rows' time (8 us) that a CTA's start and end measure there, and the
+// partials' way to memory and back at 5 TB/s, a row taking 0.85 us.  Measured against clusters of 2 to
+// 8 at n = 97 to 1024: faster everywhere but at n = 512 (equal), since clusters leave SMs idle.
+int tc_db_splits(int64_t tiles, int n_rows, int sms, int64_t partial_bytes, int most) {
+  int best = 1;
+  double best_cost = 1e30;
+  for (int s = 1; s <= most; ++s) {
+    const double cost = (double)((tiles * s + sms - 1) / sms) * ((n_rows + s - 1) / s + 9) +
+                        (s > 1 ? s * (2.0 * partial_bytes / 5e6) / 0.85 : 0.0);
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = s;
+    }
+  }
+  return best;
+}
+
 cudaError_t tc_bwd_db(const BwdArgs& a, cudaStream_t s) {
   const bool bf16 = a.dtype == TRIFAST_BF16;
   if (!a.neg_lse2 || !a.maskbits_lin) return cudaErrorInvalidValue;
-  if (a.dm.d == 128)
-    return bf16 ? launch_db<__nv_bfloat16, 128, 3, true>(a, s) : launch_db<__half, 128, 3, true>(a, s);
-  if (a.dm.d == 16)
-    return bf16 ? launch_db<__nv_bfloat16, 16, 4>(a, s) : launch_db<__half, 16, 4>(a, s);
-  if (a.dm.d == 32)
-    return bf16 ? launch_db<__nv_bfloat16, 32, 4>(a, s) : launch_db<__half, 32, 4>(a, s);
-  return bf16 ? launch_db<__nv_bfloat16, 64, 3>(a, s) : launch_db<__half, 64, 3>(a, s);
+  switch (a.dm.d) {
+    case 16: return bf16 ? launch_db<__nv_bfloat16, 16, 4>(a, s) : launch_db<__half, 16, 4>(a, s);
+    case 32: return bf16 ? launch_db<__nv_bfloat16, 32, 4>(a, s) : launch_db<__half, 32, 4>(a, s);
+    case 64: return bf16 ? launch_db<__nv_bfloat16, 64, 3>(a, s) : launch_db<__half, 64, 3>(a, s);
+    default: return bf16 ? launch_db<__nv_bfloat16, 128, 3, true>(a, s) : launch_db<__half, 128, 3, true>(a, s);
+  }
 }
 
 }  // namespace trifast
