@@ -214,8 +214,7 @@ class HostPipeline:
                                              C.c_size_t(self._fws_bytes), run_stream)
                     L.check(rc, "trifast_forward")
                     plan = L.pick_plan(B, H, n, r, d, self.dtype)
-                    tc = plan["kernel"] == L.KERNEL_TCGEN05
-                    launches += 1 + (2 if self._fws_bytes else 0)
+                    launches += 1 + (1 if self._fws_bytes and (n > 128 or n % 8 or d == 128) else 0)
                     if bwd:
                         part = self.db_f32 if c == 0 else self.db_part
                         ws, wsb = C.c_void_p(self._ws.data_ptr()), C.c_size_t(self._ws_bytes)
@@ -231,9 +230,9 @@ class HostPipeline:
                             C.byref(a["v"]), C.byref(ab), C.byref(am), lse, C.byref(a["dq"]),
                             C.byref(a["dk"]), C.byref(a["dv"]), ws, wsb, run_stream)
                         L.check(rc, "trifast_backward_dqkv")
-                        # row flags, bias copies, delta, db (+ split reduce), dq, dk/dv
-                        launches += 1 + (1 if tc else 0) + (1 if tc and n % 8 else 0) + 2 + \
-                            (1 if plan["db_row_splits"] > 1 else 0) + 2
+                        # prepare, db (+ the sum of its row splits), dq / dk / dv
+                        launches += 2 + (1 if plan["db_row_splits"] > 1 and d != 128 else 0) + \
+                            (1 if plan["bwd_fused"] else 2)
                     ev_run[c] = self.s_run.record_event()
                 # ---- device -> host
                 with torch.cuda.stream(self.s_out):
