@@ -45,7 +45,12 @@ def _newest(paths) -> float:
 
 
 def _ops_commands(nvcc: str, obj: str):
-    """Compile and link commands of the operator library."""
+    """Compile and link commands of the operator library.
+
+    It links the shared C++ runtime by its file name: a compiler that has only the static one
+    (``libstdc++.a``) would put a second copy into the process beside PyTorch's, and the two
+    disagree about the facets of a locale: the first error message with a number in it crashes.
+    """
     import torch
     from torch.utils.cpp_extension import include_paths
     root = os.path.dirname(os.path.dirname(os.path.realpath(nvcc)))
@@ -55,8 +60,8 @@ def _ops_commands(nvcc: str, obj: str):
     compile_cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-Wall",
                    f"-D_GLIBCXX_USE_CXX11_ABI={abi}", *inc, "-c", OPS_SRC, "-o", obj]
     link_cmd = [os.environ.get("CXX", "g++"), "-shared", "-o", OPS_LIB, obj, "-L", PKG,
-                "-l:libtrifast_b200.so", "-L", libs, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda",
-                "-ltorch", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + libs]
+                "-l:libtrifast_b200.so", "-l:libstdc++.so.6", "-L", libs, "-lc10", "-lc10_cuda",
+                "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + libs]
     return compile_cmd, link_cmd
 
 
