@@ -41,3 +41,24 @@ def test_messages_with_numbers(name, value, want):
     r = run_python(CALL_CUDA_KERNEL % (name, value))
     assert r.returncode == 0, (r.returncode, r.stderr[-2000:])
     assert r.stdout.strip() == want
+
+
+def small(dtype="float32"):
+    import torch
+    q, k, v = (torch.randn(1, 2, 16, 16, 32, device="cuda", dtype=getattr(torch, dtype)) for _ in range(3))
+    return q, k, v, torch.zeros(1, 2, 16, 16, device="cuda", dtype=q.dtype), \
+        torch.zeros(1, 16, 16, dtype=torch.bool, device="cuda")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("value", ["abc", "1x", "0x1", " "])
+def test_flags_override_must_be_a_decimal_integer(monkeypatch, value):
+    from trifast_b200 import triangle_attention
+    monkeypatch.setenv("TRIFAST_B200_FLAGS", value)
+    with pytest.raises(ValueError):
+        triangle_attention(*small())
+    with pytest.raises(ValueError):       # the same rule in the Python layer
+        from trifast_b200 import _lib
+        _lib.flags_choice()
+    monkeypatch.setenv("TRIFAST_B200_FLAGS", "1")
+    assert triangle_attention(*small()).shape == (1, 2, 16, 16, 32)

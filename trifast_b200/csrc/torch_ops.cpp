@@ -16,6 +16,7 @@
 #include <torch/library.h>
 
 #include <atomic>
+#include <cctype>
 #include <cstdlib>
 #include <cstring>
 
@@ -134,8 +135,13 @@ trifast_shape make_shape(const Problem& p, const Tensor& b, const Tensor& mask) 
     else
       TORCH_CHECK_VALUE(!strcasecmp(e, "auto"), "TRIFAST_B200_KERNEL=", e);
   }
-  const char* f = std::getenv("TRIFAST_B200_FLAGS");
-  int32_t flags = f && *f ? (int32_t)std::strtol(f, nullptr, 0) : 0;
+  int32_t flags = 0;
+  if (const char* f = std::getenv("TRIFAST_B200_FLAGS"); f && *f) {
+    char* end = nullptr;
+    flags = (int32_t)std::strtol(f, &end, 10);
+    while (std::isspace((unsigned char)*end)) ++end;
+    TORCH_CHECK_VALUE(end != f && !*end, "TRIFAST_B200_FLAGS=", f, " is not a decimal integer");
+  }
   if (!as_they_lie(b, mask, p.n)) flags |= TRIFAST_FLAG_STRIDED;
   return {(int32_t)p.batch, (int32_t)p.heads, (int32_t)p.n, (int32_t)p.rows, (int32_t)p.d,
           dtype_code(b.scalar_type()), kernel, flags};
