@@ -289,7 +289,8 @@ int trifast_snapshot_device_status(uint32_t* host_word, void* stream);
  * write when a wait gives up (and the next call's first kernel again while the status is set).  A binding
  * looks at it at the start of each call; when it is non-zero it calls
  * trifast_check_device_status() and then sets the word to zero.  The first call on a device
- * allocates the word: make it outside stream capture.  (No reference counterpart.) */
+ * allocates the word and waits for one small copy on a stream of its own; streams that are
+ * being captured do not notice.  (No reference counterpart.) */
 int trifast_host_status_word(uint32_t** host_word);
 
 /* Test support for that path: launches one warp that waits, with the same bounded

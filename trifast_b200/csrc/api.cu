@@ -660,15 +660,24 @@ int trifast_host_status_word(uint32_t** host_word) {
   int rc = device_setup(&dev, &status);
   if (rc) return rc;
   std::call_once(g_host_word_once[dev], [dev, status] {
-    void* p = nullptr;
-    cudaError_t e = cudaHostAlloc(&p, sizeof(uint32_t), cudaHostAllocPortable | cudaHostAllocMapped);
+    // The first call may come while a stream is being captured: under the relaxed mode this
+    // thread may allocate and wait all the same, on a stream that no capture knows.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+    const bool exchanged = e == cudaSuccess;
+    void *p = nullptr, *d = nullptr;   // the word, and the address kernels write to
+    cudaStream_t own = nullptr;
+    if (e == cudaSuccess) e = cudaHostAlloc(&p, sizeof(uint32_t), cudaHostAllocPortable | cudaHostAllocMapped);
     if (e == cudaSuccess) {
       *(volatile uint32_t*)p = 0;
-      void* d = nullptr;   // the address kernels write to (the same one under unified addressing)
       e = cudaHostGetDevicePointer(&d, p, 0);
-      if (e == cudaSuccess)
-        e = cudaMemcpy((char*)status + offsetof(DeviceStatus, host), &d, sizeof(d), cudaMemcpyHostToDevice);
     }
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync((char*)status + offsetof(DeviceStatus, host), &d, sizeof(d), cudaMemcpyHostToDevice, own);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(own);
+    if (own) cudaStreamDestroy(own);
+    if (exchanged) cudaThreadExchangeStreamCaptureMode(&mode);
     g_host_word[dev] = e == cudaSuccess ? (unsigned int*)p : nullptr;
     g_host_word_error[dev] = e;
   });
