@@ -139,8 +139,10 @@ trifast_shape make_shape(const Problem& p, const Tensor& b, const Tensor& mask) 
   if (const char* f = std::getenv("TRIFAST_B200_FLAGS"); f && *f) {
     char* end = nullptr;
     flags = (int32_t)std::strtol(f, &end, 10);
+    bool ok = end != f;
     while (std::isspace((unsigned char)*end)) ++end;
-    TORCH_CHECK_VALUE(end != f && !*end, "TRIFAST_B200_FLAGS=", f, " is not a decimal integer");
+    ok = ok && !*end;
+    TORCH_CHECK_VALUE(ok, "TRIFAST_B200_FLAGS=", f, " is not a decimal integer");
   }
   if (!as_they_lie(b, mask, p.n)) flags |= TRIFAST_FLAG_STRIDED;
   return {(int32_t)p.batch, (int32_t)p.heads, (int32_t)p.n, (int32_t)p.rows, (int32_t)p.d,
