@@ -104,7 +104,10 @@ typedef struct trifast_t5 {
   int64_t stride[4];
 } trifast_t5;
 
-/* (b, h, j, k) tensor: strides in elements for b, h, j; k has stride 1. */
+/* (b, h, j, k) tensor: strides in elements for b, h, j; k has stride 1.  As a bias, b and h may
+ * have stride 0 (one map for all heads or batches): the kernels then read it without TMA, on
+ * the CUDA cores, unless the workspace holds a packed copy (n % 8 != 0, or
+ * TRIFAST_FLAG_STRIDED, which is the faster way to pass such a map). */
 typedef struct trifast_t4 {
   void* data;
   int64_t stride[3];

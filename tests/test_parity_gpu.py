@@ -434,7 +434,7 @@ def test_cuda_core_kernels_at_their_tile_edges(n, d, dtype):
 @pytest.mark.parametrize("n,d,dtype", [(48, 32, torch.float32), (40, 32, torch.bfloat16), (64, 32, torch.bfloat16),
                                        (131, 16, torch.float16), (136, 64, torch.bfloat16), (200, 128, torch.bfloat16)])
 def test_strided_bias_and_mask_equal_dense_copies(n, d, dtype):
-    """A permuted, a misaligned and an expanded bias with a transposed mask: packed by the
+    """A permuted, a misaligned and two expanded biases with a transposed mask: packed by the
     prepare kernels, bit for bit the results of dense copies."""
     torch.manual_seed(n)
     h = 3
@@ -442,7 +442,8 @@ def test_strided_bias_and_mask_equal_dense_copies(n, d, dtype):
     m = (torch.rand(1, n, n, device=DEV) < 0.3).transpose(1, 2)
     wide = torch.randn(1, h, n, n + 3, device=DEV).to(dtype)
     for b in (torch.randn(1, n, n, h, device=DEV).to(dtype).permute(0, 3, 1, 2), wide[..., 1:n + 1],
-              torch.randn(1, 1, n, n, device=DEV).to(dtype).transpose(2, 3).expand(1, h, n, n)):
+              torch.randn(1, 1, n, n, device=DEV).to(dtype).transpose(2, 3).expand(1, h, n, n),
+              torch.randn(1, 1, n, n, device=DEV).to(dtype).expand(1, h, n, n)):
         res = []
         for bias, mask in ((b, m), (b.contiguous(), m.contiguous())):
             leaves = [t.detach().requires_grad_(True) for t in (q, k, v, bias)]

@@ -62,6 +62,13 @@ cudaError_t db_reduce_splits(const BwdArgs& a, cudaStream_t s);
 cudaError_t db_cast(const float* partials, int splits, View4 db, int dtype, int batch, int heads, int n,
                     cudaStream_t s);
 
+// Whether TMA can read a 16-bit bias as it lies: base and strides of whole 16-byte units, and no
+// stride of 0 over more than one entry (an expanded view), which no tensor map describes.
+inline bool bias_fits_tma(const View4& b, const Dims& dm) {
+  if ((reinterpret_cast<uintptr_t>(b.p) & 15) || b.sj % 8 || b.sh % 8 || b.sb % 8) return false;
+  return (b.sh > 0 || dm.heads == 1) && (b.sb > 0 || dm.batch == 1);
+}
+
 // tcgen05 kernels (tc_*.cu): bf16 / fp16.
 bool tc_forward_d128_supported(const Dims& dm, int dtype, const FwdArgs* a);
 cudaError_t tc_forward_d128(const FwdArgs& a, cudaStream_t s);

@@ -538,10 +538,8 @@ bool tc_bwd_d128_supported(const BwdArgs& a) {
   if (a.dtype != TRIFAST_BF16 && a.dtype != TRIFAST_F16) return false;
   if (a.dm.d != kD || a.dm.n < kMinTensorCoreN) return false;
   if (!a.neg_lse2 || !a.maskbits_lin || !a.rowrange) return false;
-  if (!a.bias_pad) {   // the bias goes through TMA as it is
-    if (a.dm.n % 8 != 0 || ((uintptr_t)a.bias.p) & 15) return false;
-    if ((a.bias.sj * 2) % 16 || (a.bias.sh * 2) % 16 || (a.bias.sb * 2) % 16) return false;
-  }
+  // without the padded copy the bias goes through TMA as it is
+  if (!a.bias_pad && (a.dm.n % 8 != 0 || !bias_fits_tma(a.bias, a.dm))) return false;
   return get_encode_tiled() != nullptr;
 }
 

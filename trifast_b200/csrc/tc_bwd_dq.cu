@@ -509,9 +509,7 @@ bool tc_backward_supported(const BwdArgs& a) {
   if (dm.n < kMinTensorCoreN) return false;
   if (!a.maskbits || !a.rowfull || !a.delta || !a.neg_lse2) return false;
   // the bias goes through TMA: 16-byte row pitch, or the padded copy from the workspace
-  const bool bias_tma_ok = !(((uintptr_t)a.bias.p) & 15) && (a.bias.sj * 2) % 16 == 0 &&
-                           (a.bias.sh * 2) % 16 == 0 && (a.bias.sb * 2) % 16 == 0;
-  if (!bias_tma_ok && !a.bias_pad) return false;
+  if (!a.bias_pad && !bias_fits_tma(a.bias, dm)) return false;
   return tc::get_encode_tiled() != nullptr;
 }
 

@@ -721,9 +721,7 @@ bool tc_forward_supported(const Dims& dm, int dtype, const FwdArgs* a) {
     if (!have_ws) {
       // without the prepared copies the bias goes through TMA as it is (16-byte row
       // pitch) and the key mask is read four bytes at a time
-      if (dm.n % 8 != 0) return false;
-      if ((a->bias.sj * 2) % 16 || (a->bias.sh * 2) % 16 || (a->bias.sb * 2) % 16) return false;
-      if (((uintptr_t)a->bias.p) & 15) return false;
+      if (dm.n % 8 != 0 || !bias_fits_tma(a->bias, dm)) return false;
       if (((uintptr_t)a->mask.p) & 3 || a->mask.sb % 4 || a->mask.si % 4) return false;
     }
   }

@@ -520,11 +520,7 @@ bool tc_forward_d128_supported(const Dims& dm, int dtype, const FwdArgs* a) {
   if (a) {
     if (((uintptr_t)a->o.p) & 15 || (a->o.sj * 2) % 16) return false;
     if (!a->maskbits || !a->rowfull || !a->rowrange) return false;
-    if (!a->bias_pad) {
-      if (dm.n % 8 != 0) return false;
-      if ((a->bias.sj * 2) % 16 || (a->bias.sh * 2) % 16 || (a->bias.sb * 2) % 16) return false;
-      if (((uintptr_t)a->bias.p) & 15) return false;
-    }
+    if (!a->bias_pad && (dm.n % 8 != 0 || !bias_fits_tma(a->bias, dm))) return false;
   }
   return tc::get_encode_tiled() != nullptr;
 }

@@ -106,7 +106,7 @@ bool as_they_lie(const Tensor& b, const Tensor& m, int64_t n) {
   if (b.scalar_type() == at::kFloat || n % 8 != 0) return true;
   bool ok = reinterpret_cast<uintptr_t>(b.const_data_ptr()) % 16 == 0 &&
             reinterpret_cast<uintptr_t>(m.const_data_ptr()) % 4 == 0;
-  for (int a = 0; a < 3 && ok; ++a) ok = b.stride(a) % 8 == 0 || b.size(a) == 1;
+  for (int a = 0; a < 3 && ok; ++a) ok = (b.stride(a) > 0 && b.stride(a) % 8 == 0) || b.size(a) == 1;
   for (int a = 0; a < 2 && ok; ++a) ok = m.stride(a) % 4 == 0 || m.size(a) == 1;
   return ok;
 }

@@ -49,7 +49,9 @@ def _prep5(t):
 
 
 def _prep4(t):
-    return t if (t.stride(-1) == 1 and all(s >= 0 for s in t.stride())
+    """(b, h, j, k) with k contiguous; an expanded dimension (stride 0) is materialised, as TMA
+    cannot describe it."""
+    return t if (t.stride(-1) == 1 and all(s > 0 or n == 1 for s, n in zip(t.stride(), t.shape))
                  and t.stride(-2) >= t.shape[-1]) else _dense(t)
 
 
