@@ -503,6 +503,12 @@ __global__ void __launch_bounds__(kThreads) simt_bwd_kernel(View5 a1, View5 a2, 
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int a = r0 + at.y + r * F::TY, ac = min(a, n - 1);
+    if constexpr (kKv) {
+      if (dropped[r]) {   // exactly zero, also where a query's dO, lse or delta is not finite
+#pragma unroll
+        for (int e = 0; e < F::Q * 2; ++e) acc1[r][e] = acc2[r][e] = make_float2(0.f, 0.f);
+      }
+    }
     store_row<T, D, R>(acc1[r], dm.scale, row_ptr<T>(out1, b, h, i, ac), at.x, at.p, a < n);
     if constexpr (kKv) store_row<T, D, R>(acc2[r], 1.f, row_ptr<T>(out2, b, h, i, ac), at.x, at.p, a < n);
   }

@@ -447,6 +447,8 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
       constexpr int kCols = kKv ? kD : kD / 2;
       const uint32_t tAcc = tmem_base + lane_base + (kKv && half ? kAcc2 : kAcc1) + (kKv ? 0 : half * kCols);
       const float sc = (kKv && half) ? 1.f : dm.scale;
+      // a dropped key gets exactly zero, also where a query's dO, lse or delta is not finite
+      const bool zero = kKv && dropped;
       uint32_t acc[kCols];
       tmem_ld_cols<kCols>(tAcc, acc);
       tmem_wait_ld();
@@ -462,6 +464,7 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
           u.y = pack2<T>(__uint_as_float(acc[e + 2]) * sc, __uint_as_float(acc[e + 3]) * sc);
           u.z = pack2<T>(__uint_as_float(acc[e + 4]) * sc, __uint_as_float(acc[e + 5]) * sc);
           u.w = pack2<T>(__uint_as_float(acc[e + 6]) * sc, __uint_as_float(acc[e + 7]) * sc);
+          if (zero) u = make_uint4(0u, 0u, 0u, 0u);
           *reinterpret_cast<uint4*>(dst + e) = u;
         }
       }
