@@ -340,6 +340,7 @@ int fill_bwd(const trifast_shape* shape, const Common& c, const trifast_t5* d_o,
   a->db_partials = (float*)(base + w.partial_off);
   a->kv_scratch = w.kv_scratch_bytes ? (float*)(base + w.kv_scratch_off) : nullptr;
   a->splits = c.plan.db_row_splits;
+  a->ds_up = (float*)(base + w.db_off);   // (where it is used, see pick_bwd)
   a->dm = c.dm;
   a->dtype = shape->dtype;
   a->reserve_sms = (shape->flags & TRIFAST_FLAG_SHARE_GPU)
@@ -363,9 +364,14 @@ enum BwdKernels { kBwdSimt, kBwdFused, kBwdSplit, kBwdD128 };
 
 int pick_bwd(const trifast_shape* shape, const Common& c, BwdArgs* a, BwdKernels* kern) {
   *kern = kBwdSimt;
+  float* const ds_up = a->ds_up;
+  a->ds_up = nullptr;
   if (wants_bwd_d128(shape)) {
     if (!tc_bwd_d128_supported(*a)) return TRIFAST_OK;
     *kern = kBwdD128;
+    // fp16: the row scales lie where db is summed, so dq / dk / dv run before db (and between
+    // trifast_backward_db, whose db is the caller's, and trifast_backward_dqkv the place is free)
+    if (shape->dtype == TRIFAST_F16) a->ds_up = ds_up;
   } else {
     if (c.plan.kernel != TRIFAST_KERNEL_TCGEN05) return TRIFAST_OK;
     if (!tc_backward_supported(*a))
@@ -595,9 +601,12 @@ int trifast_backward(const trifast_shape* shape, const trifast_t5* d_o, const tr
   a.dv = make_view(dv);
   cudaStream_t s = (cudaStream_t)stream;
   BwdKernels kern;
-  if ((rc = pick_bwd(shape, c, &a, &kern)) || (rc = cuda_rc(bwd_prepare(a, s))) ||
-      (rc = run_db(a, kern, s)) || (rc = run_dqkv(a, kern, s)))
-    return rc;
+  if ((rc = pick_bwd(shape, c, &a, &kern)) || (rc = cuda_rc(bwd_prepare(a, s)))) return rc;
+  if (a.ds_up)
+    rc = (rc = run_dqkv(a, kern, s)) ? rc : run_db(a, kern, s);
+  else
+    rc = (rc = run_db(a, kern, s)) ? rc : run_dqkv(a, kern, s);
+  if (rc) return rc;
   const bool partials = a.splits > 1 && kern != kBwdD128;
   return cuda_rc(db_cast(partials ? a.db_partials : a.db_f32, partials ? a.splits : 1, make_view(db),
                          shape->dtype, shape->batch, shape->heads, shape->n, s));

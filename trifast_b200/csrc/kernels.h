@@ -43,6 +43,9 @@ struct BwdArgs {
   float* db_f32;         // (b, h, n, n) fp32 result of the row reduction
   float* db_partials;    // (splits, b, h, n, n) fp32, used when splits > 1
   int splits;
+  // (b, h, n_rows) powers of two that put a pair row's dS into the range of fp16 (head dim 128,
+  // fp16; made by the prepare step), or null
+  float* ds_up;
   Dims dm;
   int dtype;
   float* kv_scratch;     // per-CTA fp32 dK / dV partials of rows walked in several query chunks, or null

@@ -27,8 +27,11 @@ struct Prep {
   uint16_t *bias_t, *bias_pad;
   Dims dm;
   unsigned int* status;
-  // block ranges, in this order: one row of the mask each; 64 x 64 bias tiles; the rest delta
-  int mask_blocks, bias_tiles, bias_blocks;
+  View5 v;
+  float* ds_up;
+  // block ranges, in this order: one row of the mask each; 64 x 64 bias tiles; one (b, h, i) of
+  // ds_up each; the rest delta
+  int mask_blocks, bias_tiles, bias_blocks, scale_blocks;
 };
 
 // ---------------------------------------------------------------------------
@@ -211,6 +214,58 @@ __device__ void prepare_delta(const View5& o, const View5& d_o, const float* lse
   }
 }
 
+// ---------------------------------------------------------------------------
+// ds_up[b, h, i] (fp16, D = 128): the power of two that scales the pair row's dS to at most
+// 2^15.  dS = P (dP - delta) with P <= 1 and |dP|, |delta| <= D max|dO| max|v|, the largest finite
+// values of the row, v over its open keys.  Without it a gradient of 1e-5 leaves dS among fp16's
+// subnormals and one of 1e4 beyond its range.  Bound by memory: dO and v once more (120 us at
+// n = 512, h = 4).
+// ---------------------------------------------------------------------------
+template <int D>
+__device__ void prepare_row_scale(const Prep& a, const View5& d_o, int w) {
+  constexpr int kParts = D / 8, kRows = kPrepThreads / kParts;   // 16-byte parts of a row, rows at a time
+  const int n = a.dm.n, i = w % a.dm.n_rows, bh = w / a.dm.n_rows, b = bh / a.dm.heads, h = bh % a.dm.heads;
+  const uint8_t* mrow = a.mask.p + b * a.mask.sb + (int64_t)i * a.mask.si;
+  int open = 0;
+  for (int k = threadIdx.x; k < n; k += kPrepThreads) open |= mrow[k * a.mask.sk] == 0;
+  const bool row_full = !__syncthreads_or(open);
+  const int part = threadIdx.x % kParts * 8;
+  const __half* po = (const __half*)d_o.p + b * d_o.sb + h * d_o.sh + (int64_t)i * d_o.si + part;
+  const __half* pv = (const __half*)a.v.p + b * a.v.sb + h * a.v.sh + (int64_t)i * a.v.si + part;
+  // magnitudes as 16-bit integers, in order; 0x7c00 and above are not finite
+  uint32_t most_o = 0u, most_v = 0u;
+  auto most = [](uint32_t m, uint32_t u) {
+    u &= 0x7fff7fffu;
+    return __vmaxu2(m, u & __vcmpltu2(u, 0x7c007c00u));
+  };
+#pragma unroll 4
+  for (int r = threadIdx.x / kParts; r < n; r += kRows) {
+    const uint4 g = __ldg(reinterpret_cast<const uint4*>(po + (int64_t)r * d_o.sj));
+    most_o = most(most(most(most(most_o, g.x), g.y), g.z), g.w);
+    if (row_full || mrow[r * a.mask.sk] == 0) {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(pv + (int64_t)r * a.v.sj));
+      most_v = most(most(most(most(most_v, u.x), u.y), u.z), u.w);
+    }
+  }
+  __shared__ uint32_t shared_most[2];
+  if (threadIdx.x < 2) shared_most[threadIdx.x] = 0u;
+  __syncthreads();
+  const uint32_t mo = __reduce_max_sync(0xffffffffu, max(most_o & 0xffffu, most_o >> 16));
+  const uint32_t mv = __reduce_max_sync(0xffffffffu, max(most_v & 0xffffu, most_v >> 16));
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(&shared_most[0], mo);
+    atomicMax(&shared_most[1], mv);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const float fo = __half2float(__ushort_as_half((unsigned short)shared_most[0]));
+    const float fv = __half2float(__ushort_as_half((unsigned short)shared_most[1]));
+    // |x| < 2^(ilogb(x) + 1); 2 D = 2^8
+    static_assert(D == 128, "exponent of 2 D");
+    a.ds_up[w] = fo > 0.f && fv > 0.f ? ldexpf(1.f, 15 - 8 - (ilogbf(fo) + 1) - (ilogbf(fv) + 1)) : 1.f;
+  }
+}
+
 __global__ void __launch_bounds__(kPrepThreads) fwd_prepare_kernel(Prep a) {
   int w = blockIdx.x;
   if (w == 0 && threadIdx.x == 0) repeat_status(a.status);
@@ -226,7 +281,11 @@ __global__ void __launch_bounds__(kPrepThreads) bwd_prepare_kernel(Prep a, View5
   if (w < a.mask_blocks) return prepare_mask_row(a, w);
   w -= a.mask_blocks;
   if (w < a.bias_blocks) return prepare_bias_tile(a, w);
-  prepare_delta<T, D>(o, d_o, lse, delta, neg_lse2, a.dm, w - a.bias_blocks);
+  w -= a.bias_blocks;
+  if constexpr (std::is_same<T, __half>::value && D == 128) {
+    if (w < a.scale_blocks) return prepare_row_scale<D>(a, d_o, w);
+  }
+  prepare_delta<T, D>(o, d_o, lse, delta, neg_lse2, a.dm, w - a.scale_blocks);
 }
 
 // ---------------------------------------------------------------------------
@@ -327,12 +386,16 @@ cudaError_t bwd_prepare(const BwdArgs& a, cudaStream_t s) {
   p.bias_pad = (uint16_t*)a.bias_pad;
   p.status = a.status;
   p.bias_blocks = a.bias_t || a.bias_pad ? p.bias_tiles * p.bias_tiles * dm.batch * dm.heads : 0;
+  p.v = a.v;
+  p.ds_up = a.ds_up;
+  p.scale_blocks = a.ds_up ? dm.batch * dm.heads * dm.n_rows : 0;
   return dispatch(a.dtype, dm.d, [&](auto* tp, auto dc) {
     using T = std::remove_pointer_t<decltype(tp)>;
     constexpr int D = decltype(dc)::value;
     constexpr int kRows = DeltaCfg<T, D>::kRows;
     const int64_t rows = (int64_t)dm.batch * dm.heads * dm.n_rows * dm.n;
-    const unsigned blocks = (unsigned)(p.mask_blocks + p.bias_blocks + (rows + kRows - 1) / kRows);
+    const unsigned blocks =
+        (unsigned)(p.mask_blocks + p.bias_blocks + p.scale_blocks + (rows + kRows - 1) / kRows);
     bwd_prepare_kernel<T, D><<<blocks, kPrepThreads, 0, s>>>(p, a.o, a.d_o, a.lse, a.delta, a.neg_lse2);
   });
 }

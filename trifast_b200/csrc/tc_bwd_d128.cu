@@ -7,9 +7,19 @@
 //            S = Q K^T, dP = dO V^T,  dS = P (dP - delta),    dQ += dS K
 //     dk/dv: resident K, V (128 keys),      streamed Q, dO;   lanes = keys
 //            S^T = K Q^T, dP^T = V dO^T,                      dV += P^T dO,  dK += dS^T Q
-// with P = exp2(S c + bias log2e - lse log2e).  A row of 128 elements is two 128-byte swizzle
-// spans: every tile is two [rows x 64] halves (two TMA boxes); K-major operands take their K
-// slices from one half or the other, MN-major ones get the halves as their two N atoms.
+// with P = exp2(S c + bias log2e - lse log2e).
+//
+// Precision: P and dS enter the products as the sum of two 16-bit operands each, the rounded value
+// and the remainder (split2), so every accumulating product runs twice.  dq, dk and dv then
+// carry the rounding of the result and no more: against float64 at n = 512, dq 1.707e-3 (bf16) and
+// 2.133e-4 (fp16) in the 2-norm, the digits that fp32 products on the CUDA cores give; with P
+// and dS rounded to one operand 2.391e-3 and 2.988e-4.  fp16 has a range to keep to as well: P is
+// held times 2^15, dS times a power of two per pair row that the prepare step takes from the
+// largest |dO| and |v| (ds_up), both undone on the accumulators.
+//
+// A row of 128 elements is two 128-byte swizzle spans: every tile is two [rows x 64] halves (two
+// TMA boxes); K-major operands take their K slices from one half or the other, MN-major ones
+// get the halves as their two N atoms.
 //
 // The bias tile is the one operand that is not transposed with the rest: lanes = keys read
 // it down its columns, 2 bytes per lane and query from unswizzled 256-byte rows (a warp reads
@@ -20,11 +30,12 @@
 // columns each); 8 TMA; 9 S / dP MMAs and the TMEM allocation; 10 accumulating MMAs; 11
 // completes the warpgroup whose registers are handed over.  Work items are persistent over
 // the SMs, and three stages are kept in flight: a stage is held for two steps plus its load
-// latency, so two stages would stall on it.  A step costs about 2450 (dq) and 3150 (dk/dv)
-// cycles, of which the MMAs hold the tensor pipe for about 770 and 1020: the hops between the
-// warps bound it, as in the kernels for smaller head dims.  Measured at n = 512, h = 4, bf16:
-// dq 574 us, dk/dv 737 us, where the CUDA-core kernels took 44.3 ms and 41.3 ms (db, one row
-// as two stages of half the head dim in tc_bwd_db.cu: 379 us against 22.3 ms).
+// latency, so two stages would stall on it.  A step of dq and one of dk/dv cost about 6900 cycles
+// together, of which the MMAs hold the tensor pipe for about 2500: the hops between the warps
+// bound it, as in the kernels for smaller head dims.  Measured at n = 512, h = 4: dq and dk/dv
+// together 1.56 ms in bf16 and 1.75 ms in fp16 (1.32 and 1.39 ms with P and dS in one 16-bit operand
+// each), where the CUDA-core kernels took 85.6 ms (db, one row as two stages of half the head
+// dim in tc_bwd_db.cu: 379 us against 22.3 ms).
 //
 // Stands in for `_bwd_q` and `_bwd_kv` of the reference (src/trifast/triton.py:268-383,
 // :137-263).  Masked keys weigh exactly zero; rows whose keys are all masked use P = 1/n
@@ -72,15 +83,18 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
                    const __grid_constant__ CUtensorMap map_nlse,
                    const __grid_constant__ CUtensorMap map_delta, View5 out1, View5 out2,
                    const float* __restrict__ neg_lse2, const float* __restrict__ delta,
-                   const uint8_t* __restrict__ rowfull, const uint32_t* __restrict__ maskbits_lin,
+                   const float* __restrict__ ds_up, const uint8_t* __restrict__ rowfull, const uint32_t* __restrict__ maskbits_lin,
                    int mask_words, const uint32_t* __restrict__ rowrange, Dims dm, Grid grid,
                    unsigned int* status) {
-  // TMEM columns: SB buffers of S, dP (64 each), then dS (and P) as 16-bit pairs, then the
-  // accumulators
+  // TMEM columns: SB buffers of S, dP (64 each), then dS (and P) as 16-bit pairs, the rounded
+  // values and the remainders (32 columns each), then the accumulators
   constexpr int SB = kKv ? 1 : 2;
-  constexpr int kDsCol = SB * 128, kPCol = kDsCol + 32;
-  constexpr int kAcc1 = kKv ? kPCol + 32 : kDsCol + 32;   // dQ, or dK
+  constexpr int kDsCol = SB * 128, kPCol = kDsCol + 64;
+  constexpr int kAcc1 = kKv ? kPCol + 64 : kDsCol + 64;   // dQ, or dK
   constexpr int kAcc2 = kAcc1 + kD;                       // dV
+  // fp16: P times 2^15 and dS times ds_up, so that neither leaves the type's normal range
+  constexpr bool kUp = std::is_same<T, __half>::value;
+  constexpr float kUpLog2 = kUp ? 15.f : 0.f, kUpP = kUp ? 32768.f : 1.f;
   static_assert((kKv ? kAcc2 : kAcc1) + kD <= 512, "TMEM columns");
   constexpr int A_FULL = 0, A_EMPTY = 1, FULL = 2, EMPTY = FULL + kStages, S_FULL = EMPTY + kStages,
                 S_FREE = S_FULL + 2, P_READY = S_FREE + 2, ACC_DONE = P_READY + 2,
@@ -281,13 +295,17 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
             if (kKv) {
 #pragma unroll
               for (int ks = 0; ks < kStep / 16; ++ks)
-                umma_ts(tmem_base + kAcc2, tmem_base + kPCol + ks * 8, e2 + ks * 128, idesc,
-                        st > lo || ks > 0);
+#pragma unroll
+                for (int lo_part = 0; lo_part < 2; ++lo_part)
+                  umma_ts(tmem_base + kAcc2, tmem_base + kPCol + lo_part * 32 + ks * 8, e2 + ks * 128, idesc,
+                          st > lo || ks > 0 || lo_part > 0);
             }
 #pragma unroll
             for (int ks = 0; ks < kStep / 16; ++ks)
-              umma_ts(tmem_base + kAcc1, tmem_base + kDsCol + ks * 8, e1 + ks * 128, idesc,
-                      st > lo || ks > 0);
+#pragma unroll
+              for (int lo_part = 0; lo_part < 2; ++lo_part)
+                umma_ts(tmem_base + kAcc1, tmem_base + kDsCol + lo_part * 32 + ks * 8, e1 + ks * 128, idesc,
+                        st > lo || ks > 0 || lo_part > 0);
             umma_commit(bar(ACC_DONE + (g & 1)));
             umma_commit(bar(EMPTY + s));
           }
@@ -306,7 +324,7 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
     const uint32_t tDS = tmem_base + lane_base + kDsCol + half * 16;
     const uint32_t tP = tmem_base + lane_base + kPCol + half * 16;
     const float c1 = dm.scale * kLog2e;
-    const float uniform = 1.f / (float)n;
+    const float uniform = kUpP / (float)n;
 
     int g = 0;
     bool ok = true;
@@ -331,15 +349,18 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
       const bool row_full = rowfull[b * dm.n_rows + i] != 0;
       // key mask in key order (bit set = dropped or beyond n; on a fully masked row only beyond n)
       const uint32_t* mrow = maskbits_lin + ((int64_t)b * dm.n_rows + i) * mask_words;
-      float nl_row = 0.f, dl_row = 0.f;
+      // dS is P (dP - delta) times `up`, of which P already carries kUpP
+      const float up = kUp ? __ldg(ds_up + ((int64_t)b * dm.heads + h) * dm.n_rows + i) : 1.f;
+      const float up_dp = up / kUpP;
+      float nl_row = 0.f, ndl_row = 0.f;
       uint32_t mw_next = 0u;
       bool dropped = false;
       if (kKv) {
         dropped = ((__ldg(mrow + im.tile * 4 + wq) >> lane) & 1u) != 0u;
       } else {
         const int64_t at = (((int64_t)b * dm.heads + h) * dm.n_rows + i) * dm.n_pad + min(row, n - 1);
-        nl_row = __ldg(neg_lse2 + at);
-        dl_row = __ldg(delta + at);
+        nl_row = __ldg(neg_lse2 + at) + kUpLog2;
+        ndl_row = -__ldg(delta + at) * up_dp;
         mw_next = __ldg(mrow + lo * 2 + half);
       }
       auto steps = [&](auto full_tag) {
@@ -362,13 +383,13 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
           __syncwarp();
           if (lane == 0) mbar_arrive(bar(S_FREE + (g & 1)));
 
-          uint32_t pp[16], pd[16];
+          uint32_t pp[16], pp_lo[16], pd[16], pd_lo[16];
           const uint8_t* bias_s = gbase + bias_off(s);
           const float4* nl4 = reinterpret_cast<const float4*>(gbase + vec_off(s)) + half * 8;
           const float4* dl4 = nl4 + kVecBytes / 16;
 #pragma unroll
           for (int q8 = 0; q8 < 4; ++q8) {
-            float bv[8], nl[8], dl[8];
+            float bv[8], nl[8], dl[8];   // (dl: delta, or -delta up_dp where the query is this thread's)
             if (kKv) {
               const float4 da = dl4[q8 * 2], db = dl4[q8 * 2 + 1];
               dl[0] = da.x; dl[1] = da.y; dl[2] = da.z; dl[3] = da.w;
@@ -385,7 +406,7 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
 #pragma unroll
               for (int e = 0; e < 8; ++e) {
                 nl[e] = nl_row;
-                dl[e] = dl_row;
+                dl[e] = ndl_row;
               }
               if (!kRowFull) {
                 const uint4 u = *reinterpret_cast<const uint4*>(bias_s + t * 128 + (((half * 4 + q8) ^ (t & 7)) << 4));
@@ -401,6 +422,7 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
               float p0 = uniform, p1 = uniform;
               if (!kRowFull) {
                 float t0, t1, a0, a1;
+                if (kKv && kUp) fadd2(nl[e], nl[e + 1], nl[e], nl[e + 1], kUpLog2, kUpLog2);
                 ffma2(t0, t1, bv[e], bv[e + 1], kLog2e, kLog2e, nl[e], nl[e + 1]);
                 ffma2(a0, a1, x[col], x[col + 1], c1, c1, t0, t1);
                 p0 = ex2(a0);
@@ -413,11 +435,16 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
                 p0 = ((mw >> col) & 1u) ? 0.f : p0;
                 p1 = ((mw >> (col + 1)) & 1u) ? 0.f : p1;
               }
-              float s0, s1, d0, d1;
-              ffma2(s0, s1, dl[e], dl[e + 1], -1.f, -1.f, gd[col], gd[col + 1]);   // dP - delta
+              float s0, s1, d0, d1;   // (dP - delta) up_dp
+              if (kKv && !kUp) {
+                ffma2(s0, s1, dl[e], dl[e + 1], -1.f, -1.f, gd[col], gd[col + 1]);
+              } else {
+                if (kKv) fmul2(dl[e], dl[e + 1], dl[e], dl[e + 1], -up_dp, -up_dp);
+                ffma2(s0, s1, gd[col], gd[col + 1], up_dp, up_dp, dl[e], dl[e + 1]);
+              }
               fmul2(d0, d1, p0, p1, s0, s1);
-              if (kKv) pp[col >> 1] = pack2<T>(p0, p1);
-              pd[col >> 1] = pack2<T>(d0, d1);
+              if (kKv) split2<T>(p0, p1, pp[col >> 1], pp_lo[col >> 1]);
+              split2<T>(d0, d1, pd[col >> 1], pd_lo[col >> 1]);
             }
           }
           __syncwarp();
@@ -428,8 +455,12 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
                                                         ((g - 1) >> 1) & 1, abort_flag));
             if (!ok) break;
           }
-          if (kKv) tmem_st16(tP, pp);
+          if (kKv) {
+            tmem_st16(tP, pp);
+            tmem_st16(tP + 32, pp_lo);
+          }
           tmem_st16(tDS, pd);
+          tmem_st16(tDS + 32, pd_lo);
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
@@ -446,7 +477,7 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
       tc_fence_after();
       constexpr int kCols = kKv ? kD : kD / 2;
       const uint32_t tAcc = tmem_base + lane_base + (kKv && half ? kAcc2 : kAcc1) + (kKv ? 0 : half * kCols);
-      const float sc = (kKv && half) ? 1.f : dm.scale;
+      const float sc = (kKv && half) ? 1.f / kUpP : dm.scale / up;
       // a dropped key gets exactly zero, also where a query's dO, lse or delta is not finite
       const bool zero = kKv && dropped;
       uint32_t acc[kCols];
@@ -530,8 +561,8 @@ cudaError_t launch(const BwdArgs& a, cudaStream_t stream) {
   grid.total = grid.tiles * dm.n_rows * dm.heads * dm.batch;
   const int sms = sm_count() - a.reserve_sms > 0 ? sm_count() - a.reserve_sms : 1;
   kern<<<grid.total < sms ? grid.total : sms, 384, kSmemBytes, stream>>>(
-      a1, a2, b1, b2, mb, mnl, mdl, kKv ? a.dk : a.dq, kKv ? a.dv : a.dq, a.neg_lse2, a.delta, a.rowfull,
-      a.maskbits_lin, a.mask_words, a.rowrange, dm, grid, a.status);
+      a1, a2, b1, b2, mb, mnl, mdl, kKv ? a.dk : a.dq, kKv ? a.dv : a.dq, a.neg_lse2, a.delta, a.ds_up,
+      a.rowfull, a.maskbits_lin, a.mask_words, a.rowrange, dm, grid, a.status);
   return cudaGetLastError();
 }
 
