@@ -254,12 +254,12 @@ class DirectStep:
         plan = L.pick_plan(bs, h, n, rows, d, q.dtype)
         self.plan = plan
         # launches per step: forward 1 (+ its prepare kernel on the tensor-core path, where there
-        # is anything to prepare); backward: prepare, db, the sum of db's row splits (at d = 128
-        # inside the db kernel), dq / dk / dv in one or two, db's cast
+        # is anything to prepare); backward: prepare, db, the sum of db's partials if there are
+        # several, dq / dk / dv in one or two, db's cast
         self.launches = 1 + (1 if plan["fwd_kernel"] == 2 and (n > 128 or n % 8 or d == 128) else 0)
         if w.backward:
-            self.launches += 2 + (1 if plan["db_row_splits"] > 1 and d != 128 else 0) + \
-                (1 if plan["bwd_fused"] else 2) + 1
+            partials = self.lib.trifast_backward_db_partials(C.byref(self.shape))
+            self.launches += 2 + (1 if partials > 1 else 0) + (1 if plan["bwd_fused"] else 2) + 1
         self.exposed = None   # (event after dq/dk/dv, event after the all-reduce wait)
         self.reducer = None
         if w.backward and group_size > 1 and db_reduce == "push":

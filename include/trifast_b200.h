@@ -137,7 +137,9 @@ typedef struct trifast_plan {
   int32_t block_k;       /* key tile */
   int32_t rows_per_cta;  /* pair rows sharing one bias tile in the forward */
   int32_t stages;        /* K/V/bias pipeline depth */
-  int32_t db_row_splits; /* row groups whose db partials are summed in fixed order */
+  int32_t db_row_splits; /* row groups whose db partials are summed in fixed order: as many as the
+                            workspace holds.  The tensor-core kernels take the number up to this
+                            that ends first (trifast_backward_db_partials) */
   int32_t bwd_fused;     /* 1: dq, dk, dv come from one kernel (one exponential per score) */
   int32_t bwd_chunks;    /* query chunks a row is walked in by that kernel (1: dQ of a row fits TMEM) */
   int32_t fwd_kernel;    /* trifast_kernel of the forward: differs from `kernel` for head dim 128.
@@ -161,6 +163,12 @@ const char* trifast_last_cuda_error(void);
  * (src/trifast/autotune.py:110-156): same key (n, h, d, dtype), but a table
  * instead of benchmarking and an on-disk cache.  Pure host code. */
 int trifast_pick_plan(const trifast_shape* shape, trifast_plan* plan);
+
+/* The fp32 partials of db that a backward of this shape writes and then sums in one more launch;
+ * 1 when db is written as it is (one row group, or row groups summed inside a thread-block
+ * cluster at head dim 128).  For a bias that TMA can read or has packed.  Negative: the
+ * trifast_status of an invalid shape.  (No reference counterpart.) */
+int32_t trifast_backward_db_partials(const trifast_shape* shape);
 
 /* Bytes of caller-provided workspace the backward needs (delta, packed masks, fp32
  * db and its row-split partials, bias copies).  Returns 0 on an invalid shape. */

@@ -67,6 +67,7 @@ SIGNATURES = {
     "trifast_copy_blocks": (C.c_int, [C.c_void_p, C.c_size_t, C.c_void_p, C.c_size_t, C.c_size_t,
                                       C.c_size_t, C.c_int, C.c_void_p]),
     "trifast_pick_plan": (C.c_int, [_P(Shape), _P(Plan)]),
+    "trifast_backward_db_partials": (C.c_int32, [_P(Shape)]),
     "trifast_backward_workspace_bytes": (C.c_size_t, [_P(Shape)]),
     "trifast_forward_workspace_bytes": (C.c_size_t, [_P(Shape)]),
     "trifast_forward": (C.c_int, [_P(Shape), _P(T5), _P(T5), _P(T5), _P(T4), _P(Mask), _P(T5),

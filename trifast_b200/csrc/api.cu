@@ -362,6 +362,15 @@ int cuda_rc(cudaError_t e) {
 // The kernels a backward runs on.
 enum BwdKernels { kBwdSimt, kBwdFused, kBwdSplit, kBwdD128 };
 
+// Row splits of db on the tensor-core kernels.
+int tc_splits(const trifast_shape* shape, const trifast_plan& plan) {
+  const int64_t t = (shape->n + 127) / 128, bh = (int64_t)shape->heads * shape->batch;
+  if (shape->d == 128)   // (summed inside a cluster, without partials)
+    return tc_db_cluster_splits(t * t * bh, shape->n_rows, sm_count());
+  // (the workspace holds the plan's number of partials)
+  return tc_db_splits(t * t * bh, shape->n_rows, sm_count(), bh * shape->n * shape->n * 4, plan.db_row_splits);
+}
+
 int pick_bwd(const trifast_shape* shape, const Common& c, BwdArgs* a, BwdKernels* kern) {
   *kern = kBwdSimt;
   float* const ds_up = a->ds_up;
@@ -378,11 +387,7 @@ int pick_bwd(const trifast_shape* shape, const Common& c, BwdArgs* a, BwdKernels
       return shape->kernel == TRIFAST_KERNEL_TCGEN05 ? TRIFAST_ERR_KERNEL_CHOICE : TRIFAST_OK;
     *kern = c.plan.bwd_fused && tc_bwd_fused_supported(*a) ? kBwdFused : kBwdSplit;
   }
-  const int64_t t = (shape->n + 127) / 128, bh = (int64_t)shape->heads * shape->batch;
-  if (*kern == kBwdD128)   // (summed inside a cluster, without partials)
-    a->splits = tc_db_cluster_splits(t * t * bh, shape->n_rows, sm_count());
-  else                     // (the workspace holds the plan's number of partials)
-    a->splits = tc_db_splits(t * t * bh, shape->n_rows, sm_count(), bh * shape->n * shape->n * 4, c.plan.db_row_splits);
+  a->splits = tc_splits(shape, c.plan);
   return TRIFAST_OK;
 }
 
@@ -457,6 +462,14 @@ const char* trifast_status_str(int status) {
 int trifast_pick_plan(const trifast_shape* shape, trifast_plan* plan) {
   if (!plan) return TRIFAST_ERR_NULL;
   return pick_plan(shape, plan);
+}
+
+int32_t trifast_backward_db_partials(const trifast_shape* shape) {
+  trifast_plan plan;
+  const int rc = pick_plan(shape, &plan);
+  if (rc) return rc;
+  if (wants_bwd_d128(shape)) return 1;
+  return plan.kernel == TRIFAST_KERNEL_TCGEN05 ? tc_splits(shape, plan) : plan.db_row_splits;
 }
 
 size_t trifast_backward_workspace_bytes(const trifast_shape* shape) {

@@ -230,9 +230,9 @@ class HostPipeline:
                             C.byref(a["v"]), C.byref(ab), C.byref(am), lse, C.byref(a["dq"]),
                             C.byref(a["dk"]), C.byref(a["dv"]), ws, wsb, run_stream)
                         L.check(rc, "trifast_backward_dqkv")
-                        # prepare, db (+ the sum of its row splits), dq / dk / dv
-                        launches += 2 + (1 if plan["db_row_splits"] > 1 and d != 128 else 0) + \
-                            (1 if plan["bwd_fused"] else 2)
+                        # prepare, db (+ the sum of its partials), dq / dk / dv
+                        launches += 2 + (1 if plan["bwd_fused"] else 2) + \
+                            (1 if lib.trifast_backward_db_partials(C.byref(shp)) > 1 else 0)
                     ev_run[c] = self.s_run.record_event()
                 # ---- device -> host
                 with torch.cuda.stream(self.s_out):
