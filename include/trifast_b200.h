@@ -132,7 +132,7 @@ typedef struct trifast_mask_strided {
 
 /* Tile plan chosen by the heuristic (host only; no device needed). */
 typedef struct trifast_plan {
-  int32_t kernel;        /* trifast_kernel actually used (by the backward, when the two differ) */
+  int32_t kernel;        /* trifast_kernel of the plan; for head dim 128 see fwd_kernel */
   int32_t block_j;       /* query tile */
   int32_t block_k;       /* key tile */
   int32_t rows_per_cta;  /* pair rows sharing one bias tile in the forward */
@@ -291,8 +291,8 @@ int trifast_check_device_status(void* stream);
  * binding can call this after each launch and look at the word at the start of its
  * next call: a non-zero value means some earlier kernel gave up on a wait (its
  * outputs are not valid), and trifast_check_device_status() then reads and clears
- * it.  This is how the Python operators turn a device-side timeout into an
- * exception without a synchronisation per call.  (No reference counterpart.) */
+ * it.  For bindings that keep a word of their own; the Python operators use
+ * trifast_host_status_word below, which enqueues nothing.  (No reference counterpart.) */
 int trifast_snapshot_device_status(uint32_t* host_word, void* stream);
 
 /* The same without anything enqueued per call: *host_word becomes the address of a pinned

@@ -275,7 +275,7 @@ def test_expanded_views_are_materialised_by_the_python_layer():
     (4, 64, torch.float16, 224, 256),
     (4, 16, torch.bfloat16, 224, 256),
     (1, 32, torch.bfloat16, 448, 480),
-    (4, 128, torch.bfloat16, 576, 608),   # CUDA-core plan
+    (4, 128, torch.bfloat16, 576, 608),   # CUDA-core plan (of the tensor-core backward, too)
     (4, 32, torch.float32, 576, 608),
 ])
 def test_static_scratch_capacity(h, d, dtype, n_ok, n_too_large):
@@ -354,8 +354,8 @@ def test_share_gpu_flag_carries_the_number_of_free_sms():
 
 
 def test_head_dim_128_plan_and_forward_workspace():
-    """d = 128: tensor-core tiles exist for the forward only.  plan.kernel (the backward's
-    family) is CUDA cores, plan.fwd_kernel tensor cores; the forward workspace always holds
+    """d = 128: plan.fwd_kernel is tensor cores; plan.kernel is CUDA cores, the plan in whose
+    workspace the tensor-core backward runs; the forward workspace always holds
     the prepared row flags and packed masks (4 words per 128 keys and row) besides the ranges,
     and the padded bias copy only for ragged n; asking for CUDA cores gives them throughout."""
     lib = _lib.load()
@@ -367,9 +367,9 @@ def test_head_dim_128_plan_and_forward_workspace():
     size = lambda n: lib.trifast_forward_workspace_bytes(C.byref(_lib.make_shape(1, 4, n, n, 128, torch.bfloat16)))
     assert size(1024) == 4096 + 1024 + 1024 * 32 * 4                  # ranges, row flags, packed masks
     assert size(1000) < 4 * 1000 * 1000 * 2 < size(1001)              # the bias copy only when ragged
-    # the backward of d = 128 has no tensor-core family to force
+    # the tensor-core family cannot be forced onto the backward of d = 128
     shp = _lib.make_shape(1, 4, 256, 256, 128, torch.bfloat16, _lib.KERNEL_TCGEN05)
-    assert lib.trifast_backward_workspace_bytes(C.byref(shp)) > 0     # sized for the CUDA-core kernels
+    assert lib.trifast_backward_workspace_bytes(C.byref(shp)) > 0     # sized by the CUDA-core plan
 
 
 def test_host_pipeline_block_bounds():

@@ -1,7 +1,7 @@
 """Head dim 128: the forward runs on its own tensor-core kernel (csrc/tc_fwd_d128.cu: two
-128-query tiles of one pair row per CTA, P written over S in TMEM), the backward on the CUDA
-cores.  Forward against the fp64 oracle and against the CUDA-core forward; the whole op with
-autograd against the oracle."""
+128-query tiles of one pair row per CTA, P written over S in TMEM), the backward on
+csrc/tc_bwd_d128.cu and csrc/tc_bwd_db.cu.  Both against the fp64 oracle and against the CUDA-core
+kernels; the whole op with autograd against the oracle."""
 
 import pytest
 import torch
@@ -105,7 +105,7 @@ def test_forward_is_deterministic_and_ignores_masked_values():
 
 
 def test_whole_op_with_autograd():
-    """Forward on tensor cores, backward on CUDA cores, through the public op."""
+    """Forward and backward on tensor cores, through the public op."""
     n, h, dtype = 160, 2, torch.bfloat16
     q, k, v, b, m = _inputs(n, h, n, dtype, "random", seed=9)
     do = torch.randn(1, h, n, n, 128, generator=torch.Generator().manual_seed(1)).to(dtype)

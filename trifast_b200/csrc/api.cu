@@ -311,7 +311,8 @@ int fill_bwd(const trifast_shape* shape, const Common& c, const trifast_t5* d_o,
     return rc;
   if (o && (rc = check_t5(o, shape))) return rc;
   if (!lse) return TRIFAST_ERR_NULL;
-  // (head dim 128: tensor-core tiles exist for the forward only)
+  // (head dim 128: the tensor-core backward is part of TRIFAST_KERNEL_AUTO, which may fall back to
+  // the CUDA cores; the plan and its workspace are theirs, so the family cannot be forced)
   if (shape->kernel == TRIFAST_KERNEL_TCGEN05 && c.plan.kernel != TRIFAST_KERNEL_TCGEN05)
     return TRIFAST_ERR_KERNEL_CHOICE;
   const Workspace w = carve(shape, c.plan);
@@ -533,7 +534,7 @@ int trifast_forward(const trifast_shape* shape, const trifast_t5* q, const trifa
       a.rowrange = nullptr;
     else if ((rc = cuda_rc(fwd_prepare(a, s))))
       return rc;
-    return cuda_rc(d128 ? tc_forward_d128(a, s) : tc_forward(a, c.plan, s));
+    return cuda_rc(d128 ? tc_forward_d128(a, s) : tc_forward(a, s));
   }
   return cuda_rc(simt_forward(a, s));
 }

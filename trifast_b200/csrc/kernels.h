@@ -76,7 +76,7 @@ inline bool bias_fits_tma(const View4& b, const Dims& dm) {
 bool tc_forward_d128_supported(const Dims& dm, int dtype, const FwdArgs* a);
 cudaError_t tc_forward_d128(const FwdArgs& a, cudaStream_t s);
 bool tc_forward_supported(const Dims& dm, int dtype, const FwdArgs* a);
-cudaError_t tc_forward(const FwdArgs& a, const trifast_plan& plan, cudaStream_t s);
+cudaError_t tc_forward(const FwdArgs& a, cudaStream_t s);
 bool tc_backward_supported(const BwdArgs& a);
 cudaError_t tc_bwd_dq(const BwdArgs& a, cudaStream_t s);
 cudaError_t tc_bwd_dkv(const BwdArgs& a, cudaStream_t s);

@@ -728,7 +728,7 @@ bool tc_forward_supported(const Dims& dm, int dtype, const FwdArgs* a) {
   return tc::get_encode_tiled() != nullptr;
 }
 
-cudaError_t tc_forward(const FwdArgs& a, const trifast_plan&, cudaStream_t s) {
+cudaError_t tc_forward(const FwdArgs& a, cudaStream_t s) {
   const bool bf16 = a.dtype == TRIFAST_BF16;
   if (a.dm.d == 16)
     return bf16 ? launch<__nv_bfloat16, 16, 2, 3>(a, s) : launch<__half, 16, 2, 3>(a, s);
