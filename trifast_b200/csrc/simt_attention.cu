@@ -236,6 +236,14 @@ __device__ __forceinline__ void store_row(float2 (&acc)[Cfg<D, R>::Q * 2], float
   }
 }
 
+template <typename T, int D, int R>
+__device__ __forceinline__ void zero_row(T* dst, int stream, int part) {
+  using F = Cfg<D, R>;
+#pragma unroll
+  for (int q = 0; q < F::Q; ++q)
+    if (stream == q % kStreams) store4<T>(dst + (q * F::G + part) * 4, make_float4(0.f, 0.f, 0.f, 0.f));
+}
+
 // Where a thread stands: lane part p of its rows, stream x, group y.
 template <int D, int R> struct Place {
   int p, x, y;
@@ -503,14 +511,16 @@ __global__ void __launch_bounds__(kThreads) simt_bwd_kernel(View5 a1, View5 a2, 
 #pragma unroll
   for (int r = 0; r < R; ++r) {
     const int a = r0 + at.y + r * F::TY, ac = min(a, n - 1);
+    store_row<T, D, R>(acc1[r], dm.scale, row_ptr<T>(out1, b, h, i, ac), at.x, at.p, a < n);
     if constexpr (kKv) {
-      if (dropped[r]) {   // exactly zero, also where a query's dO, lse or delta is not finite
-#pragma unroll
-        for (int e = 0; e < F::Q * 2; ++e) acc1[r][e] = acc2[r][e] = make_float2(0.f, 0.f);
+      store_row<T, D, R>(acc2[r], 1.f, row_ptr<T>(out2, b, h, i, ac), at.x, at.p, a < n);
+      // a dropped key gets exactly zero, also where a query's dO, lse or delta is not finite: the
+      // lanes that stored its row overwrite it (a select on the way costs the other rows 1 %)
+      if (dropped[r] && a < n) {
+        zero_row<T, D, R>(row_ptr<T>(out1, b, h, i, a), at.x, at.p);
+        zero_row<T, D, R>(row_ptr<T>(out2, b, h, i, a), at.x, at.p);
       }
     }
-    store_row<T, D, R>(acc1[r], dm.scale, row_ptr<T>(out1, b, h, i, ac), at.x, at.p, a < n);
-    if constexpr (kKv) store_row<T, D, R>(acc2[r], 1.f, row_ptr<T>(out2, b, h, i, ac), at.x, at.p, a < n);
   }
 }
 
