@@ -77,3 +77,45 @@ def test_separate_calls_equal_the_whole_backward():
     abi_backward(do, q, k, v, b, m, o, lse, *want)
     for name, x, y in zip(("dq", "dk", "dv", "db"), got, want):
         assert torch.equal(x, y), name
+
+
+def test_static_scratch_and_graph_replay_with_row_scales():
+    """fp16: the scales share the scratch with db, and follow the values of a replay."""
+    import ctypes as C
+    lib = _lib.load()
+    g = torch.Generator(device=DEV).manual_seed(1)
+    q, k, v, do = (torch.randn(1, 2, 104, 104, 128, generator=g, device=DEV).half() for _ in range(4))
+    b = torch.randn(1, 2, 104, 104, generator=g, device=DEV).half()
+    m = torch.rand(1, 104, 104, generator=g, device=DEV) < 0.2
+    o, lse = torch.empty_like(q), torch.empty(q.shape[:4], dtype=torch.float32, device=DEV)
+    abi_forward(q, k, v, b, m, o, lse)
+
+    def step(static):
+        out = [torch.full_like(q, float("nan")) for _ in range(3)] + [torch.full_like(b, float("nan"))]
+        if not static:
+            abi_backward(do, q, k, v, b, m, o, lse, *out)
+            return out
+        t5 = lambda t: C.byref(_lib.t5(t))
+        rc = lib.trifast_backward_static_scratch(
+            C.byref(_lib.make_shape(1, 2, 104, 104, 128, q.dtype)), t5(do), t5(q), t5(k), t5(v), C.byref(_lib.t4(b)),
+            C.byref(_lib.mask_view(m.view(torch.uint8))), t5(o), C.c_void_p(lse.data_ptr()), t5(out[0]), t5(out[1]),
+            t5(out[2]), C.byref(_lib.t4(out[3])), C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        _lib.check(rc, "trifast_backward_static_scratch")
+        return out
+
+    for scale in (1.0, 1e-3):
+        do.mul_(scale)
+        for x, y in zip(step(True), step(False)):
+            assert torch.equal(x, y)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        step(False)
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = step(False)
+    do.mul_(3e3)
+    graph.replay()
+    for x, y in zip(captured, step(False)):
+        assert torch.isfinite(x).all() and torch.equal(x, y)

@@ -10,7 +10,8 @@ struct FwdArgs {
   View4 bias;
   MaskView mask;
   float* lse;
-  // forward workspace (tensor-core path with n % 8 != 0 only; null otherwise)
+  // forward workspace (tensor-core path with n % 8 != 0 or a strided bias; the row flags and masks
+  // at head dim 128, too; null otherwise)
   void* bias_pad;        // (b, h, j, n_pad) copy of the bias with a 16-byte row pitch
   uint8_t* rowfull;      // (b, n_rows)
   uint32_t* maskbits;    // (b, n_rows, mask_words)
@@ -31,7 +32,7 @@ struct BwdArgs {
   float* delta;          // (b, h, n_rows, n_pad) fp32, in the workspace
   float* neg_lse2;       // (b, h, n_rows, n_pad) fp32: -lse * log2(e), in the workspace
   void* bias_t;          // (b, h, k, n_pad) transposed bias copy in the input dtype, or null
-  void* bias_pad;        // (b, h, j, n_pad) bias copy with a 16-byte row pitch (n % 8 != 0), or null
+  void* bias_pad;        // (b, h, j, n_pad) bias copy with a 16-byte row pitch (n % 8 != 0 or strided), or null
   uint8_t* rowfull;      // (b, n_rows): 1 = every key of the row is masked
   // (b, n_rows, mask_words): bit set = key dropped or beyond n.  Per 128-key chunk c
   // four words: word c*4 + jb holds, at bit l, key c*128 + 4*l + jb.
