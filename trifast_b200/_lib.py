@@ -151,12 +151,16 @@ def raise_if_device_gave_up(device) -> None:
     if int(w[0]) == 0:
         return
     with torch.cuda.device(device):
-        load().trifast_check_device_status(
+        rc = load().trifast_check_device_status(
             C.c_void_p(torch.cuda.current_stream(device).cuda_stream))
-    w.zero_()
+    cleared = rc != -9                                     # TRIFAST_ERR_LAUNCH
+    if cleared:
+        w.zero_()
     raise RuntimeError(
         "trifast_b200: " + status_str(-11) + " in an earlier call on this device; the results "
-        "of that call and of the calls after it are invalid (status cleared, retry is possible)")
+        "of that call and of the calls after it are invalid " +
+        ("(status cleared, retry is possible)" if cleared else
+         "(the status could not be cleared here, as during a graph capture)"))
 
 
 def kernel_choice() -> int:

@@ -357,6 +357,7 @@ thread_local cudaError_t g_last_cuda_error = cudaSuccess;
 int cuda_rc(cudaError_t e) {
   if (e == cudaSuccess) return TRIFAST_OK;
   g_last_cuda_error = e;
+  cudaGetLastError();   // reported here: the next launch's check must not find it again
   return TRIFAST_ERR_LAUNCH;
 }
 
@@ -633,12 +634,12 @@ int trifast_check_device_status(void* stream) {
   if (rc) return rc;
   cudaStream_t s = (cudaStream_t)stream;
   unsigned int host = 0;
-  if (cudaMemcpyAsync(&host, status, sizeof(host), cudaMemcpyDeviceToHost, s) != cudaSuccess)
-    return TRIFAST_ERR_LAUNCH;
-  if (cudaStreamSynchronize(s) != cudaSuccess) return TRIFAST_ERR_LAUNCH;
+  if ((rc = cuda_rc(cudaMemcpyAsync(&host, status, sizeof(host), cudaMemcpyDeviceToHost, s))) ||
+      (rc = cuda_rc(cudaStreamSynchronize(s))))
+    return rc;
   if (host == 0) return TRIFAST_OK;
-  cudaMemsetAsync(status, 0, sizeof(host), s);
-  cudaStreamSynchronize(s);
+  if ((rc = cuda_rc(cudaMemsetAsync(status, 0, sizeof(host), s))) || (rc = cuda_rc(cudaStreamSynchronize(s))))
+    return rc;
   return TRIFAST_ERR_DEVICE_TIMEOUT;
 }
 

@@ -171,11 +171,15 @@ void raise_if_device_gave_up(c10::DeviceIndex dev, cudaStream_t stream) {
     words[dev].store(w, std::memory_order_release);
   }
   if (*w == 0) return;
-  trifast_check_device_status(stream);
-  *w = 0;
+  // (while the stream is being captured the status cannot be read: the word stays set, and the
+  // next call outside the capture clears both)
+  const bool cleared = trifast_check_device_status(stream) != TRIFAST_ERR_LAUNCH;
+  if (cleared) *w = 0;
   TORCH_CHECK(false, "trifast_b200: ", trifast_status_str(TRIFAST_ERR_DEVICE_TIMEOUT),
               " in an earlier call on this device; the results of that call and of the calls "
-              "after it are invalid (status cleared, retry is possible)");
+              "after it are invalid ",
+              cleared ? "(status cleared, retry is possible)"
+                      : "(the status could not be cleared here, as during a graph capture)");
 }
 
 // ------------------------------------------------------------------ CUDA implementations
