@@ -35,5 +35,7 @@ def test_dropped_keys_keep_zero_gradients(n, d, dtype, what):
     assert dropped[:, :, row].any()
     assert not dk[dropped].any() and not dv[dropped].any()     # (NaN counts as true)
     assert not torch.isfinite(dk[0, 0, row]).all()              # open keys: as the mathematics has it
+    if what == "dO inf":   # P times infinity is one, unless P has no second 16-bit part (below 2^-12 of them)
+        assert torch.isinf(dv[0, 0, row, :, 1][~m[0, row]]).float().mean() > 0.95
     others = [i for i in range(n) if i != row]
     assert all(torch.isfinite(t[:, :, others]).all() for t in (dq, dk, dv))

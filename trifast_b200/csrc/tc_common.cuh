@@ -373,16 +373,17 @@ template <> __device__ __forceinline__ uint32_t pack2<__half>(float lo, float hi
   asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
 }
-// The same with infinities and values beyond the type's range as its largest finite one.
-template <typename T> __device__ __forceinline__ uint32_t pack2_finite(float lo, float hi);
-template <> __device__ __forceinline__ uint32_t pack2_finite<__nv_bfloat16>(float lo, float hi) {
+// The same rounded toward zero, infinities and values beyond the type's range as its largest finite
+// one.
+template <typename T> __device__ __forceinline__ uint32_t pack2_toward_zero(float lo, float hi);
+template <> __device__ __forceinline__ uint32_t pack2_toward_zero<__nv_bfloat16>(float lo, float hi) {
   uint32_t r;
-  asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  asm("cvt.rz.satfinite.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
 }
-template <> __device__ __forceinline__ uint32_t pack2_finite<__half>(float lo, float hi) {
+template <> __device__ __forceinline__ uint32_t pack2_toward_zero<__half>(float lo, float hi) {
   uint32_t r;
-  asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  asm("cvt.rz.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
 }
 template <typename T> __device__ __forceinline__ void unpack2(uint32_t u, float& lo, float& hi);
@@ -397,13 +398,14 @@ template <> __device__ __forceinline__ void unpack2<__half>(uint32_t u, float& l
   hi = f.y;
 }
 
-// Two fp32 values as the sum of two 16-bit ones each, the rounded value and what the rounding
-// left: 16 (bf16) or 22 (fp16) significant bits instead of 8 or 11.  An infinity stays one (the
-// first part is finite, the second infinite).
+// Two fp32 values as the sum of two 16-bit ones each, the value rounded toward zero and what that
+// left: 16 (bf16) or 22 (fp16) significant bits instead of 8 or 11.  The parts have one sign, so
+// an infinite factor gives an infinity and not the difference of two; an infinite value stays
+// one (the first part is finite, the second infinite).
 template <typename T>
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
   float h0, h1, l0, l1;
-  hi = pack2_finite<T>(a, b);
+  hi = pack2_toward_zero<T>(a, b);
   unpack2<T>(hi, h0, h1);
   ffma2(l0, l1, h0, h1, -1.f, -1.f, a, b);
   lo = pack2<T>(l0, l1);
