@@ -136,7 +136,7 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
   auto item_steps = [&](int w) -> uint32_t {
     if (w >= grid.total) return 0u;
     const Item it = decode(w);
-    const uint32_t v = __ldg(rowrange + it.b * dm.n_rows + it.i);
+    const uint32_t v = uniform(__ldg(rowrange + it.b * dm.n_rows + it.i));
     const int lo = v & 0xffffu, hi = v >> 16;
     if (kKv) return (it.tile >= lo && it.tile < hi) ? (uint32_t)grid.steps << 16 : 0u;
     return (uint32_t)(2 * lo) | (uint32_t)min(2 * hi, grid.steps) << 16;
@@ -144,7 +144,7 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
 
   if (*reinterpret_cast<volatile unsigned int*>(status) != 0u) return;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   if (tid == 0) {
     mbar_init(bar(A_FULL), 1);
     mbar_init(bar(A_EMPTY), 1);
@@ -180,13 +180,13 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform(*tmem_slot);
 
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
     if (warp == 8) {
       // ------------------------------------------------------------ TMA producer
-      if (lane == 0) {
+      {
         int g = 0, it = 0;   // running step and (walked) item counters: barrier phases
         bool ok = true;
         uint32_t next = item_steps(blockIdx.x);
@@ -195,39 +195,45 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
           next = item_steps(w + gridDim.x);
           if (lo >= hi) continue;
           const Item im = decode(w);
-          if (it > 0) ok = mbar_wait_spin(bar(A_EMPTY), (it - 1) & 1, abort_flag);
+          if (it > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(A_EMPTY), (it - 1) & 1, abort_flag));
           if (!ok) break;
           ++it;
-          mbar_arrive_expect_tx(bar(A_FULL), 2 * kResBytes);
-#pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {
-            tma_load_5d(a1_tile + hf * kResHalf, &map_a1, bar(A_FULL), hf * 64, im.tile * 128, im.i, im.h, im.b);
-            tma_load_5d(a2_tile + hf * kResHalf, &map_a2, bar(A_FULL), hf * 64, im.tile * 128, im.i, im.h, im.b);
-          }
-          for (int st = lo; st < hi; ++st, ++g) {
-            const int s = g % kStages;
-            if (g >= kStages) ok = mbar_wait_spin(bar(EMPTY + s), (g / kStages - 1) & 1, abort_flag);
-            if (!ok) break;
-            const uint32_t full = bar(FULL + s);
-            mbar_arrive_expect_tx(full, kStageBytes + (kKv ? 2 * kVecBytes : 0));
+          if (elect_one()) {
+            mbar_arrive_expect_tx(bar(A_FULL), 2 * kResBytes);
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
-              tma_load_5d(b1_tile(s) + hf * kStrHalf, &map_b1, full, hf * 64, st * kStep, im.i, im.h, im.b);
-              tma_load_5d(b2_tile(s) + hf * kStrHalf, &map_b2, full, hf * 64, st * kStep, im.i, im.h, im.b);
+              tma_load_5d(a1_tile + hf * kResHalf, &map_a1, bar(A_FULL), hf * 64, im.tile * 128, im.i, im.h, im.b);
+              tma_load_5d(a2_tile + hf * kResHalf, &map_a2, bar(A_FULL), hf * 64, im.tile * 128, im.i, im.h, im.b);
             }
-            // (keys innermost in both cases)
-            tma_load_4d(base + bias_off(s), &map_bias, full, kKv ? im.tile * 128 : st * kStep,
-                        kKv ? st * kStep : im.tile * 128, im.h, im.b);
-            if (kKv) {
-              tma_load_4d(base + vec_off(s), &map_nlse, full, st * kStep, im.i, im.h, im.b);
-              tma_load_4d(base + vec_off(s) + kVecBytes, &map_delta, full, st * kStep, im.i, im.h, im.b);
+          }
+          __syncwarp();
+          for (int st = lo; st < hi; ++st, ++g) {
+            const int s = g % kStages;
+            if (g >= kStages)
+              ok = __all_sync(0xffffffffu, mbar_wait(bar(EMPTY + s), (g / kStages - 1) & 1, abort_flag));
+            if (!ok) break;
+            const uint32_t full = bar(FULL + s);
+            if (elect_one()) {
+              mbar_arrive_expect_tx(full, kStageBytes + (kKv ? 2 * kVecBytes : 0));
+#pragma unroll
+              for (int hf = 0; hf < 2; ++hf) {
+                tma_load_5d(b1_tile(s) + hf * kStrHalf, &map_b1, full, hf * 64, st * kStep, im.i, im.h, im.b);
+                tma_load_5d(b2_tile(s) + hf * kStrHalf, &map_b2, full, hf * 64, st * kStep, im.i, im.h, im.b);
+              }
+              // (keys innermost in both cases)
+              tma_load_4d(base + bias_off(s), &map_bias, full, kKv ? im.tile * 128 : st * kStep,
+                          kKv ? st * kStep : im.tile * 128, im.h, im.b);
+              if (kKv) {
+                tma_load_4d(base + vec_off(s), &map_nlse, full, st * kStep, im.i, im.h, im.b);
+                tma_load_4d(base + vec_off(s) + kVecBytes, &map_delta, full, st * kStep, im.i, im.h, im.b);
+              }
             }
+            __syncwarp();
           }
         }
       }
     } else if (warp == 9) {
       // ------------------------------------------------------------ S / dP issuer
-      const bool leader = lane == 0;
       constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
       constexpr uint32_t idesc = make_idesc(128, kStep, kBf16, false, false);
       int g = 0, it = 0;
@@ -239,9 +245,9 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
         if (lo >= hi) continue;
         for (int st = lo; st < hi; ++st, ++g) {
           const int s = g % kStages, gp = g - SB;   // the buffer was last read at step g - SB
-          ok = (st > lo || mbar_wait_spin(bar(A_FULL), it & 1, abort_flag)) &&
-               mbar_wait_spin2(bar(FULL + s), (g / kStages) & 1, gp >= 0, bar(S_FREE + (gp & 1)),
-                               (gp >> 1) & 1, abort_flag);
+          ok = (st > lo || mbar_wait(bar(A_FULL), it & 1, abort_flag)) &&
+               mbar_wait(bar(FULL + s), (g / kStages) & 1, abort_flag) &&
+               (gp < 0 || mbar_wait(bar(S_FREE + (gp & 1)), (gp >> 1) & 1, abort_flag));
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           tc_fence_after();
@@ -250,7 +256,7 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
           const uint64_t d2 = make_smem_desc(a2_tile, 16, 1024, kSwizzle128);
           const uint64_t e1 = make_smem_desc(b1_tile(s), 16, 1024, kSwizzle128);
           const uint64_t e2 = make_smem_desc(b2_tile(s), 16, 1024, kSwizzle128);
-          if (leader) {
+          if (elect_one()) {
             // K slice kk: 32 bytes further along the row, the upper four in the second half
 #pragma unroll
             for (int kk = 0; kk < kD / 16; ++kk)
@@ -269,7 +275,6 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
       }
     } else if (warp == 10) {
       // ------------------------------------------------------------ accumulating issuer
-      const bool leader = lane == 0;
       constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
       constexpr uint32_t idesc = make_idesc(128, kD, kBf16, false, true);
       int g = 0, it = 0;
@@ -283,15 +288,15 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
           const int s = g % kStages;
           // an item's first MMAs overwrite the accumulators: the previous item's epilogue must
           // have read them
-          ok = mbar_wait_spin2(bar(P_READY + (g & 1)), (g >> 1) & 1, st == lo && it > 0, bar(ACC_FREE),
-                               (it - 1) & 1, abort_flag);
+          ok = mbar_wait(bar(P_READY + (g & 1)), (g >> 1) & 1, abort_flag) &&
+               (st > lo || it == 0 || mbar_wait(bar(ACC_FREE), (it - 1) & 1, abort_flag));
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           tc_fence_after();
           // 16 rows of a streamed tile are 2 KiB; its two halves are the two N atoms
           const uint64_t e1 = make_smem_desc(b1_tile(s), kStrHalf, 1024, kSwizzle128);
           const uint64_t e2 = make_smem_desc(b2_tile(s), kStrHalf, 1024, kSwizzle128);
-          if (leader) {
+          if (elect_one()) {
             if (kKv) {
 #pragma unroll
               for (int ks = 0; ks < kStep / 16; ++ks)
@@ -324,7 +329,7 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
     const uint32_t tDS = tmem_base + lane_base + kDsCol + half * 16;
     const uint32_t tP = tmem_base + lane_base + kPCol + half * 16;
     const float c1 = dm.scale * kLog2e;
-    const float uniform = kUpP / (float)n;
+    const float p_full = kUpP / (float)n;
 
     int g = 0;
     bool ok = true;
@@ -370,8 +375,8 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
           const uint32_t mw = mw_next;   // dq: this warp's 32 keys, fetched one step ahead
           if (!kKv && st + 1 < hi) mw_next = __ldg(mrow + (st + 1) * 2 + half);
           ok = __all_sync(0xffffffffu,
-                          mbar_wait_spin2(bar(S_FULL + (g & 1)), (g >> 1) & 1, true, bar(FULL + s),
-                                          (g / kStages) & 1, abort_flag));
+                          mbar_wait(bar(S_FULL + (g & 1)), (g >> 1) & 1, abort_flag) &&
+                              mbar_wait(bar(FULL + s), (g / kStages) & 1, abort_flag));
           if (!ok) break;
           tc_fence_after();
           float x[32], gd[32];
@@ -419,7 +424,7 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
 #pragma unroll
             for (int e = 0; e < 8; e += 2) {   // packed fp32 pairs: two scores per instruction
               const int col = q8 * 8 + e;
-              float p0 = uniform, p1 = uniform;
+              float p0 = p_full, p1 = p_full;
               if (!kRowFull) {
                 float t0, t1, a0, a1;
                 if (kKv && kUp) fadd2(nl[e], nl[e + 1], nl[e], nl[e + 1], kUpLog2, kUpLog2);
@@ -451,7 +456,7 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
           if (lane == 0) mbar_arrive(bar(EMPTY + s));   // bias and vectors consumed by this warp
 
           if (g >= 1) {   // the previous step's accumulating MMAs still read P, dS
-            ok = __all_sync(0xffffffffu, mbar_wait_spin(bar(ACC_DONE + ((g - 1) & 1)),
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(ACC_DONE + ((g - 1) & 1)),
                                                         ((g - 1) >> 1) & 1, abort_flag));
             if (!ok) break;
           }
@@ -471,7 +476,7 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
       if (!ok) break;
 
       // epilogue: dk/dv: half 0 takes dK, half 1 dV; dq: 64 columns each
-      ok = __all_sync(0xffffffffu, mbar_wait_spin(bar(ACC_DONE + ((g - 1) & 1)), ((g - 1) >> 1) & 1,
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(ACC_DONE + ((g - 1) & 1)), ((g - 1) >> 1) & 1,
                                                   abort_flag));
       if (!ok) break;
       tc_fence_after();

@@ -120,7 +120,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
   if (!kCluster && *reinterpret_cast<volatile unsigned int*>(status) != 0u) return;
   volatile int* skip = reinterpret_cast<volatile int*>(gbase + 264);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
   const int tiles_k = (n + 127) / 128;
   const int tiles = tiles_k * tiles_k;
   // Rows of a split: a contiguous block, the same partition for every tile.
@@ -193,7 +193,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform(*tmem_slot);
   const bool skipped = kCluster && *skip != 0;
 
   if (warp >= kTmaWarp) {
@@ -206,7 +206,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
       int g = 0;
       bool ok = !skipped;
       for (int r0 = 0; r0 < im.nrows && ok; r0 += 32) {
-        for (uint32_t bits = live[r0 >> 5]; bits != 0u && ok; bits &= bits - 1u) {
+        for (uint32_t bits = uniform(live[r0 >> 5]); bits != 0u && ok; bits &= bits - 1u) {
           const int i = im.i_begin + r0 + __ffs(bits) - 1;
           const int64_t row = (int64_t)im.b * dm.n_rows + i;
           uint32_t word = 0u;
@@ -218,7 +218,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
             if (!ok) break;
             if (c == Cfg::KS - 1 && lane < 5) info[s * 8 + lane] = word;
             __syncwarp();
-            if (lane == 0) {
+            if (elect_one()) {
               const int c0 = c * Cfg::DS;
               mbar_arrive_expect_tx(bar(FULL + s), Cfg::kStageBytes);
               tma_load_5d(q_tile(s), &map_q, bar(FULL + s), c0, im.jt * 128, i, im.h, im.b);
@@ -234,7 +234,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
       }
     } else if (warp == kMmaWarp) {
       // ---------------------------------------------------------- MMA issuer
-      if (lane == 0) {
+      {
         constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
         constexpr uint32_t idesc = make_idesc(128, 128, kBf16, false, false);
         bool ok = !skipped;
@@ -242,28 +242,29 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
           const int nrows = decode(blockIdx.x).nrows;
           int g = 0;
           for (int r0 = 0; r0 < nrows && ok; r0 += 32) {
-          for (uint32_t bits = live[r0 >> 5]; bits != 0u && ok; bits &= bits - 1u) {
+          for (uint32_t bits = uniform(live[r0 >> 5]); bits != 0u && ok; bits &= bits - 1u) {
             const int u = g & 1;
             if (g >= 2) ok = mbar_wait(bar(S_FREE + u), ((g >> 1) - 1) & 1, abort_flag);
-            for (int c = 0; c < Cfg::KS && ok; ++c) {
+            for (int c = 0; c < Cfg::KS; ++c) {
               const int sg = g * Cfg::KS + c, s = sg % NS;
-              ok = mbar_wait(bar(FULL + s), (sg / NS) & 1, abort_flag);
+              ok = __all_sync(0xffffffffu, ok && mbar_wait(bar(FULL + s), (sg / NS) & 1, abort_flag));
               if (!ok) break;
               tc_fence_after();
+              const uint64_t aq = make_smem_desc(q_tile(s), 16, Cfg::kSbo, Cfg::kSwz);
+              const uint64_t bk = make_smem_desc(k_tile(s), 16, Cfg::kSbo, Cfg::kSwz);
+              const uint64_t ag = make_smem_desc(do_tile(s), 16, Cfg::kSbo, Cfg::kSwz);
+              const uint64_t bv = make_smem_desc(v_tile(s), 16, Cfg::kSbo, Cfg::kSwz);
+              if (elect_one()) {   // (a K slice of 16 elements is 32 bytes further along the row)
 #pragma unroll
-              for (int kk = 0; kk < Cfg::DS / 16; ++kk) {
-                const uint64_t aq = make_smem_desc(q_tile(s) + kk * 32, 16, Cfg::kSbo, Cfg::kSwz);
-                const uint64_t bk = make_smem_desc(k_tile(s) + kk * 32, 16, Cfg::kSbo, Cfg::kSwz);
-                umma_ss(tmem_base + u * 256, aq, bk, idesc, c > 0 || kk > 0);
-              }
+                for (int kk = 0; kk < Cfg::DS / 16; ++kk)
+                  umma_ss(tmem_base + u * 256, aq + 2 * kk, bk + 2 * kk, idesc, c > 0 || kk > 0);
 #pragma unroll
-              for (int kk = 0; kk < Cfg::DS / 16; ++kk) {
-                const uint64_t ag = make_smem_desc(do_tile(s) + kk * 32, 16, Cfg::kSbo, Cfg::kSwz);
-                const uint64_t bv = make_smem_desc(v_tile(s) + kk * 32, 16, Cfg::kSbo, Cfg::kSwz);
-                umma_ss(tmem_base + u * 256 + 128, ag, bv, idesc, c > 0 || kk > 0);
+                for (int kk = 0; kk < Cfg::DS / 16; ++kk)
+                  umma_ss(tmem_base + u * 256 + 128, ag + 2 * kk, bv + 2 * kk, idesc, c > 0 || kk > 0);
+                if (c == Cfg::KS - 1) umma_commit(bar(S_FULL + u));
+                umma_commit(bar(EMPTY + s));
               }
-              if (c == Cfg::KS - 1) umma_commit(bar(S_FULL + u));
-              umma_commit(bar(EMPTY + s));
+              __syncwarp();
             }
             if (!ok) break;
             ++g;
@@ -278,7 +279,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
     const int quarter = warp >> 2, wq = warp & 3, row = tid & 127;
     const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
     const float c1 = dm.scale * kLog2e;
-    const float uniform = 1.f / (float)n;
+    const float p_full = 1.f / (float)n;
 
     bool ok = !skipped;
     {
@@ -323,7 +324,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
       int g = 0;
       bool there = false;   // the next row's barriers, tested while this one's sums are made
       for (int r0 = 0; r0 < im.nrows && ok; r0 += 32) {
-      for (uint32_t bits = live[r0 >> 5]; bits != 0u; bits &= bits - 1u) {
+      for (uint32_t bits = uniform(live[r0 >> 5]); bits != 0u; bits &= bits - 1u) {
         // (with KS stages per row the vectors are read from the last one; the earlier ones are
         // released as they come, untouched)
         const int sg = g * Cfg::KS + Cfg::KS - 1;
@@ -369,7 +370,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
           if (row_full) {
 #pragma unroll
             for (int c = 0; c < 16; ++c) {
-              const float p = ((mh >> c) & 1u) ? 0.f : uniform;
+              const float p = ((mh >> c) & 1u) ? 0.f : p_full;
               acc[hc * 16 + c] = fmaf(p, gd[c] - dl, acc[hc * 16 + c]);
             }
           } else if (mh == 0u) {  // no dropped key: a straight block the compiler can overlap

@@ -21,8 +21,7 @@
 //
 // Warps 0-7: elementwise (thread = key; warps w and w + 4 share the TMEM lanes and
 // take 32 of the step's 64 queries each); warp 8 TMA producer; warp 9 issues the S / dP MMAs (and owns the TMEM allocation), warp 10 the dV / dK
-// MMAs, warp 11 the dQ MMAs: one thread can issue an MMA only every ~60 cycles
-// whatever its size, and no kind queues behind a wait of another.  TMEM columns: S^T [0,64), dP^T [64,128), P^T [128,160),
+// MMAs, warp 11 the dQ MMAs : no kind queues behind a wait of another.  TMEM columns: S^T [0,64), dP^T [64,128), P^T [128,160),
 // dS^T [160,192) (16-bit pairs), dK [192,192+D), dV [192+D,192+2D), dQ from 192+2D,
 // D columns per 128-query tile: a row fits when ceil(n/128) * D <= 320 - 2D
 // (d = 32: n <= 1024; d = 64: n <= 384).  A longer row is walked in query chunks of as
@@ -155,12 +154,12 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
   auto item_range = [&](int w) -> uint32_t {
     if (rowrange == nullptr || w >= grid.total) return (uint32_t)nkt << 16;
     const Item it = decode(w);
-    return __ldg(rowrange + it.b * dm.n_rows + it.i);
+    return uniform(__ldg(rowrange + it.b * dm.n_rows + it.i));
   };
 
   if (*reinterpret_cast<volatile unsigned int*>(status) != 0u) return;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
 
   if (tid == 0) {
     for (int u = 0; u < 2; ++u) {
@@ -196,7 +195,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform(*tmem_slot);
 
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
@@ -204,7 +203,6 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
       // ------------------------------------------------------------ TMA producer
       // (Every lane of an issuing warp runs the loop, so that addresses, coordinates
       // and descriptors are warp-uniform values; one lane issues.)
-      const bool leader = lane == 0;
       int g = 0, ktg = 0;  // running step and key-tile counters (barrier phases)
       bool ok = true;
       uint32_t rng_next = item_range(blockIdx.x);
@@ -218,9 +216,9 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
           const int kvb = ktg & 1;
           if (ktg >= 2)
             ok = __all_sync(0xffffffffu,
-                            mbar_wait_spin(bar(KV_EMPTY + kvb), ((ktg >> 1) - 1) & 1, abort_flag));
+                            mbar_wait(bar(KV_EMPTY + kvb), ((ktg >> 1) - 1) & 1, abort_flag));
           if (!ok) break;
-          if (leader) {
+          if (elect_one()) {
             mbar_arrive_expect_tx(bar(KV_FULL + kvb), 2 * Cfg::kKVBytes);
             tma_load_5d(k_tile(kvb), &map_k, bar(KV_FULL + kvb), 0, kt * kBKeys, im.i, im.h, im.b);
             tma_load_5d(v_tile(kvb), &map_v, bar(KV_FULL + kvb), 0, kt * kBKeys, im.i, im.h, im.b);
@@ -229,9 +227,9 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             const int s = g % NS;
             if (g >= NS)
               ok = __all_sync(0xffffffffu,
-                              mbar_wait_spin(bar(EMPTY + s), ((g / NS) - 1) & 1, abort_flag));
+                              mbar_wait(bar(EMPTY + s), ((g / NS) - 1) & 1, abort_flag));
             if (!ok) break;
-            if (leader) {
+            if (elect_one()) {
               mbar_arrive_expect_tx(bar(FULL + s),
                                     2 * Cfg::kQBytes + Cfg::kBiasBytes + 2 * Cfg::kVecBytes);
               tma_load_5d(q_tile(s), &map_q, bar(FULL + s), 0, js * kBJ, im.i, im.h, im.b);
@@ -247,7 +245,6 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
       }
     } else if (warp == 9) {
       // ------------------------------------------------------------ S^T / dP^T issuer
-      const bool leader = lane == 0;
       constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
       constexpr uint32_t idesc_s = make_idesc(128, kBJ, kBf16, false, false);
       int g = 0, ktg = 0;
@@ -264,9 +261,9 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             const int s = g % NS;
             // the S / dP buffer of this step was last read at step g - SB
             const int gp = g - SB;
-            ok = (js > js0 || mbar_wait_spin(bar(KV_FULL + kvb), (ktg >> 1) & 1, abort_flag)) &&
-                 mbar_wait_spin2(bar(FULL + s), (g / NS) & 1, gp >= 0, bar(S_FREE + (gp & 1)),
-                                 (gp >> 1) & 1, abort_flag);
+            ok = (js > js0 || mbar_wait(bar(KV_FULL + kvb), (ktg >> 1) & 1, abort_flag)) &&
+                 mbar_wait(bar(FULL + s), (g / NS) & 1, abort_flag) &&
+                 (gp < 0 || mbar_wait(bar(S_FREE + (gp & 1)), (gp >> 1) & 1, abort_flag));
             const uint32_t t_s = tmem_base + (g % SB) * 128;
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
@@ -275,7 +272,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             const uint64_t bq = make_smem_desc(q_tile(s), 16, Cfg::kSbo, Cfg::kSwz);
             const uint64_t av = make_smem_desc(v_tile(kvb), 16, Cfg::kSbo, Cfg::kSwz);
             const uint64_t bg = make_smem_desc(do_tile(s), 16, Cfg::kSbo, Cfg::kSwz);
-            if (leader) {
+            if (elect_one()) {
               // a K slice of 16 elements is 32 bytes further along the row: + 2 in the
               // descriptor's address field (16-byte units)
 #pragma unroll
@@ -293,7 +290,6 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
       }
     } else if (warp == 10) {
       // ------------------------------------------------------------ dV / dK issuer
-      const bool leader = lane == 0;
       constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
       constexpr uint32_t idesc_acc = make_idesc(128, D, kBf16, false, true);
       // 16 rows of an MN-major tile are this many 16-byte units further on
@@ -310,18 +306,17 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
           for (int js = js0; js < js1; ++js, ++g) {
             const int s = g % NS;
             // the first accumulating MMAs of a key tile overwrite dK, dV: the epilogue
-            // of the previous key tile must have read them (tested together with
-            // P_READY: each test costs a shared-memory round trip)
+            // of the previous key tile must have read them
             const bool first = js == js0 && ktg > 0;
-            ok = mbar_wait_spin2(bar(P_READY + (g & 1)), (g >> 1) & 1, first, bar(ACC_FREE),
-                                 (ktg - 1) & 1, abort_flag);
+            ok = mbar_wait(bar(P_READY + (g & 1)), (g >> 1) & 1, abort_flag) &&
+                 (!first || mbar_wait(bar(ACC_FREE), (ktg - 1) & 1, abort_flag));
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
             const uint32_t acc = (js > js0) ? 1u : 0u;
             const uint64_t b_do = make_smem_desc(do_tile(s), Cfg::kSbo, Cfg::kSbo, Cfg::kSwz);
             const uint64_t b_q = make_smem_desc(q_tile(s), Cfg::kSbo, Cfg::kSbo, Cfg::kSwz);
-            if (leader) {
+            if (elect_one()) {
 #pragma unroll
               for (int ks = 0; ks < kBJ / 16; ++ks) {  // dV += P^T dO, dK += dS^T Q, interleaved
                 umma_ts(tmem_base + Cfg::kDvCol, tmem_base + Cfg::kPCol + ks * 8,
@@ -339,7 +334,6 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
       }
     } else {
       // ------------------------------------------------------------ dQ issuer
-      const bool leader = lane == 0;
       constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
       constexpr uint32_t idesc_dq = make_idesc(128, D, kBf16, true, true);
       constexpr uint32_t kStep16Rows = (16 * Cfg::kRowBytes) >> 4;
@@ -359,8 +353,8 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             // the first dQ MMA of a chunk overwrites dQ: the previous chunk's epilogue must
             // have read it
             const bool first = with_dq && kt == kt_lo && pr == 0 && chg > 0;
-            ok = mbar_wait_spin2(bar(P_READY + (g & 1)), (g >> 1) & 1, first, bar(DQ_FREE),
-                                 (chg - 1) & 1, abort_flag);
+            ok = mbar_wait(bar(P_READY + (g & 1)), (g >> 1) & 1, abort_flag) &&
+                 (!first || mbar_wait(bar(DQ_FREE), (chg - 1) & 1, abort_flag));
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
@@ -368,7 +362,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             // read as an MN-major A operand it is dS (queries x keys)
             const uint64_t a_ds = make_smem_desc(base + pair_off(pb), Cfg::kHalfBytes, 1024, kSwizzle128);
             const uint64_t b_k = make_smem_desc(k_tile(kvb), Cfg::kSbo, Cfg::kSbo, Cfg::kSwz);
-            if (leader) {
+            if (elect_one()) {
               if (with_dq) {
                 // dQ of the 128-query tile js / 2: both halves of its dS tile are written
                 // (an odd last step leaves the second half stale: those queries lie
@@ -401,7 +395,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
       const uint32_t tAcc = tmem_base + lane_base + Cfg::kDkCol + half * Cfg::kAcc;  // dK (half 0) or dV (half 1)
       const uint32_t tDQ = tmem_base + lane_base + Cfg::kDqCol;
       const float c1 = dm.scale * kLog2e;
-      const float uniform = 1.f / (float)n;
+      const float p_full = 1.f / (float)n;
 
       int g = 0, ktg = 0, pgc = 0;
       bool ok = true;
@@ -451,13 +445,10 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
               const int gg = g0 + (js - js0);
               const int s = gg % NS;
               // S^T / dP^T of this step and its bias / lse / delta stage (implied by
-              // S_FULL, whose MMAs read Q from the same stage): tested together, each
-              // test being a shared-memory round trip.  The waits poll instead of
-              // parking: a parked thread resumes hundreds of cycles after the phase
-              // completes.
+              // S_FULL, whose MMAs read Q from the same stage).
               ok = __all_sync(0xffffffffu,
-                              mbar_wait_spin2(bar(S_FULL + (gg & 1)), (gg >> 1) & 1, true,
-                                              bar(FULL + s), (gg / NS) & 1, abort_flag));
+                              mbar_wait(bar(S_FULL + (gg & 1)), (gg >> 1) & 1, abort_flag) &&
+                                  mbar_wait(bar(FULL + s), (gg / NS) & 1, abort_flag));
               if (!ok) break;
               tc_fence_after();
               float x[32], g_[32];
@@ -494,7 +485,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
                     for (int e = 0; e < 8; ++e) p[e] = 0.f;
                   } else if (kMode == 3) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) p[e] = uniform;
+                    for (int e = 0; e < 8; ++e) p[e] = p_full;
                   } else {
                     const uint4 u = *reinterpret_cast<const uint4*>(brow + chunk);
                     const float4 la = lse4[q8 * 2];
@@ -538,7 +529,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
               if (lane == 0) mbar_arrive(bar(EMPTY + s));  // bias^T, lse, delta consumed by this warp
 
               if (gg >= 1) {  // the accumulating MMAs of the previous step still read P^T, dS^T
-                ok = __all_sync(0xffffffffu, mbar_wait_spin(bar(ACC_DONE + ((gg - 1) & 1)),
+                ok = __all_sync(0xffffffffu, mbar_wait(bar(ACC_DONE + ((gg - 1) & 1)),
                                                             ((gg - 1) >> 1) & 1, abort_flag));
                 if (!ok) break;
               }
@@ -564,7 +555,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
           // dK (warps 0-3) and dV (warps 4-7) of this key tile
           {
             const int g_last = g - 1;
-            ok = __all_sync(0xffffffffu, mbar_wait_spin(bar(ACC_DONE + (g_last & 1)), (g_last >> 1) & 1,
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(ACC_DONE + (g_last & 1)), (g_last >> 1) & 1,
                                                         abort_flag));
             if (!ok) break;
             tc_fence_after();

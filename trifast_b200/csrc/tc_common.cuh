@@ -17,6 +17,19 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
+// A value that all lanes of a converged warp hold.
+template <typename V> __device__ __forceinline__ V uniform(V v) { return __shfl_sync(0xffffffffu, v, 0); }
+// True in one lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(one));
+  return one != 0;
+}
+
 // ------------------------------------------------------------------ mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
@@ -43,9 +56,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Non-blocking test of a phase: returns at once.  Used first in every wait, because
-// the potentially-blocking try_wait costs well over a hundred cycles even when
-// the phase has already completed.
+// Non-blocking test of a phase: returns at once.
 __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
@@ -58,36 +69,26 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Same test, but the hardware may park the thread for up to `hint_ns` while the
-// phase is incomplete, instead of returning at once: a waiting warp then issues
-// next to nothing and leaves the scheduler to the warps that have work.
-__device__ __forceinline__ bool mbar_try_wait_parked(uint32_t bar, uint32_t parity,
-                                                     uint32_t hint_ns) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity), "r"(hint_ns)
-      : "memory");
-  return ok != 0;
-}
-
 // Every wait in these kernels is bounded: after kWaitCycles without the phase
 // completing (or as soon as another thread of the CTA has given up) the wait
 // returns false, the caller stops issuing work and the kernel drains and exits
 // with a status bit set; nothing traps and nothing spins forever.
+//
+// The wait is the plain try_wait, for which the hardware holds the warp until the phase completes
+// or a time of its own has passed.  From an arrive to the waiter's next instruction it measures
+// 83 cycles (95 beside 16 warps of arithmetic), a loop of non-blocking tests 138 (166), and
+// a test followed by a try_wait with a time hint 126 (145); and a warp that waits so issues
+// nothing.
 constexpr long long kWaitCycles = 2000000000LL;  // about one second
-constexpr uint32_t kParkNs = 20000;              // re-check abort flag and clock every 20 us
 
 // The wait itself, with the limit as an argument (clock cycles).
 __device__ __forceinline__ bool mbar_wait_limit(uint32_t bar, uint32_t parity,
                                                 volatile int* abort_flag, long long limit_cycles) {
-  if (mbar_test_wait(bar, parity)) return true;
+  if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
+#pragma unroll 1
   while (true) {
-    if (mbar_try_wait_parked(bar, parity, kParkNs)) return true;
+    if (mbar_try_wait(bar, parity)) return true;
     if (*abort_flag) return false;
     if (clock64() - t0 > limit_cycles) {
       *abort_flag = 1;
@@ -98,50 +99,6 @@ __device__ __forceinline__ bool mbar_wait_limit(uint32_t bar, uint32_t parity,
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   return mbar_wait_limit(bar, parity, abort_flag, kWaitCycles);
-}
-
-// The same bounded wait for the warps that issue MMAs and TMA loads: it polls with
-// the non-blocking test instead of parking the thread, because a parked thread is
-// resumed some hundreds of cycles after the phase completes and every such delay
-// sits on the critical path between a tile being ready and its MMAs being issued.
-__device__ __forceinline__ bool mbar_wait_spin(uint32_t bar, uint32_t parity,
-                                               volatile int* abort_flag) {
-  if (mbar_test_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (true) {
-#pragma unroll 1
-    for (int i = 0; i < 64; ++i)
-      if (mbar_test_wait(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if (clock64() - t0 > kWaitCycles) {
-      *abort_flag = 1;
-      return false;
-    }
-  }
-}
-
-// Two barriers at once (the second only when `with_b`): both tests are issued before
-// either result is looked at, so their shared-memory round trips overlap.
-__device__ __forceinline__ bool mbar_wait_spin2(uint32_t bar_a, uint32_t parity_a, bool with_b,
-                                                uint32_t bar_b, uint32_t parity_b,
-                                                volatile int* abort_flag) {
-  bool a = mbar_test_wait(bar_a, parity_a);
-  bool b = !with_b || mbar_test_wait(bar_b, parity_b);
-  if (a && b) return true;
-  const long long t0 = clock64();
-  while (true) {
-#pragma unroll 1
-    for (int i = 0; i < 64; ++i) {
-      if (!a) a = mbar_test_wait(bar_a, parity_a);
-      if (!b) b = mbar_test_wait(bar_b, parity_b);
-      if (a && b) return true;
-    }
-    if (*abort_flag) return false;
-    if (clock64() - t0 > kWaitCycles) {
-      *abort_flag = 1;
-      return false;
-    }
-  }
 }
 
 // ------------------------------------------------------------------ TMA loads
@@ -190,6 +147,16 @@ __device__ __forceinline__ void tc_fence_after() {
 }
 __device__ __forceinline__ void tmem_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+// The same for a load of 16 registers with other work between it and the wait: the registers pass
+// through it, so that nothing that reads them can be moved before it.
+__device__ __forceinline__ void tmem_wait_ld_regs(uint32_t* a) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]),
+                 "+r"(a[7]), "+r"(a[8]), "+r"(a[9]), "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]),
+                 "+r"(a[14]), "+r"(a[15])
+               :
+               : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -243,11 +210,29 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
       : "memory");
 }
 
-// N consecutive columns (16, or a multiple of 32) of this thread's lane.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]),
+      "r"(r[7])
+      : "memory");
+}
+
+// N consecutive columns (8, 16, or a multiple of 32) of this thread's lane.
 template <int N>
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t* r) {
-  static_assert(N == 16 || N % 32 == 0, "column count");
-  if constexpr (N == 16) {
+  static_assert(N == 8 || N == 16 || N % 32 == 0, "column count");
+  if constexpr (N == 8) {
+    tmem_ld8(taddr, r);
+  } else if constexpr (N == 16) {
     tmem_ld16(taddr, r);
   } else {
 #pragma unroll

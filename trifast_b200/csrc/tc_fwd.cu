@@ -173,7 +173,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       lo = min(lo, v & 0xffffu);
       hi = max(hi, v >> 16);
     }
-    return lo | (hi << 16);
+    return uniform(lo | (hi << 16));
   };
 
   // A wait that gave up in an earlier CTA or launch leaves the status word set:
@@ -183,7 +183,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     return;
   }
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
 
   if (tid == 0) {
     mbar_init(bar(Q_FULL), 1);
@@ -216,13 +216,16 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform(*tmem_slot);
 
   if (warp >= 4 * R) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TRIFAST_REG_DEC));
   if (warp == 4 * R) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    // (The whole warp runs the loops of the producer and the issuers; elect_one() issues, which
+    // tells the compiler that one thread does: under a lane test it wraps every MMA and TMA
+    // load in code for several, 130 cycles an MMA instead of 50.)
+    {
       int g = 0, it = 0;  // running key-tile and item counters (barrier phases)
       bool ok = true;
       uint32_t rng_next = item_range(blockIdx.x);
@@ -231,42 +234,53 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         const uint32_t rng = rng_next;
         const int kt_lo = rng & 0xffffu, kt_hi = rng >> 16;
         rng_next = item_range(w + gridDim.x);
-        if (it > 0) ok = mbar_wait(bar(Q_EMPTY), (it - 1) & 1, abort_flag);
+        if (it > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(Q_EMPTY), (it - 1) & 1, abort_flag));
         if (!ok) break;
-        rng_word[it & 1] = rng;
-        mbar_arrive_expect_tx(bar(Q_FULL), R * Cfg::kTileBytes);
-        for (int r = 0; r < R; ++r)
-          tma_load_5d(q_tile(r), &map_q, bar(Q_FULL), 0, im.jt * kBJ, slot_row(im, r), im.h, im.b);
+        if (elect_one()) {
+          rng_word[it & 1] = rng;
+          mbar_arrive_expect_tx(bar(Q_FULL), R * Cfg::kTileBytes);
+          for (int r = 0; r < R; ++r)
+            tma_load_5d(q_tile(r), &map_q, bar(Q_FULL), 0, im.jt * kBJ, slot_row(im, r), im.h, im.b);
+        }
+        __syncwarp();
         for (int kt = kt_lo; kt < kt_hi; ++kt, ++g) {
           const int s = g % NS;
-          if (g >= NS) ok = mbar_wait(bar(EMPTY + s), ((g / NS) - 1) & 1, abort_flag);
+          if (g >= NS)
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(EMPTY + s), ((g / NS) - 1) & 1, abort_flag));
           if (!ok) break;
-          mbar_arrive_expect_tx(bar(FULL + s), R * 2 * Cfg::kTileBytes + Cfg::kBiasBytes);
-          for (int r = 0; r < R; ++r) {
-            tma_load_5d(k_tile(s, r), &map_k, bar(FULL + s), 0, kt * kBK, slot_row(im, r), im.h, im.b);
-            tma_load_5d(v_tile(s, r), &map_v, bar(FULL + s), 0, kt * kBK, slot_row(im, r), im.h, im.b);
+          if (elect_one()) {
+            mbar_arrive_expect_tx(bar(FULL + s), R * 2 * Cfg::kTileBytes + Cfg::kBiasBytes);
+            for (int r = 0; r < R; ++r) {
+              tma_load_5d(k_tile(s, r), &map_k, bar(FULL + s), 0, kt * kBK, slot_row(im, r), im.h, im.b);
+              tma_load_5d(v_tile(s, r), &map_v, bar(FULL + s), 0, kt * kBK, slot_row(im, r), im.h, im.b);
+            }
+            const uint32_t bias_s = base + bias_off(s);
+            tma_load_4d(bias_s, &map_b, bar(FULL + s), kt * kBK, im.jt * kBJ, im.h, im.b);
+            tma_load_4d(bias_s + 16384, &map_b, bar(FULL + s), kt * kBK + 64, im.jt * kBJ, im.h, im.b);
           }
-          const uint32_t bias_s = base + bias_off(s);
-          tma_load_4d(bias_s, &map_b, bar(FULL + s), kt * kBK, im.jt * kBJ, im.h, im.b);
-          tma_load_4d(bias_s + 16384, &map_b, bar(FULL + s), kt * kBK + 64, im.jt * kBJ, im.h, im.b);
+          __syncwarp();
         }
       }
     }
   } else if (warp - (4 * R + 1) < R) {
     // ------------------------------------------------------------ MMA issuers (one per slot)
     const int r = warp - (4 * R + 1);
-    if (lane == 0) {
+    {
       constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
       constexpr uint32_t idesc_qk = make_idesc(128, 128, kBf16, false, false);
       constexpr uint32_t idesc_pv = make_idesc(128, D, kBf16, false, true);
-      auto issue_qk = [&](int s) {
+      auto issue_qk = [&](int s, bool last_q) {
+        const uint64_t ad = make_smem_desc(q_tile(r), 16, Cfg::kSbo, Cfg::kSwz);
+        const uint64_t bd = make_smem_desc(k_tile(s, r), 16, Cfg::kSbo, Cfg::kSwz);
+        if (elect_one()) {
+          // (a K slice of 16 elements is 32 bytes further along the row)
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          const uint64_t ad = make_smem_desc(q_tile(r) + kk * 32, 16, Cfg::kSbo, Cfg::kSwz);
-          const uint64_t bd = make_smem_desc(k_tile(s, r) + kk * 32, 16, Cfg::kSbo, Cfg::kSwz);
-          umma_ss(tmem_base + r * 256, ad, bd, idesc_qk, kk > 0);
+          for (int kk = 0; kk < D / 16; ++kk)
+            umma_ss(tmem_base + r * 256, ad + 2 * kk, bd + 2 * kk, idesc_qk, kk > 0);
+          umma_commit(bar(S_FULL + r));
+          if (last_q) umma_commit(bar(Q_EMPTY));   // last read of this item's Q tile
         }
-        umma_commit(bar(S_FULL + r));
+        __syncwarp();
       };
       int g = 0, it = 0;
       bool ok = true;
@@ -276,37 +290,41 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         ok = mbar_wait(bar(Q_FULL), it & 1, abort_flag) &&
              mbar_wait(bar(FULL + g % NS), (g / NS) & 1, abort_flag) &&
              (g == 0 || mbar_wait(bar(S_FREE + r), (g - 1) & 1, abort_flag));
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t rng = rng_word[it & 1];
+        const uint32_t rng = uniform(rng_word[it & 1]);
         const int kt_lo = rng & 0xffffu, kt_hi = rng >> 16;
-        issue_qk(g % NS);
-        if (kt_hi - kt_lo == 1) umma_commit(bar(Q_EMPTY));
+        issue_qk(g % NS, kt_hi - kt_lo == 1);
         for (int kt = kt_lo; kt < kt_hi && ok; ++kt, ++g) {
           const int s = g % NS;
           if (kt + 1 < kt_hi) {
             const int ns = (g + 1) % NS;
             ok = mbar_wait(bar(FULL + ns), ((g + 1) / NS) & 1, abort_flag) &&
                  mbar_wait(bar(S_FREE + r), g & 1, abort_flag);
+            ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
-            issue_qk(ns);
-            if (kt + 2 == kt_hi) umma_commit(bar(Q_EMPTY));  // last read of this item's Q tile
+            issue_qk(ns, kt + 2 == kt_hi);
           }
           ok = mbar_wait(bar(P_READY + r), g & 1, abort_flag);
           // the first PV of an item overwrites O: the previous item's epilogue must have read it
           if (ok && kt == kt_lo && it > 0) ok = mbar_wait(bar(O_FREE + r), (it - 1) & 1, abort_flag);
+          ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           tc_fence_after();
+          const uint64_t bd = make_smem_desc(v_tile(s, r), Cfg::kSbo, Cfg::kSbo, Cfg::kSwz);
+          const uint32_t acc = kt > kt_lo ? 1u : 0u;
+          if (elect_one()) {
+            // (16 rows of the MN-major V tile further on, in 16-byte units)
 #pragma unroll
-          for (int ks = 0; ks < kBK / 16; ++ks) {
-            const uint64_t bd = make_smem_desc(v_tile(s, r) + ks * 16 * Cfg::kRowBytes, Cfg::kSbo,
-                                               Cfg::kSbo, Cfg::kSwz);
-            umma_ts(tmem_base + r * 256 + 192, tmem_base + r * 256 + 128 + ks * 8, bd, idesc_pv,
-                    (kt > kt_lo || ks > 0) ? 1u : 0u);
+            for (int ks = 0; ks < kBK / 16; ++ks)
+              umma_ts(tmem_base + r * 256 + 192, tmem_base + r * 256 + 128 + ks * 8,
+                      bd + ks * ((16 * Cfg::kRowBytes) >> 4), idesc_pv, ks > 0 ? 1u : acc);
+            umma_commit(bar(O_DONE + r));
+            umma_commit(bar(EMPTY + s));
           }
-          umma_commit(bar(O_DONE + r));
-          umma_commit(bar(EMPTY + s));
+          __syncwarp();
         }
       }
     }
@@ -402,7 +420,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         if (!ok) break;
         tc_fence_after();
         if (kt_lo < 0) {
-          const uint32_t rng = rng_word[it & 1];
+          const uint32_t rng = uniform(rng_word[it & 1]);
           kt_lo = kt = rng & 0xffffu;
           kt_hi = rng >> 16;
         }

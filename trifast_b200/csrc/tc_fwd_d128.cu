@@ -114,7 +114,7 @@ tc_fwd_d128_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
 
   if (*reinterpret_cast<volatile unsigned int*>(status) != 0u) return;
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
 
   if (tid == 0) {
     mbar_init(bar(Q_FULL), 1);
@@ -147,17 +147,17 @@ tc_fwd_d128_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = uniform(*tmem_slot);
 
   if (warp >= 8) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegDec));
     if (warp == 8) {
       // ---------------------------------------------------------------- TMA producer
-      if (lane == 0) {
+      {
         auto item_range = [&](int w) -> uint32_t {
           if (rowrange == nullptr || w >= items.total) return (uint32_t)nkt << 16;
           const Item it = decode(w);
-          return __ldg(rowrange + it.b * dm.n_rows + it.i);
+          return uniform(__ldg(rowrange + it.b * dm.n_rows + it.i));
         };
         int g = 0, it = 0;   // running key-tile and item counters (barrier phases)
         bool ok = true;
@@ -167,105 +167,122 @@ tc_fwd_d128_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           const uint32_t rng = rng_next;
           const int kt_lo = rng & 0xffffu, kt_hi = rng >> 16;
           rng_next = item_range(w + gridDim.x);
-          if (it > 0) ok = mbar_wait(bar(Q_EMPTY), (it - 1) & 1, abort_flag);
+          if (it > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(Q_EMPTY), (it - 1) & 1, abort_flag));
           if (!ok) break;
-          rng_word[it & 1] = rng;
-          mbar_arrive_expect_tx(bar(Q_FULL), 2 * kTileBytes);
-          for (int r = 0; r < 2; ++r) {
-            const int j0 = slot_tile(im, r) * 128;
-            tma_load_5d(q_tile(r), &map_q, bar(Q_FULL), 0, j0, im.i, im.h, im.b);
-            tma_load_5d(q_tile(r) + kHalfBytes, &map_q, bar(Q_FULL), 64, j0, im.i, im.h, im.b);
+          if (elect_one()) {
+            rng_word[it & 1] = rng;
+            mbar_arrive_expect_tx(bar(Q_FULL), 2 * kTileBytes);
+            for (int r = 0; r < 2; ++r) {
+              const int j0 = slot_tile(im, r) * 128;
+              tma_load_5d(q_tile(r), &map_q, bar(Q_FULL), 0, j0, im.i, im.h, im.b);
+              tma_load_5d(q_tile(r) + kHalfBytes, &map_q, bar(Q_FULL), 64, j0, im.i, im.h, im.b);
+            }
           }
+          __syncwarp();
           for (int kt = kt_lo; kt < kt_hi; ++kt, ++g) {
-            if (g > 0) ok = mbar_wait(bar(K_EMPTY), (g - 1) & 1, abort_flag);
+            if (g > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(K_EMPTY), (g - 1) & 1, abort_flag));
             if (!ok) break;
-            mbar_arrive_expect_tx(bar(K_FULL), kTileBytes);
-            tma_load_5d(k_tile, &map_k, bar(K_FULL), 0, kt * 128, im.i, im.h, im.b);
-            tma_load_5d(k_tile + kHalfBytes, &map_k, bar(K_FULL), 64, kt * 128, im.i, im.h, im.b);
-            for (int r = 0; r < 2 && ok; ++r) {
-              if (g > 0) ok = mbar_wait(bar(B_EMPTY + r), (g - 1) & 1, abort_flag);
+            if (elect_one()) {
+              mbar_arrive_expect_tx(bar(K_FULL), kTileBytes);
+              tma_load_5d(k_tile, &map_k, bar(K_FULL), 0, kt * 128, im.i, im.h, im.b);
+              tma_load_5d(k_tile + kHalfBytes, &map_k, bar(K_FULL), 64, kt * 128, im.i, im.h, im.b);
+            }
+            __syncwarp();
+            for (int r = 0; r < 2; ++r) {
+              if (g > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(B_EMPTY + r), (g - 1) & 1, abort_flag));
               if (!ok) break;
               const uint32_t dst = base + bias_off(r);
               const int j0 = slot_tile(im, r) * 128;
-              mbar_arrive_expect_tx(bar(B_FULL + r), kBiasBytes);
-              tma_load_4d(dst, &map_b, bar(B_FULL + r), kt * 128, j0, im.h, im.b);
-              tma_load_4d(dst + 16384, &map_b, bar(B_FULL + r), kt * 128 + 64, j0, im.h, im.b);
+              if (elect_one()) {
+                mbar_arrive_expect_tx(bar(B_FULL + r), kBiasBytes);
+                tma_load_4d(dst, &map_b, bar(B_FULL + r), kt * 128, j0, im.h, im.b);
+                tma_load_4d(dst + 16384, &map_b, bar(B_FULL + r), kt * 128 + 64, j0, im.h, im.b);
+              }
+              __syncwarp();
             }
             if (!ok) break;
-            if (g > 0) ok = mbar_wait(bar(V_EMPTY), (g - 1) & 1, abort_flag);
+            if (g > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(V_EMPTY), (g - 1) & 1, abort_flag));
             if (!ok) break;
-            mbar_arrive_expect_tx(bar(V_FULL), kTileBytes);
-            tma_load_5d(v_tile, &map_v, bar(V_FULL), 0, kt * 128, im.i, im.h, im.b);
-            tma_load_5d(v_tile + kHalfBytes, &map_v, bar(V_FULL), 64, kt * 128, im.i, im.h, im.b);
+            if (elect_one()) {
+              mbar_arrive_expect_tx(bar(V_FULL), kTileBytes);
+              tma_load_5d(v_tile, &map_v, bar(V_FULL), 0, kt * 128, im.i, im.h, im.b);
+              tma_load_5d(v_tile + kHalfBytes, &map_v, bar(V_FULL), 64, kt * 128, im.i, im.h, im.b);
+            }
+            __syncwarp();
           }
         }
       }
     } else if (warp == 9) {
       // ---------------------------------------------------------------- MMA issuer
-      if (lane == 0) {
+      {
         constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
         constexpr uint32_t idesc_qk = make_idesc(128, 128, kBf16, false, false);
         constexpr uint32_t idesc_pv = make_idesc(128, 128, kBf16, false, true);
         // S_r = Q_r K^T: eight K slices of 16 elements, four in each half of the tiles
-        auto issue_qk = [&](int r) {
+        auto issue_qk = [&](int r, bool last_k, bool last_q) {
+          const uint64_t ad = make_smem_desc(q_tile(r), 16, 1024, kSwizzle128);
+          const uint64_t bd = make_smem_desc(k_tile, 16, 1024, kSwizzle128);
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < 8; ++kk) {
-            const uint32_t off = (kk >> 2) * kHalfBytes + (kk & 3) * 32;
-            const uint64_t ad = make_smem_desc(q_tile(r) + off, 16, 1024, kSwizzle128);
-            const uint64_t bd = make_smem_desc(k_tile + off, 16, 1024, kSwizzle128);
-            umma_ss(tmem_base + r * 256, ad, bd, idesc_qk, kk > 0);
+            for (int kk = 0; kk < 8; ++kk) {
+              const uint32_t off = (kk >> 2) * (kHalfBytes >> 4) + (kk & 3) * 2;
+              umma_ss(tmem_base + r * 256, ad + off, bd + off, idesc_qk, kk > 0);
+            }
+            umma_commit(bar(S_FULL + r));
+            if (last_k) umma_commit(bar(K_EMPTY));
+            if (last_q) umma_commit(bar(Q_EMPTY));   // last read of the item's Q
           }
-          umma_commit(bar(S_FULL + r));
+          __syncwarp();
         };
         // O_r (+)= P_r V: eight slices of 16 keys; V is MN-major, its two 64-element halves
         // are the two N atoms (leading offset 16 KiB), 8-key groups 1 KiB apart
         auto issue_pv = [&](int r, bool first) {
+          const uint64_t bd = make_smem_desc(v_tile, kHalfBytes, 1024, kSwizzle128);
+          const uint32_t acc = first ? 0u : 1u;
+          if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < 8; ++ks) {
-            const uint64_t bd = make_smem_desc(v_tile + ks * 2048, kHalfBytes, 1024, kSwizzle128);
-            umma_ts(tmem_base + r * 256 + 128, tmem_base + r * 256 + ks * 8, bd, idesc_pv,
-                    (!first || ks > 0) ? 1u : 0u);
+            for (int ks = 0; ks < 8; ++ks)
+              umma_ts(tmem_base + r * 256 + 128, tmem_base + r * 256 + ks * 8, bd + ks * (2048 >> 4), idesc_pv,
+                      ks > 0 ? 1u : acc);
+            umma_commit(bar(O_DONE + r));
+            if (r == 1) umma_commit(bar(V_EMPTY));
           }
-          umma_commit(bar(O_DONE + r));
+          __syncwarp();
         };
         int g = 0, it = 0;
         bool ok = true;
         for (int w = blockIdx.x; w < items.total && ok; w += gridDim.x, ++it) {
-          ok = mbar_wait_spin(bar(Q_FULL), it & 1, abort_flag) &&
-               mbar_wait_spin(bar(K_FULL), g & 1, abort_flag);
+          ok = mbar_wait(bar(Q_FULL), it & 1, abort_flag) &&
+               mbar_wait(bar(K_FULL), g & 1, abort_flag);
+          ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           tc_fence_after();
-          const uint32_t rng = rng_word[it & 1];
+          const uint32_t rng = uniform(rng_word[it & 1]);
           const int kt_lo = rng & 0xffffu, kt_hi = rng >> 16;
           // (these S overwrite the S / P columns of the previous item's last tile: its
           // O += P V were issued before them by this thread and so execute before them)
-          issue_qk(0);
-          issue_qk(1);
-          umma_commit(bar(K_EMPTY));
-          if (kt_hi - kt_lo == 1) umma_commit(bar(Q_EMPTY));
+          issue_qk(0, false, false);
+          issue_qk(1, true, kt_hi - kt_lo == 1);
           for (int kt = kt_lo; kt < kt_hi && ok; ++kt, ++g) {
             const bool more = kt + 1 < kt_hi;
             for (int r = 0; r < 2; ++r) {
-              ok = mbar_wait_spin2(bar(P_READY + r), g & 1, r == 0, bar(V_FULL), g & 1, abort_flag);
+              ok = mbar_wait(bar(P_READY + r), g & 1, abort_flag) &&
+                   (r > 0 || mbar_wait(bar(V_FULL), g & 1, abort_flag));
               // the first O += P V of an item overwrites O: the previous item's epilogue must
               // have read it
-              if (ok && kt == kt_lo && it > 0) ok = mbar_wait_spin(bar(O_FREE + r), (it - 1) & 1, abort_flag);
+              if (ok && kt == kt_lo && it > 0) ok = mbar_wait(bar(O_FREE + r), (it - 1) & 1, abort_flag);
+              ok = __all_sync(0xffffffffu, ok);
               if (!ok) break;
               tc_fence_after();
               issue_pv(r, kt == kt_lo);
-              if (r == 1) umma_commit(bar(V_EMPTY));
               if (more) {
                 // the slot's next S goes behind its O += P V (P lies over S)
                 if (r == 0) {
-                  ok = mbar_wait_spin(bar(K_FULL), (g + 1) & 1, abort_flag);
+                  ok = __all_sync(0xffffffffu, mbar_wait(bar(K_FULL), (g + 1) & 1, abort_flag));
                   if (!ok) break;
                   tc_fence_after();
                 }
-                issue_qk(r);
-                if (r == 1) {
-                  umma_commit(bar(K_EMPTY));
-                  if (kt + 2 == kt_hi) umma_commit(bar(Q_EMPTY));   // last read of the item's Q
-                }
+                issue_qk(r, r == 1, r == 1 && kt + 2 == kt_hi);
               }
             }
           }
@@ -301,7 +318,7 @@ tc_fwd_d128_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
           if (!ok) break;
           tc_fence_after();
           if (kt_lo < 0) {
-            const uint32_t rng = rng_word[it & 1];
+            const uint32_t rng = uniform(rng_word[it & 1]);
             kt_lo = kt = rng & 0xffffu;
             kt_hi = rng >> 16;
           }
