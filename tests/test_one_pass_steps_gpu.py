@@ -1,0 +1,50 @@
+"""The one-pass dq / dk / dv kernel where its walk changes: steps per key tile odd and even, one
+step per tile, the row lengths at which a TMEM buffer goes (dQ takes its columns) and at which a
+row is split into query chunks, with several rows per CTA and rows that skip key tiles."""
+
+import pytest
+import torch
+
+from tests.test_backward_gpu import NAMES, _inputs, _run_abi
+from trifast_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [  # n, heads, d, dtype, rows; buffers of dP and of dK, dV, chunks
+    (64, 5, 32, torch.bfloat16, 64),      # one step per key tile
+    (129, 4, 32, torch.float16, 90),      # three steps, the last key tile with one key
+    (256, 2, 32, torch.bfloat16, 160),    # 2, 2
+    (257, 2, 32, torch.bfloat16, 90),     # 2, 1
+    (512, 1, 32, torch.float16, 160),
+    (513, 1, 32, torch.bfloat16, 150),    # 1, 1
+    (768, 1, 16, torch.bfloat16, 20),
+    (769, 1, 32, torch.bfloat16, 150),    # chunks of 4 and 3 query tiles
+    (1100, 1, 32, torch.float16, 12),
+    (128, 4, 64, torch.float16, 90),
+    (257, 1, 64, torch.bfloat16, 150),    # 1, 1
+    (385, 1, 64, torch.bfloat16, 40),     # two chunks of 2
+    (900, 1, 64, torch.float16, 8),       # three chunks, the last one short
+]
+
+
+@pytest.mark.parametrize("n,h,d,dtype,rows", SHAPES)
+def test_every_walk_gives_the_two_kernel_results(n, h, d, dtype, rows):
+    args = _inputs(n, h, d, dtype, "random", rows, seed=n)
+    one = _run_abi(args)
+    for x, y in zip(one, _run_abi(args)):
+        assert torch.equal(x, y)
+    # head dim 16 has no two-kernel backward: the CUDA-core kernels, whose P and dS stay in fp32
+    two = _run_abi(args, kernel=_lib.KERNEL_SIMT) if d == 16 else _run_abi(args, flags=_lib.FLAG_SPLIT_BWD)
+    chunks = _lib.pick_plan(1, h, n, rows, d, dtype)["bwd_chunks"]
+    for name, x, y in zip(NAMES, one, two):
+        x, y = x.float(), y.float()
+        assert not torch.isnan(x).any(), name
+        if d == 16:
+            # P and dS rounded to 8 bits: 2^-9 each, uncorrelated over the sums; four times that
+            assert float((x - y).norm()) <= 4 * 2.0 ** -9 * float(y.norm()), name
+        elif chunks > 1 and name in ("dk", "dv"):
+            # summed per chunk, the fp32 partials added: last places of a few elements
+            assert float((x - y).abs().max()) <= 2.0 ** -7 * float(y.abs().max()), name
+            assert float((x != y).float().mean()) < 0.02, name
+        else:
+            assert torch.equal(x, y), name
