@@ -29,10 +29,66 @@ struct Prep {
   unsigned int* status;
   View5 v;
   float* ds_up;
+  // forward at head dims up to 64: rows without an open key are finished here (o: the mean of
+  // all values, lse: the sentinel) and their range of key tiles is empty
+  View5 o;
+  float* lse;
+  int dtype;
   // block ranges, in this order: one row of the mask each; 64 x 64 bias tiles; one (b, h, i) of
   // ds_up each; the rest delta
   int mask_blocks, bias_tiles, bias_blocks, scale_blocks;
 };
+
+// ---------------------------------------------------------------------------
+// Output of a pair row (b, i) without an open key, all heads: the mean of its n values for every
+// query, which the tensor-core kernel would spend a walk over all keys on.  One block, 16 bytes per
+// thread and load, sums in fp32.
+// ---------------------------------------------------------------------------
+__device__ void fill_masked_row(const Prep& a, int b, int i) {
+  __shared__ float sums[8][kPrepThreads];
+  const int n = a.dm.n, parts = a.dm.d / 8, part = threadIdx.x % parts, first = threadIdx.x / parts;
+  const int rows = kPrepThreads / parts;
+  const bool bf16 = a.dtype == TRIFAST_BF16;
+  for (int h = 0; h < a.dm.heads; ++h) {
+    const uint16_t* v = (const uint16_t*)a.v.p + b * a.v.sb + h * a.v.sh + (int64_t)i * a.v.si + part * 8;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+    for (int k = first; k < n; k += rows) {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(v + (int64_t)k * a.v.sj));
+      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const uint16_t x = (uint16_t)(w[e >> 1] >> (16 * (e & 1)));
+        acc[e] += bf16 ? __uint_as_float((uint32_t)x << 16) : __half2float(__ushort_as_half(x));
+      }
+    }
+    __syncthreads();   // (the previous head's sums have been read)
+#pragma unroll
+    for (int e = 0; e < 8; ++e) sums[e][threadIdx.x] = acc[e];
+    for (int half = kPrepThreads / 2; half >= parts; half >>= 1) {
+      __syncthreads();
+      if (threadIdx.x < half)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) sums[e][threadIdx.x] += sums[e][threadIdx.x + half];
+    }
+    __syncthreads();
+    const float inv = 1.f / (float)n;
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+      const float lo = sums[e][part] * inv, hi = sums[e + 1][part] * inv;
+      w[e >> 1] = bf16 ? (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(lo)) |
+                             (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(hi)) << 16
+                       : (uint32_t)__half_as_ushort(__float2half_rn(lo)) |
+                             (uint32_t)__half_as_ushort(__float2half_rn(hi)) << 16;
+    }
+    uint16_t* o = (uint16_t*)a.o.p + b * a.o.sb + h * a.o.sh + (int64_t)i * a.o.si + part * 8;
+    for (int j = first; j < n; j += rows)
+      *reinterpret_cast<uint4*>(o + (int64_t)j * a.o.sj) = make_uint4(w[0], w[1], w[2], w[3]);
+    float* lse = a.lse + (((int64_t)b * a.dm.heads + h) * a.dm.n_rows + i) * n;
+    for (int j = threadIdx.x; j < n; j += kPrepThreads) lse[j] = a.dm.sentinel;
+  }
+}
 
 // ---------------------------------------------------------------------------
 // One pair row of the mask: rowfull = 1 when every key is masked, the packed key masks, the
@@ -43,19 +99,24 @@ __device__ void prepare_mask_row(const Prep& a, int bi) {
   const int b = bi / n_rows, i = bi % n_rows;
   const uint8_t* row = a.mask.p + b * a.mask.sb + (int64_t)i * a.mask.si;
   const int64_t sk = a.mask.sk;
-  __shared__ int first_open, last_open;
+  __shared__ int first_open, last_open, dropped_any;
   if (threadIdx.x == 0) {
     first_open = n;
     last_open = -1;
+    dropped_any = 0;
   }
   __syncthreads();
   int lo = n, hi = -1;
+  bool dropped = false;
   for (int k = threadIdx.x; k < n; k += kPrepThreads) {
     if (row[k * sk] == 0) {
       lo = min(lo, k);
       hi = max(hi, k);
+    } else {
+      dropped = true;
     }
   }
+  if (dropped) dropped_any = 1;
   if (hi >= 0) {
     atomicMin(&first_open, lo);
     atomicMax(&last_open, hi);
@@ -65,13 +126,15 @@ __device__ void prepare_mask_row(const Prep& a, int bi) {
   if (threadIdx.x == 0) {
     if (a.rowfull) a.rowfull[bi] = open ? 0 : 1;
     // 128-key tiles [first, last + 1) that hold an open key: the tensor-core kernels walk
-    // only those.  A fully masked row weighs all n keys: every tile.
+    // only those.  A fully masked row weighs all n keys: every tile, or none where it is
+    // finished here; there, the top bit says that no key is dropped.
     if (a.rowrange) {
-      const uint32_t t0 = open ? (uint32_t)(first_open >> 7) : 0u;
-      const uint32_t t1 = open ? (uint32_t)(last_open >> 7) + 1u : (uint32_t)((n + 127) >> 7);
-      a.rowrange[bi] = t0 | (t1 << 16);
+      const uint32_t t0 = open ? (uint32_t)(first_open >> 7) : a.lse ? 0xffffu : 0u;
+      const uint32_t t1 = open ? (uint32_t)(last_open >> 7) + 1u : a.lse ? 0u : (uint32_t)((n + 127) >> 7);
+      a.rowrange[bi] = t0 | (t1 << 16) | (a.lse && !dropped_any ? 0x80000000u : 0u);
     }
   }
+  if (!open && a.lse) fill_masked_row(a, b, i);
   if (!a.maskbits) return;
   // Packed key mask (bit set = key dropped or beyond n).  A fully masked row keeps
   // all n keys with uniform weight, so only the keys beyond n stay set.  Layout per
@@ -411,6 +474,12 @@ cudaError_t fwd_prepare(const FwdArgs& a, cudaStream_t s) {
   p.bias_pad = (uint16_t*)a.bias_pad;
   p.status = a.status;
   p.bias_blocks = a.bias_pad ? p.bias_tiles * p.bias_tiles * a.dm.batch * a.dm.heads : 0;
+  if (a.dm.d <= 64) {
+    p.v = a.v;
+    p.o = a.o;
+    p.lse = a.lse;
+    p.dtype = a.dtype;
+  }
   fwd_prepare_kernel<<<p.mask_blocks + p.bias_blocks, kPrepThreads, 0, s>>>(p);
   return cudaGetLastError();
 }

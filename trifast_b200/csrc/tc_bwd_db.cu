@@ -278,7 +278,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
     // ------------------------------------------------------------ elementwise warpgroups
     const int quarter = warp >> 2, wq = warp & 3, row = tid & 127;
     const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
-    const float c1 = dm.scale * kLog2e;
+    const float c1 = in_register(dm.scale * kLog2e), log2e = in_register(kLog2e);
     const float p_full = 1.f / (float)n;
 
     bool ok = !skipped;
@@ -378,7 +378,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
             for (int c = 0; c < 16; c += 2) {  // packed fp32 pairs: two scores per FMA instruction
               float b0, b1, t0, t1, a0, a1, s0, s1;
               unpack2<T>(bp[(hc * 16 + c) >> 1], b0, b1);
-              ffma2(t0, t1, b0, b1, kLog2e, kLog2e, nl, nl);
+              ffma2(t0, t1, b0, b1, log2e, log2e, nl, nl);
               ffma2(a0, a1, x[c], x[c + 1], c1, c1, t0, t1);
               const float p0 = ex2(a0), p1 = ex2(a1);
               fadd2(s0, s1, gd[c], gd[c + 1], ndl, ndl);
@@ -390,7 +390,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
             for (int c = 0; c < 16; c += 2) {
               float b0, b1, t0, t1, a0, a1, s0, s1;
               unpack2<T>(bp[(hc * 16 + c) >> 1], b0, b1);
-              ffma2(t0, t1, b0, b1, kLog2e, kLog2e, nl, nl);
+              ffma2(t0, t1, b0, b1, log2e, log2e, nl, nl);
               ffma2(a0, a1, x[c], x[c + 1], c1, c1, t0, t1);
               float p0 = ex2(a0), p1 = ex2(a1);
               p0 = ((mh >> c) & 1u) ? 0.f : p0;

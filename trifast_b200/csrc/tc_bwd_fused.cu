@@ -586,7 +586,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
       const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
       const uint32_t tS0 = tmem_base + lane_base + half * 32;
       const uint32_t tDP0 = tmem_base + lane_base + Cfg::kDpCol + half * 32;
-      const float c1 = dm.scale * kLog2e;
+      const float c1 = in_register(dm.scale * kLog2e), log2e = in_register(kLog2e), minus = in_register(-1.f);
       const float p_full = 1.f / (float)n;
 
       int g = 0, pgc = 0;
@@ -707,7 +707,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
 #pragma unroll
                     for (int e = 0; e < 8; e += 2) {
                       float t0, t1, a0, a1;
-                      ffma2(t0, t1, bv[e], bv[e + 1], kLog2e, kLog2e, nl[e], nl[e + 1]);
+                      ffma2(t0, t1, bv[e], bv[e + 1], log2e, log2e, nl[e], nl[e + 1]);
                       ffma2(a0, a1, x[q8 * 8 + e], x[q8 * 8 + e + 1], c1, c1, t0, t1);
                       p[e] = ex2(a0);
                       p[e + 1] = ex2(a1);
@@ -717,7 +717,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
                   for (int e = 0; e < 8; e += 2) {
                     const int col = q8 * 8 + e;
                     float s0, s1, d0, d1;
-                    ffma2(s0, s1, dl[e], dl[e + 1], -1.f, -1.f, g_[hq * 16 + col], g_[hq * 16 + col + 1]);   // dP - delta
+                    ffma2(s0, s1, dl[e], dl[e + 1], minus, minus, g_[hq * 16 + col], g_[hq * 16 + col + 1]);   // dP - delta
                     fmul2(d0, d1, p[e], p[e + 1], s0, s1);
                     uint32_t wp = pack2<T>(p[e], p[e + 1]);
                     uint32_t wd = pack2<T>(d0, d1);

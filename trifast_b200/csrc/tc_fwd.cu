@@ -1,33 +1,44 @@
 // Forward triangle attention on the 5th-generation tensor cores (bf16 / fp16).
 //
-// Work item = one 128-query tile (h, j-tile) of R = 2 consecutive pair rows i
-// ("slots"), walked over the keys in tiles of 128.  The slots share every bias
-// tile, which is the dominant shared-memory stream (32 KiB per step against
-// 8-16 KiB of K+V per slot), and give the tensor pipe independent work while the
-// softmax of the other slot runs.  CTAs are persistent: one per SM, each looping
-// over work items, so that the loads and the first MMA of the next item overlap
-// the tail of the current one instead of paying a pipeline fill per item.
+// Work item = one 128-query tile (h, j-tile) of R = 4 consecutive pair rows i
+// ("slots"), walked over the keys in steps of 64.  The slots share every bias
+// tile, the dominant shared-memory stream, and cover each other's waits: a slot's
+// step is a chain (S -> weights -> O += P V -> the next S), and four of them on an SM are what
+// keeps the exponential unit fed.  CTAs are persistent: one per SM, each looping over work
+// items, so that the loads and the first MMA of the next item overlap the tail of the current
+// one.
 //
-//   warps 0 .. 4R-1 : softmax warpgroups, one per slot; thread t owns query row t:
+//   warps 0 .. 15   : softmax warpgroups, one per slot; thread t owns query row t:
 //                     S (TMEM) -> registers, + bias (shared memory), mask, online
-//                     softmax in fp32, P -> TMEM as 16-bit pairs, O rescale when
+//                     softmax in fp32, P -> TMEM as 16-bit pairs over S, O rescale when
 //                     the row maximum moves, final O / l and lse
-//   warp 4R         : TMA producer (one lane): Q per item, then K, V (per slot)
-//                     and the bias tile per key step through an NS-deep ring
-//   warps 4R+1, 4R+2: MMA issuers, one per slot (one lane each): S = Q K^T (SS,
-//                     both operands K-major) and O += P V (A = P from TMEM, B = V as
-//                     an MN-major tile); a slot's MMAs never wait behind the other's
-//   warp 4R + 3     : idle; it completes the warpgroup whose registers are handed
-//                     to the softmax warpgroups (setmaxnreg)
+//   warp 16         : TMA producer: Q per item, then K, V (per slot) and the bias tile per
+//                     key step through an NS-deep ring; it also finds the items (those whose rows
+//                     all have no open key are left out) and hands them to the other roles
+//   warps 17, 18    : MMA issuers, two slots each: O += P V (A = P from TMEM, B = V as
+//                     an MN-major tile), then the slot's next S = Q K^T (SS, both operands
+//                     K-major), whose result overwrites that P: MMAs of one thread execute in
+//                     the order of their issue, so nothing waits in between, and a step's S
+//                     is complete only when the O += P V before it is
+//   warp 19         : idle; it completes the warpgroup whose registers are handed over
 //
-// TMEM columns per slot r (base r * 256): S [0,128) fp32, P [128,192) packed
-// 16-bit pairs, O [192, 192 + D) fp32.
+// What bounds it: a slot's step takes about 3400 cycles, two thirds of them in its own arithmetic
+// beside the other slots', the rest on the way to the MMAs and back; the issue slots are 63 % used
+// (8.8 instructions a score), the exponential unit 60 %.  Time at h = 4, before (two slots of eight warps,
+// steps of 128 keys, P beside S) and after: d = 32 bf16 n = 512 (15 % padding) 259 -> 232 us, n = 1024 1.81 -> 1.54 ms,
+// n = 2048 (10 % padding) 13.1 -> 11.0 ms; d = 64 fp16 n = 1024 2.17 -> 1.88 ms; n = 64 14.3 -> 12.3 us.
+// Measured and left (n = 1024, d = 32): P beside S, the next S issued as soon as this one is read, 1.67 ms,
+// all slots then keep in step; the same with two pairs of slots taking turns in the exponentials
+// 1.62 ms.
+//
+// TMEM columns per slot r (base r * 128): S [0,64) fp32, P over it [0,32) packed 16-bit pairs,
+// O [64, 64 + D) fp32.
 //
 // Semantics follow the PyTorch path of the reference (src/trifast/equiv.py:42-69):
-// masked keys weigh exactly zero; rows whose keys are all masked get uniform
-// weights over all n keys and lse = finfo(dtype).min.  The kernel stands in for
-// `_fwd` of the reference (src/trifast/triton.py:14-132); unlike it, the scale
-// d^-0.5 is applied to the fp32 accumulator, not to Q in 16 bits.
+// masked keys weigh exactly zero; rows whose keys are all masked get the mean of all n
+// values and lse = finfo(dtype).min (written by the prepare kernel where it runs).  The
+// kernel stands in for `_fwd` of the reference (src/trifast/triton.py:14-132); unlike it, the
+// scale d^-0.5 is applied to the fp32 accumulator, not to Q in 16 bits.
 
 #include <math.h>
 
@@ -40,104 +51,81 @@ namespace trifast {
 namespace {
 using namespace tc;
 
-// Registers per thread after the warpgroups rebalance (setmaxnreg): the last
-// warpgroup drops to TRIFAST_REG_DEC, the softmax warpgroups rise to
-// TRIFAST_REG_INC.  The hand-over must balance: 384 threads launch with 168
-// registers each, and a request beyond what the issue warpgroup released would
-// block forever.
-#ifndef TRIFAST_REG_DEC
-#define TRIFAST_REG_DEC 56
-#endif
-#ifndef TRIFAST_REG_INC
-#define TRIFAST_REG_INC 224
-#endif
-static_assert(256 * TRIFAST_REG_INC + 128 * TRIFAST_REG_DEC <= 384 * 168, "setmaxnreg pool");
+// Register hand-over (setmaxnreg): 640 threads launch with 96 registers each; what the
+// softmax warpgroups gain must not exceed what the issue warpgroup releases, or the request
+// blocks forever.
+constexpr int kRegsLaunch = 96, kRegsIssue = 32, kRegsMath = 112;
+static_assert(512 * kRegsMath + 128 * kRegsIssue <= 640 * kRegsLaunch, "setmaxnreg pool");
 
-constexpr int kBJ = 128, kBK = 128;
+constexpr int kR = 4;             // slots: pair rows of an item
+constexpr int kBJ = 128, kBK = 64;
+constexpr int kTmaWarp = 16;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kMaxInit = -1e30f;
-// A tile moves the running maximum only when it exceeds it by more than the lazy threshold
+// A step moves the running maximum only when it exceeds it by more than the lazy threshold
 // (natural-log units).  0 = always track the exact maximum: the largest weight of a
 // row is then exactly 1 before rounding to 16 bits, which keeps the error of peaked
 // rows lowest; a positive value (FlashAttention-style lazy rescale) trades that for
-// fewer rescales of O.  Measured at n = 1024: 2.7 % of the forward at d = 64 (64 columns of
-// O per rescale), 1.5 % at d = 32, 1 % at d = 16, for a maximum error against the fp64 oracle
-// about a third larger: taken at d = 64 only.
-template <int D> constexpr float lazy_tau() { return D >= 64 ? 5.5f : 0.f; }
+// fewer rescales of O, 64 columns at d = 64.  There (n = 300, fp16, relative 2-norm error of o against
+// float64; forward of n = 512, h = 8): 0 2.50e-4, 547 us; 2 2.74e-4, 537 us; 5.5 2.83e-4, 523 us, and
+// 2.75e-4 before the steps were 64 keys long.
+template <int D> constexpr float lazy_tau() { return D >= 64 ? 1.5f : 0.f; }
 constexpr int kSmemLimit = 232448;  // 227 KiB opt-in limit per CTA
-constexpr int kHeaderBytes = 512;
+constexpr int kHeaderBytes = 1024;
 
-template <int D, int R, int NS>
-struct FwdCfg {
+template <int D> struct FwdCfg {
+  static constexpr int NS = D == 64 ? 2 : D == 32 ? 3 : 4;  // stages of the ring
   static constexpr int kRowBytes = D * 2;
-  static constexpr int kTileBytes = 128 * kRowBytes;      // one Q / K / V tile
-  static constexpr int kBiasBytes = 128 * 128 * 2;        // two [128 x 64] boxes
-  static constexpr int kStageBytes = 2 * R * kTileBytes + kBiasBytes;
-  static constexpr int kTilesBytes = R * kTileBytes + NS * kStageBytes;
-  static constexpr int kThreads = R * 128 + 128;
+  static constexpr int kQBytes = kBJ * kRowBytes;           // Q tile of a slot
+  static constexpr int kKVBytes = kBK * kRowBytes;          // K or V tile of a slot
+  static constexpr int kBiasBytes = kBJ * kBK * 2;
+  static constexpr int kStageBytes = 2 * kR * kKVBytes + kBiasBytes;
+  static constexpr int kSmemBytes = kHeaderBytes + kR * kQBytes + NS * kStageBytes;
+  static constexpr int kThreads = 640;
   static constexpr uint64_t kSwz = RowSwizzle<D>::kDesc;
-  static constexpr int kSbo = 8 * kRowBytes;              // pitch of 8-row groups
-  // per slot: 4 mask words per 128-key chunk, one or two buffers (this item's and the next's)
-  static int mask_bytes(int n, int bufs) { return bufs * R * ((n + kBK - 1) / kBK) * 16; }
-  static int smem_with(int n, int bufs) {
-    const int head = (kHeaderBytes + mask_bytes(n, bufs) + 1023) / 1024 * 1024;
-    return 1024 + head + kTilesBytes;                     // 1024: manual base alignment
-  }
-  // two mask buffers (the next item's words are made ahead) when they fit, else one
-  static int mask_bufs(int n) { return smem_with(n, 2) <= kSmemLimit ? 2 : 1; }
-  static int smem_bytes(int n) {
-    const int head = (kHeaderBytes + mask_bytes(n, mask_bufs(n)) + 1023) / 1024 * 1024;
-    return 1024 + head + kTilesBytes;                     // 1024: manual base alignment
-  }
+  static constexpr int kSbo = 8 * kRowBytes;                // pitch of 8-row groups
+  static_assert(kSmemBytes <= kSmemLimit, "shared memory");
 };
 
-// Work items in launch order: j-tile fastest, then row pair, then (b, h): the CTAs
+// Work items in launch order: j-tile fastest, then row group, then (b, h): the CTAs
 // running at one time share bias strips and K/V rows in L2.
+// The first `full` row groups' items have kR rows; those after it are halves of two rows each, so
+// that a last round that would fill at most half of the CTAs fills them all and ends earlier
+// (a half item takes about 0.6 of a whole one).
 struct ItemGrid {
-  int njt, nrp, total;
+  int njt, nrg, full, total;
 };
 
-// MB: mask buffers per softmax warp (2: the next item's words are made ahead).
-template <typename T, int D, int R, int NS, int MB>
-__global__ void __launch_bounds__(R * 128 + 128, 1)
+// kWords: the key mask comes as the prepare step's packed words, else as the caller's bytes.
+template <typename T, int D, bool kWords>
+__global__ void __launch_bounds__(640, 1)
 tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_b,
-              View5 o, float* __restrict__ lse, MaskView mask, const uint8_t* __restrict__ ws_rowfull,
+              View5 v, View5 o, float* __restrict__ lse, MaskView mask,
               const uint32_t* __restrict__ ws_maskbits, int ws_mask_words,
               const uint32_t* __restrict__ ws_rowrange, Dims dm, ItemGrid items,
               unsigned int* status) {
-  using Cfg = FwdCfg<D, R, NS>;
-  static_assert(R == 2, "two slots: the exp phases alternate between them");
-  constexpr int Q_FULL = 0, Q_EMPTY = 1, FULL = 2, EMPTY = FULL + NS, S_FULL = EMPTY + NS,
-                S_FREE = S_FULL + R, P_READY = S_FREE + R, O_DONE = P_READY + R,
-                O_FREE = O_DONE + R, TOKEN = O_FREE + R, NBARS = TOKEN + R;
-  static_assert(NBARS * 8 <= 256, "barrier area");
+  using Cfg = FwdCfg<D>;
+  constexpr int NS = Cfg::NS;
+  constexpr int ITEM = 0, Q_FULL = 4, Q_EMPTY = 5, FULL = 6, EMPTY = FULL + NS, S_FULL = EMPTY + NS,
+                P_READY = S_FULL + kR, O_DONE = P_READY + kR, O_FREE = O_DONE + kR, NBARS = O_FREE + kR;
+  static_assert(NBARS * 8 <= 512, "barrier area");
 
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t raw = smem_u32(smem_raw);
-  const uint32_t base = (raw + 1023u) & ~1023u;
-  uint8_t* gbase = smem_raw + (base - raw);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + 256);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + 260);
-  uint32_t* maskbits = reinterpret_cast<uint32_t*>(gbase + kHeaderBytes);  // [R slots][MB][nkt][4]
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const uint32_t base = smem_u32(smem_raw);
+  uint8_t* gbase = smem_raw;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + 512);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + 516);
 
   const int n = dm.n;
-  const int nkt = (n + kBK - 1) / kBK;
-  const uint32_t tiles_off = (kHeaderBytes + MB * R * nkt * 16 + 1023u) & ~1023u;
-  const uint32_t tiles = base + tiles_off;
+  constexpr uint32_t tiles_off = kHeaderBytes;
+  constexpr uint32_t stages_off = tiles_off + kR * Cfg::kQBytes;
   auto bar = [&](int i) -> uint32_t { return base + 8u * i; };
-  auto q_tile = [&](int r) -> uint32_t { return tiles + r * Cfg::kTileBytes; };
-  auto stage_base = [&](int s) -> uint32_t {
-    return tiles + R * Cfg::kTileBytes + s * Cfg::kStageBytes;
-  };
-  auto k_tile = [&](int s, int r) -> uint32_t { return stage_base(s) + r * Cfg::kTileBytes; };
-  auto v_tile = [&](int s, int r) -> uint32_t {
-    return stage_base(s) + (R + r) * Cfg::kTileBytes;
-  };
-  auto bias_off = [&](int s) -> uint32_t {  // byte offset from gbase
-    return tiles_off + R * Cfg::kTileBytes + s * Cfg::kStageBytes + 2 * R * Cfg::kTileBytes;
-  };
+  auto q_tile = [&](int r) -> uint32_t { return base + tiles_off + r * Cfg::kQBytes; };
+  auto k_tile = [&](int s, int r) -> uint32_t { return base + stages_off + s * Cfg::kStageBytes + r * Cfg::kKVBytes; };
+  auto v_tile = [&](int s, int r) -> uint32_t { return k_tile(s, kR + r); };
+  auto bias_off = [&](int s) -> uint32_t { return stages_off + s * Cfg::kStageBytes + 2 * kR * Cfg::kKVBytes; };
   // item -> (j tile, first row, head, batch); a slot beyond the last row re-does the
   // last row (its loads stay in range, its results are not stored)
   struct Item {
@@ -145,36 +133,24 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   };
   auto decode = [&](int w) -> Item {
     Item it;
+    const int half = w - items.full;
+    if (half >= 0) w = items.full + (half >> 1);
     it.jt = w % items.njt;
     const int rest = w / items.njt;
-    it.i0 = (rest % items.nrp) * R;
-    const int bh = rest / items.nrp;
+    it.i0 = (rest % items.nrg) * kR + (half >= 0 ? 2 * (half & 1) : 0);
+    const int bh = rest / items.nrg;
     it.h = bh % dm.heads;
     it.b = bh / dm.heads;
     return it;
   };
   auto slot_row = [&](const Item& it, int r) -> int { return min(it.i0 + r, dm.n_rows - 1); };
-  // Key tiles [lo, hi) an item walks, as lo | hi << 16: the union of the live ranges of its
-  // rows (tiles outside it hold no open key of either row and weigh exactly zero).  Only the
-  // producer computes it (one item ahead; it alone is off the critical path) and hands it to
-  // the other roles through a shared-memory word per item parity, written before its arrive
-  // on Q_FULL: the issuers read it after their wait on Q_FULL, the softmax warps after the
-  // item's first S_FULL, which the issuers' MMAs complete.  The producer is never more than
-  // one item ahead of the issuers (Q_EMPTY) nor the issuers of the softmax warps (S_FREE),
-  // so a word is rewritten only after every reader of its previous value has moved on.
-  volatile uint32_t* rng_word = reinterpret_cast<volatile uint32_t*>(gbase + 264);   // [2]
-  auto item_range = [&](int w) -> uint32_t {
-    if (ws_rowrange == nullptr || w >= items.total) return (uint32_t)nkt << 16;
-    const Item it = decode(w);
-    uint32_t lo = 0xffffu, hi = 0u;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const uint32_t v = __ldg(ws_rowrange + it.b * dm.n_rows + slot_row(it, r));
-      lo = min(lo, v & 0xffffu);
-      hi = max(hi, v >> 16);
-    }
-    return uniform(lo | (hi << 16));
-  };
+  // The producer hands an item to the other roles through a ring of four records and barriers: number
+  // (-1 at the end), a word that holds its key steps [lo, hi) in bits 0-11 and 16-27, and per slot r
+  // whether the row has no dropped key, bit 12 + r, and whether it has no open one, bit 28 + r;
+  // first query, first row, head, batch.  It is never more than two items ahead of a reader: an item's
+  // Q is loaded behind Q_EMPTY of the one before, whose MMAs are issued behind P_READY of
+  // the one before that.
+  volatile int* records = reinterpret_cast<volatile int*>(gbase + 544);   // [4][8]
 
   // A wait that gave up in an earlier CTA or launch leaves the status word set:
   // stop doing work until the host has read and cleared it.
@@ -183,31 +159,32 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     return;
   }
 
+  // (what every lane of a warp shares goes through uniform(), so that the compiler keeps it, and the
+  // descriptors made of it, in uniform registers, where the MMAs want them)
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
 
   if (tid == 0) {
+    for (int u = 0; u < 4; ++u) mbar_init(bar(ITEM + u), 1);
     mbar_init(bar(Q_FULL), 1);
-    mbar_init(bar(Q_EMPTY), R);
+    mbar_init(bar(Q_EMPTY), kR);
     for (int s = 0; s < NS; ++s) {
       mbar_init(bar(FULL + s), 1);
-      mbar_init(bar(EMPTY + s), R * 5);  // per slot: 1 MMA commit + 4 softmax warps
+      mbar_init(bar(EMPTY + s), kR * 5);  // per slot: 1 MMA commit + 4 softmax warps
     }
-    for (int r = 0; r < R; ++r) {
+    for (int r = 0; r < kR; ++r) {
       mbar_init(bar(S_FULL + r), 1);
-      mbar_init(bar(S_FREE + r), 4);
       mbar_init(bar(P_READY + r), 4);
       mbar_init(bar(O_DONE + r), 1);
       mbar_init(bar(O_FREE + r), 4);
-      mbar_init(bar(TOKEN + r), 4);
     }
     *abort_flag = 0;
     mbar_fence_init();
   }
-  if (warp == 4 * R + 1) {
+  if (warp == kTmaWarp + 1) {
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
   }
-  if (warp == 4 * R && lane == 0) {
+  if (warp == kTmaWarp && lane == 0) {
     tma_prefetch_desc(&map_q);
     tma_prefetch_desc(&map_k);
     tma_prefetch_desc(&map_v);
@@ -218,337 +195,312 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   tc_fence_after();
   const uint32_t tmem_base = uniform(*tmem_slot);
 
-  if (warp >= 4 * R) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(TRIFAST_REG_DEC));
-  if (warp == 4 * R) {
+  if (warp >= kTmaWarp) {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
+  // (The whole warp runs the loops of the producer and the issuers; elect_one() issues, which
+  // tells the compiler that one thread does: under a lane test it wraps every MMA and TMA
+  // load in code for several, 130 cycles an MMA instead of 50.)
+  if (warp == kTmaWarp) {
     // ------------------------------------------------------------ TMA producer
-    // (The whole warp runs the loops of the producer and the issuers; elect_one() issues, which
-    // tells the compiler that one thread does: under a lane test it wraps every MMA and TMA
-    // load in code for several, 130 cycles an MMA instead of 50.)
-    {
-      int g = 0, it = 0;  // running key-tile and item counters (barrier phases)
-      bool ok = true;
-      uint32_t rng_next = item_range(blockIdx.x);
-      for (int w = blockIdx.x; w < items.total && ok; w += gridDim.x, ++it) {
-        const Item im = decode(w);
-        const uint32_t rng = rng_next;
-        const int kt_lo = rng & 0xffffu, kt_hi = rng >> 16;
-        rng_next = item_range(w + gridDim.x);
-        if (it > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(Q_EMPTY), (it - 1) & 1, abort_flag));
+    // key steps an item walks: the union of the live ranges of its rows (in 128-key tiles; a row
+    // without an open key has none), fetched one item ahead
+    auto item_range = [&](int w) -> uint32_t {
+      const uint32_t steps = (uint32_t)(n + kBK - 1) / kBK;
+      if (ws_rowrange == nullptr || w >= items.total) return steps << 16;
+      const Item it = decode(w);
+      uint32_t lo = 0xffffu, hi = 0u, flags = 0u;
+      for (int r = 0; r < (w < items.full ? kR : 2); ++r) {
+        const uint32_t u = __ldg(ws_rowrange + it.b * dm.n_rows + slot_row(it, r));
+        const uint32_t l = u & 0xffffu, h = (u >> 16) & 0x7fffu;
+        lo = min(lo, l);
+        hi = max(hi, h);
+        flags |= ((u >> 31) << (12 + r)) | ((l >= h ? 1u : 0u) << (28 + r));
+      }
+      return uniform(lo >= hi ? 0u : 2 * lo | min(2 * hi, steps) << 16 | flags);
+    };
+    int g = 0, it = 0;  // running key-step and item counters (barrier phases)
+    bool ok = true;
+    uint32_t rng_next = item_range(blockIdx.x);
+    for (int w = blockIdx.x; w < items.total && ok; w += gridDim.x) {
+      const uint32_t rng = rng_next;
+      const int lo = rng & 0xfffu, hi = (rng >> 16) & 0xfffu;
+      rng_next = item_range(w + gridDim.x);
+      if (lo >= hi) continue;
+      const Item im = decode(w);
+      const int slots = w < items.full ? kR : 2;
+      if (it > 0) ok = __all_sync(0xffffffffu, mbar_wait(bar(Q_EMPTY), (it - 1) & 1, abort_flag));
+      if (!ok) break;
+      if (elect_one()) {
+        volatile int* rec = records + (it & 3) * 8;
+        rec[0] = w;
+        rec[1] = (int)rng;
+        rec[2] = im.jt * kBJ;
+        rec[3] = im.i0;
+        rec[4] = im.h;
+        rec[5] = im.b;
+        mbar_arrive(bar(ITEM + (it & 3)));
+        mbar_arrive_expect_tx(bar(Q_FULL), slots * Cfg::kQBytes);
+        for (int r = 0; r < slots; ++r)
+          tma_load_5d(q_tile(r), &map_q, bar(Q_FULL), 0, im.jt * kBJ, slot_row(im, r), im.h, im.b);
+      }
+      __syncwarp();
+      ++it;
+      for (int st = lo; st < hi; ++st, ++g) {
+        const int s = g % NS;
+        if (g >= NS)
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(EMPTY + s), ((g / NS) - 1) & 1, abort_flag));
         if (!ok) break;
         if (elect_one()) {
-          rng_word[it & 1] = rng;
-          mbar_arrive_expect_tx(bar(Q_FULL), R * Cfg::kTileBytes);
-          for (int r = 0; r < R; ++r)
-            tma_load_5d(q_tile(r), &map_q, bar(Q_FULL), 0, im.jt * kBJ, slot_row(im, r), im.h, im.b);
+          mbar_arrive_expect_tx(bar(FULL + s), 2 * slots * Cfg::kKVBytes + Cfg::kBiasBytes);
+          for (int r = 0; r < slots; ++r) {
+            tma_load_5d(k_tile(s, r), &map_k, bar(FULL + s), 0, st * kBK, slot_row(im, r), im.h, im.b);
+            tma_load_5d(v_tile(s, r), &map_v, bar(FULL + s), 0, st * kBK, slot_row(im, r), im.h, im.b);
+          }
+          tma_load_4d(base + bias_off(s), &map_b, bar(FULL + s), st * kBK, im.jt * kBJ, im.h, im.b);
         }
         __syncwarp();
-        for (int kt = kt_lo; kt < kt_hi; ++kt, ++g) {
-          const int s = g % NS;
-          if (g >= NS)
-            ok = __all_sync(0xffffffffu, mbar_wait(bar(EMPTY + s), ((g / NS) - 1) & 1, abort_flag));
-          if (!ok) break;
-          if (elect_one()) {
-            mbar_arrive_expect_tx(bar(FULL + s), R * 2 * Cfg::kTileBytes + Cfg::kBiasBytes);
-            for (int r = 0; r < R; ++r) {
-              tma_load_5d(k_tile(s, r), &map_k, bar(FULL + s), 0, kt * kBK, slot_row(im, r), im.h, im.b);
-              tma_load_5d(v_tile(s, r), &map_v, bar(FULL + s), 0, kt * kBK, slot_row(im, r), im.h, im.b);
-            }
-            const uint32_t bias_s = base + bias_off(s);
-            tma_load_4d(bias_s, &map_b, bar(FULL + s), kt * kBK, im.jt * kBJ, im.h, im.b);
-            tma_load_4d(bias_s + 16384, &map_b, bar(FULL + s), kt * kBK + 64, im.jt * kBJ, im.h, im.b);
-          }
-          __syncwarp();
-        }
       }
     }
-  } else if (warp - (4 * R + 1) < R) {
-    // ------------------------------------------------------------ MMA issuers (one per slot)
-    const int r = warp - (4 * R + 1);
-    {
-      constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
-      constexpr uint32_t idesc_qk = make_idesc(128, 128, kBf16, false, false);
-      constexpr uint32_t idesc_pv = make_idesc(128, D, kBf16, false, true);
-      auto issue_qk = [&](int s, bool last_q) {
-        const uint64_t ad = make_smem_desc(q_tile(r), 16, Cfg::kSbo, Cfg::kSwz);
-        const uint64_t bd = make_smem_desc(k_tile(s, r), 16, Cfg::kSbo, Cfg::kSwz);
-        if (elect_one()) {
-          // (a K slice of 16 elements is 32 bytes further along the row)
+    if (ok && elect_one()) {
+      records[(it & 3) * 8] = -1;
+      mbar_arrive(bar(ITEM + (it & 3)));
+    }
+    __syncwarp();
+  } else if (warp < kTmaWarp + 3) {
+    // ------------------------------------------------------------ MMA issuers (two slots each)
+    const int r0 = (warp - kTmaWarp - 1) * 2;
+    constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
+    constexpr uint32_t idesc_qk = make_idesc(128, kBK, kBf16, false, false);
+    constexpr uint32_t idesc_pv = make_idesc(128, D, kBf16, false, true);
+    // (a K slice of 16 elements is 32 bytes further along the row; 16 rows of the MN-major V tile
+    // are kStep16Rows units of 16 bytes further on)
+    constexpr uint32_t kStep16Rows = (16 * Cfg::kRowBytes) >> 4;
+    auto qk = [&](int r, int s, bool last_q) {   // in the elected lane
+      const uint64_t ad = make_smem_desc(q_tile(r), 16, Cfg::kSbo, Cfg::kSwz);
+      const uint64_t bd = make_smem_desc(k_tile(s, r), 16, Cfg::kSbo, Cfg::kSwz);
 #pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk)
-            umma_ss(tmem_base + r * 256, ad + 2 * kk, bd + 2 * kk, idesc_qk, kk > 0);
-          umma_commit(bar(S_FULL + r));
-          if (last_q) umma_commit(bar(Q_EMPTY));   // last read of this item's Q tile
+      for (int kk = 0; kk < D / 16; ++kk)
+        umma_ss(tmem_base + r * 128, ad + 2 * kk, bd + 2 * kk, idesc_qk, kk > 0);
+      umma_commit(bar(S_FULL + r));
+      if (last_q) umma_commit(bar(Q_EMPTY));   // last read of this item's Q tile
+    };
+    int g = 0, gs = 0;   // running key steps of all items (ring) and of those this warp's slots walk
+    int its = 0;         // running items of this warp's slots
+    bool ok = true;
+    for (int it = 0; ok; ++it) {
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(ITEM + (it & 3)), (it >> 2) & 1, abort_flag));
+      if (!ok) break;
+      const int w = uniform(records[(it & 3) * 8]);
+      if (w < 0) break;
+      const uint32_t rng = uniform(records[(it & 3) * 8 + 1]);
+      const int steps = ((rng >> 16) & 0xfffu) - (rng & 0xfffu);
+      ok = mbar_wait(bar(Q_FULL), it & 1, abort_flag) &&
+           mbar_wait(bar(FULL + g % NS), (g / NS) & 1, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      if (w >= items.full && r0 > 0) {   // half an item: these slots' share of the arrivals
+        if (lane == 0) mbar_arrive_n(bar(Q_EMPTY), 2);
+        for (int st = 0; st < steps && ok; ++st, ++g) {
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(FULL + g % NS), (g / NS) & 1, abort_flag));
+          if (ok && lane == 0) mbar_arrive_n(bar(EMPTY + g % NS), 2 * 5);
         }
-        __syncwarp();
-      };
-      int g = 0, it = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; w < items.total && ok; w += gridDim.x, ++it) {
-        // S of the item's first key tile: needs Q, the first stage, and the S columns
-        // released by the softmax of the previous item's last tile
-        ok = mbar_wait(bar(Q_FULL), it & 1, abort_flag) &&
-             mbar_wait(bar(FULL + g % NS), (g / NS) & 1, abort_flag) &&
-             (g == 0 || mbar_wait(bar(S_FREE + r), (g - 1) & 1, abort_flag));
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t rng = uniform(rng_word[it & 1]);
-        const int kt_lo = rng & 0xffffu, kt_hi = rng >> 16;
-        issue_qk(g % NS, kt_hi - kt_lo == 1);
-        for (int kt = kt_lo; kt < kt_hi && ok; ++kt, ++g) {
-          const int s = g % NS;
-          if (kt + 1 < kt_hi) {
-            const int ns = (g + 1) % NS;
-            ok = mbar_wait(bar(FULL + ns), ((g + 1) / NS) & 1, abort_flag) &&
-                 mbar_wait(bar(S_FREE + r), g & 1, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            tc_fence_after();
-            issue_qk(ns, kt + 2 == kt_hi);
-          }
-          ok = mbar_wait(bar(P_READY + r), g & 1, abort_flag);
+        continue;
+      }
+      // S of the first step (the P under it is read by MMAs issued before)
+      tc_fence_after();
+      if (elect_one()) {
+        qk(r0, g % NS, steps == 1);
+        qk(r0 + 1, g % NS, steps == 1);
+      }
+      __syncwarp();
+      for (int st = 0; st < steps && ok; ++st, ++g, ++gs) {
+        const int s = g % NS, ns = (g + 1) % NS;
+        const bool more = st + 1 < steps;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int r = r0 + u;
           // the first PV of an item overwrites O: the previous item's epilogue must have read it
-          if (ok && kt == kt_lo && it > 0) ok = mbar_wait(bar(O_FREE + r), (it - 1) & 1, abort_flag);
+          ok = ok && mbar_wait(bar(P_READY + r), gs & 1, abort_flag) &&
+               (st > 0 || its == 0 || mbar_wait(bar(O_FREE + r), (its - 1) & 1, abort_flag));
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
           tc_fence_after();
           const uint64_t bd = make_smem_desc(v_tile(s, r), Cfg::kSbo, Cfg::kSbo, Cfg::kSwz);
-          const uint32_t acc = kt > kt_lo ? 1u : 0u;
+          const uint32_t t_r = tmem_base + r * 128, acc = st > 0 ? 1u : 0u;
           if (elect_one()) {
-            // (16 rows of the MN-major V tile further on, in 16-byte units)
 #pragma unroll
             for (int ks = 0; ks < kBK / 16; ++ks)
-              umma_ts(tmem_base + r * 256 + 192, tmem_base + r * 256 + 128 + ks * 8,
-                      bd + ks * ((16 * Cfg::kRowBytes) >> 4), idesc_pv, ks > 0 ? 1u : acc);
-            umma_commit(bar(O_DONE + r));
+              umma_ts(t_r + 64, t_r + ks * 8, bd + ks * kStep16Rows, idesc_pv, ks > 0 ? 1u : acc);
+            if (!more) umma_commit(bar(O_DONE + r));
             umma_commit(bar(EMPTY + s));
           }
           __syncwarp();
+          if (more) {   // (the next stage may still be on its way: only this slot waits for it)
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(FULL + ns), ((g + 1) / NS) & 1, abort_flag));
+            if (!ok) break;
+            tc_fence_after();
+            if (elect_one()) qk(r, ns, st + 2 == steps);
+            __syncwarp();
+          }
         }
       }
+      ++its;
     }
   }
   } else {
-  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(TRIFAST_REG_INC));
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegsMath));
   {
     // ------------------------------------------------------------ softmax warpgroups
-    const int r = warp / 4, wq = warp & 3, t = tid & 127;
+    const int r = warp >> 2, wq = warp & 3, t = tid & 127;
     const uint32_t lane_base = (uint32_t)(wq * 32) << 16;
-    const uint32_t tS = tmem_base + lane_base + r * 256;
-    const uint32_t tP = tS + 128, tO = tS + 192;
-    // One copy per slot: the four warps of a slot work on the same row, each makes the
-    // same words and writes them to the same place, and reads them back after its own
-    // writes: whatever the interleaving, every read sees the one value all warps write.
-    uint32_t* mb = maskbits + r * MB * nkt * 4;
+    const uint32_t tS = tmem_base + lane_base + r * 128, tP = tS, tO = tS + 64;
 
-    // Key mask of a row as bit words (bit set = key dropped or beyond n), made one item
-    // ahead so that the loads run under the last PV of the current item.  Lane l reads
-    // keys 4l .. 4l+3 of a 128-key chunk as one word; word j of the chunk then holds,
-    // at bit l, key 4l + j.
-    struct RowMask {
-      const uint32_t* words;
-      bool full;
-    };
-    auto row_mask = [&](int w, uint32_t* dst) -> RowMask {
-      const Item im = decode(w);
-      const int i = slot_row(im, r), b = im.b;
-      RowMask rm;
-      if (ws_maskbits != nullptr) {
-        // made by the prepare step (n % 8 != 0: the mask rows are not word-aligned)
-        rm.words = ws_maskbits + ((int64_t)b * dm.n_rows + i) * ws_mask_words;
-        rm.full = ws_rowfull[b * dm.n_rows + i] != 0;
-        return rm;
-      }
-      const uint8_t* mrow = mask.p + b * mask.sb + (int64_t)i * mask.si;
-      uint32_t open = 0;
-      // four chunks at a time: the loads go out together, so a batch costs one
-      // memory latency instead of four
-      for (int c0 = 0; c0 < nkt; c0 += 4) {
-        uint32_t u[4];
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-          const int key4 = (c0 + cc) * kBK + 4 * lane;
-          u[cc] = (c0 + cc < nkt && key4 < n) ? __ldg(reinterpret_cast<const uint32_t*>(mrow + key4))
-                                              : 0x01010101u;
-        }
-#pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-          const int c = c0 + cc;
-          if (c < nkt) {
-            const uint32_t vm = __ballot_sync(0xffffffffu, c * kBK + 4 * lane < n);
-#pragma unroll
-            for (int jb = 0; jb < 4; ++jb) {
-              const uint32_t bits = __ballot_sync(0xffffffffu, ((u[cc] >> (8 * jb)) & 0xffu) != 0u);
-              if (lane == 0) dst[c * 4 + jb] = bits;
-              open |= ~bits & vm;
-            }
-          }
-        }
-      }
-      __syncwarp();
-      rm.words = dst;
-      rm.full = open == 0u;
-      return rm;
-    };
-
-    int g = 0, it = 0;
+    const float log2e = in_register(kLog2e), scale = in_register(dm.scale);
+    // (as the issuers count, but with the ring's stage and phase and the slot's phase kept as such:
+    // made from running counters they cost some forty instructions a step)
+    int s = 0;
+    uint32_t ring = 0u, turn = 0u;   // phase of the stage, of the slot's barriers
     bool ok = true;
-    constexpr bool ahead = MB == 2;
-    RowMask next_mask{mb, false};
-    if (ahead && (int)blockIdx.x < items.total) next_mask = row_mask(blockIdx.x, mb);
-    for (int w = blockIdx.x; w < items.total && ok; w += gridDim.x, ++it) {
-      const Item im = decode(w);
-      const int i = slot_row(im, r);
-      const bool do_store = im.i0 + r < dm.n_rows;
-      const int b = im.b, h = im.h, jt = im.jt;
-      if (!ahead) next_mask = row_mask(w, mb);  // one buffer: made at the top of the item
-      const bool row_full = next_mask.full;
-      const uint32_t* mbr = next_mask.words;
+    struct {
+      int w, j0, i0, h, b;
+      uint32_t rng;
+    } im, nx;
+    auto next_item = [&](int it) {
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(ITEM + (it & 3)), (it >> 2) & 1, abort_flag));
+      const volatile int* rec = records + (it & 3) * 8;
+      nx.w = ok ? uniform(rec[0]) : -1;
+      nx.rng = uniform((uint32_t)rec[1]);
+      nx.j0 = rec[2];
+      nx.i0 = rec[3];
+      nx.h = rec[4];
+      nx.b = rec[5];
+    };
+    next_item(0);
+    for (int it = 0; ok && nx.w >= 0; ++it) {
+      im = nx;
+      const uint32_t rng = im.rng;
+      const int lo = rng & 0xfffu, hi = (rng >> 16) & 0xfffu;
+      if (im.w >= items.full && r >= 2) break;   // half an item: the last one
+      const int i = min(im.i0 + r, dm.n_rows - 1), b = im.b, h = im.h;
+
+      // Key mask of a step, fetched one step ahead.  Bytes: lane l < 16 reads keys 4l .. 4l + 3 as
+      // one word.  Words: those of the 128-key chunk, of which the step is one half.
+      const uint8_t* mrow = mask.p + b * mask.sb + (int64_t)i * mask.si;
+      const uint32_t* mwords = ws_maskbits + ((int64_t)b * dm.n_rows + i) * ws_mask_words;
+      uint4 m_next;
+      auto fetch_mask = [&](int st) {
+        if constexpr (kWords) {
+          m_next = __ldg(reinterpret_cast<const uint4*>(mwords + (st >> 1) * 4));
+        } else {
+          const int key4 = st * kBK + 4 * lane;
+          m_next.x = lane >= 16 ? 0u : key4 < n ? __ldg(reinterpret_cast<const uint32_t*>(mrow + key4)) : 0x01010101u;
+        }
+      };
+      // (a row without a dropped key needs its mask for the step at the row's end alone)
+      const int masked_from = (rng >> (12 + r)) & 1u ? n / kBK : lo;
+      if (masked_from <= lo) fetch_mask(lo);
 
       float m_run = kMaxInit, l_run = 0.f;
-      // The key loop exists in two copies, chosen once per row: the fully-masked-row
-      // case (every score is 0) must not merge with the regular case inside the
-      // loop, or the 128 live scores get duplicated and spill.
-      auto key_loop = [&](auto row_full_tag) {
-      constexpr bool kRowFull = decltype(row_full_tag)::value;
-      // (the item's tile range is read after its first S_FULL: see rng_word)
-      int kt_lo = -1, kt_hi = 1;
-      for (int kt = 0; kt < kt_hi; ++kt, ++g) {
-        const int s = g % NS;
-        ok = __all_sync(0xffffffffu, mbar_wait(bar(S_FULL + r), g & 1, abort_flag));
+      bool any_open = false;
+      for (int st = lo; st < hi; ++st) {
+        // mask words of this step (uniform over the warp): key c of the step is bit c >> 2 of word c & 3
+        uint32_t mw[4] = {0u, 0u, 0u, 0u};
+        bool clean = true;
+        if (st >= masked_from) {
+          if constexpr (kWords) {
+            const int sh = (st & 1) * 16;
+            mw[0] = (m_next.x >> sh) & 0xffffu;
+            mw[1] = (m_next.y >> sh) & 0xffffu;
+            mw[2] = (m_next.z >> sh) & 0xffffu;
+            mw[3] = (m_next.w >> sh) & 0xffffu;
+          } else {
+#pragma unroll
+            for (int jb = 0; jb < 4; ++jb)
+              mw[jb] = __ballot_sync(0xffffffffu, ((m_next.x >> (8 * jb)) & 0xffu) != 0u);
+          }
+          clean = (mw[0] | mw[1] | mw[2] | mw[3]) == 0u;
+          any_open = any_open || (mw[0] & mw[1] & mw[2] & mw[3]) != 0xffffu;
+        }
+        if (st + 1 >= masked_from && st + 1 < hi) fetch_mask(st + 1);
+
+        ok = mbar_wait(bar(FULL + s), ring, abort_flag) && mbar_wait(bar(S_FULL + r), turn, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        if (kt_lo < 0) {
-          const uint32_t rng = uniform(rng_word[it & 1]);
-          kt_lo = kt = rng & 0xffffu;
-          kt_hi = rng >> 16;
-        }
-        float x[128];
-        {
-          uint32_t* xr = reinterpret_cast<uint32_t*>(x);
-          tmem_ld32(tS + 0, xr + 0);
-          tmem_ld32(tS + 32, xr + 32);
-          tmem_ld32(tS + 64, xr + 64);
-          tmem_ld32(tS + 96, xr + 96);
-          tmem_wait_ld();
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(S_FREE + r));
+        float x[64];
+        tmem_ld32(tS, reinterpret_cast<uint32_t*>(x));
+        tmem_ld32(tS + 32, reinterpret_cast<uint32_t*>(x) + 32);
+        tmem_wait_ld();
 
-        // mask words of this key tile (uniform over the warp); column c of the tile
-        // is bit (c >> 2) of word (c & 3)
-        uint32_t mw[4];
+        const uint8_t* brow = gbase + bias_off(s) + t * 128;
 #pragma unroll
-        for (int jb = 0; jb < 4; ++jb) {
-          if (kRowFull) {  // only keys beyond n stay dropped: key 4l + jb of the chunk
-            const int rem = n - kt * kBK - jb;             // keys 4l + jb < n  <=>  l < ceil(rem / 4)
-            const int groups = rem <= 0 ? 0 : (rem + 3) / 4;
-            mw[jb] = groups >= 32 ? 0u : ~((1u << groups) - 1u);
-          } else {
-            mw[jb] = mbr[kt * 4 + jb];
-          }
-        }
-        const bool clean = (mw[0] | mw[1] | mw[2] | mw[3]) == 0u;
-
-        ok = __all_sync(0xffffffffu, mbar_wait(bar(FULL + s), (g / NS) & 1, abort_flag));
-        if (!ok) break;
-        if (kRowFull) {
-#pragma unroll
-          for (int c = 0; c < 128; ++c) x[c] = 0.f;
-        } else {
-          const uint8_t* brow = gbase + bias_off(s) + t * 128;
-#pragma unroll
-          for (int gq = 0; gq < 16; ++gq) {
-            const uint4 u = *reinterpret_cast<const uint4*>(brow + (gq >> 3) * 16384 +
-                                                            (((gq & 7) ^ (t & 7)) << 4));
-            float b0, b1;
-            unpack2<T>(u.x, b0, b1);
-            ffma2(x[gq * 8 + 0], x[gq * 8 + 1], x[gq * 8 + 0], x[gq * 8 + 1], dm.scale, dm.scale, b0, b1);
-            unpack2<T>(u.y, b0, b1);
-            ffma2(x[gq * 8 + 2], x[gq * 8 + 3], x[gq * 8 + 2], x[gq * 8 + 3], dm.scale, dm.scale, b0, b1);
-            unpack2<T>(u.z, b0, b1);
-            ffma2(x[gq * 8 + 4], x[gq * 8 + 5], x[gq * 8 + 4], x[gq * 8 + 5], dm.scale, dm.scale, b0, b1);
-            unpack2<T>(u.w, b0, b1);
-            ffma2(x[gq * 8 + 6], x[gq * 8 + 7], x[gq * 8 + 6], x[gq * 8 + 7], dm.scale, dm.scale, b0, b1);
-          }
+        for (int gq = 0; gq < 8; ++gq) {
+          const uint4 u = *reinterpret_cast<const uint4*>(brow + ((gq ^ (t & 7)) << 4));
+          float b0, b1;
+          unpack2<T>(u.x, b0, b1);
+          ffma2(x[gq * 8 + 0], x[gq * 8 + 1], x[gq * 8 + 0], x[gq * 8 + 1], scale, scale, b0, b1);
+          unpack2<T>(u.y, b0, b1);
+          ffma2(x[gq * 8 + 2], x[gq * 8 + 3], x[gq * 8 + 2], x[gq * 8 + 3], scale, scale, b0, b1);
+          unpack2<T>(u.z, b0, b1);
+          ffma2(x[gq * 8 + 4], x[gq * 8 + 5], x[gq * 8 + 4], x[gq * 8 + 5], scale, scale, b0, b1);
+          unpack2<T>(u.w, b0, b1);
+          ffma2(x[gq * 8 + 6], x[gq * 8 + 7], x[gq * 8 + 6], x[gq * 8 + 7], scale, scale, b0, b1);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(EMPTY + s));  // bias tile consumed by this warp
 
         if (!clean) {
 #pragma unroll
-          for (int c = 0; c < 128; ++c)
+          for (int c = 0; c < 64; ++c)
             if ((mw[c & 3] >> (c >> 2)) & 1u) x[c] = -INFINITY;
         }
-        // Four independent chains for the row maximum and the row sum: with two
-        // warps per scheduler a single dependent chain of 128 would be latency-bound.
+        // four independent chains for the row maximum and the row sum
         float mx[4] = {x[0], x[1], x[2], x[3]};
 #pragma unroll
-        for (int c = 4; c < 124; c += 8) {  // 3-input max: two scores per instruction
+        for (int c = 4; c < 60; c += 8) {  // 3-input max: two scores per instruction
           mx[0] = fmax3(mx[0], x[c + 0], x[c + 1]);
           mx[1] = fmax3(mx[1], x[c + 2], x[c + 3]);
           mx[2] = fmax3(mx[2], x[c + 4], x[c + 5]);
           mx[3] = fmax3(mx[3], x[c + 6], x[c + 7]);
         }
-        mx[0] = fmax3(mx[0], x[124], x[125]);
-        mx[1] = fmax3(mx[1], x[126], x[127]);
-        const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+        mx[0] = fmax3(mx[0], x[60], x[61]);
+        mx[1] = fmax3(mx[1], x[62], x[63]);
+        const float mt = fmaxf(fmax3(mx[0], mx[1], mx[2]), mx[3]);
         // running maximum (see lazy_tau)
         const float m_new = (mt > m_run + lazy_tau<D>()) ? mt : m_run;
         const float neg = -m_new * kLog2e;
         // (difference first: exactly 1 when the maximum stays, also at the initial value,
         // where a fused m_run * log2e + neg would leave the rounding residue of 1e30 * log2e
-        // in the exponent and turn a key tile with no open key into inf * 0)
+        // in the exponent and turn a key step with no open key into inf * 0)
         const float alpha = ex2((m_run - m_new) * kLog2e);
         m_run = m_new;
 
-        if (kt > kt_lo) {
-          // PV of the previous key tile must be done before O is rescaled and P reused.
-          ok = __all_sync(0xffffffffu, mbar_wait(bar(O_DONE + r), (g - 1) & 1, abort_flag));
-          if (!ok) break;
-          tc_fence_after();
-          if (__any_sync(0xffffffffu, alpha != 1.f)) {
-            if constexpr (D == 16) {
-              uint32_t acc[16];
-              tmem_ld16(tO, acc);
-              tmem_wait_ld();
+        // (this S being complete, so is the O += P V before it)
+        if (st > lo && __any_sync(0xffffffffu, alpha != 1.f)) {
+          constexpr int kCols = D == 32 ? 32 : 16;   // (d = 64: registers)
 #pragma unroll
-              for (int e = 0; e < 16; ++e) acc[e] = __float_as_uint(__uint_as_float(acc[e]) * alpha);
-              tmem_st16(tO, acc);
-            } else {
+          for (int c = 0; c < D; c += kCols) {
+            uint32_t acc[kCols];
+            tmem_ld_cols<kCols>(tO + c, acc);
+            tmem_wait_ld();
+            float* f = reinterpret_cast<float*>(acc);
 #pragma unroll
-              for (int c = 0; c < D / 32; ++c) {
-                uint32_t acc[32];
-                tmem_ld32(tO + 32 * c, acc);
-                tmem_wait_ld();
-#pragma unroll
-                for (int e = 0; e < 32; ++e) acc[e] = __float_as_uint(__uint_as_float(acc[e]) * alpha);
-                tmem_st32(tO + 32 * c, acc);
-              }
-            }
+            for (int e = 0; e < kCols; e += 2) fmul2(f[e], f[e + 1], f[e], f[e + 1], alpha, alpha);
+            tmem_st_cols<kCols>(tO + c, acc);
           }
         }
-        // The two slots take turns in the exp phase, so that one slot's loads, bias
-        // FMAs and maximum overlap the other's exponentials instead of both phases
-        // running in lockstep.  Slot 0 goes first; each slot passes the turn on
-        // after issuing its exponentials.
-        ok = __all_sync(0xffffffffu,
-                        mbar_wait(bar(TOKEN + r), (r == 0) ? ((g & 1) ^ 1) : (g & 1), abort_flag));
-        if (!ok) break;
         // exp and P store in chunks of 32 keys, so a packed chunk leaves the
         // registers as soon as it is made; four independent partial sums.
         float sm[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int ch = 0; ch < 4; ++ch) {
+        for (int ch = 0; ch < 2; ++ch) {
           uint32_t pk[16];
 #pragma unroll
           for (int e = 0; e < 32; e += 4) {
             const int c = ch * 32 + e;
             float a0, a1, a2, a3;
-            ffma2(a0, a1, x[c + 0], x[c + 1], kLog2e, kLog2e, neg, neg);
-            ffma2(a2, a3, x[c + 2], x[c + 3], kLog2e, kLog2e, neg, neg);
+            ffma2(a0, a1, x[c + 0], x[c + 1], log2e, log2e, neg, neg);
+            ffma2(a2, a3, x[c + 2], x[c + 3], log2e, log2e, neg, neg);
             const float p0 = ex2(a0), p1 = ex2(a1), p2 = ex2(a2), p3 = ex2(a3);
             fadd2(sm[0], sm[1], sm[0], sm[1], p0, p1);
             fadd2(sm[2], sm[3], sm[2], sm[3], p2, p3);
@@ -558,27 +510,28 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
           tmem_st16(tP + ch * 16, pk);
         }
         l_run = fmaf(l_run, alpha, (sm[0] + sm[1]) + (sm[2] + sm[3]));
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar(TOKEN + (r ^ 1)));
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(P_READY + r));
+        turn ^= 1u;
+        if (++s == NS) {
+          s = 0;
+          ring ^= 1u;
+        }
       }
-      };
-      if (row_full) key_loop(std::true_type{}); else key_loop(std::false_type{});
       if (!ok) break;
 
-      // the next item's mask words, while the last PV of this item runs
-      if (ahead && w + (int)gridDim.x < items.total)
-        next_mask = row_mask(w + gridDim.x, mb + ((it + 1) & 1) * nkt * 4);
-
-      // epilogue of the item: O / l and lse
-      ok = __all_sync(0xffffffffu, mbar_wait(bar(O_DONE + r), (g - 1) & 1, abort_flag));
+      // epilogue of the item: O / l and lse.  A row without an open key is left to the prepare
+      // kernel (which marks it with an empty range) or, where none runs, done here.
+      const bool row_full = ws_rowrange == nullptr ? !any_open : (rng >> (28 + r)) & 1u;
+      next_item(it + 1);   // (its record and, below, O arrive in each other's shadow)
+      if (!ok) break;
+      const bool do_store = im.i0 + r < dm.n_rows && !(row_full && ws_rowrange != nullptr);
+      ok = __all_sync(0xffffffffu, mbar_wait(bar(O_DONE + r), it & 1, abort_flag));
       if (!ok) break;
       tc_fence_after();
-      const int j = jt * kBJ + t;
-      const float inv = 1.f / l_run;
+      const int j = im.j0 + t;
       T* dst = reinterpret_cast<T*>(o.p) + b * o.sb + h * o.sh + (int64_t)i * o.si + (int64_t)j * o.sj;
       uint32_t acc[D];
       tmem_ld_cols<D>(tO, acc);
@@ -587,6 +540,26 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(O_FREE + r));  // the next item's first PV may overwrite O
       if (do_store && j < n) {
+        float inv = 1.f / l_run;
+        if (row_full) {   // (at most 128 keys: no prepare kernel)
+          const T* vr = reinterpret_cast<const T*>(v.p) + b * v.sb + h * v.sh + (int64_t)i * v.si;
+          inv = 1.f / (float)n;
+#pragma unroll
+          for (int e = 0; e < D; ++e) acc[e] = 0u;
+          for (int k = 0; k < n; ++k)
+#pragma unroll
+            for (int e = 0; e < D; e += 8) {
+              const uint4 u = __ldg(reinterpret_cast<const uint4*>(vr + (int64_t)k * v.sj + e));
+              const uint32_t u4[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                float a0, a1;
+                unpack2<T>(u4[c], a0, a1);
+                acc[e + 2 * c] = __float_as_uint(__uint_as_float(acc[e + 2 * c]) + a0);
+                acc[e + 2 * c + 1] = __float_as_uint(__uint_as_float(acc[e + 2 * c + 1]) + a1);
+              }
+            }
+        }
 #pragma unroll
         for (int e = 0; e < D; e += 8) {
           uint4 u;
@@ -615,29 +588,30 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     if (tid == 0) set_status(status, kStatusTimeoutFwd);
     __syncthreads();
   }
-  if (warp == 4 * R + 1) {
+  if (warp == kTmaWarp + 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
   }
 }
 
-template <typename T, int D, int R, int NS>
+template <typename T, int D>
 cudaError_t launch(const FwdArgs& a, cudaStream_t stream) {
-  using Cfg = FwdCfg<D, R, NS>;
+  using Cfg = FwdCfg<D>;
   const Dims& dm = a.dm;
   const bool bf16 = std::is_same<T, __nv_bfloat16>::value;
   const uint64_t eb = 2;
   CUtensorMap mq, mk, mv, mbias;
   const uint64_t dims5[5] = {(uint64_t)D, (uint64_t)dm.n, (uint64_t)dm.n_rows, (uint64_t)dm.heads,
                              (uint64_t)dm.batch};
-  const uint32_t box5[5] = {(uint32_t)D, 128, 1, 1, 1};
+  const uint32_t box_q[5] = {(uint32_t)D, kBJ, 1, 1, 1}, box_kv[5] = {(uint32_t)D, kBK, 1, 1, 1};
   const CUtensorMapSwizzle swz = (CUtensorMapSwizzle)RowSwizzle<D>::kTma;
-  auto map5 = [&](CUtensorMap* m, const View5& v) {
+  auto map5 = [&](CUtensorMap* m, const View5& v, const uint32_t* box5) {
     const uint64_t st[4] = {(uint64_t)v.sj * eb, (uint64_t)v.si * eb, (uint64_t)v.sh * eb,
                             (uint64_t)v.sb * eb};
     return make_tensor_map(m, bf16, 5, v.p, dims5, st, box5, swz);
   };
-  if (!map5(&mq, a.q) || !map5(&mk, a.k) || !map5(&mv, a.v)) return cudaErrorInvalidValue;
+  if (!map5(&mq, a.q, box_q) || !map5(&mk, a.k, box_kv) || !map5(&mv, a.v, box_kv))
+    return cudaErrorInvalidValue;
   {
     // the bias itself when its rows are 16-byte pitched, else the padded copy
     const uint64_t n = dm.n, np = dm.n_pad;
@@ -649,21 +623,22 @@ cudaError_t launch(const FwdArgs& a, cudaStream_t stream) {
                          a.bias_pad ? st_pad : st_user, box4, CU_TENSOR_MAP_SWIZZLE_128B))
       return cudaErrorInvalidValue;
   }
-  const int smem = Cfg::smem_bytes(dm.n);
-  const bool two = Cfg::mask_bufs(dm.n) == 2;
-  constexpr auto kern2 = tc_fwd_kernel<T, D, R, NS, 2>;
-  constexpr auto kern1 = tc_fwd_kernel<T, D, R, NS, 1>;
-  const auto kern = two ? kern2 : kern1;
-  cudaError_t e = two ? opt_in_smem<kern2>(smem) : opt_in_smem<kern1>(smem);
+  const bool words = a.maskbits != nullptr;
+  constexpr auto kern_w = tc_fwd_kernel<T, D, true>;
+  constexpr auto kern_b = tc_fwd_kernel<T, D, false>;
+  const auto kern = words ? kern_w : kern_b;
+  cudaError_t e = words ? opt_in_smem<kern_w>(Cfg::kSmemBytes) : opt_in_smem<kern_b>(Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
   ItemGrid items;
   items.njt = (dm.n + kBJ - 1) / kBJ;
-  items.nrp = (dm.n_rows + R - 1) / R;
-  items.total = items.njt * items.nrp * dm.batch * dm.heads;
-  const int grid = items.total < sm_count() ? items.total : sm_count();
-  kern<<<grid, Cfg::kThreads, smem, stream>>>(mq, mk, mv, mbias, a.o, a.lse, a.mask, a.rowfull,
-                                              a.maskbits, a.mask_words, a.rowrange, dm, items,
-                                              a.status);
+  items.nrg = (dm.n_rows + kR - 1) / kR;
+  const int sms = sm_count(), groups = items.njt * items.nrg * dm.batch * dm.heads;
+  const int rest = groups % sms;
+  items.full = 2 * rest <= sms ? groups - rest : groups;
+  items.total = items.full + 2 * (groups - items.full);
+  const int grid = items.total < sms ? items.total : sms;
+  kern<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(mq, mk, mv, mbias, a.v, a.o, a.lse, a.mask, a.maskbits,
+                                                         a.mask_words, a.rowrange, dm, items, a.status);
   return cudaGetLastError();
 }
 
@@ -729,10 +704,6 @@ bool tc_forward_supported(const Dims& dm, int dtype, const FwdArgs* a) {
   if (dtype != TRIFAST_BF16 && dtype != TRIFAST_F16) return false;
   if (dm.d != 16 && dm.d != 32 && dm.d != 64) return false;
   if (dm.n < kMinTensorCoreN) return false;
-  const int smem = (dm.d == 16)   ? FwdCfg<16, 2, 3>::smem_bytes(dm.n)
-                   : (dm.d == 32) ? FwdCfg<32, 2, 3>::smem_bytes(dm.n)
-                                  : FwdCfg<64, 2, 2>::smem_bytes(dm.n);
-  if (smem > kSmemLimit) return false;
   if (a) {
     if (((uintptr_t)a->o.p) & 15 || (a->o.sj * 2) % 16) return false;
     const bool have_ws = a->bias_pad && a->maskbits && a->rowfull;
@@ -748,11 +719,11 @@ bool tc_forward_supported(const Dims& dm, int dtype, const FwdArgs* a) {
 
 cudaError_t tc_forward(const FwdArgs& a, cudaStream_t s) {
   const bool bf16 = a.dtype == TRIFAST_BF16;
-  if (a.dm.d == 16)
-    return bf16 ? launch<__nv_bfloat16, 16, 2, 3>(a, s) : launch<__half, 16, 2, 3>(a, s);
-  if (a.dm.d == 32)
-    return bf16 ? launch<__nv_bfloat16, 32, 2, 3>(a, s) : launch<__half, 32, 2, 3>(a, s);
-  return bf16 ? launch<__nv_bfloat16, 64, 2, 2>(a, s) : launch<__half, 64, 2, 2>(a, s);
+  switch (a.dm.d) {
+    case 16: return bf16 ? launch<__nv_bfloat16, 16>(a, s) : launch<__half, 16>(a, s);
+    case 32: return bf16 ? launch<__nv_bfloat16, 32>(a, s) : launch<__half, 32>(a, s);
+    default: return bf16 ? launch<__nv_bfloat16, 64>(a, s) : launch<__half, 64>(a, s);
+  }
 }
 
 }  // namespace trifast
