@@ -116,6 +116,32 @@ __device__ __forceinline__ void set_status(unsigned int* status, unsigned int bi
   mirror_status(status, atomicOr(status, bits) | bits);
 }
 
+// Kernels of a call are launched with programmatic serialization (launch_early): the launch itself
+// and the placing of the blocks need not wait until the kernel before has been flushed out; the
+// blocks wait here for that, first of all and before any early return, so that a kernel that is
+// complete implies that all before it are.  No kernel lets the next one start before its own
+// blocks have ended (griddepcontrol.launch_dependents at their start was slower for all but the
+// smallest calls: n = 384 445 us a step, n = 733 717 us a forward).
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Launches a kernel that calls after_previous().  Against plain launches, h = 4, d = 32, calls back to
+// back: forward and backward (six kernels) at n = 256 154.8 -> 143.8 us, n = 384 428 -> 415, n = 512 (15 %
+// padding) 823 -> 813; forward alone at n = 733 703 -> 699 us.
+template <typename... P, typename... A>
+cudaError_t launch_early(void (*kernel)(P...), dim3 grid, int threads, size_t smem, cudaStream_t s, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // SMs of the current device.
 int sm_count();
 

@@ -311,6 +311,7 @@ __global__ void __launch_bounds__(kThreads) simt_fwd_kernel(View5 q, View5 k, Vi
   using F = Cfg<D, R>;
   using S = FwdSmem<D, R>;
   extern __shared__ __align__(16) float sm[];
+  after_previous();
   const int n = dm.n, i = blockIdx.y, b = blockIdx.z / dm.heads, h = blockIdx.z % dm.heads;
   const int j0 = blockIdx.x * F::BR;
   const Place<D, R> at;
@@ -427,6 +428,7 @@ __global__ void __launch_bounds__(kThreads) simt_bwd_kernel(View5 a1, View5 a2, 
   using F = Cfg<D, R>;
   using S = BwdSmem<D, R, kKv>;
   extern __shared__ __align__(16) float sm[];
+  after_previous();
   const int n = dm.n, i = blockIdx.y, b = blockIdx.z / dm.heads, h = blockIdx.z % dm.heads;
   const int r0 = blockIdx.x * F::BR;
   const Place<D, R> at;
@@ -543,6 +545,7 @@ __global__ void __launch_bounds__(TILE / EA * (TILE / EC), 2) simt_db_kernel(Vie
   using S = DbSmem<T, D, EA, EC, TILE>;
   constexpr int NC = D / S::DC;
   extern __shared__ __align__(16) float sm[];
+  after_previous();
   const int n = dm.n, tiles_k = (n + S::TILE - 1) / S::TILE;
   const int j0 = blockIdx.x / tiles_k * S::TILE, k0 = blockIdx.x % tiles_k * S::TILE;
   const int split = blockIdx.y, bh = blockIdx.z, b = bh / dm.heads, h = bh % dm.heads;
@@ -663,8 +666,7 @@ cudaError_t launch_fwd(const FwdArgs& a, cudaStream_t s) {
   constexpr auto kern = simt_fwd_kernel<T, D, R>;
   if (cudaError_t e = opt_in_smem<kern>(kBytes)) return e;
   const dim3 grid((dm.n + Cfg<D, R>::BR - 1) / Cfg<D, R>::BR, dm.n_rows, dm.batch * dm.heads);
-  kern<<<grid, kThreads, kBytes, s>>>(a.q, a.k, a.v, a.bias, a.mask, a.o, a.lse, dm);
-  return cudaGetLastError();
+  return launch_early(kern, grid, kThreads, kBytes, s, a.q, a.k, a.v, a.bias, a.mask, a.o, a.lse, dm);
 }
 
 template <typename T, int D, int R, bool kKv>
@@ -674,10 +676,9 @@ cudaError_t launch_bwd(const BwdArgs& a, cudaStream_t s) {
   constexpr auto kern = simt_bwd_kernel<T, D, R, kKv>;
   if (cudaError_t e = opt_in_smem<kern>(kBytes)) return e;
   const dim3 grid((dm.n + Cfg<D, R>::BR - 1) / Cfg<D, R>::BR, dm.n_rows, dm.batch * dm.heads);
-  kern<<<grid, kThreads, kBytes, s>>>(kKv ? a.k : a.q, kKv ? a.v : a.d_o, kKv ? a.q : a.k, kKv ? a.d_o : a.v,
+  return launch_early(kern, grid, kThreads, kBytes, s, kKv ? a.k : a.q, kKv ? a.v : a.d_o, kKv ? a.q : a.k, kKv ? a.d_o : a.v,
                                       a.bias, kKv ? a.dk : a.dq, kKv ? a.dv : a.dq, a.lse, a.delta, a.rowfull,
                                       a.maskbits_lin, a.mask_words, dm);
-  return cudaGetLastError();
 }
 
 template <typename T, int D, int EA, int EC, int TILE>
@@ -687,10 +688,9 @@ cudaError_t launch_db(const BwdArgs& a, cudaStream_t s) {
   constexpr auto kern = simt_db_kernel<T, D, EA, EC, TILE>;
   if (cudaError_t e = opt_in_smem<kern>(S::kBytes)) return e;
   const int t = (dm.n + S::TILE - 1) / S::TILE;
-  kern<<<dim3(t * t, a.splits, dm.batch * dm.heads), S::NT, S::kBytes, s>>>(
-      a.q, a.k, a.v, a.bias, a.d_o, a.lse, a.delta, a.rowfull, a.maskbits_lin, a.mask_words,
+  return launch_early(
+      kern, dim3(t * t, a.splits, dm.batch * dm.heads), S::NT, S::kBytes, s, a.q, a.k, a.v, a.bias, a.d_o, a.lse, a.delta, a.rowfull, a.maskbits_lin, a.mask_words,
       a.splits > 1 ? a.db_partials : a.db_f32, a.splits, dm);
-  return cudaGetLastError();
 }
 
 }  // namespace

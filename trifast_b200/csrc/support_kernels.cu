@@ -330,6 +330,7 @@ __device__ void prepare_row_scale(const Prep& a, const View5& d_o, int w) {
 }
 
 __global__ void __launch_bounds__(kPrepThreads) fwd_prepare_kernel(Prep a) {
+  after_previous();
   int w = blockIdx.x;
   if (w == 0 && threadIdx.x == 0) repeat_status(a.status);
   if (w < a.mask_blocks) return prepare_mask_row(a, w);
@@ -339,6 +340,7 @@ __global__ void __launch_bounds__(kPrepThreads) fwd_prepare_kernel(Prep a) {
 template <typename T, int D>
 __global__ void __launch_bounds__(kPrepThreads) bwd_prepare_kernel(Prep a, View5 o, View5 d_o, const float* lse,
                                                                    float* delta, float* neg_lse2) {
+  after_previous();
   int w = blockIdx.x;
   if (w == 0 && threadIdx.x == 0) repeat_status(a.status);
   if (w < a.mask_blocks) return prepare_mask_row(a, w);
@@ -358,6 +360,7 @@ __global__ void __launch_bounds__(kPrepThreads) bwd_prepare_kernel(Prep a, View5
 // ---------------------------------------------------------------------------
 template <typename T, bool kWide>
 __global__ void db_finish_kernel(const float* partials, int splits, View4 db, int heads, int n, int64_t count) {
+  after_previous();
   constexpr int V = kWide ? 4 : 1;
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx * V >= count) return;
@@ -399,10 +402,8 @@ cudaError_t launch_finish(const float* partials, int splits, View4 db, int batch
   const int64_t threads = wide ? count / 4 : count;
   const unsigned blocks = (unsigned)((threads + 255) / 256);
   if (wide)
-    db_finish_kernel<T, true><<<blocks, 256, 0, s>>>(partials, splits, db, heads, n, count);
-  else
-    db_finish_kernel<T, false><<<blocks, 256, 0, s>>>(partials, splits, db, heads, n, count);
-  return cudaGetLastError();
+    return launch_early(db_finish_kernel<T, true>, blocks, 256, 0, s, partials, splits, db, heads, n, count);
+  return launch_early(db_finish_kernel<T, false>, blocks, 256, 0, s, partials, splits, db, heads, n, count);
 }
 
 Prep make_prep(const MaskView& mask, const View4& bias, const Dims& dm) {
@@ -419,13 +420,12 @@ template <typename F>
 cudaError_t dispatch(int dtype, int d, F&& f) {
   auto on_d = [&](auto* tp) -> cudaError_t {
     switch (d) {
-      case 16: f(tp, std::integral_constant<int, 16>{}); break;
-      case 32: f(tp, std::integral_constant<int, 32>{}); break;
-      case 64: f(tp, std::integral_constant<int, 64>{}); break;
-      case 128: f(tp, std::integral_constant<int, 128>{}); break;
+      case 16: return f(tp, std::integral_constant<int, 16>{});
+      case 32: return f(tp, std::integral_constant<int, 32>{});
+      case 64: return f(tp, std::integral_constant<int, 64>{});
+      case 128: return f(tp, std::integral_constant<int, 128>{});
       default: return cudaErrorInvalidValue;
     }
-    return cudaGetLastError();
   };
   switch (dtype) {
     case TRIFAST_F32: return on_d((float*)nullptr);
@@ -459,7 +459,7 @@ cudaError_t bwd_prepare(const BwdArgs& a, cudaStream_t s) {
     const int64_t rows = (int64_t)dm.batch * dm.heads * dm.n_rows * dm.n;
     const unsigned blocks =
         (unsigned)(p.mask_blocks + p.bias_blocks + p.scale_blocks + (rows + kRows - 1) / kRows);
-    bwd_prepare_kernel<T, D><<<blocks, kPrepThreads, 0, s>>>(p, a.o, a.d_o, a.lse, a.delta, a.neg_lse2);
+    return launch_early(bwd_prepare_kernel<T, D>, blocks, kPrepThreads, 0, s, p, a.o, a.d_o, a.lse, a.delta, a.neg_lse2);
   });
 }
 
@@ -480,8 +480,7 @@ cudaError_t fwd_prepare(const FwdArgs& a, cudaStream_t s) {
     p.lse = a.lse;
     p.dtype = a.dtype;
   }
-  fwd_prepare_kernel<<<p.mask_blocks + p.bias_blocks, kPrepThreads, 0, s>>>(p);
-  return cudaGetLastError();
+  return launch_early(fwd_prepare_kernel, p.mask_blocks + p.bias_blocks, kPrepThreads, 0, s, p);
 }
 
 cudaError_t db_reduce_splits(const BwdArgs& a, cudaStream_t s) {

@@ -142,6 +142,19 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
     return (uint32_t)(2 * lo) | (uint32_t)min(2 * hi, grid.steps) << 16;
   };
 
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&map_a1);
+    tma_prefetch_desc(&map_a2);
+    tma_prefetch_desc(&map_b1);
+    tma_prefetch_desc(&map_b2);
+    tma_prefetch_desc(&map_bias);
+    if (kKv) {
+      tma_prefetch_desc(&map_nlse);
+      tma_prefetch_desc(&map_delta);
+    }
+  }
+  after_previous();
+
   if (*reinterpret_cast<volatile unsigned int*>(status) != 0u) return;
 
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
@@ -165,17 +178,6 @@ tc_bwd_d128_kernel(const __grid_constant__ CUtensorMap map_a1, const __grid_cons
   if (warp == 9) {
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
-  }
-  if (warp == 8 && lane == 0) {
-    tma_prefetch_desc(&map_a1);
-    tma_prefetch_desc(&map_a2);
-    tma_prefetch_desc(&map_b1);
-    tma_prefetch_desc(&map_b2);
-    tma_prefetch_desc(&map_bias);
-    if (kKv) {
-      tma_prefetch_desc(&map_nlse);
-      tma_prefetch_desc(&map_delta);
-    }
   }
   tc_fence_before();
   __syncthreads();
@@ -565,10 +567,9 @@ cudaError_t launch(const BwdArgs& a, cudaStream_t stream) {
   grid.steps = (dm.n + kStep - 1) / kStep;
   grid.total = grid.tiles * dm.n_rows * dm.heads * dm.batch;
   const int sms = sm_count() - a.reserve_sms > 0 ? sm_count() - a.reserve_sms : 1;
-  kern<<<grid.total < sms ? grid.total : sms, 384, kSmemBytes, stream>>>(
+  return launch_early(kern, grid.total < sms ? grid.total : sms, 384, kSmemBytes, stream, 
       a1, a2, b1, b2, mb, mnl, mdl, kKv ? a.dk : a.dq, kKv ? a.dv : a.dq, a.neg_lse2, a.delta, a.ds_up,
       a.rowfull, a.maskbits_lin, a.mask_words, a.rowrange, dm, grid, a.status);
-  return cudaGetLastError();
 }
 
 }  // namespace

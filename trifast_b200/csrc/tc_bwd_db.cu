@@ -123,6 +123,16 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
   auto nlse_off = [&](int s) -> uint32_t { return stage_off(s) + 4 * Cfg::kTileBytes; };
   auto delta_off = [&](int s) -> uint32_t { return nlse_off(s) + Cfg::kVecBytes; };
 
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&map_q);
+    tma_prefetch_desc(&map_do);
+    tma_prefetch_desc(&map_k);
+    tma_prefetch_desc(&map_v);
+    tma_prefetch_desc(&map_nlse);
+    tma_prefetch_desc(&map_delta);
+  }
+  after_previous();
+
   // (a cluster's CTAs must all reach its barriers: they skip the rows instead)
   if (!kCluster && *reinterpret_cast<volatile unsigned int*>(status) != 0u) return;
   volatile int* skip = reinterpret_cast<volatile int*>(gbase + 264);
@@ -198,14 +208,6 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
   }
   // (the roles walk the set bits word by word: one shared-memory read per 32 rows, nothing
   // per row)
-  if (warp == kTmaWarp && lane == 0) {
-    tma_prefetch_desc(&map_q);
-    tma_prefetch_desc(&map_do);
-    tma_prefetch_desc(&map_k);
-    tma_prefetch_desc(&map_v);
-    tma_prefetch_desc(&map_nlse);
-    tma_prefetch_desc(&map_delta);
-  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -607,24 +609,25 @@ cudaError_t launch_db(const BwdArgs& a, cudaStream_t stream) {
   }
   if (kCluster) {
     cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = a.splits;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // (as launch_early)
+    at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(Cfg::kThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kern, mq, mdo, mk, mv, mnl, mdl, bias, (const uint8_t*)a.rowfull,
                               (const uint32_t*)a.maskbits_lin, a.mask_words, (const uint32_t*)a.rowrange,
                               out, a.splits, dm, a.status);
   }
-  kern<<<grid, Cfg::kThreads, smem, stream>>>(mq, mdo, mk, mv, mnl, mdl, bias, a.rowfull,
+  return launch_early(kern, grid, Cfg::kThreads, smem, stream, mq, mdo, mk, mv, mnl, mdl, bias, a.rowfull,
                                               a.maskbits_lin, a.mask_words, a.rowrange, out, a.splits,
                                               dm, a.status);
-  return cudaGetLastError();
 }
 
 }  // namespace

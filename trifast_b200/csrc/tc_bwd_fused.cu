@@ -168,6 +168,17 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
     return uniform(__ldg(rowrange + it.b * dm.n_rows + it.i));
   };
 
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&map_k);
+    tma_prefetch_desc(&map_v);
+    tma_prefetch_desc(&map_q);
+    tma_prefetch_desc(&map_do);
+    tma_prefetch_desc(&map_bt);
+    tma_prefetch_desc(&map_lse);
+    tma_prefetch_desc(&map_delta);
+  }
+  after_previous();
+
   if (*reinterpret_cast<volatile unsigned int*>(status) != 0u) return;
 
   // (what every lane of a warp shares goes through uniform(), so that the compiler keeps it, and the
@@ -200,15 +211,6 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
   if (warp == kTmaWarp + 1) {
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
-  }
-  if (warp == kTmaWarp && lane == 0) {
-    tma_prefetch_desc(&map_k);
-    tma_prefetch_desc(&map_v);
-    tma_prefetch_desc(&map_q);
-    tma_prefetch_desc(&map_do);
-    tma_prefetch_desc(&map_bt);
-    tma_prefetch_desc(&map_lse);
-    tma_prefetch_desc(&map_delta);
   }
   tc_fence_before();
   __syncthreads();
@@ -840,10 +842,9 @@ cudaError_t launch_fused(const BwdArgs& a, cudaStream_t stream) {
     const int waves = (grid.total + keep - 1) / keep;
     ctas = (grid.total + waves - 1) / waves;
   }
-  kern<<<ctas, Cfg::kThreads, smem, stream>>>(mk, mv, mq, mdo, mbt, mlse, mdelta, a.dq, a.dk, a.dv,
+  return launch_early(kern, ctas, Cfg::kThreads, smem, stream, mk, mv, mq, mdo, mbt, mlse, mdelta, a.dq, a.dk, a.dv,
                                               a.rowfull, a.maskbits_lin, a.mask_words, a.rowrange, dm,
                                               grid, a.kv_scratch, a.status);
-  return cudaGetLastError();
 }
 
 // Second buffers of dP and of dK, dV where the row's dQ leaves room for them.

@@ -152,6 +152,14 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   // the one before that.
   volatile int* records = reinterpret_cast<volatile int*>(gbase + 544);   // [4][8]
 
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&map_q);
+    tma_prefetch_desc(&map_k);
+    tma_prefetch_desc(&map_v);
+    tma_prefetch_desc(&map_b);
+  }
+  after_previous();
+
   // A wait that gave up in an earlier CTA or launch leaves the status word set:
   // stop doing work until the host has read and cleared it.
   if (*reinterpret_cast<volatile unsigned int*>(status) != 0u) {
@@ -183,12 +191,6 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   if (warp == kTmaWarp + 1) {
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
-  }
-  if (warp == kTmaWarp && lane == 0) {
-    tma_prefetch_desc(&map_q);
-    tma_prefetch_desc(&map_k);
-    tma_prefetch_desc(&map_v);
-    tma_prefetch_desc(&map_b);
   }
   tc_fence_before();
   __syncthreads();
@@ -637,9 +639,8 @@ cudaError_t launch(const FwdArgs& a, cudaStream_t stream) {
   items.full = 2 * rest <= sms ? groups - rest : groups;
   items.total = items.full + 2 * (groups - items.full);
   const int grid = items.total < sms ? items.total : sms;
-  kern<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(mq, mk, mv, mbias, a.v, a.o, a.lse, a.mask, a.maskbits,
-                                                         a.mask_words, a.rowrange, dm, items, a.status);
-  return cudaGetLastError();
+  return launch_early(kern, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, mq, mk, mv, mbias, a.v, a.o, a.lse, a.mask,
+                      a.maskbits, a.mask_words, a.rowrange, dm, items, a.status);
 }
 
 }  // namespace

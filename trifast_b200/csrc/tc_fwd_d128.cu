@@ -112,6 +112,14 @@ tc_fwd_d128_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   // without one: it repeats slot 0's tile (its loads stay in range) and stores nothing
   auto slot_tile = [&](const Item& it, int r) -> int { return min(2 * it.jp + r, items.njt - 1); };
 
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&map_q);
+    tma_prefetch_desc(&map_k);
+    tma_prefetch_desc(&map_v);
+    tma_prefetch_desc(&map_b);
+  }
+  after_previous();
+
   if (*reinterpret_cast<volatile unsigned int*>(status) != 0u) return;
 
   const int tid = threadIdx.x, warp = uniform(tid >> 5), lane = tid & 31;
@@ -137,12 +145,6 @@ tc_fwd_d128_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_const
   if (warp == 9) {
     tmem_alloc(smem_u32(tmem_slot), 512);
     tmem_relinquish();
-  }
-  if (warp == 8 && lane == 0) {
-    tma_prefetch_desc(&map_q);
-    tma_prefetch_desc(&map_k);
-    tma_prefetch_desc(&map_v);
-    tma_prefetch_desc(&map_b);
   }
   tc_fence_before();
   __syncthreads();
@@ -522,9 +524,8 @@ cudaError_t launch128(const FwdArgs& a, cudaStream_t stream) {
   items.total = items.njp * dm.n_rows * dm.batch * dm.heads;
   const int sms = sm_count();
   const int grid = items.total < sms ? items.total : sms;
-  kern<<<grid, 384, kSmemBytes, stream>>>(mq, mk, mv, mbias, a.o, a.lse, a.rowfull, a.maskbits,
+  return launch_early(kern, grid, 384, kSmemBytes, stream, mq, mk, mv, mbias, a.o, a.lse, a.rowfull, a.maskbits,
                                           a.mask_words, a.rowrange, dm, items, a.status);
-  return cudaGetLastError();
 }
 
 }  // namespace
