@@ -39,44 +39,68 @@ struct Prep {
   int mask_blocks, bias_tiles, bias_blocks, scale_blocks;
 };
 
+// (volatile: the loads of a thread go out together, in this order)
+__device__ __forceinline__ uint4 load_once(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
+
 // ---------------------------------------------------------------------------
 // Output of a pair row (b, i) without an open key, all heads: the mean of its n values for every
-// query, which the tensor-core kernel would spend a walk over all keys on.  One block, 16 bytes per
-// thread and load, sums in fp32.
+// query, which the tensor-core kernel would spend a walk over all keys on.  One block; a thread
+// owns 16 bytes of a head's row and every so-manieth key, so that all heads' loads are in flight
+// together (head after head the block took 25 us at n = 512, h = 4, so 11).  Sums in fp32.
 // ---------------------------------------------------------------------------
 __device__ void fill_masked_row(const Prep& a, int b, int i) {
   __shared__ float sums[8][kPrepThreads];
-  const int n = a.dm.n, parts = a.dm.d / 8, part = threadIdx.x % parts, first = threadIdx.x / parts;
-  const int rows = kPrepThreads / parts;
+  const int n = a.dm.n, parts = a.dm.d / 8, columns = parts * a.dm.heads;
+  int wide = 1;   // columns of a pass, a power of two
+  while (wide < columns && wide < kPrepThreads / 2) wide *= 2;
+  const int rows = kPrepThreads / wide, first = threadIdx.x / wide;
   const bool bf16 = a.dtype == TRIFAST_BF16;
-  for (int h = 0; h < a.dm.heads; ++h) {
-    const uint16_t* v = (const uint16_t*)a.v.p + b * a.v.sb + h * a.v.sh + (int64_t)i * a.v.si + part * 8;
+  for (int c0 = 0; c0 < columns; c0 += wide) {
+    const int column = c0 + threadIdx.x % wide, h = column / parts, part = column % parts;
+    const bool mine = column < columns;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
-    for (int k = first; k < n; k += rows) {
-      const uint4 u = __ldg(reinterpret_cast<const uint4*>(v + (int64_t)k * a.v.sj));
-      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    if (mine) {
+      const uint16_t* v = (const uint16_t*)a.v.p + b * a.v.sb + h * a.v.sh + (int64_t)i * a.v.si + part * 8;
+      constexpr int U = 8;   // loads in flight
+      for (int k0 = first; k0 < n; k0 += U * rows) {
+        uint4 u[U];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const uint16_t x = (uint16_t)(w[e >> 1] >> (16 * (e & 1)));
-        acc[e] += bf16 ? __uint_as_float((uint32_t)x << 16) : __half2float(__ushort_as_half(x));
+        for (int c = 0; c < U; ++c) u[c] = load_once(v + (int64_t)min(k0 + c * rows, n - 1) * a.v.sj);
+#pragma unroll
+        for (int c = 0; c < U; ++c) {
+          const uint32_t w[4] = {u[c].x, u[c].y, u[c].z, u[c].w};
+          const bool in = k0 + c * rows < n;
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const uint16_t x = in ? (uint16_t)(w[e >> 1] >> (16 * (e & 1))) : (uint16_t)0;
+            acc[e] += bf16 ? __uint_as_float((uint32_t)x << 16) : __half2float(__ushort_as_half(x));
+          }
+        }
       }
     }
-    __syncthreads();   // (the previous head's sums have been read)
+    __syncthreads();   // (the previous pass's sums have been read)
 #pragma unroll
     for (int e = 0; e < 8; ++e) sums[e][threadIdx.x] = acc[e];
-    for (int half = kPrepThreads / 2; half >= parts; half >>= 1) {
+    for (int half = kPrepThreads / 2; half >= wide; half >>= 1) {
       __syncthreads();
       if (threadIdx.x < half)
 #pragma unroll
         for (int e = 0; e < 8; ++e) sums[e][threadIdx.x] += sums[e][threadIdx.x + half];
     }
     __syncthreads();
+    if (!mine) continue;
     const float inv = 1.f / (float)n;
+    const int at = threadIdx.x % wide;
     uint32_t w[4];
 #pragma unroll
     for (int e = 0; e < 8; e += 2) {
-      const float lo = sums[e][part] * inv, hi = sums[e + 1][part] * inv;
+      const float lo = sums[e][at] * inv, hi = sums[e + 1][at] * inv;
       w[e >> 1] = bf16 ? (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(lo)) |
                              (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(hi)) << 16
                        : (uint32_t)__half_as_ushort(__float2half_rn(lo)) |
@@ -85,6 +109,8 @@ __device__ void fill_masked_row(const Prep& a, int b, int i) {
     uint16_t* o = (uint16_t*)a.o.p + b * a.o.sb + h * a.o.sh + (int64_t)i * a.o.si + part * 8;
     for (int j = first; j < n; j += rows)
       *reinterpret_cast<uint4*>(o + (int64_t)j * a.o.sj) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  for (int h = 0; h < a.dm.heads; ++h) {
     float* lse = a.lse + (((int64_t)b * a.dm.heads + h) * a.dm.n_rows + i) * n;
     for (int j = threadIdx.x; j < n; j += kPrepThreads) lse[j] = a.dm.sentinel;
   }
@@ -222,15 +248,6 @@ template <typename T, int D> struct DeltaCfg {
   static constexpr int U = kSteps == 1 ? 4 : kSteps == 2 ? 2 : 1;
   static constexpr int kRows = kPrepThreads / G * U;   // rows of a block
 };
-
-// (volatile: the loads of a thread go out together, in this order)
-__device__ __forceinline__ uint4 load_once(const void* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
-  return v;
-}
 
 template <typename T, int D>
 __device__ void prepare_delta(const View5& o, const View5& d_o, const float* lse, float* delta,
