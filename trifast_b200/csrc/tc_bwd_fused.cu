@@ -119,7 +119,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
   // (g >> 1) & 1), which leaves every waiter a whole step of slack before a parity
   // could be mistaken for the one two steps earlier.
   constexpr int KV_FULL = 0, KV_EMPTY = 2, FULL = 4, EMPTY = FULL + NS, S_FULL = EMPTY + NS,
-                DP_FULL = S_FULL + SB, DP_FREE = DP_FULL + 2, P_READY = DP_FREE + 2, DQ_PAIR = P_READY + 4,
+                DP_FULL = S_FULL + SB, DP_FREE = DP_FULL + 2, P_READY = DP_FREE + 2, ACC_DONE = P_READY + 4, DQ_PAIR = ACC_DONE + SB,
                 ACC_FREE = DQ_PAIR + 2, TILE_DONE = ACC_FREE + AB, DQ_DONE = TILE_DONE + AB,
                 DQ_FREE = DQ_DONE + 1, NBARS = DQ_FREE + Cfg::kMaxJTiles;
   static_assert(NBARS * 8 <= 512, "barrier area");
@@ -193,7 +193,10 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
       mbar_init(bar(DP_FREE + u), 8);
       mbar_init(bar(DQ_PAIR + u), 1);
     }
-    for (int u = 0; u < SB; ++u) mbar_init(bar(S_FULL + u), 1);
+    for (int u = 0; u < SB; ++u) {
+      mbar_init(bar(S_FULL + u), 1);
+      mbar_init(bar(ACC_DONE + u), 1);
+    }
     for (int u = 0; u < 4; ++u) mbar_init(bar(P_READY + u), 8);
     for (int s = 0; s < NS; ++s) {
       mbar_init(bar(FULL + s), 1);
@@ -264,7 +267,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
         }
       }
     } else if (warp == kTmaWarp + 1) {
-      // ------------------------------------------------------------ dP^T issuer
+      // ------------------------------------------------------------ S^T / dP^T issuer
       constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
       constexpr uint32_t idesc_s = make_idesc(128, kBJ, kBf16, false, false);
       int g = 0, ktg = 0;
@@ -278,19 +281,35 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
         for (int kt = kt_lo; kt < kt_hi && ok; ++kt, ++ktg) {
           const int kvb = ktg & 1;
           for (int js = js0; js < js1; ++js, ++g) {
-            const int s = g % NS, gp = g - PB;   // the buffer was last read at step g - PB
+            const int s = g % NS, sb = g % SB;
+            // S^T: its buffer held P^T, dS^T of step g - SB, which the dV / dK MMAs have read
             ok = (js > js0 || mbar_wait(bar(KV_FULL + kvb), (ktg >> 1) & 1, abort_flag)) &&
                  mbar_wait(bar(FULL + s), (g / NS) & 1, abort_flag) &&
-                 (gp < 0 || mbar_wait(bar(DP_FREE + (gp & 1)), (gp >> 1) & 1, abort_flag));
+                 (g < SB || mbar_wait(bar(ACC_DONE + sb), (g / SB - 1) & 1, abort_flag));
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t t_dp = tmem_base + Cfg::kDpCol + (g % PB) * 64;
+            const uint64_t ak = make_smem_desc(k_tile(kvb), 16, Cfg::kSbo, Cfg::kSwz);
+            const uint64_t bq = make_smem_desc(q_tile(s), 16, Cfg::kSbo, Cfg::kSwz);
             const uint64_t av = make_smem_desc(v_tile(kvb), 16, Cfg::kSbo, Cfg::kSwz);
             const uint64_t bg = make_smem_desc(do_tile(s), 16, Cfg::kSbo, Cfg::kSwz);
+            const uint32_t t_s = tmem_base + sb * 64, t_dp = tmem_base + Cfg::kDpCol + (g % PB) * 64;
             if (elect_one()) {
               // a K slice of 16 elements is 32 bytes further along the row: + 2 in the
               // descriptor's address field (16-byte units)
+#pragma unroll
+              for (int kk = 0; kk < D / 16; ++kk)
+                umma_ss(t_s, ak + 2 * kk, bq + 2 * kk, idesc_s, kk > 0);
+              umma_commit(bar(S_FULL + sb));
+            }
+            __syncwarp();
+            const int gp = g - PB;   // dP^T: its buffer was last read at step g - PB
+            if (gp >= 0) {
+              ok = __all_sync(0xffffffffu, mbar_wait(bar(DP_FREE + (gp & 1)), (gp >> 1) & 1, abort_flag));
+              if (!ok) break;
+              tc_fence_after();
+            }
+            if (elect_one()) {
 #pragma unroll
               for (int kk = 0; kk < D / 16; ++kk)
                 umma_ss(t_dp, av + 2 * kk, bg + 2 * kk, idesc_s, kk > 0);
@@ -302,65 +321,12 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
         }
       }
     } else if (warp == kTmaWarp + 2) {
-      // ------------------------------------------------------------ S^T, dV / dK issuer
-      // After the dV / dK MMAs of step g come the S^T MMAs of step g + SB, whose result overwrites
-      // the P^T and dS^T those read: MMAs of one thread execute in the order of their issue,
-      // so nothing has to wait in between.
+      // ------------------------------------------------------------ dV / dK issuer
       constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
-      constexpr uint32_t idesc_s = make_idesc(128, kBJ, kBf16, false, false);
       constexpr uint32_t idesc_acc = make_idesc(128, D, kBf16, false, true);
       // 16 rows of an MN-major tile are this many 16-byte units further on
       constexpr uint32_t kStep16Rows = (16 * Cfg::kRowBytes) >> 4;
       bool ok = true;
-      // the step whose S^T is next: item, its range of key tiles, chunk, key tile, query step
-      struct {
-        int w, lo, hi, c, kt, js, js1, ktg, g;
-        uint32_t rng;
-      } nx;
-      nx.w = blockIdx.x;
-      nx.rng = item_range(nx.w);
-      nx.c = nx.ktg = nx.g = nx.js = 0;
-      nx.js1 = min(njs, jsc);
-      nx.lo = nx.kt = nx.rng & 0xffffu;
-      nx.hi = nx.rng >> 16;
-      nx.rng = item_range(nx.w + gridDim.x);
-      auto issue_s = [&]() {
-        if (nx.w >= grid.total) return;
-        const int js0 = nx.c * jsc, s = nx.g % NS, kvb = nx.ktg & 1;
-        ok = (nx.js > js0 || mbar_wait(bar(KV_FULL + kvb), (nx.ktg >> 1) & 1, abort_flag)) &&
-             mbar_wait(bar(FULL + s), (nx.g / NS) & 1, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) return;
-        tc_fence_after();
-        const uint64_t ak = make_smem_desc(k_tile(kvb), 16, Cfg::kSbo, Cfg::kSwz);
-        const uint64_t bq = make_smem_desc(q_tile(s), 16, Cfg::kSbo, Cfg::kSwz);
-        const uint32_t t_s = tmem_base + (nx.g % SB) * 64;
-        if (elect_one()) {
-#pragma unroll
-          for (int kk = 0; kk < D / 16; ++kk) umma_ss(t_s, ak + 2 * kk, bq + 2 * kk, idesc_s, kk > 0);
-          umma_commit(bar(S_FULL + nx.g % SB));
-        }
-        __syncwarp();
-        ++nx.g;
-        ++nx.js;
-        if (nx.js < nx.js1) return;
-        ++nx.ktg;
-        ++nx.kt;
-        if (nx.kt == nx.hi) {
-          nx.kt = nx.lo;
-          ++nx.c;
-          if (nx.c == nch) {
-            nx.c = 0;
-            nx.w += gridDim.x;
-            nx.lo = nx.kt = nx.rng & 0xffffu;
-            nx.hi = nx.rng >> 16;
-            nx.rng = item_range(nx.w + gridDim.x);
-          }
-        }
-        nx.js = nx.c * jsc;
-        nx.js1 = min(njs, nx.js + jsc);
-      };
-      for (int u = 0; u < SB && ok; ++u) issue_s();
       int g = 0, ktg = 0;
       uint32_t rng_next = item_range(blockIdx.x);
       for (int w = blockIdx.x; w < grid.total && ok; w += gridDim.x) {
@@ -392,11 +358,11 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
                 umma_ts(t_acc + Cfg::kDkCol, t_p + ks * 16 + 8, b_q + ks * kStep16Rows, idesc_acc,
                         (ks > 0) ? 1u : acc);
               }
+              umma_commit(bar(ACC_DONE + g % SB));
               umma_commit(bar(EMPTY + s));
               if (js == js1 - 1) umma_commit(bar(TILE_DONE + ab));
             }
             __syncwarp();
-            issue_s();
           }
         }
         }
