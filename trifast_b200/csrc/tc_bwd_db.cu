@@ -20,11 +20,14 @@
 // vectors per row, NS-deep ring); warp 17 MMA issuer; warps 18-19 idle.  TMEM: two buffers of S [0,128) and
 // dP [128,256), so the MMAs of row i+1 overlap the elementwise work of row i.
 //
-// What bounds it: the exponential unit (1100 cycles per row and tile) and the issue slots (as
-// many), and the waits between them.  A barrier test takes 110 cycles even when the phase is
-// over and a global load several hundred, so the next row's barriers are tested under this
-// row's sums and its mask words come with the stage.  Measured at n = 1024, h = 4, d = 32, bf16:
-// 1.50 ms (two waits and two global loads at the top of every row: 1.87 ms).
+// What bounds it: the exponential unit (1024 cycles per row and tile) and the issue slots (58 % used, 6.4
+// instructions a score), and the waits between them; at large n the card's power limit.  The next row's
+// barriers are tested under this row's sums and its mask words come with the stage (two waits and two
+// global loads at the top of every row: n = 1024 1.87 ms against 1.50).  The elementwise warps walk a
+// count of rows with running stages and phases: with the prepare step, h = 4, d = 32, bf16, n = 384
+// 120 -> 114 us, n = 733 680 -> 630 us, n = 1024 1.50 -> 1.49 ms (each row found in the bitmap, its stage and
+// phases made from its number).  Bias kept as fp32 times log2(e) in place of 16-bit pairs, columns
+// in eights for the registers: 1.62 ms.
 //
 // Stands in for `_bwd_b` of the reference (src/trifast/triton.py:388-501), which
 // loops over all rows with 16-32 wide tiles.
@@ -383,24 +386,32 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
           }
         }
       }
-      int g = 0;
+      // live rows of the item (which ones they are is the producer's business)
+      int count = 0;
+      for (int w0 = lane; w0 * 32 < im.nrows; w0 += 32) count += __popc(live[w0]);
+      count = __reduce_add_sync(0xffffffffu, count);
+      // stage and phases kept as such: made from the row's number they cost twenty instructions a row
+      int s = 0, g = 0;
+      uint32_t ring = 0u, u = 0u, turn = 0u;
+      auto next_stage = [&]() {
+        if (++s == NS) {
+          s = 0;
+          ring ^= 1u;
+        }
+      };
       bool there = false;   // the next row's barriers, tested while this one's sums are made
-      for (int r0 = 0; r0 < im.nrows && ok; r0 += 32) {
-      for (uint32_t bits = uniform(live[r0 >> 5]); bits != 0u; bits &= bits - 1u) {
+      for (; g < count; ++g) {
         // (with KS stages per row the vectors are read from the last one; the earlier ones are
         // released as they come, untouched)
-        const int sg = g * Cfg::KS + Cfg::KS - 1;
-        const int s = sg % NS, u = g & 1;
         if (Cfg::KS > 1) {
-          const int s0 = (sg - 1) % NS;
-          ok = __all_sync(0xffffffffu, mbar_wait(bar(FULL + s0), ((sg - 1) / NS) & 1, abort_flag));
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(FULL + s), ring, abort_flag));
           if (!ok) break;
-          if (lane == 0) mbar_arrive(bar(EMPTY + s0));
+          if (lane == 0) mbar_arrive(bar(EMPTY + s));
+          next_stage();
         }
         if (!__all_sync(0xffffffffu, there)) {
-          const bool a = mbar_wait(bar(FULL + s), (sg / NS) & 1, abort_flag);
-          const bool c = mbar_wait(bar(S_FULL + u), (g >> 1) & 1, abort_flag);
-          ok = __all_sync(0xffffffffu, a && c);
+          ok = mbar_wait(bar(FULL + s), ring, abort_flag) && mbar_wait(bar(S_FULL + u), turn, abort_flag);
+          ok = __all_sync(0xffffffffu, ok);
           if (!ok) break;
         }
         tc_fence_after();
@@ -424,9 +435,11 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
               mbar_arrive(bar(S_FREE + u));
               mbar_arrive(bar(EMPTY + s));   // (the vectors and the mask, read above)
             }
-            const int sn = sg + Cfg::KS;
-            there = mbar_test_wait(bar(FULL + sn % NS), (sn / NS) & 1) &&
-                    mbar_test_wait(bar(S_FULL + (u ^ 1)), ((g + 1) >> 1) & 1);
+            next_stage();
+            turn ^= u;
+            u ^= 1u;
+            if constexpr (Cfg::KS == 1)
+              there = mbar_test_wait(bar(FULL + s), ring) && mbar_test_wait(bar(S_FULL + u), turn);
           }
           const uint32_t mh = (mw >> (hc * 16)) & 0xffffu;
           if (!Cfg::kMaskedApart && row_full) {
@@ -463,25 +476,22 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
             }
           }
         }
-        ++g;
-      }
       }
       if constexpr (Cfg::kMaskedApart) {
-        const int u = g & 1;
         int sg = g;
         float dsum = 0.f;
         for (int r0 = 0; r0 < im.nrows && ok; r0 += 32) {
           for (uint32_t bits = uniform(masked[r0 >> 5]); bits != 0u; bits &= bits - 1u, ++sg) {
-            const int s = sg % NS;
-            ok = __all_sync(0xffffffffu, mbar_wait(bar(FULL + s), (sg / NS) & 1, abort_flag));
+            ok = __all_sync(0xffffffffu, mbar_wait(bar(FULL + s), ring, abort_flag));
             if (!ok) break;
             dsum += reinterpret_cast<const float*>(gbase + delta_off(s))[row];
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(EMPTY + s));
+            next_stage();
           }
         }
         if (ok && sg > g) {
-          ok = __all_sync(0xffffffffu, mbar_wait(bar(S_FULL + u), (g >> 1) & 1, abort_flag));
+          ok = __all_sync(0xffffffffu, mbar_wait(bar(S_FULL + u), turn, abort_flag));
           tc_fence_after();
           float gd[32];
           tmem_ld32(tmem_base + lane_base + u * 256 + 128 + quarter * 32, reinterpret_cast<uint32_t*>(gd));
