@@ -10,19 +10,20 @@ from trifast_b200 import _lib
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [  # n, heads, d, dtype, rows; buffers of dP and of dK, dV, chunks
+SHAPES = [  # n, heads, d, dtype, rows; buffers of S, dP, (dK, dV); chunks
     (64, 5, 32, torch.bfloat16, 64),      # one step per key tile
     (129, 4, 32, torch.float16, 90),      # three steps, the last key tile with one key
-    (256, 2, 32, torch.bfloat16, 160),    # 2, 2
-    (257, 2, 32, torch.bfloat16, 90),     # 2, 1
+    (256, 2, 32, torch.bfloat16, 160),    # 3, 2, 2
+    (257, 2, 32, torch.bfloat16, 90),     # 3, 2, 1
     (512, 1, 32, torch.float16, 160),
-    (513, 1, 32, torch.bfloat16, 150),    # 1, 1
+    (513, 1, 32, torch.bfloat16, 150),    # 3, 1, 1
     (768, 1, 16, torch.bfloat16, 20),
-    (769, 1, 32, torch.bfloat16, 150),    # chunks of 4 and 3 query tiles
-    (1100, 1, 32, torch.float16, 12),
-    (128, 4, 64, torch.float16, 90),
-    (257, 1, 64, torch.bfloat16, 150),    # 1, 1
-    (385, 1, 64, torch.bfloat16, 40),     # two chunks of 2
+    (769, 1, 32, torch.bfloat16, 150),    # 2, 1, 1
+    (1100, 1, 32, torch.float16, 12),     # chunks of five and four query tiles: 3, 1, 1
+    (2000, 1, 32, torch.bfloat16, 5),     # chunks of eight: 2, 1, 1
+    (128, 4, 64, torch.float16, 90),      # 2, 2, 1
+    (257, 1, 64, torch.bfloat16, 150),    # 2, 1, 1
+    (385, 1, 64, torch.bfloat16, 40),     # two chunks of two: 2, 2, 1
     (900, 1, 64, torch.float16, 8),       # three chunks, the last one short
 ]
 

@@ -17,7 +17,8 @@ struct FwdArgs {
   uint32_t* maskbits;    // (b, n_rows, mask_words)
   int mask_words;
   // (b, n_rows): live key tiles [lo, hi) of each row as lo | hi << 16 (tensor-core path,
-  // every n; null otherwise)
+  // null otherwise).  d <= 64: empty (lo = 0xffff) for a row without an open key, whose output the
+  // prepare kernel writes; the top bit is set for a row without a dropped one
   uint32_t* rowrange;
   Dims dm;
   int dtype;

@@ -20,23 +20,25 @@
 // both with one exponential per score.
 //
 // Warps 0-15: elementwise, two groups of eight that take the steps in turn; 16 TMA producer;
-// 17 issues the dP MMAs (and owns the TMEM allocation), 18 the S and the dV / dK MMAs, 19 the dQ
-// MMAs; 20-23 write dK, dV and dQ.  TMEM columns: SB buffers of S^T (64 each, overwritten by the
-// step's P^T and dS^T as 16-bit pairs), PB buffers of dP^T (64), AB pairs of dK and dV (D each), dQ
-// with D columns per 128-query tile.  Rows whose dQ does not fit (d = 32: n > 768; d = 64:
-// n > 384) are walked in query chunks of equal length: per chunk all key tiles are swept again
-// (S, P, dS of a chunk's queries are still evaluated once), dQ of the chunk leaves at its end, and
-// dK / dV of a key tile are completed over the chunks: the partial of the earlier chunks waits as
-// fp32 in a per-CTA scratch (written and read by the same thread, L2-resident).
+// 17 issues the S and dP MMAs (and owns the TMEM allocation), 18 the dV / dK MMAs (and, with two S
+// buffers, S), 19 the dQ MMAs; 20-23 write dK, dV and dQ.  TMEM columns: SB buffers of S^T (64 each,
+// overwritten by the step's P^T and dS^T as 16-bit pairs), PB buffers of dP^T (64), AB pairs of dK and
+// dV (D each), dQ with D columns per 128-query tile.  The dQ of eight tiles (d = 32: n = 1024) or
+// three (d = 64: n = 384) fits beside the fewest buffers.  Longer rows are walked in query chunks of
+// equal length: per chunk all key tiles are swept again (S, P, dS of a chunk's queries are still evaluated
+// once), dQ of the chunk leaves at its end, and dK / dV of a key tile are completed over the chunks:
+// the partial of the earlier chunks waits as fp32 in a per-CTA scratch (written and read by the same
+// thread, L2-resident).
 //
 // What bounds it: the chain of a step, S^T -> registers -> P^T, dS^T -> accumulating MMAs -> the
-// next S^T in that place, which takes about 2800 cycles, of which a group's arithmetic takes
-// 1700 (the issue slots are half used, the exponential unit 512 cycles a step, the tensor pipe 560).  With
-// three buffers and two groups a step is started every 1350 cycles.  Time at h = 4, bf16, before
-// and after (one group of eight warps that also wrote the results, S and P in places of their own):
-// d = 32, n = 256 86 -> 65 us, n = 512 456 -> 360 us, n = 1024 3.20 -> 2.59 ms; d = 64, n = 1024
-// 8.90 -> 5.70 ms.  Two S buffers instead of three: 70 us, 408 us, 2.76 ms at d = 32; at d = 64, where
-// the third would leave dQ two tiles instead of three, three take 7.80 ms.
+// next S^T in that place, which takes about 3400 cycles, of which a group's arithmetic takes
+// 1800 (the issue slots are 63 % used, the exponential unit 512 cycles a step, the tensor pipe 560).  With
+// three S buffers (as far as six tiles of dQ) a step is started every 1250 cycles, with two every
+// 1550.  Time at h = 4, bf16, before and after (one group of eight warps that also wrote the results, S and P
+// in places of their own): d = 32, n = 256 86 -> 61 us, n = 512 (15 % padding) 456 -> 333, n = 733 1354 -> 977,
+// n = 1024 3.20 -> 2.83 ms, n = 2048 (10 %) 26.4 -> 21.3 ms; d = 64, n = 1024 8.90 -> 5.7 ms.  n = 1024 in two chunks with
+// three S buffers takes 2.47 ms, but sums dk and dv in another order and needs the scratch.
+// At d = 64 the third S buffer would leave dQ two tiles instead of three: 7.80 ms.
 //
 // Masked keys weigh exactly zero; rows whose keys are all masked use P = 1/n over
 // the n keys (the PyTorch semantics, src/trifast/equiv.py:42-69).
@@ -62,9 +64,8 @@ constexpr int kFusedMaxCtas = 160;  // grid cap: the per-CTA dK / dV scratch is 
 constexpr int kRegsLaunch = 80, kRegsIssue = 40, kRegsOut = 56, kRegsMath = 96;
 static_assert(512 * kRegsMath + 128 * (kRegsIssue + kRegsOut) <= 768 * kRegsLaunch, "setmaxnreg pool");
 constexpr int kTmaWarp = 16, kOutWarp = 20;
-// Stages of the ring and S^T buffers (measured above).
+// Stages of the ring.
 template <int D> constexpr int kFusedStages = D == 64 ? 3 : 5;
-template <int D> constexpr int kFusedSBuffers = D == 64 ? 2 : 3;
 
 template <int D, int NS, int SB, int PB, int AB>
 struct FusedCfg {
@@ -87,7 +88,7 @@ struct FusedCfg {
   static constexpr int kDpCol = SB * 64, kDkCol = kDpCol + PB * 64, kDvCol = kDkCol + kAcc;
   static constexpr int kDqCol = kDkCol + AB * 2 * kAcc;     // first dQ column
   static constexpr int kMaxJTiles = (512 - kDqCol) / kAcc;  // 128-query tiles whose dQ fits
-  static constexpr bool kChunks = PB == 1 && AB == 1;       // rows may be walked in several query chunks
+  static constexpr bool kChunks = AB == 1;                  // rows may be walked in several query chunks
   static constexpr int kVecOff = 1024, kHeader = (kVecOff + NS * 2 * kVecBytes + 1023) / 1024 * 1024;
   static constexpr int kSmemBytes = kHeader + kTilesBytes;   // (the base is aligned to 1024 bytes)
 };
@@ -122,6 +123,10 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
                 DP_FULL = S_FULL + SB, DP_FREE = DP_FULL + 2, P_READY = DP_FREE + 2, ACC_DONE = P_READY + 4, DQ_PAIR = ACC_DONE + SB,
                 ACC_FREE = DQ_PAIR + 2, TILE_DONE = ACC_FREE + AB, DQ_DONE = TILE_DONE + AB,
                 DQ_FREE = DQ_DONE + 1, NBARS = DQ_FREE + Cfg::kMaxJTiles;
+  // With two S^T buffers the next S^T is what a step waits for: it is issued behind the MMAs that
+  // free its place (n = 1024, h = 4, d = 32: 2.83 ms; by the dP issuer behind their commit 2.93 ms).  With
+  // three it is not urgent, and out of the way of the next step's accumulation (n = 512 372 -> 350 us).
+  constexpr bool kBehind = SB == 2;
   static_assert(NBARS * 8 <= 512, "barrier area");
   static_assert(Cfg::kDqCol + Cfg::kMaxJTiles * Cfg::kAcc <= 512, "TMEM columns");
 
@@ -285,7 +290,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             // S^T: its buffer held P^T, dS^T of step g - SB, which the dV / dK MMAs have read
             ok = (js > js0 || mbar_wait(bar(KV_FULL + kvb), (ktg >> 1) & 1, abort_flag)) &&
                  mbar_wait(bar(FULL + s), (g / NS) & 1, abort_flag) &&
-                 (g < SB || mbar_wait(bar(ACC_DONE + sb), (g / SB - 1) & 1, abort_flag));
+                 (kBehind || g < SB || mbar_wait(bar(ACC_DONE + sb), (g / SB - 1) & 1, abort_flag));
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after();
@@ -294,7 +299,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
             const uint64_t av = make_smem_desc(v_tile(kvb), 16, Cfg::kSbo, Cfg::kSwz);
             const uint64_t bg = make_smem_desc(do_tile(s), 16, Cfg::kSbo, Cfg::kSwz);
             const uint32_t t_s = tmem_base + sb * 64, t_dp = tmem_base + Cfg::kDpCol + (g % PB) * 64;
-            if (elect_one()) {
+            if (!kBehind && elect_one()) {
               // a K slice of 16 elements is 32 bytes further along the row: + 2 in the
               // descriptor's address field (16-byte units)
 #pragma unroll
@@ -322,11 +327,65 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
       }
     } else if (warp == kTmaWarp + 2) {
       // ------------------------------------------------------------ dV / dK issuer
+      // kBehind: after the dV / dK MMAs of step g come the S^T MMAs of step g + SB, whose result
+      // overwrites the P^T and dS^T those read: MMAs of one thread execute in the order of their
+      // issue, so nothing has to wait in between.
       constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
+      constexpr uint32_t idesc_s = make_idesc(128, kBJ, kBf16, false, false);
       constexpr uint32_t idesc_acc = make_idesc(128, D, kBf16, false, true);
       // 16 rows of an MN-major tile are this many 16-byte units further on
       constexpr uint32_t kStep16Rows = (16 * Cfg::kRowBytes) >> 4;
       bool ok = true;
+      // the step whose S^T is next: item, its range of key tiles, chunk, key tile, query step
+      struct {
+        int w, lo, hi, c, kt, js, js1, ktg, g;
+        uint32_t rng;
+      } nx;
+      nx.w = blockIdx.x;
+      nx.rng = item_range(nx.w);
+      nx.c = nx.ktg = nx.g = nx.js = 0;
+      nx.js1 = min(njs, jsc);
+      nx.lo = nx.kt = nx.rng & 0xffffu;
+      nx.hi = nx.rng >> 16;
+      nx.rng = item_range(nx.w + gridDim.x);
+      auto issue_s = [&]() {
+        if (nx.w >= grid.total) return;
+        const int js0 = nx.c * jsc, s = nx.g % NS, kvb = nx.ktg & 1;
+        ok = (nx.js > js0 || mbar_wait(bar(KV_FULL + kvb), (nx.ktg >> 1) & 1, abort_flag)) &&
+             mbar_wait(bar(FULL + s), (nx.g / NS) & 1, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) return;
+        tc_fence_after();
+        const uint64_t ak = make_smem_desc(k_tile(kvb), 16, Cfg::kSbo, Cfg::kSwz);
+        const uint64_t bq = make_smem_desc(q_tile(s), 16, Cfg::kSbo, Cfg::kSwz);
+        const uint32_t t_s = tmem_base + (nx.g % SB) * 64;
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk) umma_ss(t_s, ak + 2 * kk, bq + 2 * kk, idesc_s, kk > 0);
+          umma_commit(bar(S_FULL + nx.g % SB));
+        }
+        __syncwarp();
+        ++nx.g;
+        ++nx.js;
+        if (nx.js < nx.js1) return;
+        ++nx.ktg;
+        ++nx.kt;
+        if (nx.kt == nx.hi) {
+          nx.kt = nx.lo;
+          ++nx.c;
+          if (nx.c == nch) {
+            nx.c = 0;
+            nx.w += gridDim.x;
+            nx.lo = nx.kt = nx.rng & 0xffffu;
+            nx.hi = nx.rng >> 16;
+            nx.rng = item_range(nx.w + gridDim.x);
+          }
+        }
+        nx.js = nx.c * jsc;
+        nx.js1 = min(njs, nx.js + jsc);
+      };
+      if constexpr (kBehind)
+        for (int u = 0; u < SB && ok; ++u) issue_s();
       int g = 0, ktg = 0;
       uint32_t rng_next = item_range(blockIdx.x);
       for (int w = blockIdx.x; w < grid.total && ok; w += gridDim.x) {
@@ -358,11 +417,12 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
                 umma_ts(t_acc + Cfg::kDkCol, t_p + ks * 16 + 8, b_q + ks * kStep16Rows, idesc_acc,
                         (ks > 0) ? 1u : acc);
               }
-              umma_commit(bar(ACC_DONE + g % SB));
+              if (!kBehind) umma_commit(bar(ACC_DONE + g % SB));
               umma_commit(bar(EMPTY + s));
               if (js == js1 - 1) umma_commit(bar(TILE_DONE + ab));
             }
             __syncwarp();
+            if constexpr (kBehind) issue_s();
           }
         }
         }
@@ -791,7 +851,7 @@ cudaError_t launch_fused(const BwdArgs& a, cudaStream_t stream) {
   grid.nkt = (dm.n + kBKeys - 1) / kBKeys;
   grid.njs = (dm.n + kBJ - 1) / kBJ;
   grid.njt = (dm.n + 127) / 128;
-  grid.nch = (grid.njt + Cfg::kMaxJTiles - 1) / Cfg::kMaxJTiles;
+  grid.nch = tc_bwd_fused_chunks(dm.n, D);
   grid.jsc = 2 * ((grid.njt + grid.nch - 1) / grid.nch);
   if (grid.nch > 1 && !a.kv_scratch) return cudaErrorInvalidValue;
   int sms = sm_count();
@@ -813,17 +873,21 @@ cudaError_t launch_fused(const BwdArgs& a, cudaStream_t stream) {
                                               grid, a.kv_scratch, a.status);
 }
 
-// Second buffers of dP and of dK, dV where the row's dQ leaves room for them.
-template <int D, int PB, int AB> using CfgFor = FusedCfg<D, kFusedStages<D>, kFusedSBuffers<D>, PB, AB>;
+// The number of chunks follows from the fewest buffers; then the most buffers that the dQ of a chunk
+// leaves room for are taken: a third S (d <= 32), a second dP, and, for rows walked at once, a second
+// pair of dK, dV.
 template <typename T, int D>
 cudaError_t launch_d(const BwdArgs& a, cudaStream_t s) {
-  constexpr int NS = kFusedStages<D>, SB = kFusedSBuffers<D>;
-  const int njt = (a.dm.n + 127) / 128;
-  if constexpr (CfgFor<D, 2, 2>::kMaxJTiles > 0) {
-    if (njt <= CfgFor<D, 2, 2>::kMaxJTiles) return launch_fused<T, D, NS, SB, 2, 2>(a, s);
+  constexpr int NS = kFusedStages<D>, SB = D == 64 ? 2 : 3;
+  const int njt = (a.dm.n + 127) / 128, nch = tc_bwd_fused_chunks(a.dm.n, D), per = (njt + nch - 1) / nch;
+  if constexpr (FusedCfg<D, NS, SB, 2, 2>::kMaxJTiles > 0) {
+    if (nch == 1 && per <= FusedCfg<D, NS, SB, 2, 2>::kMaxJTiles) return launch_fused<T, D, NS, SB, 2, 2>(a, s);
   }
-  if (njt <= CfgFor<D, 2, 1>::kMaxJTiles) return launch_fused<T, D, NS, SB, 2, 1>(a, s);
-  return launch_fused<T, D, NS, SB, 1, 1>(a, s);
+  if (per <= FusedCfg<D, NS, SB, 2, 1>::kMaxJTiles) return launch_fused<T, D, NS, SB, 2, 1>(a, s);
+  if constexpr (SB == 3) {
+    if (per <= FusedCfg<D, NS, SB, 1, 1>::kMaxJTiles) return launch_fused<T, D, NS, SB, 1, 1>(a, s);
+  }
+  return launch_fused<T, D, NS, 2, 1, 1>(a, s);
 }
 template <typename T>
 cudaError_t launch_for(const BwdArgs& a, cudaStream_t s) {
@@ -845,9 +909,9 @@ bool tc_bwd_fused_supported(const BwdArgs& a) {
 
 int tc_bwd_fused_chunks(int n, int d) {
   const int njt = (n + 127) / 128;
-  const int max_tiles = (d == 16)   ? CfgFor<16, 1, 1>::kMaxJTiles
-                        : (d == 32) ? CfgFor<32, 1, 1>::kMaxJTiles
-                                    : CfgFor<64, 1, 1>::kMaxJTiles;
+  const int max_tiles = (d == 16)   ? FusedCfg<16, kFusedStages<16>, 2, 1, 1>::kMaxJTiles
+                        : (d == 32) ? FusedCfg<32, kFusedStages<32>, 2, 1, 1>::kMaxJTiles
+                                    : FusedCfg<64, kFusedStages<64>, 2, 1, 1>::kMaxJTiles;
   return (njt + max_tiles - 1) / max_tiles;
 }
 
