@@ -120,6 +120,9 @@ __device__ void fill_masked_row(const Prep& a, int b, int i) {
 // One pair row of the mask: rowfull = 1 when every key is masked, the packed key masks, the
 // range of 128-key tiles that hold an open key.
 // ---------------------------------------------------------------------------
+// (kFill: the forward's, which also finishes rows without an open key; its shared memory would cost the
+// backward's prepare kernel blocks.)
+template <bool kFill>
 __device__ void prepare_mask_row(const Prep& a, int bi) {
   const int n = a.dm.n, n_rows = a.dm.n_rows;
   const int b = bi / n_rows, i = bi % n_rows;
@@ -160,7 +163,8 @@ __device__ void prepare_mask_row(const Prep& a, int bi) {
       a.rowrange[bi] = t0 | (t1 << 16) | (a.lse && !dropped_any ? 0x80000000u : 0u);
     }
   }
-  if (!open && a.lse) fill_masked_row(a, b, i);
+  if constexpr (kFill)
+    if (!open && a.lse) fill_masked_row(a, b, i);
   if (!a.maskbits) return;
   // Packed key mask (bit set = key dropped or beyond n).  A fully masked row keeps
   // all n keys with uniform weight, so only the keys beyond n stay set.  Layout per
@@ -350,7 +354,7 @@ __global__ void __launch_bounds__(kPrepThreads) fwd_prepare_kernel(Prep a) {
   after_previous();
   int w = blockIdx.x;
   if (w == 0 && threadIdx.x == 0) repeat_status(a.status);
-  if (w < a.mask_blocks) return prepare_mask_row(a, w);
+  if (w < a.mask_blocks) return prepare_mask_row<true>(a, w);
   prepare_bias_tile(a, w - a.mask_blocks);
 }
 
@@ -360,7 +364,7 @@ __global__ void __launch_bounds__(kPrepThreads) bwd_prepare_kernel(Prep a, View5
   after_previous();
   int w = blockIdx.x;
   if (w == 0 && threadIdx.x == 0) repeat_status(a.status);
-  if (w < a.mask_blocks) return prepare_mask_row(a, w);
+  if (w < a.mask_blocks) return prepare_mask_row<false>(a, w);
   w -= a.mask_blocks;
   if (w < a.bias_blocks) return prepare_bias_tile(a, w);
   w -= a.bias_blocks;
