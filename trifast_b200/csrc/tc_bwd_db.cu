@@ -12,7 +12,7 @@
 // A row without an open key has P = 1/n throughout, so its share needs no S and no weights: the dP of all
 // such rows of the item are summed by the MMAs themselves, in one accumulator, and enter the sums
 // once at the end, less the sum of their deltas (d <= 64; n = 512 with 15 % of the rows padded
-// 262 -> 227 us with the rows below).
+// 262 -> 238 us).
 //
 // Warps 0-15: four elementwise warpgroups, one per 32-key quarter of the tile, so
 // that four warps per scheduler cover each other's barrier, TMEM-load and MUFU
