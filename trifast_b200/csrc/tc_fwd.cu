@@ -145,11 +145,11 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   };
   auto slot_row = [&](const Item& it, int r) -> int { return min(it.i0 + r, dm.n_rows - 1); };
   // The producer hands an item to the other roles through a ring of four records and barriers: number
-  // (-1 at the end), a word that holds its key steps [lo, hi) in bits 0-11 and 16-27, and per slot r
-  // whether the row has no dropped key, bit 12 + r, and whether it has no open one, bit 28 + r;
-  // first query, first row, head, batch.  It is never more than two items ahead of a reader: an item's
-  // Q is loaded behind Q_EMPTY of the one before, whose MMAs are issued behind P_READY of
-  // the one before that.
+  // (-1 at the end), its key steps [lo, hi) as lo | hi << 16 (twice the 15 bits of a row's key tiles),
+  // first query, first row, head with the flags above its 16 bits, batch.  Flags: per slot r whether
+  // the row has no dropped key, bit r, and whether it has no open one, bit 4 + r.  It is never more
+  // than two items ahead of a reader: an item's Q is loaded behind Q_EMPTY of the one before, whose
+  // MMAs are issued behind P_READY of the one before that.
   volatile int* records = reinterpret_cast<volatile int*>(gbase + 544);   // [4][8]
 
   if (threadIdx.x == 0) {
@@ -206,9 +206,12 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     // ------------------------------------------------------------ TMA producer
     // key steps an item walks: the union of the live ranges of its rows (in 128-key tiles; a row
     // without an open key has none), fetched one item ahead
-    auto item_range = [&](int w) -> uint32_t {
+    struct Range {
+      uint32_t steps, flags;   // as in the record
+    };
+    auto item_range = [&](int w) -> Range {
       const uint32_t steps = (uint32_t)(n + kBK - 1) / kBK;
-      if (ws_rowrange == nullptr || w >= items.total) return steps << 16;
+      if (ws_rowrange == nullptr || w >= items.total) return {steps << 16, 0u};
       const Item it = decode(w);
       uint32_t lo = 0xffffu, hi = 0u, flags = 0u;
       for (int r = 0; r < (w < items.full ? kR : 2); ++r) {
@@ -216,16 +219,16 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         const uint32_t l = u & 0xffffu, h = (u >> 16) & 0x7fffu;
         lo = min(lo, l);
         hi = max(hi, h);
-        flags |= ((u >> 31) << (12 + r)) | ((l >= h ? 1u : 0u) << (28 + r));
+        flags |= ((u >> 31) << r) | ((l >= h ? 1u : 0u) << (4 + r));
       }
-      return uniform(lo >= hi ? 0u : 2 * lo | min(2 * hi, steps) << 16 | flags);
+      return {uniform(lo >= hi ? 0u : 2 * lo | min(2 * hi, steps) << 16), uniform(flags)};
     };
     int g = 0, it = 0;  // running key-step and item counters (barrier phases)
     bool ok = true;
-    uint32_t rng_next = item_range(blockIdx.x);
+    Range rng_next = item_range(blockIdx.x);
     for (int w = blockIdx.x; w < items.total && ok; w += gridDim.x) {
-      const uint32_t rng = rng_next;
-      const int lo = rng & 0xfffu, hi = (rng >> 16) & 0xfffu;
+      const Range rng = rng_next;
+      const int lo = rng.steps & 0xffffu, hi = rng.steps >> 16;
       rng_next = item_range(w + gridDim.x);
       if (lo >= hi) continue;
       const Item im = decode(w);
@@ -235,10 +238,10 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       if (elect_one()) {
         volatile int* rec = records + (it & 3) * 8;
         rec[0] = w;
-        rec[1] = (int)rng;
+        rec[1] = (int)rng.steps;
         rec[2] = im.jt * kBJ;
         rec[3] = im.i0;
-        rec[4] = im.h;
+        rec[4] = im.h | (int)(rng.flags << 16);
         rec[5] = im.b;
         mbar_arrive(bar(ITEM + (it & 3)));
         mbar_arrive_expect_tx(bar(Q_FULL), slots * Cfg::kQBytes);
@@ -295,7 +298,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       const int w = uniform(records[(it & 3) * 8]);
       if (w < 0) break;
       const uint32_t rng = uniform(records[(it & 3) * 8 + 1]);
-      const int steps = ((rng >> 16) & 0xfffu) - (rng & 0xfffu);
+      const int steps = (rng >> 16) - (rng & 0xffffu);
       ok = mbar_wait(bar(Q_FULL), it & 1, abort_flag) &&
            mbar_wait(bar(FULL + g % NS), (g / NS) & 1, abort_flag);
       ok = __all_sync(0xffffffffu, ok);
@@ -364,8 +367,8 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     uint32_t ring = 0u, turn = 0u;   // phase of the stage, of the slot's barriers
     bool ok = true;
     struct {
-      int w, j0, i0, h, b;
-      uint32_t rng;
+      int w, j0, i0, b;
+      uint32_t rng, hf;   // head and flags
     } im, nx;
     auto next_item = [&](int it) {
       ok = __all_sync(0xffffffffu, mbar_wait(bar(ITEM + (it & 3)), (it >> 2) & 1, abort_flag));
@@ -374,16 +377,15 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       nx.rng = uniform((uint32_t)rec[1]);
       nx.j0 = rec[2];
       nx.i0 = rec[3];
-      nx.h = rec[4];
+      nx.hf = (uint32_t)rec[4];
       nx.b = rec[5];
     };
     next_item(0);
     for (int it = 0; ok && nx.w >= 0; ++it) {
       im = nx;
-      const uint32_t rng = im.rng;
-      const int lo = rng & 0xfffu, hi = (rng >> 16) & 0xfffu;
+      const int lo = im.rng & 0xffffu, hi = im.rng >> 16;
       if (im.w >= items.full && r >= 2) break;   // half an item: the last one
-      const int i = min(im.i0 + r, dm.n_rows - 1), b = im.b, h = im.h;
+      const int i = min(im.i0 + r, dm.n_rows - 1), b = im.b, h = im.hf & 0xffffu;
 
       // Key mask of a step, fetched one step ahead.  Bytes: lane l < 16 reads keys 4l .. 4l + 3 as
       // one word.  Words: those of the 128-key chunk, of which the step is one half.
@@ -399,7 +401,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         }
       };
       // (a row without a dropped key needs its mask for the step at the row's end alone)
-      const int masked_from = (rng >> (12 + r)) & 1u ? n / kBK : lo;
+      const int masked_from = (im.hf >> (16 + r)) & 1u ? n / kBK : lo;
       if (masked_from <= lo) fetch_mask(lo);
 
       float m_run = kMaxInit, l_run = 0.f;
@@ -526,7 +528,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
 
       // epilogue of the item: O / l and lse.  A row without an open key is left to the prepare
       // kernel (which marks it with an empty range) or, where none runs, done here.
-      const bool row_full = ws_rowrange == nullptr ? !any_open : (rng >> (28 + r)) & 1u;
+      const bool row_full = ws_rowrange == nullptr ? !any_open : (im.hf >> (20 + r)) & 1u;
       next_item(it + 1);   // (its record and, below, O arrive in each other's shadow)
       if (!ok) break;
       const bool do_store = im.i0 + r < dm.n_rows && !(row_full && ws_rowrange != nullptr);
