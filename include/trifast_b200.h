@@ -134,9 +134,10 @@ typedef struct trifast_mask_strided {
 typedef struct trifast_plan {
   int32_t kernel;        /* trifast_kernel of the plan; for head dim 128 see fwd_kernel */
   int32_t block_j;       /* query tile */
-  int32_t block_k;       /* key tile */
+  int32_t block_k;       /* key tile: of the backward, and of the ranges of open keys that all kernels walk
+                            (the forward at head dims up to 64 does so in steps of 64 keys) */
   int32_t rows_per_cta;  /* pair rows sharing one bias tile in the forward */
-  int32_t stages;        /* K/V/bias pipeline depth */
+  int32_t stages;        /* K/V/bias pipeline depth of the forward */
   int32_t db_row_splits; /* row groups whose db partials are summed in fixed order: as many as the
                             workspace holds.  The tensor-core kernels take the number up to this
                             that ends first (trifast_backward_db_partials) */

@@ -62,6 +62,18 @@ def test_heuristic_table(n, h, d, dtype, kernel):
         assert (plan["block_j"], plan["block_k"]) == (128, 128)
 
 
+@pytest.mark.parametrize("d,stages", [(16, 4), (32, 3), (64, 2)])
+@pytest.mark.parametrize("n", [64, 733, 2048])
+def test_plan_of_the_forward(n, d, stages):
+    """The tensor-core forward shares a bias tile among four pair rows; the depth of its ring is what
+    227 KB of shared memory hold of them."""
+    plan = _lib.pick_plan(1, 4, n, n, d, torch.float16)
+    assert (plan["rows_per_cta"], plan["stages"]) == (4, stages)
+    # Q of the rows; per stage their K and V of 64 keys and a 128 x 64 bias tile
+    bytes_of = lambda s: 1024 + 4 * 128 * d * 2 + s * (2 * 4 * 64 * d * 2 + 128 * 64 * 2)
+    assert bytes_of(stages) <= 232448
+
+
 def test_forward_workspace_sizes():
     """Tensor-core plan: the live key-tile range of every row (4 bytes per row, 256-byte
     granules); ragged n adds the padded bias copy, packed masks and row flags.  CUDA-core

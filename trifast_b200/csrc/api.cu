@@ -250,8 +250,8 @@ int pick_plan(const trifast_shape* s, trifast_plan* p) {
   if (kernel == TRIFAST_KERNEL_TCGEN05) {
     p->block_j = 128;
     p->block_k = 128;
-    p->rows_per_cta = 2;
-    p->stages = (s->d <= 32) ? 3 : 2;
+    p->rows_per_cta = kFwdRows;
+    p->stages = tc_forward_stages(s->d);
   } else {
     p->block_j = 64;
     p->block_k = (s->d <= 32) ? 64 : 32;

@@ -79,6 +79,9 @@ bool tc_forward_d128_supported(const Dims& dm, int dtype, const FwdArgs* a);
 cudaError_t tc_forward_d128(const FwdArgs& a, cudaStream_t s);
 bool tc_forward_supported(const Dims& dm, int dtype, const FwdArgs* a);
 cudaError_t tc_forward(const FwdArgs& a, cudaStream_t s);
+// its pair rows per bias tile and stages of its ring of K, V and bias tiles (also what the plan reports)
+constexpr int kFwdRows = 4;
+constexpr int tc_forward_stages(int d) { return d == 64 ? 2 : d == 32 ? 3 : 4; }
 bool tc_backward_supported(const BwdArgs& a);
 cudaError_t tc_bwd_dq(const BwdArgs& a, cudaStream_t s);
 cudaError_t tc_bwd_dkv(const BwdArgs& a, cudaStream_t s);

@@ -57,7 +57,7 @@ using namespace tc;
 constexpr int kRegsLaunch = 96, kRegsIssue = 32, kRegsMath = 112;
 static_assert(512 * kRegsMath + 128 * kRegsIssue <= 640 * kRegsLaunch, "setmaxnreg pool");
 
-constexpr int kR = 4;             // slots: pair rows of an item
+constexpr int kR = kFwdRows;      // slots: pair rows of an item
 constexpr int kBJ = 128, kBK = 64;
 constexpr int kTmaWarp = 16;
 constexpr float kLog2e = 1.4426950408889634f;
@@ -75,7 +75,7 @@ constexpr int kSmemLimit = 232448;  // 227 KiB opt-in limit per CTA
 constexpr int kHeaderBytes = 1024;
 
 template <int D> struct FwdCfg {
-  static constexpr int NS = D == 64 ? 2 : D == 32 ? 3 : 4;  // stages of the ring
+  static constexpr int NS = tc_forward_stages(D);           // stages of the ring
   static constexpr int kRowBytes = D * 2;
   static constexpr int kQBytes = kBJ * kRowBytes;           // Q tile of a slot
   static constexpr int kKVBytes = kBK * kRowBytes;          // K or V tile of a slot
