@@ -205,14 +205,17 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   if (warp == kTmaWarp) {
     // ------------------------------------------------------------ TMA producer
     // key steps an item walks: the union of the live ranges of its rows (in 128-key tiles; a row
-    // without an open key has none), fetched one item ahead
+    // without an open key has none), fetched one item ahead; none for the second half of a group
+    // of one or two rows
     struct Range {
       uint32_t steps, flags;   // as in the record
     };
     auto item_range = [&](int w) -> Range {
       const uint32_t steps = (uint32_t)(n + kBK - 1) / kBK;
-      if (ws_rowrange == nullptr || w >= items.total) return {steps << 16, 0u};
+      if (w >= items.total) return {0u, 0u};
       const Item it = decode(w);
+      if (it.i0 >= dm.n_rows) return {0u, 0u};
+      if (ws_rowrange == nullptr) return {steps << 16, 0u};
       uint32_t lo = 0xffffu, hi = 0u, flags = 0u;
       for (int r = 0; r < (w < items.full ? kR : 2); ++r) {
         const uint32_t u = __ldg(ws_rowrange + it.b * dm.n_rows + slot_row(it, r));
