@@ -112,7 +112,8 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
   uint8_t* gbase = smem_raw + (base - raw);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + 256);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gbase + 260);
-  // per stage: the row's key-mask words of this key tile (four, bit set = dropped) and its flag
+  // per stage: the row's key-mask words of this key tile (four, bit set = dropped) and, where rows
+  // without an open key are not kept apart, its flag
   volatile uint32_t* info = reinterpret_cast<volatile uint32_t*>(gbase + 320);   // [NS][8]
 
   const int n = dm.n;
@@ -221,8 +222,9 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegsIssue));
     if (warp == kTmaWarp) {
       // ---------------------------------------------------------- TMA producer
-      // (The whole warp runs the loop: lanes 0-4 bring the row's key-mask words of this key tile
-      // and its flag, which travel with the stage.)
+      // (The whole warp runs the loop: its first lanes bring what info holds, which travels with
+      // the stage.)
+      constexpr int kInfo = Cfg::kMaskedApart ? 4 : 5;
       const Item im = decode(blockIdx.x);
       int g = 0;
       bool ok = !skipped;
@@ -232,12 +234,12 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
           const int64_t row = (int64_t)im.b * dm.n_rows + i;
           uint32_t word = 0u;
           if (lane < 4) word = __ldg(maskbits + row * mask_words + im.kt * 4 + lane);
-          if (lane == 4) word = rowfull[row];
+          if (!Cfg::kMaskedApart && lane == 4) word = rowfull[row];
           for (int c = 0; c < Cfg::KS; ++c, ++g) {
             const int s = g % NS;
             if (g >= NS) ok = __all_sync(0xffffffffu, mbar_wait(bar(EMPTY + s), ((g / NS) - 1) & 1, abort_flag));
             if (!ok) break;
-            if (c == Cfg::KS - 1 && lane < 5) info[s * 8 + lane] = word;
+            if (c == Cfg::KS - 1 && lane < kInfo) info[s * 8 + lane] = word;
             __syncwarp();
             if (elect_one()) {
               const int c0 = c * Cfg::DS;
@@ -418,7 +420,8 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
         const float nl = reinterpret_cast<const float*>(gbase + nlse_off(s))[row];
         const float dl = reinterpret_cast<const float*>(gbase + delta_off(s))[row];
         const uint32_t mw = info[s * 8 + quarter];
-        const bool row_full = info[s * 8 + 4] != 0u;
+        bool row_full = false;
+        if constexpr (!Cfg::kMaskedApart) row_full = info[s * 8 + 4] != 0u;
         const float ndl = -dl;
         const uint32_t tS = tmem_base + lane_base + u * 256 + quarter * 32;
         const uint32_t tDP = tS + 128;
@@ -442,7 +445,7 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
               there = mbar_test_wait(bar(FULL + s), ring) && mbar_test_wait(bar(S_FULL + u), turn);
           }
           const uint32_t mh = (mw >> (hc * 16)) & 0xffffu;
-          if (!Cfg::kMaskedApart && row_full) {
+          if (row_full) {
 #pragma unroll
             for (int c = 0; c < 16; ++c) {
               const float p = ((mh >> c) & 1u) ? 0.f : p_full;
