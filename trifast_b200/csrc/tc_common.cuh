@@ -151,16 +151,6 @@ __device__ __forceinline__ void tc_fence_after() {
 __device__ __forceinline__ void tmem_wait_ld() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-// The same for a load of 16 registers with other work between it and the wait: the registers pass
-// through it, so that nothing that reads them can be moved before it.
-__device__ __forceinline__ void tmem_wait_ld_regs(uint32_t* a) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]),
-                 "+r"(a[7]), "+r"(a[8]), "+r"(a[9]), "+r"(a[10]), "+r"(a[11]), "+r"(a[12]), "+r"(a[13]),
-                 "+r"(a[14]), "+r"(a[15])
-               :
-               : "memory");
-}
 __device__ __forceinline__ void tmem_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
@@ -213,14 +203,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t* r) {
       : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t* r) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-        "=r"(r[7])
-      : "r"(taddr)
-      : "memory");
-}
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
@@ -229,13 +211,11 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
       : "memory");
 }
 
-// N consecutive columns (8, 16, or a multiple of 32) of this thread's lane.
+// N consecutive columns (16, or a multiple of 32) of this thread's lane.
 template <int N>
 __device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t* r) {
-  static_assert(N == 8 || N == 16 || N % 32 == 0, "column count");
-  if constexpr (N == 8) {
-    tmem_ld8(taddr, r);
-  } else if constexpr (N == 16) {
+  static_assert(N == 16 || N % 32 == 0, "column count");
+  if constexpr (N == 16) {
     tmem_ld16(taddr, r);
   } else {
 #pragma unroll
