@@ -147,7 +147,9 @@ int sm_count();
 
 // Opts a kernel in to `bytes` of dynamic shared memory: one runtime call per kernel, device
 // and growth of the size, not one per launch.
-template <auto Kernel>
+// kFirst: the kernel's tiles count on the dynamic shared memory lying first, on the SM's 1024-byte
+// boundary (the atoms of the swizzles); with static shared memory before it the kernel is refused.
+template <auto Kernel, bool kFirst = false>
 cudaError_t opt_in_smem(int bytes) {
   static std::atomic<int> have[64];
   int dev = 0;
@@ -157,6 +159,11 @@ cudaError_t opt_in_smem(int bytes) {
   if (have[dev].load(std::memory_order_acquire) >= bytes) return cudaSuccess;
   e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (e != cudaSuccess) return e;
+  if (kFirst) {
+    cudaFuncAttributes at;
+    if ((e = cudaFuncGetAttributes(&at, Kernel)) != cudaSuccess) return e;
+    if (at.sharedSizeBytes != 0) return cudaErrorInvalidValue;
+  }
   int seen = have[dev].load(std::memory_order_relaxed);
   while (seen < bytes && !have[dev].compare_exchange_weak(seen, bytes, std::memory_order_release)) {
   }

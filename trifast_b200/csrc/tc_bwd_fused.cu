@@ -130,7 +130,7 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
   static_assert(NBARS * 8 <= 512, "barrier area");
   static_assert(Cfg::kDqCol + Cfg::kMaxJTiles * Cfg::kAcc <= 512, "TMEM columns");
 
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];   // (see opt_in_smem)
   const uint32_t base = smem_u32(smem_raw);
   uint8_t* gbase = smem_raw;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + 512);
@@ -844,7 +844,7 @@ cudaError_t launch_fused(const BwdArgs& a, cudaStream_t stream) {
   }
   const int smem = Cfg::kSmemBytes;
   constexpr auto kern = tc_dqkv_kernel<T, D, NS, SB, PB, AB>;
-  cudaError_t e = opt_in_smem<kern>(smem);
+  cudaError_t e = opt_in_smem<kern, true>(smem);
   if (e != cudaSuccess) return e;
   FusedGrid grid;
   grid.total = dm.batch * dm.heads * dm.n_rows;

@@ -112,7 +112,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
                 P_READY = S_FULL + kR, O_DONE = P_READY + kR, O_FREE = O_DONE + kR, NBARS = O_FREE + kR;
   static_assert(NBARS * 8 <= 512, "barrier area");
 
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];   // (see opt_in_smem)
   const uint32_t base = smem_u32(smem_raw);
   uint8_t* gbase = smem_raw;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gbase + 512);
@@ -634,7 +634,7 @@ cudaError_t launch(const FwdArgs& a, cudaStream_t stream) {
   constexpr auto kern_w = tc_fwd_kernel<T, D, true>;
   constexpr auto kern_b = tc_fwd_kernel<T, D, false>;
   const auto kern = words ? kern_w : kern_b;
-  cudaError_t e = words ? opt_in_smem<kern_w>(Cfg::kSmemBytes) : opt_in_smem<kern_b>(Cfg::kSmemBytes);
+  cudaError_t e = words ? opt_in_smem<kern_w, true>(Cfg::kSmemBytes) : opt_in_smem<kern_b, true>(Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
   ItemGrid items;
   items.njt = (dm.n + kBJ - 1) / kBJ;
