@@ -21,6 +21,8 @@ SHAPES = [  # n, heads, rows, d, dtype
     (257, 1, 21, 16, torch.bfloat16),
     (520, 1, 6, 32, torch.bfloat16),
     (1100, 1, 2, 64, torch.float16),      # the second half of the one group is beyond the rows
+    (136, 20, 9, 64, torch.float16),      # heads x d > 1024: rows without an open key in several passes
+    (200, 33, 6, 32, torch.bfloat16),     # the last pass with one head
 ]
 
 
