@@ -676,9 +676,9 @@ cudaError_t launch_bwd(const BwdArgs& a, cudaStream_t s) {
   constexpr auto kern = simt_bwd_kernel<T, D, R, kKv>;
   if (cudaError_t e = opt_in_smem<kern>(kBytes)) return e;
   const dim3 grid((dm.n + Cfg<D, R>::BR - 1) / Cfg<D, R>::BR, dm.n_rows, dm.batch * dm.heads);
-  return launch_early(kern, grid, kThreads, kBytes, s, kKv ? a.k : a.q, kKv ? a.v : a.d_o, kKv ? a.q : a.k, kKv ? a.d_o : a.v,
-                                      a.bias, kKv ? a.dk : a.dq, kKv ? a.dv : a.dq, a.lse, a.delta, a.rowfull,
-                                      a.maskbits_lin, a.mask_words, dm);
+  return launch_early(kern, grid, kThreads, kBytes, s, kKv ? a.k : a.q, kKv ? a.v : a.d_o, kKv ? a.q : a.k,
+                      kKv ? a.d_o : a.v, a.bias, kKv ? a.dk : a.dq, kKv ? a.dv : a.dq, a.lse, a.delta, a.rowfull,
+                      a.maskbits_lin, a.mask_words, dm);
 }
 
 template <typename T, int D, int EA, int EC, int TILE>
@@ -688,9 +688,9 @@ cudaError_t launch_db(const BwdArgs& a, cudaStream_t s) {
   constexpr auto kern = simt_db_kernel<T, D, EA, EC, TILE>;
   if (cudaError_t e = opt_in_smem<kern>(S::kBytes)) return e;
   const int t = (dm.n + S::TILE - 1) / S::TILE;
-  return launch_early(
-      kern, dim3(t * t, a.splits, dm.batch * dm.heads), S::NT, S::kBytes, s, a.q, a.k, a.v, a.bias, a.d_o, a.lse, a.delta, a.rowfull, a.maskbits_lin, a.mask_words,
-      a.splits > 1 ? a.db_partials : a.db_f32, a.splits, dm);
+  return launch_early(kern, dim3(t * t, a.splits, dm.batch * dm.heads), S::NT, S::kBytes, s, a.q, a.k, a.v, a.bias,
+                      a.d_o, a.lse, a.delta, a.rowfull, a.maskbits_lin, a.mask_words,
+                      a.splits > 1 ? a.db_partials : a.db_f32, a.splits, dm);
 }
 
 }  // namespace

@@ -120,8 +120,9 @@ __device__ void fill_masked_row(const Prep& a, int b, int i) {
 // One pair row of the mask: rowfull = 1 when every key is masked, the packed key masks, the
 // range of 128-key tiles that hold an open key.
 // ---------------------------------------------------------------------------
-// kFill: the forward's, which also finishes rows without an open key (the backward's kernel is spared
-// the registers and shared memory of that).
+// kFill: the forward's, which also finishes rows without an open key.  The backward's kernel is spared
+// the registers and shared memory of that, 64 and 16.7 KB instead of 47 and 8.5 (d = 32); its time was the
+// same with them (n = 1024, h = 4: 116 us).
 template <bool kFill>
 __device__ void prepare_mask_row(const Prep& a, int bi) {
   const int n = a.dm.n, n_rows = a.dm.n_rows;

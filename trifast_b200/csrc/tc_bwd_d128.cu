@@ -33,9 +33,10 @@
 // latency, so two stages would stall on it.  A step of dq and one of dk/dv cost about 6900 cycles
 // together, of which the MMAs hold the tensor pipe for about 2500: the hops between the warps
 // bound it, as in the kernels for smaller head dims.  Measured at n = 512, h = 4: dq and dk/dv
-// together 1.56 ms in bf16 and 1.75 ms in fp16 (1.32 and 1.39 ms with P and dS in one 16-bit operand
-// each), where the CUDA-core kernels took 85.6 ms (db, one row as two stages of half the head
-// dim in tc_bwd_db.cu: 379 us against 22.3 ms).
+// together 1.42 ms in bf16 and 1.50 ms in fp16 (1.56 and 1.75 before an elected lane issued the
+// MMAs, and then 1.32 and 1.39 with P and dS in one 16-bit operand each), where the CUDA-core
+// kernels took 85.6 ms (db, one row as two stages of half the head dim in tc_bwd_db.cu: 379 us
+// against 22.3 ms).
 //
 // Stands in for `_bwd_q` and `_bwd_kv` of the reference (src/trifast/triton.py:268-383,
 // :137-263).  Masked keys weigh exactly zero; rows whose keys are all masked use P = 1/n
@@ -567,7 +568,8 @@ cudaError_t launch(const BwdArgs& a, cudaStream_t stream) {
   grid.steps = (dm.n + kStep - 1) / kStep;
   grid.total = grid.tiles * dm.n_rows * dm.heads * dm.batch;
   const int sms = sm_count() - a.reserve_sms > 0 ? sm_count() - a.reserve_sms : 1;
-  return launch_early(kern, grid.total < sms ? grid.total : sms, 384, kSmemBytes, stream, 
+  return launch_early(
+      kern, grid.total < sms ? grid.total : sms, 384, kSmemBytes, stream,
       a1, a2, b1, b2, mb, mnl, mdl, kKv ? a.dk : a.dq, kKv ? a.dv : a.dq, a.neg_lse2, a.delta, a.ds_up,
       a.rowfull, a.maskbits_lin, a.mask_words, a.rowrange, dm, grid, a.status);
 }

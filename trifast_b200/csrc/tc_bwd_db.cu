@@ -20,8 +20,9 @@
 // vectors per row, NS-deep ring); warp 17 MMA issuer; warps 18-19 idle.  TMEM: two buffers of S [0,128) and
 // dP [128,256), so the MMAs of row i+1 overlap the elementwise work of row i.
 //
-// What bounds it: the exponential unit (1024 cycles per row and tile) and the issue slots (58 % used, 6.4
-// instructions a score), and the waits between them; at large n the card's power limit.  The next row's
+// What bounds it: the exponential unit (1024 cycles per row and tile) and the issue slots, and the waits
+// between them (n = 1024, d = 32, 148 rows: 6.1 instructions a score, issue slots 56 %, exponential unit
+// 74 %); at large n the card's power limit.  The next row's
 // barriers are tested under this row's sums and its mask words come with the stage (two waits and two
 // global loads at the top of every row: n = 1024 1.87 ms against 1.50).  The elementwise warps walk a
 // count of rows with running stages and phases: with the prepare step, h = 4, d = 32, bf16, n = 384

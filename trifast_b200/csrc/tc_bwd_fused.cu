@@ -32,7 +32,8 @@
 //
 // What bounds it: the chain of a step, S^T -> registers -> P^T, dS^T -> accumulating MMAs -> the
 // next S^T in that place, which takes about 3400 cycles, of which a group's arithmetic takes
-// 1800 (the issue slots are 63 % used, the exponential unit 512 cycles a step, the tensor pipe 560).  With
+// 1800 (the exponential unit 512 cycles a step, the tensor pipe 560; n = 1024, d = 32, 148 rows, two S buffers:
+// 12.2 instructions a score, issue slots 53 %, exponential unit 35 %).  With
 // three S buffers (as far as six tiles of dQ) a step is started every 1250 cycles, with two every
 // 1550.  Time at h = 4, bf16, before and after (one group of eight warps that also wrote the results, S and P
 // in places of their own): d = 32, n = 256 86 -> 61 us, n = 512 (15 % padding) 456 -> 333, n = 733 1354 -> 977,
@@ -116,9 +117,16 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
                int mask_words, const uint32_t* __restrict__ rowrange, Dims dm, FusedGrid grid,
                float* __restrict__ kv_scratch, unsigned int* status) {
   using Cfg = FusedCfg<D, NS, SB, PB, AB>;
-  // Barriers.  The per-step ones exist once per step parity (index g & 1, phase
-  // (g >> 1) & 1), which leaves every waiter a whole step of slack before a parity
-  // could be mistaken for the one two steps earlier.
+  // Barriers of step g: S_FULL, ACC_DONE g % SB; DP_FULL, DP_FREE g & 1; P_READY g & 3; FULL, EMPTY
+  // g % NS; DQ_PAIR by the parity of its pair.  A wait names a phase by its parity, so a waiter must be
+  // neither a phase early nor two late.  Late: what would complete the phase after comes behind the
+  // waiter's own arrive (step g + 4 of P_READY: the elementwise warps wait for the dQ of the pair
+  // two before, which the dQ issuer commits after its waits for that pair's steps).  Early:
+  // a role that waits for every step in turn cannot be.  An elementwise group sees every other step,
+  // and where a barrier's successive steps are not all its own (SB, NS odd) the phase between has
+  // completed because of what the group has waited for: S_FULL (SB = 3) by DP_FULL of the same step,
+  // whose commit follows those of S up to this step; FULL by the S of its own step before,
+  // issued after those of all earlier steps; DQ_PAIR by that of an earlier pair, all committed in order.
   constexpr int KV_FULL = 0, KV_EMPTY = 2, FULL = 4, EMPTY = FULL + NS, S_FULL = EMPTY + NS,
                 DP_FULL = S_FULL + SB, DP_FREE = DP_FULL + 2, P_READY = DP_FREE + 2, ACC_DONE = P_READY + 4, DQ_PAIR = ACC_DONE + SB,
                 ACC_FREE = DQ_PAIR + 2, TILE_DONE = ACC_FREE + AB, DQ_DONE = TILE_DONE + AB,
@@ -328,8 +336,11 @@ tc_dqkv_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant_
     } else if (warp == kTmaWarp + 2) {
       // ------------------------------------------------------------ dV / dK issuer
       // kBehind: after the dV / dK MMAs of step g come the S^T MMAs of step g + SB, whose result
-      // overwrites the P^T and dS^T those read: MMAs of one thread execute in the order of their
-      // issue, so nothing has to wait in between.
+      // overwrites the P^T and dS^T those read, with no wait in between.  This counts on the tensor
+      // core taking one thread's MMAs in the order of their issue; the PTX documentation says so
+      // for MMAs of one accumulator and shape, and these differ in both.  What bears it are
+      // results equal to the two-kernel path's bit for bit (tests/test_one_pass_steps_gpu.py);
+      // with three S buffers ACC_DONE stands between, the documented way.
       constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
       constexpr uint32_t idesc_s = make_idesc(128, kBJ, kBf16, false, false);
       constexpr uint32_t idesc_acc = make_idesc(128, D, kBf16, false, true);

@@ -17,9 +17,12 @@
 //                     all have no open key are left out) and hands them to the other roles
 //   warps 17, 18    : MMA issuers, two slots each: O += P V (A = P from TMEM, B = V as
 //                     an MN-major tile), then the slot's next S = Q K^T (SS, both operands
-//                     K-major), whose result overwrites that P: MMAs of one thread execute in
-//                     the order of their issue, so nothing waits in between, and a step's S
-//                     is complete only when the O += P V before it is
+//                     K-major), whose result overwrites that P with no wait in between, and a
+//                     step's S is complete only when the O += P V before it is.  This counts on
+//                     the tensor core taking one thread's MMAs in the order of their issue; the
+//                     PTX documentation says so for MMAs of one accumulator and shape, and these
+//                     differ in both.  What bears it are results that repeat bit for bit and
+//                     agree with float64 (tests/test_forward_steps_gpu.py)
 //   warp 19         : idle; it completes the warpgroup whose registers are handed over
 //
 // What bounds it: a slot's step takes about 3400 cycles, two thirds of them in its own arithmetic
