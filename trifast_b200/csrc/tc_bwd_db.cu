@@ -9,10 +9,12 @@
 // accumulators.  The partial of every row split is written as fp32 and the splits
 // are added in split order afterwards, so the result is deterministic: no atomics.
 //
-// A row without an open key has P = 1/n throughout, so its share needs no S and no weights: the dP of all
-// such rows of the item are summed by the MMAs themselves, in one accumulator, and enter the sums
-// once at the end, less the sum of their deltas (d <= 64; n = 512 with 15 % of the rows padded
-// 262 -> 238 us).
+// A row without an open key has P = 1/n throughout, so it needs no S and no weights (d <= 64): its dP is
+// added as it is, less its delta, before the other rows, while the sums are small (n = 512, h = 4, with
+// the prepare step, all rows without: 264 us walked like others, 147 so).  Summed over the rows by the
+// MMAs and added once it took 118 us, and 217 in place of 221 with 15 % of the rows padded, but the
+// accumulator cuts off where an fp32 addition rounds: relative error of such sums against float64 1.9e-6
+// to 4e-6, row by row 1.6e-7.
 //
 // Warps 0-15: four elementwise warpgroups, one per 32-key quarter of the tile, so
 // that four warps per scheduler cover each other's barrier, TMEM-load and MUFU
@@ -229,6 +231,22 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
       const Item im = decode(blockIdx.x);
       int g = 0;
       bool ok = !skipped;
+      if constexpr (Cfg::kMaskedApart) {
+        for (int r0 = 0; r0 < im.nrows && ok; r0 += 32) {
+          for (uint32_t bits = uniform(masked[r0 >> 5]); bits != 0u && ok; bits &= bits - 1u, ++g) {
+            const int i = im.split + (r0 + __ffs(bits) - 1) * splits, s = g % NS;
+            if (g >= NS) ok = __all_sync(0xffffffffu, mbar_wait(bar(EMPTY + s), ((g / NS) - 1) & 1, abort_flag));
+            if (!ok) break;
+            if (elect_one()) {
+              mbar_arrive_expect_tx(bar(FULL + s), 2 * Cfg::kTileBytes + Cfg::kVecBytes);
+              tma_load_5d(do_tile(s), &map_do, bar(FULL + s), 0, im.jt * 128, i, im.h, im.b);
+              tma_load_5d(v_tile(s), &map_v, bar(FULL + s), 0, im.kt * 128, i, im.h, im.b);
+              tma_load_4d(base + delta_off(s), &map_delta, bar(FULL + s), im.jt * 128, i, im.h, im.b);
+            }
+            __syncwarp();
+          }
+        }
+      }
       for (int r0 = 0; r0 < im.nrows && ok; r0 += 32) {
         for (uint32_t bits = uniform(live[r0 >> 5]); bits != 0u && ok; bits &= bits - 1u) {
           const int i = im.split + (r0 + __ffs(bits) - 1) * splits;
@@ -256,22 +274,6 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
           }
         }
       }
-      if constexpr (Cfg::kMaskedApart) {
-        for (int r0 = 0; r0 < im.nrows && ok; r0 += 32) {
-          for (uint32_t bits = uniform(masked[r0 >> 5]); bits != 0u && ok; bits &= bits - 1u, ++g) {
-            const int i = im.split + (r0 + __ffs(bits) - 1) * splits, s = g % NS;
-            if (g >= NS) ok = __all_sync(0xffffffffu, mbar_wait(bar(EMPTY + s), ((g / NS) - 1) & 1, abort_flag));
-            if (!ok) break;
-            if (elect_one()) {
-              mbar_arrive_expect_tx(bar(FULL + s), 2 * Cfg::kTileBytes + Cfg::kVecBytes);
-              tma_load_5d(do_tile(s), &map_do, bar(FULL + s), 0, im.jt * 128, i, im.h, im.b);
-              tma_load_5d(v_tile(s), &map_v, bar(FULL + s), 0, im.kt * 128, i, im.h, im.b);
-              tma_load_4d(base + delta_off(s), &map_delta, bar(FULL + s), im.jt * 128, i, im.h, im.b);
-            }
-            __syncwarp();
-          }
-        }
-      }
     } else if (warp == kMmaWarp) {
       // ---------------------------------------------------------- MMA issuer
       {
@@ -281,6 +283,28 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
         {
           const int nrows = decode(blockIdx.x).nrows;
           int g = 0;
+          if constexpr (Cfg::kMaskedApart) {   // rows without an open key: dP alone
+            for (int r0 = 0; r0 < nrows && ok; r0 += 32) {
+              for (uint32_t bits = uniform(masked[r0 >> 5]); bits != 0u; bits &= bits - 1u, ++g) {
+                const int s = g % NS, u = g & 1;
+                ok = (g < 2 || mbar_wait(bar(S_FREE + u), ((g >> 1) - 1) & 1, abort_flag)) &&
+                     mbar_wait(bar(FULL + s), (g / NS) & 1, abort_flag);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                tc_fence_after();
+                const uint64_t ag = make_smem_desc(do_tile(s), 16, Cfg::kSbo, Cfg::kSwz);
+                const uint64_t bv = make_smem_desc(v_tile(s), 16, Cfg::kSbo, Cfg::kSwz);
+                if (elect_one()) {
+#pragma unroll
+                  for (int kk = 0; kk < Cfg::DS / 16; ++kk)
+                    umma_ss(tmem_base + u * 256 + 128, ag + 2 * kk, bv + 2 * kk, idesc, kk > 0);
+                  umma_commit(bar(S_FULL + u));
+                  umma_commit(bar(EMPTY + s));
+                }
+                __syncwarp();
+              }
+            }
+          }
           for (int r0 = 0; r0 < nrows && ok; r0 += 32) {
           for (uint32_t bits = uniform(live[r0 >> 5]); bits != 0u && ok; bits &= bits - 1u) {
             const int u = g & 1;
@@ -309,34 +333,6 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
             if (!ok) break;
             ++g;
           }
-          }
-          if constexpr (Cfg::kMaskedApart) {   // the sum of dP over the rows without an open key
-            const int u = g & 1;
-            int sg = g;
-            for (int r0 = 0; r0 < nrows && ok; r0 += 32) {
-              for (uint32_t bits = uniform(masked[r0 >> 5]); bits != 0u && ok; bits &= bits - 1u, ++sg) {
-                const int s = sg % NS;
-                ok = (sg > g || g < 2 || mbar_wait(bar(S_FREE + u), ((g >> 1) - 1) & 1, abort_flag)) &&
-                     mbar_wait(bar(FULL + s), (sg / NS) & 1, abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                tc_fence_after();
-                const uint64_t ag = make_smem_desc(do_tile(s), 16, Cfg::kSbo, Cfg::kSwz);
-                const uint64_t bv = make_smem_desc(v_tile(s), 16, Cfg::kSbo, Cfg::kSwz);
-                const uint32_t acc = sg > g ? 1u : 0u;
-                if (elect_one()) {
-#pragma unroll
-                  for (int kk = 0; kk < Cfg::DS / 16; ++kk)
-                    umma_ss(tmem_base + u * 256 + 128, ag + 2 * kk, bv + 2 * kk, idesc, kk > 0 ? 1u : acc);
-                  umma_commit(bar(EMPTY + s));
-                }
-                __syncwarp();
-              }
-            }
-            if (ok && sg > g) {
-              if (elect_one()) umma_commit(bar(S_FULL + u));
-              __syncwarp();
-            }
           }
         }
       }
@@ -402,8 +398,34 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
           ring ^= 1u;
         }
       };
+      if constexpr (Cfg::kMaskedApart) {
+        int without = 0;   // rows without an open key
+        for (int w0 = lane; w0 * 32 < im.nrows; w0 += 32) without += __popc(masked[w0]);
+        without = __reduce_add_sync(0xffffffffu, without);
+        for (int e = 0; e < without; ++e) {
+          ok = mbar_wait(bar(FULL + s), ring, abort_flag) && mbar_wait(bar(S_FULL + u), turn, abort_flag);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after();
+          const float dl = reinterpret_cast<const float*>(gbase + delta_off(s))[row];
+          float gd[32];
+          tmem_ld32(tmem_base + lane_base + u * 256 + 128 + quarter * 32, reinterpret_cast<uint32_t*>(gd));
+          tmem_wait_ld();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive(bar(S_FREE + u));
+            mbar_arrive(bar(EMPTY + s));
+          }
+          next_stage();
+          turn ^= u;
+          u ^= 1u;
+#pragma unroll
+          for (int c = 0; c < 32; ++c) acc[c] = fmaf(p_full, gd[c] - dl, acc[c]);
+        }
+      }
       bool there = false;   // the next row's barriers, tested while this one's sums are made
-      for (; g < count; ++g) {
+      for (; ok && g < count; ++g) {
         // (with KS stages per row the vectors are read from the last one; the earlier ones are
         // released as they come, untouched)
         if (Cfg::KS > 1) {
@@ -479,30 +501,6 @@ tc_db_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ 
                     acc[hc * 16 + c + 1]);
             }
           }
-        }
-      }
-      if constexpr (Cfg::kMaskedApart) {
-        int sg = g;
-        float dsum = 0.f;
-        for (int r0 = 0; r0 < im.nrows && ok; r0 += 32) {
-          for (uint32_t bits = uniform(masked[r0 >> 5]); bits != 0u; bits &= bits - 1u, ++sg) {
-            ok = __all_sync(0xffffffffu, mbar_wait(bar(FULL + s), ring, abort_flag));
-            if (!ok) break;
-            dsum += reinterpret_cast<const float*>(gbase + delta_off(s))[row];
-            __syncwarp();
-            if (lane == 0) mbar_arrive(bar(EMPTY + s));
-            next_stage();
-          }
-        }
-        if (ok && sg > g) {
-          ok = __all_sync(0xffffffffu, mbar_wait(bar(S_FULL + u), turn, abort_flag));
-          tc_fence_after();
-          float gd[32];
-          tmem_ld32(tmem_base + lane_base + u * 256 + 128 + quarter * 32, reinterpret_cast<uint32_t*>(gd));
-          tmem_wait_ld();
-          tc_fence_before();
-#pragma unroll
-          for (int c = 0; c < 32; ++c) acc[c] = fmaf(p_full, gd[c] - dsum, acc[c]);
         }
       }
       if (kCluster) {
