@@ -105,7 +105,7 @@ template <typename T, int D, bool kWords>
 __global__ void __launch_bounds__(640, 1)
 tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_b,
-              View5 v, View5 o, float* __restrict__ lse, MaskView mask,
+              View5 o, float* __restrict__ lse, MaskView mask,
               const uint32_t* __restrict__ ws_maskbits, int ws_mask_words,
               const uint32_t* __restrict__ ws_rowrange, Dims dm, ItemGrid items,
               unsigned int* status) {
@@ -397,13 +397,24 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       // one word.  Words: those of the 128-key chunk, of which the step is one half.
       const uint8_t* mrow = mask.p + b * mask.sb + (int64_t)i * mask.si;
       const uint32_t* mwords = ws_maskbits + ((int64_t)b * dm.n_rows + i) * ws_mask_words;
+      // A row without an open key is left to the prepare kernel, which marks it with an empty range.
+      // Where none runs (at most 128 keys, one word a lane) it is found here and every score
+      // is 0: its weights are 1 and O / l the mean.
+      bool row_full = (im.hf >> (20 + r)) & 1u;
+      if constexpr (!kWords)
+        if (ws_rowrange == nullptr)
+          row_full = __all_sync(0xffffffffu, 4 * lane >= n ||
+                                                 __vcmpeq4(__ldg(reinterpret_cast<const uint32_t*>(mrow + 4 * lane)), 0u) == 0u);
+      const bool uniform_row = !kWords && ws_rowrange == nullptr && row_full;
       uint4 m_next;
       auto fetch_mask = [&](int st) {
         if constexpr (kWords) {
           m_next = __ldg(reinterpret_cast<const uint4*>(mwords + (st >> 1) * 4));
         } else {
           const int key4 = st * kBK + 4 * lane;
-          m_next.x = lane >= 16 ? 0u : key4 < n ? __ldg(reinterpret_cast<const uint32_t*>(mrow + key4)) : 0x01010101u;
+          m_next.x = lane >= 16 || uniform_row && key4 < n ? 0u
+                     : key4 < n                            ? __ldg(reinterpret_cast<const uint32_t*>(mrow + key4))
+                                                           : 0x01010101u;
         }
       };
       // (a row without a dropped key needs its mask for the step at the row's end alone)
@@ -411,7 +422,6 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       if (masked_from <= lo) fetch_mask(lo);
 
       float m_run = kMaxInit, l_run = 0.f;
-      bool any_open = false;
       for (int st = lo; st < hi; ++st) {
         // mask words of this step (uniform over the warp): key c of the step is bit c >> 2 of word c & 3
         uint32_t mw[4] = {0u, 0u, 0u, 0u};
@@ -429,7 +439,6 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
               mw[jb] = __ballot_sync(0xffffffffu, ((m_next.x >> (8 * jb)) & 0xffu) != 0u);
           }
           clean = (mw[0] | mw[1] | mw[2] | mw[3]) == 0u;
-          any_open = any_open || (mw[0] & mw[1] & mw[2] & mw[3]) != 0xffffu;
         }
         if (st + 1 >= masked_from && st + 1 < hi) fetch_mask(st + 1);
 
@@ -459,6 +468,10 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(EMPTY + s));  // bias tile consumed by this warp
 
+        if constexpr (!kWords)
+          if (uniform_row)
+#pragma unroll
+            for (int c = 0; c < 64; ++c) x[c] = 0.f;
         if (!clean) {
 #pragma unroll
           for (int c = 0; c < 64; ++c)
@@ -532,9 +545,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       }
       if (!ok) break;
 
-      // epilogue of the item: O / l and lse.  A row without an open key is left to the prepare
-      // kernel (which marks it with an empty range) or, where none runs, done here.
-      const bool row_full = ws_rowrange == nullptr ? !any_open : (im.hf >> (20 + r)) & 1u;
+      // epilogue of the item: O / l and lse
       next_item(it + 1);   // (its record and, below, O arrive in each other's shadow)
       if (!ok) break;
       const bool do_store = im.i0 + r < dm.n_rows && !(row_full && ws_rowrange != nullptr);
@@ -550,26 +561,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(O_FREE + r));  // the next item's first PV may overwrite O
       if (do_store && j < n) {
-        float inv = 1.f / l_run;
-        if (row_full) {   // (at most 128 keys: no prepare kernel)
-          const T* vr = reinterpret_cast<const T*>(v.p) + b * v.sb + h * v.sh + (int64_t)i * v.si;
-          inv = 1.f / (float)n;
-#pragma unroll
-          for (int e = 0; e < D; ++e) acc[e] = 0u;
-          for (int k = 0; k < n; ++k)
-#pragma unroll
-            for (int e = 0; e < D; e += 8) {
-              const uint4 u = __ldg(reinterpret_cast<const uint4*>(vr + (int64_t)k * v.sj + e));
-              const uint32_t u4[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-              for (int c = 0; c < 4; ++c) {
-                float a0, a1;
-                unpack2<T>(u4[c], a0, a1);
-                acc[e + 2 * c] = __float_as_uint(__uint_as_float(acc[e + 2 * c]) + a0);
-                acc[e + 2 * c + 1] = __float_as_uint(__uint_as_float(acc[e + 2 * c + 1]) + a1);
-              }
-            }
-        }
+        const float inv = 1.f / l_run;
 #pragma unroll
         for (int e = 0; e < D; e += 8) {
           uint4 u;
@@ -647,7 +639,7 @@ cudaError_t launch(const FwdArgs& a, cudaStream_t stream) {
   items.full = 2 * rest <= sms ? groups - rest : groups;
   items.total = items.full + 2 * (groups - items.full);
   const int grid = items.total < sms ? items.total : sms;
-  return launch_early(kern, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, mq, mk, mv, mbias, a.v, a.o, a.lse, a.mask,
+  return launch_early(kern, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, mq, mk, mv, mbias, a.o, a.lse, a.mask,
                       a.maskbits, a.mask_words, a.rowrange, dm, items, a.status);
 }
 
