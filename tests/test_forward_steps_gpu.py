@@ -38,12 +38,39 @@ def _mask(n, rows, g):
     return m
 
 
+def _ranges(n, rows, g):
+    """Rows of a group that walk different key tiles: one tile each, all but the first or the last
+    ones, every tile, none."""
+    tile, m = torch.arange(n) // 128, torch.rand(1, rows, n, generator=g) < 0.1
+    for i in range(rows):
+        kind, at = (i + i // 4) % 6, i % int(tile[-1] + 1)
+        m[0, i] |= [tile != at, tile < at, tile > at, tile < 0, tile >= 0, tile != 0][kind]
+        if kind != 4 and i % 3 == 0:
+            m[0, i] = ~(~m[0, i] | (torch.arange(n) == n - 1))      # and the last key
+    return m
+
+
 @pytest.mark.parametrize("n,h,rows,d,dtype", SHAPES)
 def test_forward_and_lse_against_float64(n, h, rows, d, dtype):
+    _check(n, h, rows, d, dtype, _mask)
+
+
+@pytest.mark.parametrize("n,h,rows,d,dtype", [
+    (257, 2, 50, 32, torch.bfloat16),
+    (384, 2, 13, 64, torch.float16),
+    (640, 3, 65, 32, torch.float16),
+    (700, 1, 30, 64, torch.bfloat16),
+    (520, 2, 26, 16, torch.bfloat16),
+])
+def test_rows_of_a_group_with_different_steps(n, h, rows, d, dtype):
+    _check(n, h, rows, d, dtype, _ranges)
+
+
+def _check(n, h, rows, d, dtype, make_mask):
     g = torch.Generator().manual_seed(n + d)
     q, k, v = (torch.randn(1, h, rows, n, d, generator=g).to(dtype).to(DEV) for _ in range(3))
     bias = torch.randn(1, h, n, n, generator=g).to(dtype).to(DEV)
-    mask = _mask(n, rows, g).to(DEV)
+    mask = make_mask(n, rows, g).to(DEV)
     o = torch.full_like(q, float("nan"))
     lse = torch.full(q.shape[:4], float("nan"), device=DEV)
     abi_forward(q, k, v, bias, mask, o, lse)

@@ -149,10 +149,9 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
   auto slot_row = [&](const Item& it, int r) -> int { return min(it.i0 + r, dm.n_rows - 1); };
   // The producer hands an item to the other roles through a ring of four records and barriers: number
   // (-1 at the end), its key steps [lo, hi) as lo | hi << 16 (twice the 15 bits of a row's key tiles),
-  // first query, first row, head with the flags above its 16 bits, batch.  Flags: per slot r whether
-  // the row has no dropped key, bit r, and whether it has no open one, bit 4 + r.  It is never more
-  // than two items ahead of a reader: an item's Q is loaded behind Q_EMPTY of the one before, whose
-  // MMAs are issued behind P_READY of the one before that.
+  // first query, first row, head, batch.  It is never more than two items ahead of a reader: an
+  // item's Q is loaded behind Q_EMPTY of the one before, whose MMAs are issued behind P_READY of
+  // the one before that.
   volatile int* records = reinterpret_cast<volatile int*>(gbase + 544);   // [4][8]
 
   if (threadIdx.x == 0) {
@@ -210,31 +209,26 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     // key steps an item walks: the union of the live ranges of its rows (in 128-key tiles; a row
     // without an open key has none), fetched one item ahead; none for the second half of a group
     // of one or two rows
-    struct Range {
-      uint32_t steps, flags;   // as in the record
-    };
-    auto item_range = [&](int w) -> Range {
+    auto item_range = [&](int w) -> uint32_t {
       const uint32_t steps = (uint32_t)(n + kBK - 1) / kBK;
-      if (w >= items.total) return {0u, 0u};
+      if (w >= items.total) return 0u;
       const Item it = decode(w);
-      if (it.i0 >= dm.n_rows) return {0u, 0u};
-      if (ws_rowrange == nullptr) return {steps << 16, 0u};
-      uint32_t lo = 0xffffu, hi = 0u, flags = 0u;
+      if (it.i0 >= dm.n_rows) return 0u;
+      if (ws_rowrange == nullptr) return steps << 16;
+      uint32_t lo = 0xffffu, hi = 0u;
       for (int r = 0; r < (w < items.full ? kR : 2); ++r) {
         const uint32_t u = __ldg(ws_rowrange + it.b * dm.n_rows + slot_row(it, r));
-        const uint32_t l = u & 0xffffu, h = (u >> 16) & 0x7fffu;
-        lo = min(lo, l);
-        hi = max(hi, h);
-        flags |= ((u >> 31) << r) | ((l >= h ? 1u : 0u) << (4 + r));
+        lo = min(lo, u & 0xffffu);
+        hi = max(hi, (u >> 16) & 0x7fffu);
       }
-      return {uniform(lo >= hi ? 0u : 2 * lo | min(2 * hi, steps) << 16), uniform(flags)};
+      return uniform(lo >= hi ? 0u : 2 * lo | min(2 * hi, steps) << 16);
     };
     int g = 0, it = 0;  // running key-step and item counters (barrier phases)
     bool ok = true;
-    Range rng_next = item_range(blockIdx.x);
+    uint32_t rng_next = item_range(blockIdx.x);
     for (int w = blockIdx.x; w < items.total && ok; w += gridDim.x) {
-      const Range rng = rng_next;
-      const int lo = rng.steps & 0xffffu, hi = rng.steps >> 16;
+      const uint32_t rng = rng_next;
+      const int lo = rng & 0xffffu, hi = rng >> 16;
       rng_next = item_range(w + gridDim.x);
       if (lo >= hi) continue;
       const Item im = decode(w);
@@ -244,10 +238,10 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       if (elect_one()) {
         volatile int* rec = records + (it & 3) * 8;
         rec[0] = w;
-        rec[1] = (int)rng.steps;
+        rec[1] = (int)rng;
         rec[2] = im.jt * kBJ;
         rec[3] = im.i0;
-        rec[4] = im.h | (int)(rng.flags << 16);
+        rec[4] = im.h;
         rec[5] = im.b;
         mbar_arrive(bar(ITEM + (it & 3)));
         mbar_arrive_expect_tx(bar(Q_FULL), slots * Cfg::kQBytes);
@@ -373,8 +367,8 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
     uint32_t ring = 0u, turn = 0u;   // phase of the stage, of the slot's barriers
     bool ok = true;
     struct {
-      int w, j0, i0, b;
-      uint32_t rng, hf;   // head and flags
+      int w, j0, i0, h, b;
+      uint32_t rng, own;   // key steps of the item; the row's word of ws_rowrange
     } im, nx;
     auto next_item = [&](int it) {
       ok = __all_sync(0xffffffffu, mbar_wait(bar(ITEM + (it & 3)), (it >> 2) & 1, abort_flag));
@@ -383,15 +377,19 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       nx.rng = uniform((uint32_t)rec[1]);
       nx.j0 = rec[2];
       nx.i0 = rec[3];
-      nx.hf = (uint32_t)rec[4];
+      nx.h = rec[4];
       nx.b = rec[5];
+      nx.own = ws_rowrange && nx.w >= 0 ? __ldg(ws_rowrange + nx.b * dm.n_rows + min(nx.i0 + r, dm.n_rows - 1)) : 0x7fff0000u;
     };
     next_item(0);
     for (int it = 0; ok && nx.w >= 0; ++it) {
       im = nx;
-      const int lo = im.rng & 0xffffu, hi = im.rng >> 16;
       if (im.w >= items.full && r >= 2) break;   // half an item: the last one
-      const int i = min(im.i0 + r, dm.n_rows - 1), b = im.b, h = im.hf & 0xffffu;
+      const int i = min(im.i0 + r, dm.n_rows - 1), b = im.b, h = im.h;
+      // the row's own steps [lo, hi) within the item's [from, to): none for a row without an open key
+      const uint32_t own = uniform(im.own);
+      const int from = im.rng & 0xffffu, to = im.rng >> 16;
+      const int lo = min(2 * (int)(own & 0xffffu), to), hi = max(lo, min(2 * (int)((own >> 16) & 0x7fffu), to));
 
       // Key mask of a step, fetched one step ahead.  Bytes: lane l < 16 reads keys 4l .. 4l + 3 as
       // one word.  Words: those of the 128-key chunk, of which the step is one half.
@@ -400,7 +398,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       // A row without an open key is left to the prepare kernel, which marks it with an empty range.
       // Where none runs (at most 128 keys, one word a lane) it is found here and every score
       // is 0: its weights are 1 and O / l the mean.
-      bool row_full = (im.hf >> (20 + r)) & 1u;
+      bool row_full = hi == lo;
       if constexpr (!kWords)
         if (ws_rowrange == nullptr)
           row_full = __all_sync(0xffffffffu, 4 * lane >= n ||
@@ -418,8 +416,37 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         }
       };
       // (a row without a dropped key needs its mask for the step at the row's end alone)
-      const int masked_from = (im.hf >> (16 + r)) & 1u ? n / kBK : lo;
-      if (masked_from <= lo) fetch_mask(lo);
+      const int masked_from = own >> 31 ? n / kBK : lo;
+      if (masked_from <= lo && lo < hi) fetch_mask(lo);
+
+      // Steps of the item's other rows: weights of zero, as a walk would give, and nothing else moves.
+      auto pass_steps = [&](int count) {
+        for (; count > 0; --count) {
+          ok = mbar_wait(bar(FULL + s), ring, abort_flag) && mbar_wait(bar(S_FULL + r), turn, abort_flag);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          tc_fence_after();
+          uint32_t zero[16];
+#pragma unroll
+          for (int e = 0; e < 16; ++e) zero[e] = 0u;
+          tmem_st16(tP, zero);
+          tmem_st16(tP + 16, zero);
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            mbar_arrive(bar(EMPTY + s));
+            mbar_arrive(bar(P_READY + r));
+          }
+          turn ^= 1u;
+          if (++s == NS) {
+            s = 0;
+            ring ^= 1u;
+          }
+        }
+      };
+      pass_steps(lo - from);
+      if (!ok) break;
 
       float m_run = kMaxInit, l_run = 0.f;
       for (int st = lo; st < hi; ++st) {
@@ -543,6 +570,9 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
           ring ^= 1u;
         }
       }
+      if (!ok) break;
+
+      pass_steps(to - hi);
       if (!ok) break;
 
       // epilogue of the item: O / l and lse
