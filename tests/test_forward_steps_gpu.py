@@ -21,8 +21,9 @@ SHAPES = [  # n, heads, rows, d, dtype
     (257, 1, 21, 16, torch.bfloat16),
     (520, 1, 6, 32, torch.bfloat16),
     (1100, 1, 2, 64, torch.float16),      # the second half of the one group is beyond the rows
-    (136, 20, 9, 64, torch.float16),      # heads x d > 1024: rows without an open key in several passes
-    (200, 33, 6, 32, torch.bfloat16),     # the last pass with one head
+    (136, 20, 9, 64, torch.float16),      # few rows, many heads: a block for each in rows without an open key
+    (200, 33, 130, 32, torch.bfloat16),   # four blocks with eight or nine heads
+    (136, 70, 136, 64, torch.float16),    # more than 1024 columns a block: several passes
 ]
 
 

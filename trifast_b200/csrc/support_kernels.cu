@@ -34,8 +34,9 @@ struct Prep {
   View5 o;
   float* lse;
   int dtype;
-  // block ranges, in this order: one row of the mask each; 64 x 64 bias tiles; one (b, h, i) of
-  // ds_up each; the rest delta
+  int fill_blocks;   // blocks per row, which share its heads
+  // block ranges, in this order: one row of the mask each (or fill_blocks of them); 64 x 64 bias
+  // tiles; one (b, h, i) of ds_up each; the rest delta
   int mask_blocks, bias_tiles, bias_blocks, scale_blocks;
 };
 
@@ -49,20 +50,20 @@ __device__ __forceinline__ uint4 load_once(const void* p) {
 }
 
 // ---------------------------------------------------------------------------
-// Output of a pair row (b, i) without an open key, all heads: the mean of its n values for every
-// query, which the tensor-core kernel would spend a walk over all keys on.  One block; a thread
+// Output of a pair row (b, i) without an open key, `heads` heads from h0 on: the mean of its n values for
+// every query, which the tensor-core kernel would spend a walk over all keys on.  A thread
 // owns 16 bytes of a head's row and every so-manieth key, so that all heads' loads are in flight
 // together (head after head the block took 25 us at n = 512, h = 4, so 11).  Sums in fp32.
 // ---------------------------------------------------------------------------
-__device__ void fill_masked_row(const Prep& a, int b, int i) {
+__device__ void fill_masked_row(const Prep& a, int b, int i, int h0, int heads) {
   __shared__ float sums[8][kPrepThreads];
-  const int n = a.dm.n, parts = a.dm.d / 8, columns = parts * a.dm.heads;
+  const int n = a.dm.n, parts = a.dm.d / 8, columns = parts * heads;
   int wide = 1;   // columns of a pass, a power of two
   while (wide < columns && wide < kPrepThreads / 2) wide *= 2;
   const int rows = kPrepThreads / wide, first = threadIdx.x / wide;
   const bool bf16 = a.dtype == TRIFAST_BF16;
   for (int c0 = 0; c0 < columns; c0 += wide) {
-    const int column = c0 + threadIdx.x % wide, h = column / parts, part = column % parts;
+    const int column = c0 + threadIdx.x % wide, h = h0 + column / parts, part = column % parts;
     const bool mine = column < columns;
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (mine) {
@@ -110,7 +111,7 @@ __device__ void fill_masked_row(const Prep& a, int b, int i) {
     for (int j = first; j < n; j += rows)
       *reinterpret_cast<uint4*>(o + (int64_t)j * a.o.sj) = make_uint4(w[0], w[1], w[2], w[3]);
   }
-  for (int h = 0; h < a.dm.heads; ++h) {
+  for (int h = h0; h < h0 + heads; ++h) {
     float* lse = a.lse + (((int64_t)b * a.dm.heads + h) * a.dm.n_rows + i) * n;
     for (int j = threadIdx.x; j < n; j += kPrepThreads) lse[j] = a.dm.sentinel;
   }
@@ -124,8 +125,9 @@ __device__ void fill_masked_row(const Prep& a, int b, int i) {
 // the registers and shared memory of that, 64 and 16.7 KB instead of 47 and 8.5 (d = 32); its time was the
 // same with them (n = 1024, h = 4: 116 us).
 template <bool kFill>
-__device__ void prepare_mask_row(const Prep& a, int bi) {
+__device__ void prepare_mask_row(const Prep& a, int block) {
   const int n = a.dm.n, n_rows = a.dm.n_rows;
+  const int bi = kFill ? block / a.fill_blocks : block, share = kFill ? block % a.fill_blocks : 0;
   const int b = bi / n_rows, i = bi % n_rows;
   const uint8_t* row = a.mask.p + b * a.mask.sb + (int64_t)i * a.mask.si;
   const int64_t sk = a.mask.sk;
@@ -153,7 +155,7 @@ __device__ void prepare_mask_row(const Prep& a, int bi) {
   }
   __syncthreads();
   const int open = last_open >= 0;
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && share == 0) {
     if (a.rowfull) a.rowfull[bi] = open ? 0 : 1;
     // 128-key tiles [first, last + 1) that hold an open key: the tensor-core kernels walk
     // only those.  A fully masked row weighs all n keys: every tile, or none where it is
@@ -165,8 +167,11 @@ __device__ void prepare_mask_row(const Prep& a, int bi) {
     }
   }
   if constexpr (kFill)
-    if (!open && a.lse) fill_masked_row(a, b, i);
-  if (!a.maskbits) return;
+    if (!open && a.lse) {
+      const int h0 = share * a.dm.heads / a.fill_blocks;
+      fill_masked_row(a, b, i, h0, (share + 1) * a.dm.heads / a.fill_blocks - h0);
+    }
+  if (!a.maskbits || share > 0) return;
   // Packed key mask (bit set = key dropped or beyond n).  A fully masked row keeps
   // all n keys with uniform weight, so only the keys beyond n stay set.  Layout per
   // 128-key chunk c: word c*4 + jb holds, at bit l, key c*128 + 4*l + jb (the order
@@ -434,6 +439,7 @@ Prep make_prep(const MaskView& mask, const View4& bias, const Dims& dm) {
   p.bias = bias;
   p.dm = dm;
   p.mask_blocks = dm.batch * dm.n_rows;
+  p.fill_blocks = 1;
   p.bias_tiles = (dm.n + 63) / 64;
   return p;
 }
@@ -501,6 +507,13 @@ cudaError_t fwd_prepare(const FwdArgs& a, cudaStream_t s) {
     p.o = a.o;
     p.lse = a.lse;
     p.dtype = a.dtype;
+    // A row's heads are shared by as many blocks as one round holds (four blocks an SM): beside few
+    // rows the kernel lasts as long as its slowest one.  The forward with one row of eight without an
+    // open key, one block a row and so: n = 1024, h = 8, d = 64 82 -> 46 us, n = 2048 230 -> 145 us,
+    // n = 4096, h = 4, d = 32 271 -> 232 us.
+    const int most = 4 * sm_count() / p.mask_blocks;
+    p.fill_blocks = most < 1 ? 1 : most < a.dm.heads ? most : a.dm.heads;
+    p.mask_blocks *= p.fill_blocks;
   }
   return launch_early(fwd_prepare_kernel, p.mask_blocks + p.bias_blocks, kPrepThreads, 0, s, p);
 }
