@@ -100,8 +100,10 @@ struct ItemGrid {
   int njt, nrg, full, total;
 };
 
-// kWords: the key mask comes as the prepare step's packed words, else as the caller's bytes.
-template <typename T, int D, bool kWords>
+// The key mask: the prepare step's packed words, or the caller's bytes; kAlone: bytes, and no prepare
+// step has run (at most 128 keys: the mask of a row is one word a lane, and the ranges are all keys).
+enum Masks { kWords, kBytes, kAlone };
+template <typename T, int D, Masks M>
 __global__ void __launch_bounds__(640, 1)
 tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
               const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_b,
@@ -214,7 +216,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       if (w >= items.total) return 0u;
       const Item it = decode(w);
       if (it.i0 >= dm.n_rows) return 0u;
-      if (ws_rowrange == nullptr) return steps << 16;
+      if (M == kAlone) return steps << 16;
       uint32_t lo = 0xffffu, hi = 0u;
       for (int r = 0; r < (w < items.full ? kR : 2); ++r) {
         const uint32_t u = __ldg(ws_rowrange + it.b * dm.n_rows + slot_row(it, r));
@@ -379,7 +381,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       nx.i0 = rec[3];
       nx.h = rec[4];
       nx.b = rec[5];
-      nx.own = ws_rowrange && nx.w >= 0 ? __ldg(ws_rowrange + nx.b * dm.n_rows + min(nx.i0 + r, dm.n_rows - 1)) : 0x7fff0000u;
+      if (M != kAlone && nx.w >= 0) nx.own = __ldg(ws_rowrange + nx.b * dm.n_rows + min(nx.i0 + r, dm.n_rows - 1));
     };
     next_item(0);
     for (int it = 0; ok && nx.w >= 0; ++it) {
@@ -387,32 +389,35 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       if (im.w >= items.full && r >= 2) break;   // half an item: the last one
       const int i = min(im.i0 + r, dm.n_rows - 1), b = im.b, h = im.h;
       // the row's own steps [lo, hi) within the item's [from, to): none for a row without an open key
-      const uint32_t own = uniform(im.own);
       const int from = im.rng & 0xffffu, to = im.rng >> 16;
-      const int lo = min(2 * (int)(own & 0xffffu), to), hi = max(lo, min(2 * (int)((own >> 16) & 0x7fffu), to));
+      const uint32_t own = M == kAlone ? 0u : uniform(im.own);
+      const int lo = M == kAlone ? from : min(2 * (int)(own & 0xffffu), to);
+      const int hi = M == kAlone ? to : max(lo, min(2 * (int)((own >> 16) & 0x7fffu), to));
 
       // Key mask of a step, fetched one step ahead.  Bytes: lane l < 16 reads keys 4l .. 4l + 3 as
       // one word.  Words: those of the 128-key chunk, of which the step is one half.
       const uint8_t* mrow = mask.p + b * mask.sb + (int64_t)i * mask.si;
       const uint32_t* mwords = ws_maskbits + ((int64_t)b * dm.n_rows + i) * ws_mask_words;
       // A row without an open key is left to the prepare kernel, which marks it with an empty range.
-      // Where none runs (at most 128 keys, one word a lane) it is found here and every score
-      // is 0: its weights are 1 and O / l the mean.
+      // Where none runs (at most 128 keys, one word a lane: the mask of both steps) it is found here
+      // and every score is 0: its weights are 1 and O / l the mean.
       bool row_full = hi == lo;
-      if constexpr (!kWords)
-        if (ws_rowrange == nullptr)
-          row_full = __all_sync(0xffffffffu, 4 * lane >= n ||
-                                                 __vcmpeq4(__ldg(reinterpret_cast<const uint32_t*>(mrow + 4 * lane)), 0u) == 0u);
-      const bool uniform_row = !kWords && ws_rowrange == nullptr && row_full;
+      uint32_t both = 0x01010101u;
+      if (M == kAlone) {
+        if (4 * lane < n) both = __ldg(reinterpret_cast<const uint32_t*>(mrow + 4 * lane));
+        row_full = __all_sync(0xffffffffu, __vcmpeq4(both, 0u) == 0u);
+        if (row_full && 4 * lane < n) both = 0u;
+      }
       uint4 m_next;
       auto fetch_mask = [&](int st) {
-        if constexpr (kWords) {
+        if constexpr (M == kWords) {
           m_next = __ldg(reinterpret_cast<const uint4*>(mwords + (st >> 1) * 4));
+        } else if constexpr (M == kAlone) {
+          m_next.x = __shfl_sync(0xffffffffu, both, st * 16 + (lane & 15));
+          if (lane >= 16) m_next.x = 0u;
         } else {
           const int key4 = st * kBK + 4 * lane;
-          m_next.x = lane >= 16 || uniform_row && key4 < n ? 0u
-                     : key4 < n                            ? __ldg(reinterpret_cast<const uint32_t*>(mrow + key4))
-                                                           : 0x01010101u;
+          m_next.x = lane >= 16 ? 0u : key4 < n ? __ldg(reinterpret_cast<const uint32_t*>(mrow + key4)) : 0x01010101u;
         }
       };
       // (a row without a dropped key needs its mask for the step at the row's end alone)
@@ -445,7 +450,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
           }
         }
       };
-      pass_steps(lo - from);
+      if (M != kAlone) pass_steps(lo - from);
       if (!ok) break;
 
       float m_run = kMaxInit, l_run = 0.f;
@@ -454,7 +459,7 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         uint32_t mw[4] = {0u, 0u, 0u, 0u};
         bool clean = true;
         if (st >= masked_from) {
-          if constexpr (kWords) {
+          if constexpr (M == kWords) {
             const int sh = (st & 1) * 16;
             mw[0] = (m_next.x >> sh) & 0xffffu;
             mw[1] = (m_next.y >> sh) & 0xffffu;
@@ -495,8 +500,8 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(EMPTY + s));  // bias tile consumed by this warp
 
-        if constexpr (!kWords)
-          if (uniform_row)
+        if constexpr (M == kAlone)
+          if (row_full)
 #pragma unroll
             for (int c = 0; c < 64; ++c) x[c] = 0.f;
         if (!clean) {
@@ -572,13 +577,13 @@ tc_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__
       }
       if (!ok) break;
 
-      pass_steps(to - hi);
+      if (M != kAlone) pass_steps(to - hi);
       if (!ok) break;
 
       // epilogue of the item: O / l and lse
       next_item(it + 1);   // (its record and, below, O arrive in each other's shadow)
       if (!ok) break;
-      const bool do_store = im.i0 + r < dm.n_rows && !(row_full && ws_rowrange != nullptr);
+      const bool do_store = im.i0 + r < dm.n_rows && !(row_full && M != kAlone);
       ok = __all_sync(0xffffffffu, mbar_wait(bar(O_DONE + r), it & 1, abort_flag));
       if (!ok) break;
       tc_fence_after();
@@ -655,11 +660,13 @@ cudaError_t launch(const FwdArgs& a, cudaStream_t stream) {
                          a.bias_pad ? st_pad : st_user, box4, CU_TENSOR_MAP_SWIZZLE_128B))
       return cudaErrorInvalidValue;
   }
-  const bool words = a.maskbits != nullptr;
-  constexpr auto kern_w = tc_fwd_kernel<T, D, true>;
-  constexpr auto kern_b = tc_fwd_kernel<T, D, false>;
-  const auto kern = words ? kern_w : kern_b;
-  cudaError_t e = words ? opt_in_smem<kern_w, true>(Cfg::kSmemBytes) : opt_in_smem<kern_b, true>(Cfg::kSmemBytes);
+  constexpr auto kern_w = tc_fwd_kernel<T, D, kWords>;
+  constexpr auto kern_b = tc_fwd_kernel<T, D, kBytes>;
+  constexpr auto kern_a = tc_fwd_kernel<T, D, kAlone>;
+  const auto kern = a.maskbits ? kern_w : a.rowrange ? kern_b : kern_a;
+  cudaError_t e = a.maskbits   ? opt_in_smem<kern_w, true>(Cfg::kSmemBytes)
+                  : a.rowrange ? opt_in_smem<kern_b, true>(Cfg::kSmemBytes)
+                               : opt_in_smem<kern_a, true>(Cfg::kSmemBytes);
   if (e != cudaSuccess) return e;
   ItemGrid items;
   items.njt = (dm.n + kBJ - 1) / kBJ;
