@@ -662,9 +662,11 @@ int tc_db_cluster_splits(int64_t tiles, int n_rows, int sms) {
 
 // Row splits of a tile whose partials go through global memory (d <= 64), up to `most`: the same
 // estimate with the 9 rows' time (8 us) that a CTA's start and end measure there, and the
-// partials' way to memory and back at 5 TB/s, a row taking 0.85 us.  The constants were fitted at
-// d = 32; timed against every count up to `most` at d = 16, 32 and 64 (h = 4, n = 97, 128, 192, 256,
-// 384, 512, 733, 1024), the pick was the fastest or within 0.8 % of it each time.  Against clusters of
+// partials' way to memory and back at 5 TB/s, a row taking 0.85 us (by now about 0.75; the picks below are the same).
+// The constants were fitted at d = 32; timed with this kernel against every count up to `most` at d = 16,
+// 32 and 64 (h = 4, n = 97, 128, 192, 256, 384, 512, 733, 1024), the pick was the fastest each time, and
+// so with 15 % of rows and keys padded, which the host does not know of, but for n = 1024, where 3 splits
+// in place of 4 take 4 % less (d = 32 1271 against 1323 us).  Against clusters of
 // 2 to 8 at n = 97 to 1024 (d = 32): faster everywhere but at n = 512 (equal), since clusters leave
 // SMs idle.
 int tc_db_splits(int64_t tiles, int n_rows, int sms, int64_t partial_bytes, int most) {

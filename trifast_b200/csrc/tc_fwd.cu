@@ -26,10 +26,11 @@
 //   warp 19         : idle; it completes the warpgroup whose registers are handed over
 //
 // What bounds it: a slot's step takes about 3400 cycles, two thirds of them in its own arithmetic
-// beside the other slots', the rest on the way to the MMAs and back; the issue slots are 63 % used
-// (8.8 instructions a score), the exponential unit 60 %.  Time at h = 4, before (two slots of eight warps,
-// steps of 128 keys, P beside S) and after: d = 32 bf16 n = 512 (15 % padding) 259 -> 232 us, n = 1024 1.81 -> 1.54 ms,
-// n = 2048 (10 % padding) 13.1 -> 11.0 ms; d = 64 fp16 n = 1024 2.17 -> 1.88 ms; n = 64 14.3 -> 12.3 us.
+// beside the other slots', the rest on the way to the MMAs and back (n = 1024, d = 32, 148 rows: 7.4
+// instructions a score, issue slots 58 %, exponential unit 64 %).  Time at h = 4 by the C ABI, back to back,
+// before (two slots of eight warps, steps of 128 keys, P beside S) and after: d = 32 bf16 n = 64 10.3 -> 5.7 us, n = 512
+// (15 % padding) 271 -> 207 us, n = 1024 1.94 -> 1.55 ms, n = 2048 (10 % padding) 14.1 -> 10.5 ms; d = 64 fp16
+// n = 1024 2.33 -> 2.03 ms.
 // Measured and left (n = 1024, d = 32): P beside S, the next S issued as soon as this one is read, 1.67 ms,
 // all slots then keep in step; the same with two pairs of slots taking turns in the exponentials
 // 1.62 ms.
@@ -71,8 +72,10 @@ constexpr float kMaxInit = -1e30f;
 // row is then exactly 1 before rounding to 16 bits, which keeps the error of peaked
 // rows lowest; a positive value (FlashAttention-style lazy rescale) trades that for
 // fewer rescales of O, 64 columns at d = 64.  There (n = 300, fp16, relative 2-norm error of o against
-// float64; forward of n = 512, h = 8): 0 2.50e-4, 547 us; 2 2.74e-4, 537 us; 5.5 2.83e-4, 523 us, and
-// 2.75e-4 before the steps were 64 keys long.
+// float64; forward of n = 512, h = 8, one session): 0 2.50e-4, 547 us; 2 2.74e-4, 537 us; 5.5 2.83e-4, 523 us, and
+// 2.75e-4 before the steps were 64 keys long.  1.5 against 0, in turn: n = 512, h = 8, fp16 2.73e-4, 527 us
+// and 2.54e-4, 531 us (bf16 2.18e-3, 544 and 2.03e-3, 551); n = 1024, h = 4, 5 % random mask 2.76e-4, 2.09 to
+// 2.14 ms and 2.58e-4, 2.15 to 2.17 ms.
 template <int D> constexpr float lazy_tau() { return D >= 64 ? 1.5f : 0.f; }
 constexpr int kSmemLimit = 232448;  // 227 KiB opt-in limit per CTA
 constexpr int kHeaderBytes = 1024;
